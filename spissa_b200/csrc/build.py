@@ -53,6 +53,7 @@ MODULES = {
     "flash_tc": "flash_tc.cu",
     "decode_layers": "decode_layers.cu",
     "tc_stream": "tc_stream.cu",
+    "tc_mid": "tc_mid.cu",
     "host_step": "host_step.cu",
     "seqmix": "seqmix_kernels.cu",
     "diff_flash": "diff_flash.cu",

@@ -9,9 +9,9 @@
 // the other libraries' own entry points; their addresses are handed over once (sp_host_step_bind) and the choice of
 // product kernel by the number of tokens is the same as in the Python path (the thresholds come with the binding).
 //
-// From 17 to 64 tokens (and head sizes 64 and 128) a layer is five launches instead of eight: the RMS norms, the
-// rotation and the cache write ride in the epilogues of the products (sp_tc_stream_fused: see EpiArgs there), as in
-// the Python runner of larger prompt steps.
+// From 17 tokens on (and head sizes 64 and 128) a layer is five launches instead of eight: the RMS norms, the rotation
+// and the cache write ride in the epilogues of the products (sp_tc_mid, or sp_tc_stream_fused up to 64 tokens where gate
+// and up rows lie in blocks of 64: see EpiArgs there), as in the Python runner of larger prompt steps.
 //
 // There are no kernels in this file. It allocates nothing: the step's activations live in buffers of the caller.
 #include "common.cuh"
@@ -37,6 +37,8 @@ typedef int (*FlashPrefillFn)(const void*, void*, const void*, const void*, cons
 typedef int (*TcStreamFusedFn)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, int*, cudaStream_t);
 typedef int (*RopeTableFn)(const int*, const int*, const int*, const int*, int, int, const float*, int, int, void*, int*, cudaStream_t);
 typedef int (*NormPrepareFn)(const float*, const void*, void*, float*, int, int, cudaStream_t);
+typedef int (*TcMidFn)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, int, float, float,
+                       float, int*, cudaStream_t);
 typedef const char* (*LastErrorFn)();
 }
 
@@ -76,12 +78,15 @@ struct HostKernels {
     TcStreamFusedFn tc_stream_fused;
     RopeTableFn rope_table;
     NormPrepareFn norm_prepare;
+    TcMidFn tc_mid;
+    TcStreamSupportedFn tc_mid_supported;
+    LastErrorFn err_tc_mid;
     int gemv_tokens;           // up to this many tokens the weight-streaming kernel takes a product
     int stream_tokens;         // up to this many the tensor-core kernel that streams the weight
     int flash_query_tile;      // query rows per CTA of the prompt attention
-    int pad;
+    int mid_tokens;            // up to this many the one with the tokens as the instruction's N
 };
-static_assert(sizeof(HostKernels) == 19 * 8 + 16, "the host packs this layout");
+static_assert(sizeof(HostKernels) == 22 * 8 + 16, "the host packs this layout");
 
 // One layer: a pre-norm block of an RMS norm, a rotary grouped-query attention and a SwiGLU. All pointers are device
 // addresses; weights are bfloat16 [out, in] row-major, the gate/up weight interleaves ``gu_pair`` gate rows and their
@@ -124,7 +129,7 @@ struct HostStep {
     float* ssq[2];
     void* cs;
     int* tok_page;
-    int T, H, n_seqs, max_pages, page_size, n_q_tiles, fused, pad1;
+    int T, H, n_seqs, max_pages, page_size, n_q_tiles, fused, mid;     // mid: sp_tc_mid takes the products of the fused sequence
 };
 static_assert(sizeof(HostStep) == 19 * 8 + 8 * 4, "the host packs this layout");
 
@@ -152,6 +157,11 @@ int linear(const void* x, const void* W, void* out, int out_dt, int M, int N, in
         if (k.gemv(x, W, out, out_dt, M, N, K, K, K, ldo, mode, pair, stream)) return fail_from(k.err_gemv, "host step");
         return 0;
     }
+    if (M <= k.mid_tokens && k.tc_mid_supported(x, W, M, N, K, K, K, mode, pair) == 0 && ((uintptr_t)out & 15) == 0 && ldo % 4 == 0) {
+        if (k.tc_mid(x, W, out, out_dt, M, N, K, K, K, ldo, mode, pair, nullptr, SP_ACT_SILU, 1.0f, 0.0f, 0.0f, status, stream))
+            return fail_from(k.err_tc_mid, "host step");
+        return 0;
+    }
     if (M <= k.stream_tokens && k.tc_stream_supported(x, W, M, N, K, K, K, mode, pair) == 0) {
         if (k.tc_stream(x, W, out, out_dt, M, N, K, K, K, ldo, mode, pair, status, stream)) return fail_from(k.err_tc_stream, "host step");
         return 0;
@@ -168,6 +178,21 @@ int linear(const void* x, const void* W, void* out, int out_dt, int M, int N, in
     return 0;
 }
 
+// A product of the fused sequence with its epilogue's arguments.
+int fused_product(const void* x, const void* W, void* out, int out_dt, int N, int K, int ldo, int mode, int pair, const EpiArgs* ep,
+                  const HostStep& st, cudaStream_t stream) {
+    const HostKernels& k = kernels;
+    ++launches;
+    if (st.mid) {
+        if (k.tc_mid(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode, pair, ep, SP_ACT_SILU, 1.0f, 0.0f, 0.0f, st.status, stream))
+            return fail_from(k.err_tc_mid, "host step");
+        return 0;
+    }
+    if (k.tc_stream_fused(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode, pair, ep, st.status, stream))
+        return fail_from(k.err_tc_stream, "host step");
+    return 0;
+}
+
 // One layer of the fused sequence. ``n_ssq``: partial sums per row that st.ssq[0] holds for this layer's first norm.
 int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, int& n_ssq, cudaStream_t stream) {
     const HostKernels& k = kernels;
@@ -180,9 +205,7 @@ int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, i
     ep.cs = st.cs; ep.tok_page = st.tok_page; ep.positions = st.positions;
     ep.q_out = st.q; ep.kpool = L.k_pool; ep.vpool = L.v_pool;
     ep.nh = L.nh; ep.nkv = L.nkv; ep.hd = L.hd; ep.page_size = st.page_size;
-    ++launches;
-    if (k.tc_stream_fused(st.xw[0], L.w_qkv, nullptr, DT_BF16, st.T, nqkv, st.H, st.H, st.H, 0, MODE_STREAM_QKV_ROPE, 0, &ep,
-                          st.status, stream)) return fail_from(k.err_tc_stream, "host step");
+    if (fused_product(st.xw[0], L.w_qkv, nullptr, DT_BF16, nqkv, st.H, 0, MODE_STREAM_QKV_ROPE, 0, &ep, st, stream)) return 1;
     ++launches;
     if (k.flash_prefill(st.q, st.ctx, L.k_pool, L.v_pool, st.seq_start, st.positions, st.seq_row, st.page_table, st.max_pages,
                         st.page_size, st.n_seqs, st.n_q_tiles, L.nh, L.nkv, L.hd, L.window, L.scale, stream))
@@ -190,26 +213,18 @@ int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, i
     // output projection into the residual; the same epilogue writes residual ⊙ second norm weight and its statistics
     memset(&ep, 0, sizeof(ep));
     ep.xw = st.xw[1]; ep.next_w = L.norm2; ep.ssq_out = st.ssq[1];
-    ++launches;
-    if (k.tc_stream_fused(st.ctx, L.w_o, st.h, DT_F32, st.T, st.H, nq, nq, nq, st.H, MODE_ACCUMULATE, 0, &ep, st.status, stream))
-        return fail_from(k.err_tc_stream, "host step");
+    if (fused_product(st.ctx, L.w_o, st.h, DT_F32, st.H, nq, st.H, MODE_ACCUMULATE, 0, &ep, st, stream)) return 1;
     // gate/up on it, scaled by 1/rms, with silu(gate)·up
     memset(&ep, 0, sizeof(ep));
     ep.row_ssq = st.ssq[1]; ep.n_ssq = tiles; ep.norm_width = st.H; ep.eps = L.eps2;
-    ++launches;
-    if (k.tc_stream_fused(st.xw[1], L.w_gu, st.act, DT_BF16, st.T, 2 * L.I, st.H, st.H, st.H, L.I, MODE_SILU_MUL, L.gu_pair, &ep,
-                          st.status, stream)) return fail_from(k.err_tc_stream, "host step");
+    if (fused_product(st.xw[1], L.w_gu, st.act, DT_BF16, 2 * L.I, st.H, L.I, MODE_SILU_MUL, L.gu_pair, &ep, st, stream)) return 1;
     // down projection into the residual, preparing the next layer's first norm
-    ++launches;
+    memset(&ep, 0, sizeof(ep));
     if (next) {
-        memset(&ep, 0, sizeof(ep));
         ep.xw = st.xw[0]; ep.next_w = next->norm1; ep.ssq_out = st.ssq[0];
-        if (k.tc_stream_fused(st.act, L.w_down, st.h, DT_F32, st.T, st.H, L.I, L.I, L.I, st.H, MODE_ACCUMULATE, 0, &ep, st.status,
-                              stream)) return fail_from(k.err_tc_stream, "host step");
         n_ssq = tiles;
-    } else if (k.tc_stream(st.act, L.w_down, st.h, DT_F32, st.T, st.H, L.I, L.I, L.I, st.H, MODE_ACCUMULATE, 0, st.status, stream)) {
-        return fail_from(k.err_tc_stream, "host step");
     }
+    if (fused_product(st.act, L.w_down, st.h, DT_F32, st.H, L.I, st.H, MODE_ACCUMULATE, 0, &ep, st, stream)) return 1;
     return 0;
 }
 
@@ -219,7 +234,7 @@ SP_API int sp_host_step_bind(const void* table, int bytes) {
     if (bytes != (int)sizeof(HostKernels)) SP_FAIL("host step: the kernel table has %d bytes, %d are expected", bytes, (int)sizeof(HostKernels));
     memcpy(&kernels, table, sizeof(kernels));
     if (!kernels.rmsnorm || !kernels.gemv || !kernels.tc_stream || !kernels.tc_gemm || !kernels.rope_kv_write ||
-        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.rope_table || !kernels.norm_prepare)
+        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.rope_table || !kernels.norm_prepare)
         SP_FAIL("host step: an entry point is missing from the kernel table");
     bound = true;
     return 0;

@@ -402,6 +402,9 @@ STATUS_TEXT = {101: "the TMA loader waited too long for a free pipeline stage",
                121: "tc_stream: the TMA loader waited too long for a free pipeline stage",
                122: "tc_stream: the MMA issuer waited too long for operands",
                123: "tc_stream: the epilogue warps waited too long for the accumulator",
+               131: "tc_mid: the TMA loader waited too long for a free pipeline stage",
+               132: "tc_mid: the MMA issuer waited too long for operands",
+               133: "tc_mid: the epilogue warps waited too long for the accumulator",
                201: "decode layers: the copy warp waited too long for a free stage of the weight ring",
                202: "decode layers: a consumer warp waited too long for a weight tile",
                203: "decode layers: a CTA waited too long at the grid barrier",
@@ -570,8 +573,8 @@ def _fused_product(module, a, w, out, mode, width, n_tiles, row_ssq, norm_width,
         ep.nh, ep.nkv, ep.hd, ep.page_size = int(r["nh"]), int(r["nkv"]), int(r["hd"]), int(r["page_size"])
         _declare_bounds(module, lib, r.get("declared_pages", r["k_pool"].shape[0]), 0, a.device)
         c_ptr, c_dt, ldc = None, BF16, 0
-        if module == "tc_stream":
-            code = 4                                   # 3 is the greedy head's mode there
+        if module != "tc_gemm":
+            code = 4                                   # 3 is the greedy head's mode in tc_stream
     else:
         want_cols = N // 2 if mode == TC_SILU_MUL else N
         if out.shape[0] != M or out.shape[1] != want_cols or out.stride(1) != 1:
@@ -579,6 +582,12 @@ def _fused_product(module, a, w, out, mode, width, n_tiles, row_ssq, norm_width,
         c_ptr, c_dt, ldc = _ptr(out), dt_code(out), out.stride(0)
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"{module} takes bfloat16 operands")
+    if module == "tc_mid":
+        _check(module, lib.sp_tc_mid(
+            c_void_p(_ptr(a)), c_void_p(_ptr(w)), c_void_p(c_ptr), c_dt, M, N, K, a.stride(0), w.stride(0), ldc, code, width,
+            ctypes.byref(ep), ACT_SILU, c_float(1.0), c_float(0.0), c_float(0.0), c_void_p(_ptr(status_word(a.device))),
+            c_void_p(_stream())))
+        return
     fn = lib.sp_tc_gemm_fused if module == "tc_gemm" else lib.sp_tc_stream_fused
     _check(module, fn(
         c_void_p(_ptr(a)), c_void_p(_ptr(w)), c_void_p(c_ptr), c_dt, M, N, K, a.stride(0), w.stride(0), ldc,
@@ -967,6 +976,50 @@ def tc_stream(x, w, out, mode=TC_STORE, pair=0, act=ACT_SILU, mult: float = 1.0,
     _check("tc_stream", lib.sp_tc_stream(
         c_void_p(_ptr(x)), c_void_p(_ptr(w)), c_void_p(_ptr(out)), dt_code(out), M, N, K, x.stride(0), w.stride(0),
         out.stride(0), int(mode), int(pair), c_void_p(_ptr(status_word(x.device))), c_void_p(_stream())))
+
+
+# ------------------------------------------------------------------ tensor-core product for dozens to hundreds of tokens
+def tc_mid_supported(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode=TC_STORE, pair: int = 0) -> bool:
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.dim() != 2 or w.dim() != 2:
+        return False
+    if x.stride(1) != 1 or w.stride(1) != 1 or x.shape[1] != w.shape[1] or out.data_ptr() % 16 or out.stride(0) % 4:
+        return False
+    return load("tc_mid").sp_tc_mid_supported(
+        c_void_p(_ptr(x)), c_void_p(_ptr(w)), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
+        int(mode), int(pair)) == 0
+
+
+def tc_mid(x, w, out, mode=TC_STORE, pair=0, act=ACT_SILU, mult: float = 1.0, limit: float = 0.0, slope: float = 0.0):
+    """out = x · wᵀ for some dozens to some hundreds of tokens on the tensor cores: rows of ``w`` as the instruction's M, up
+    to 256 tokens as its N, tiles of tokens and pieces of K chosen together by the sizes. Modes as ``tc_gemm``; for
+    TC_SILU_MUL gate and up rows alternate in blocks of ``pair`` = 128."""
+    lib = load("tc_mid")
+    M, K = x.shape
+    N = w.shape[0]
+    want_cols = N // 2 if mode == TC_SILU_MUL else N
+    if out.shape[0] != M or out.shape[1] != want_cols or out.stride(1) != 1:
+        raise KernelError(f"tc_mid: out {tuple(out.shape)} does not fit x {tuple(x.shape)}, w {tuple(w.shape)}")
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        raise KernelError("tc_mid takes bfloat16 operands")
+    _check("tc_mid", lib.sp_tc_mid(
+        c_void_p(_ptr(x)), c_void_p(_ptr(w)), c_void_p(_ptr(out)), dt_code(out), M, N, K, x.stride(0), w.stride(0),
+        out.stride(0), int(mode), int(pair), c_void_p(None), int(act), c_float(mult), c_float(limit), c_float(slope),
+        c_void_p(_ptr(status_word(x.device))), c_void_p(_stream())))
+
+
+def tc_mid_fused(a, w, out, mode, pair=0, row_ssq=None, norm_width=0, eps=0.0, xw=None, next_w=None, ssq_out=None,
+                 rope=None):
+    """``tc_mid`` with the epilogues of ``tc_stream_fused``; ``ssq_out`` is [M, tc_stream_n_tiles(N)] as there."""
+    _fused_product("tc_mid", a, w, out, mode, int(pair), tc_stream_n_tiles(w.shape[0]), row_ssq, norm_width, eps, xw,
+                   next_w, ssq_out, rope)
+
+
+def tc_mid_plan(mode, M: int, N: int, K: int) -> tuple:
+    """(token tiles, tokens per tile, pieces of K, stages) of a product of these sizes."""
+    out = (c_int * 4)()
+    if load("tc_mid").sp_tc_mid_plan(int(mode), int(M), int(N), int(K), out):
+        raise KernelError(f"tc_mid: no division of {M} tokens x {N} x {K}")
+    return tuple(out)
 
 
 # ------------------------------------------------------------------ seqmix: other mixers, their norm and activation

@@ -3,9 +3,10 @@
 Part by part a layer is eight launches: norm, QKV, rotate-and-store, attention, output projection, norm, gate/up,
 down. When every layer's parts describe themselves through ``fused_fields()`` (the same pre-norm / RMS norm / rotary
 grouped-query attention / SwiGLU, bfloat16 description that the one-kernel decode path reads) a step of 17 tokens
-to 64 (a prompt, or a decode step of that many sequences: the kernel that streams the weights, ``tc_stream``) or of
-more than 128 (the tile kernel, ``tc_gemm``) runs each layer as five. Between them the tile kernel splits K over a
-cluster, which has no such epilogues, and is faster than either fused form (a 100-token step: 2.1 ms against 2.6):
+or more runs each layer as five: up to ``MID_TOKENS`` on ``tc_mid`` (a prompt, or a decode step of that many sequences),
+beyond on the tile kernel, ``tc_gemm``. Where gate and up rows lie in blocks of 64 ``tc_mid`` does not take the layer:
+``tc_stream`` does up to 64 tokens and ``tc_gemm`` from 129 on, and between them the step runs part by part (the tile
+kernel then splits K over a cluster, which has no such epilogues):
 
 * QKV product on ``xw`` = residual ⊙ norm weight, its result multiplied by each row's 1/rms, rotated, q stored and
   k, v written into the paged cache in the product's epilogue;
@@ -24,7 +25,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import lib as K
-from ..parts.linear import STREAM_TOKENS, sm_count, tile_width
+from ..parts.linear import MID_TOKENS, STREAM_TOKENS, sm_count, tile_width
 from .fused_decode import collect_fused_fields, five_launch_from
 from ..phases import phase
 
@@ -32,8 +33,13 @@ MIN_TOKENS = 17          # up to 16 tokens the weight-streaming kernels (or the 
 TILE_TOKENS = 129        # from here on the tile kernel's epilogues
 
 
-def fuses(n_tokens: int) -> bool:
-    return MIN_TOKENS <= n_tokens <= STREAM_TOKENS or n_tokens >= TILE_TOKENS
+def mid_layers(fields: list) -> bool:
+    """Whether ``tc_mid`` takes every product of these layers."""
+    return all(f["ffn"]["pair"] == 128 and f["mixer"]["hidden_size"] % 8 == 0 for f in fields)
+
+
+def fuses(n_tokens: int, mid: bool) -> bool:
+    return MIN_TOKENS <= n_tokens <= (MID_TOKENS if mid else STREAM_TOKENS) or n_tokens >= TILE_TOKENS
 
 
 class FusedPrefill:
@@ -42,6 +48,7 @@ class FusedPrefill:
         self.fields = fields
         self.H = fields[0]["mixer"]["hidden_size"]
         self.hd = fields[0]["mixer"]["head_dim"]
+        self.mid = mid_layers(fields)
         self.runs = 0
         self.layer_bytes = max(sum(w.numel() * w.element_size() for w in (f["mixer"]["qkv"], f["mixer"]["o"], f["ffn"]["gate_up"],
                                                                      f["ffn"]["down"])) for f in fields)
@@ -73,7 +80,7 @@ class FusedPrefill:
 
     def takes(self, step, cache) -> bool:
         # (a decode step of up to 16 sequences comes here too where large layers make this the faster way)
-        if not (fuses(step.n_tokens) or (step.all_single and step.n_tokens >= five_launch_from(self.layer_bytes))):
+        if not (fuses(step.n_tokens, self.mid) or (step.all_single and step.n_tokens >= five_launch_from(self.layer_bytes))):
             return False
         for e in self.model.spec.schedule:
             g = cache.kv_groups.get(cache.cache_group.get(e.cache))
@@ -99,23 +106,26 @@ class FusedPrefill:
         T, H, hd = step.n_tokens, self.H, self.hd
         dev, bf = h.device, torch.bfloat16
         sms = sm_count(dev)
-        stream = T <= STREAM_TOKENS                    # the kernel that streams the weights takes these few tokens
+        mid = self.mid and T <= MID_TOKENS
+        stream = not mid and T <= STREAM_TOKENS        # the kernel that streams the weights takes these few tokens
         schedule = self.model.spec.schedule
 
         def product(a, w, out, mode, bn, pair=0, **kw):
-            if stream:
+            if mid:
+                K.tc_mid_fused(a, w, out, mode, pair, **kw)
+            elif stream:
                 K.tc_stream_fused(a, w, out, mode, pair, **kw)
             else:
                 K.tc_gemm_fused(a, w, out, mode, bn, **kw)
 
         def res_tiles(bn):
-            return K.tc_stream_n_tiles(H) if stream else K.tc_gemm_n_tiles(H, bn)
+            return K.tc_stream_n_tiles(H) if mid or stream else K.tc_gemm_n_tiles(H, bn)
 
         def into_residual(a, w, next_w):
             """h += a·wᵀ, and the next norm's input: (residual ⊙ next_w in bfloat16, the rows' sums of squares)."""
             bn = tile_width(T, H, sms)
             xw = torch.empty(T, H, dtype=bf, device=dev)
-            if not stream and K.tc_gemm_splits(T, H, a.shape[1], bn) > 1:
+            if not (mid or stream) and K.tc_gemm_splits(T, H, a.shape[1], bn) > 1:
                 # few tiles and a long K (the down projection of a few hundred tokens): the kernel that splits K over a
                 # cluster has the plain epilogues only, so the norm's input is a small kernel of its own behind it
                 ssq = torch.empty(T, 1, dtype=torch.float32, device=dev)
@@ -161,6 +171,8 @@ class FusedPrefill:
             with phase("down_projection+mlp_residual_ms"):
                 if i + 1 < len(self.fields):
                     xw, ssq = into_residual(act, ff["down"], self.fields[i + 1]["mixer_norm"]["weight"])
+                elif mid:
+                    K.tc_mid(act, ff["down"], h, K.TC_ACCUMULATE)
                 elif stream:
                     K.tc_stream(act, ff["down"], h, K.TC_ACCUMULATE)
                 else:

@@ -5,7 +5,7 @@ microseconds each, and from Python each costs ten microseconds or more. When eve
 through ``fused_fields()`` (the description the one-kernel decode path and the fused prompt path read), a prompt step
 of at most 128 tokens hands the whole sequence to ``csrc/host_step.cu``: a table of layer descriptors built once per
 cache, the step's arrays and its activation buffers. Up to 16 tokens the kernels are the same as part by part, chosen
-by the same thresholds (``parts/linear.py``), so the results are bit-identical to the Python path. From 17 to 64 tokens
+by the same thresholds (``parts/linear.py``), so the results are bit-identical to the Python path. From 17 tokens on
 (head sizes 64 and 128) a layer is five launches instead of eight: the norms, the rotation and the cache write ride in
 the products' epilogues, the same kernels with the same arguments as ``engine/fused_prefill.py`` launches them, so
 those results are bit-identical to that runner's. Anything else (another mixer, 32-bit, a larger step, a profiled
@@ -29,8 +29,9 @@ class _Kernels(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in (
         "rmsnorm", "gemv", "gemv_supported", "tc_stream", "tc_stream_supported", "tc_gemm", "tc_gemm_supported",
         "gemm_generic", "silu_mul", "rope_kv_write", "flash_prefill", "err_generic", "err_gemv", "err_tc_stream",
-        "err_tc_gemm", "err_attention", "tc_stream_fused", "rope_table", "norm_prepare")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
-                                            ("flash_query_tile", c_int), ("pad", c_int)]
+        "err_tc_gemm", "err_attention", "tc_stream_fused", "rope_table", "norm_prepare", "tc_mid", "tc_mid_supported",
+        "err_tc_mid")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
+                                            ("flash_query_tile", c_int), ("mid_tokens", c_int)]
 
 
 class _Layer(ctypes.Structure):
@@ -43,7 +44,7 @@ class _Step(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("h", "x", "qkv", "q", "ctx", "act", "gu", "token_seq", "positions", "seq_row",
                                         "page_table", "seq_start", "status", "xw0", "xw1", "ssq0", "ssq1", "cs",
                                         "tok_page")] + \
-               [(n, c_int) for n in ("T", "H", "n_seqs", "max_pages", "page_size", "n_q_tiles", "fused", "pad1")]
+               [(n, c_int) for n in ("T", "H", "n_seqs", "max_pages", "page_size", "n_q_tiles", "fused", "mid")]
 
 
 def _address(lib, name) -> int:
@@ -63,7 +64,7 @@ def _bind() -> ctypes.CDLL:
         want = int(getattr(host, f"sp_host_step_{size}_bytes")())
         if ctypes.sizeof(struct) != want:
             raise K.KernelError(f"host step: the {size} record has {ctypes.sizeof(struct)} bytes here, {want} in the library")
-    generic, gemv, stream, gemm, att = (K.load(m) for m in ("generic", "gemv", "tc_stream", "tc_gemm", "attention"))
+    generic, gemv, stream, gemm, att, mid = (K.load(m) for m in ("generic", "gemv", "tc_stream", "tc_gemm", "attention", "tc_mid"))
     t = _Kernels()
     t.rmsnorm, t.gemm_generic = _address(generic, "sp_rmsnorm"), _address(generic, "sp_gemm_generic")
     t.silu_mul, t.rope_kv_write = _address(generic, "sp_silu_mul"), _address(generic, "sp_rope_kv_write")
@@ -76,7 +77,9 @@ def _bind() -> ctypes.CDLL:
     t.err_generic, t.err_gemv = _address(generic, "sp_generic_last_error"), _address(gemv, "sp_gemv_last_error")
     t.err_tc_stream, t.err_tc_gemm = _address(stream, "sp_tc_stream_last_error"), _address(gemm, "sp_tc_gemm_last_error")
     t.err_attention = _address(att, "sp_attention_last_error")
-    t.gemv_tokens, t.stream_tokens = L.GEMV_TOKENS, L.STREAM_TOKENS
+    t.tc_mid, t.tc_mid_supported = _address(mid, "sp_tc_mid"), _address(mid, "sp_tc_mid_supported")
+    t.err_tc_mid = _address(mid, "sp_tc_mid_last_error")
+    t.gemv_tokens, t.stream_tokens, t.mid_tokens = L.GEMV_TOKENS, L.STREAM_TOKENS, L.MID_TOKENS
     t.flash_query_tile = K.flash_query_tile()
     K._check("host_step", host.sp_host_step_bind(ctypes.byref(t), ctypes.sizeof(t)))
     _bound = True
@@ -105,8 +108,9 @@ class HostStep:
             if hd % 16 or not 16 <= hd <= 128 or m["num_heads"] // m["num_kv_heads"] > 16:
                 return None                              # the prompt attention kernel's sizes
         runner = cls(model, fields)
-        from .fused_prefill import FusedPrefill
+        from .fused_prefill import FusedPrefill, mid_layers
         runner.can_fuse = FusedPrefill.plan(model) is not None
+        runner.mid = mid_layers(fields)
         return runner
 
     def takes(self, step, cache) -> bool:
@@ -171,7 +175,7 @@ class HostStep:
         st.ctx, off = off, off + T * self.max_q * 2
         st.act = off
         from .fused_prefill import fuses
-        fused = self.can_fuse and self.model.fuse_prefill and fuses(T)
+        fused = self.can_fuse and self.model.fuse_prefill and fuses(T, self.mid)
         if fused:
             tiles = K.tc_stream_n_tiles(self.H)
             hd = self.layers[0].hd
@@ -184,7 +188,7 @@ class HostStep:
             st.ssq1, off = off, off + T * tiles * 4
             st.cs, off = off, off + T * hd * 4                # (cos, sin) pairs of hd / 2 angles
             st.tok_page = off
-            st.fused = 1
+            st.fused, st.mid = 1, int(self.mid)
             self.extra = extra
         pt = step.page_tables[self.group]
         st.token_seq, st.positions, st.seq_row = step.token_seq.data_ptr(), step.positions.data_ptr(), step.seq_row.data_ptr()
@@ -192,7 +196,7 @@ class HostStep:
         st.status = K.status_word(dev).data_ptr()
         st.T, st.H, st.n_seqs, st.max_pages, st.page_size = T, self.H, step.n_seqs, pt.shape[1], cache.page_size
         st.n_q_tiles = K.query_tiles(step.host["new_counts"], K.flash_query_tile())
-        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream"):       # the debug build's bounds, library by library
+        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream", "tc_mid"):       # the debug build's bounds, library by library
             K._declare_bounds(module, K.load(module), cache.kv_groups[self.group].n_pages, pt.shape[0], dev)
         stream = K._stream()
         rc = host.sp_host_step_prompt_layers(self.layers, len(self.fields), ctypes.byref(st), c_void_p(stream))

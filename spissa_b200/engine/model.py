@@ -68,7 +68,7 @@ class Model:
             walk(p)
         if act_dtype != torch.bfloat16:
             return ["generic"] + own
-        mods = ["generic", "gemv", "tc_gemm", "tc_stream"] + own
+        mods = ["generic", "gemv", "tc_gemm", "tc_mid", "tc_stream"] + own
         kinds = {layer.mixer.kind for layer in self.spec.layers}
         if "attention" in kinds:
             mods.append("attention")

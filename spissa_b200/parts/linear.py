@@ -2,9 +2,8 @@
 
 ``Linear`` holds one weight matrix and picks the kernel for a call by the operands'
 storage types and sizes: bfloat16 activations on a bfloat16 weight go to the weight-streaming
-kernel for a few tokens (decoding), to the tcgen05 kernel that streams the weight with its rows as the
-instruction's M for a few dozen tokens, and to the tcgen05 tile kernel otherwise, when the rows are
-multiples of 16 bytes; everything else, and the whole 32-bit path, goes to the FFMA kernel.
+kernel for a few tokens (decoding), to the tcgen05 kernel with the weight's rows as the instruction's M for some dozens
+to some hundreds of tokens, and to the tcgen05 tile kernel otherwise, when the rows are multiples of 16 bytes; everything else, and the whole 32-bit path, goes to the FFMA kernel.
 """
 from __future__ import annotations
 
@@ -23,8 +22,13 @@ def sm_count(device=None) -> int:
     return _SM_COUNT[index]
 GEMV_TOKENS = 16          # up to this many tokens the weight-streaming kernel runs instead of 128-row tiles
 GATED_GEMV_TOKENS = 16    # the same for the gate/up product
-STREAM_TOKENS = 64        # from there up to this many tokens the weight streams through tcgen05 with the tokens as the
-#                           instruction's N (at 64 tokens: QKV 9.4 vs 12.8 us, gate/up 29 vs 40 us, down 14.4 vs 19.5 us)
+MID_TOKENS = 1023         # from there up to this many tokens the weight's rows are the instruction's M and the tokens its N
+#                           (tc_mid.cu). Per layer of the 1B shape (QKV + output + gate/up + down, us) against what ran before
+#                           (tc_stream.cu up to 64 tokens, tc_gemm.cu's tiles of 128 tokens beyond): 33 tokens 44 / 47, 64: 47 / 50,
+#                           100: 53 / 92, 301: 67 / 122, 512: 83 / 108, 1,000: 138 / 201; of the 8B shape 100: 110 / 149,
+#                           301: 171 / 254, 700: 321 / 416, 1,000: 430 / 435. From 1,024 tokens on tc_gemm.cu has enough tiles for
+#                           pairs of CTAs, which read half as much per product
+STREAM_TOKENS = 64        # what tc_mid.cu does not take (gate and up rows in blocks of 64): tc_stream.cu up to this many tokens
 
 
 def tile_width(M: int, N: int, sms: int | None = None) -> int:
@@ -61,6 +65,8 @@ class Linear:
         mode = K.TC_ACCUMULATE if accumulate else K.TC_STORE
         if x.shape[0] <= GEMV_TOKENS and K.gemv_supported(x, self.weight):
             K.gemv(x, self.weight, out, mode)
+        elif x.shape[0] <= MID_TOKENS and K.tc_mid_supported(x, self.weight, out, mode):
+            K.tc_mid(x, self.weight, out, mode)
         elif x.shape[0] <= STREAM_TOKENS and K.tc_stream_supported(x, self.weight, mode):
             K.tc_stream(x, self.weight, out, mode)
         elif K.tc_gemm_supported(x, self.weight):
@@ -106,6 +112,8 @@ class GatedLinear:
         kw = dict(act=self.act, mult=self.mult, limit=self.limit, slope=self.slope)
         if self.block and x.shape[0] <= GATED_GEMV_TOKENS and K.gemv_supported(x, self.weight):
             K.gemv(x, self.weight, out, K.TC_SILU_MUL, self.block, **kw)
+        elif self.block and x.shape[0] <= MID_TOKENS and K.tc_mid_supported(x, self.weight, out, K.TC_SILU_MUL, self.block):
+            K.tc_mid(x, self.weight, out, K.TC_SILU_MUL, self.block, **kw)
         elif self.block and x.shape[0] <= STREAM_TOKENS and K.tc_stream_supported(x, self.weight, K.TC_SILU_MUL, self.block):
             K.tc_stream(x, self.weight, out, K.TC_SILU_MUL, self.block, **kw)
         elif self.block and K.tc_gemm_supported(x, self.weight):

@@ -1,0 +1,152 @@
+"""The product with W's rows as the instruction's M and up to 256 tokens as its N (tc_mid.cu), at the sizes where its tiles
+end: tokens that are no multiple of 16, several token tiles, pieces of K that are not equally long, rows of W that do not
+fill a tile; and every epilogue in the divisions that the sizes choose."""
+import pytest
+import torch
+
+import kernel_harness as KH
+from plain import llama_plain as P
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def K():
+    from spissa_b200.csrc import lib
+    yield lib
+    lib.check_status(DEV)
+
+
+def within(got, a, w, extra=None, rel=0.0):
+    """Against the exact sum of the bfloat16 products. A float32 sum of K terms in any order is off by less than
+    K · 2^-23 · Σ|a||w| (2^-24 for each addition that rounds to nearest, twice that where it truncates); ``rel``: the
+    storage's rounding of the result."""
+    ref, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    if extra is not None:
+        ref, size = ref + extra.double(), size + extra.double().abs()
+    bound = a.shape[1] * 2.0 ** -23 * size + rel * ref.abs() + 1e-30
+    assert bool(((got.double() - ref).abs() <= bound).all())
+
+
+def operands(M, N, Kd, seed=0):
+    torch.manual_seed(M * 7 + N + Kd + seed)
+    return torch.randn(M, Kd, device=DEV).bfloat16(), (torch.randn(N, Kd, device=DEV) * 0.1).bfloat16()
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 160, 161, 256, 257, 301, 1023])
+@pytest.mark.parametrize("N,Kd", [(8, 8), (136, 72), (128, 2048), (3072, 2048), (72, 1096)])
+def test_store_and_accumulate(K, M, N, Kd):
+    a, w = operands(M, N, Kd)
+    tiles, nt, pieces, stages = K.tc_mid_plan(K.TC_STORE, M, N, Kd)
+    assert nt % 16 == 0 and nt <= 256 and (tiles - 1) * nt < M <= tiles * nt and stages >= 1
+    blocks = -(-Kd // 64)
+    assert (pieces - 1) * -(-blocks // pieces) < blocks                 # no CTA of a cluster without a block of K
+    out = torch.full((M, N), float("nan"), device=DEV)
+    assert K.tc_mid_supported(a, w, out)
+    K.tc_mid(a, w, out)
+    within(out, a, w)
+    short = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    K.tc_mid(a, w, short)
+    within(short, a, w, rel=2.0 ** -8)
+    c0 = torch.randn(M, N, device=DEV)
+    acc, again = c0.clone(), c0.clone()
+    K.tc_mid(a, w, acc, K.TC_ACCUMULATE)
+    within(acc, a, w, extra=c0)
+    K.tc_mid(a, w, again, K.TC_ACCUMULATE)
+    assert torch.equal(acc, again)                                      # a fixed order of sums
+
+
+def test_rows_further_apart_than_they_are_long(K):
+    a, w = operands(70, 264, 136)
+    wide_a, wide_w, wide_c = (torch.full((t.shape[0], t.shape[1] + 24), 9.0, dtype=t.dtype, device=DEV)
+                              for t in (a, w, torch.empty(70, 264)))
+    wide_a[:, :136], wide_w[:, :136] = a, w
+    K.tc_mid(wide_a[:, :136], wide_w[:, :136], wide_c[:, :264])
+    within(wide_c[:, :264], a, w)
+    assert bool((wide_c[:, 264:] == 9.0).all())
+
+
+def test_operands_it_does_not_take(K):
+    a, w = operands(64, 256, 128)
+    out = torch.empty(64, 256, device=DEV)
+    assert K.tc_mid_supported(a, w, out)
+    assert not K.tc_mid_supported(a, w, torch.empty(64, 258, device=DEV)[:, 1:257])          # C off a 16-byte boundary
+    assert not K.tc_mid_supported(a[:, 1:125], w[:, 1:125], out)
+    assert not K.tc_mid_supported(a, w[:252], out[:, :252])                                  # rows of W in eights
+    assert not K.tc_mid_supported(a, w, torch.empty(64, 128, device=DEV), K.TC_SILU_MUL, 64)
+    with pytest.raises(K.KernelError):
+        K.tc_mid(a, w, torch.empty(64, 128, device=DEV), K.TC_SILU_MUL, 64)
+    with pytest.raises(K.KernelError):
+        K.tc_mid(a, w, torch.empty(64, 256, dtype=torch.bfloat16, device=DEV), K.TC_ACCUMULATE)
+    K.check_status(DEV)
+
+
+@pytest.mark.parametrize("M,I,H", [(20, 128, 264), (64, 8192, 2048), (100, 8192, 2048), (301, 1024, 512), (700, 2048, 2048), (257, 128, 4096)])
+@pytest.mark.parametrize("act", ["silu", "gelu", "clamped"])
+def test_gated_rows(K, M, I, H, act):
+    """With rows scaled by 1/rms (silu) and without (the other activations); one piece of K and several."""
+    x, w = operands(M, 2 * I, H)
+    v = w.reshape(I // 128, 2, 128, H)
+    g, u = (x.double() @ v[:, i].reshape(I, H).double().t() for i in (0, 1))
+    out = torch.full((M, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+    if act == "silu":
+        ssq = torch.rand(M, 5, device=DEV) * H
+        K.tc_mid_fused(x, w, out, K.TC_SILU_MUL, 128, row_ssq=ssq, norm_width=H, eps=1e-6)
+        rs = 1.0 / torch.sqrt(ssq.double().sum(1, keepdim=True) / H + 1e-6)
+        ref = P.silu(g * rs) * (u * rs)
+    elif act == "gelu":
+        K.tc_mid(x, w, out, K.TC_SILU_MUL, 128, act=K.ACT_GELU, mult=0.5)
+        ref = torch.nn.functional.gelu(g, approximate="tanh") * u * 0.5
+    else:
+        K.tc_mid(x, w, out, K.TC_SILU_MUL, 128, act=K.ACT_CLAMPED, limit=2.0, slope=1.702)
+        gc, uc = g.clamp(max=2.0), u.clamp(-2.0, 2.0)
+        ref = gc * torch.sigmoid(1.702 * gc) * (uc + 1.0)
+    # bfloat16 rounds by 2^-9; the float32 sums of H terms and the activation are far below that
+    assert float((out.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max())
+    assert float((out.double() - ref).norm() / ref.norm()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,N,Kd", [(17, 520, 264), (100, 2048, 8192), (301, 2048, 2048), (1000, 256, 2048)])
+def test_accumulate_prepares_the_next_norm(K, M, N, Kd):
+    a, w = operands(M, N, Kd)
+    c0 = torch.randn(M, N, device=DEV)
+    next_w = (1 + 0.2 * torch.randn(N, device=DEV)).bfloat16()
+    c = c0.clone()
+    xw = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ssq = torch.full((M, K.tc_stream_n_tiles(N)), float("nan"), device=DEV)
+    K.tc_mid_fused(a, w, c, K.TC_ACCUMULATE, xw=xw, next_w=next_w, ssq_out=ssq)
+    within(c, a, w, extra=c0)
+    assert torch.equal(xw, (c * next_w.float()).bfloat16())             # of the very sums it stored
+    want = (c.double() ** 2).sum(1)
+    assert float(((ssq.double().sum(1) - want) / want).abs().max()) <= 128 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 6, 2), (64, 5, 1), (64, 32, 8), (128, 4, 2), (128, 3, 1)])
+@pytest.mark.parametrize("new_counts,before", [([9, 7, 1], [0, 100, 61]), ([130, 7, 70], [0, 100, 61]), ([400, 1, 330], [0, 64, 5])])
+def test_qkv_rotates_and_writes_the_cache(K, hd, nh, nkv, new_counts, before):
+    torch.manual_seed(hd + nh)
+    H, T, N = 1032, sum(new_counts), (nh + 2 * nkv) * hd
+    meta = KH.paged_meta(new_counts, before, DEV, seed=hd)
+    x, w = operands(T, N, H)
+    ssq = torch.rand(T, 3, device=DEV) * H
+    inv_freq = P.rope_inv_freq(10000.0, hd).to(DEV)
+    cs, tok_page = torch.empty(T, hd // 2, 2, device=DEV), torch.empty(T, dtype=torch.int32, device=DEV)
+    K.rope_table(meta, inv_freq, hd // 2, cs, tok_page)
+    pools = [torch.full((meta.n_pages, nkv, 64, hd), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    q = torch.full((T, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    K.tc_mid_fused(x, w, None, K.TC_QKV_ROPE, row_ssq=ssq, norm_width=H, eps=1e-5,
+                   rope=dict(cs=cs, tok_page=tok_page, positions=meta.positions, q_out=q, k_pool=pools[0], v_pool=pools[1],
+                             nh=nh, nkv=nkv, hd=hd, page_size=64))
+    rows = (x.double() @ w.double().t()) / torch.sqrt(ssq.double().sum(1, keepdim=True) / H + 1e-5)
+    rows = rows.reshape(T, nh + 2 * nkv, hd)
+    c, s = cs[..., 0].double()[:, None], cs[..., 1].double()[:, None]
+    lo, hi = rows[..., :hd // 2], rows[..., hd // 2:]
+    turned = torch.cat([lo * c - hi * s, hi * c + lo * s], dim=-1)
+    want = [turned[:, :nh], turned[:, nh:nh + nkv], rows[:, nh + nkv:]]
+    page, at = tok_page.long(), meta.positions.long() % 64
+    for got, ref in zip([q.view(T, nh, hd)] + [p[page, :, at] for p in pools], want):
+        assert float((got.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max())
+    for p in pools:                                                     # nothing else was written
+        p[page, :, at] = 7.0
+        assert bool((p == 7.0).all())
