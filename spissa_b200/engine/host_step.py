@@ -179,13 +179,14 @@ class HostStep:
         if fused:
             tiles = K.tc_stream_n_tiles(self.H)
             hd = self.layers[0].hd
-            extra = torch.empty(2 * T * self.H * 2 + 2 * T * tiles * 4 + T * hd * 4 + T * 4 + 64, dtype=torch.uint8, device=dev)
+            extra = torch.empty(2 * T * self.H * 2 + 2 * T * tiles * 4 + T * hd * 4 + T * 4 + 96, dtype=torch.uint8, device=dev)
             off = extra.data_ptr()
             off += (-off) % 16
             st.xw0, off = off, off + T * self.H * 2
             st.xw1, off = off, off + T * self.H * 2
             st.ssq0, off = off, off + T * tiles * 4
             st.ssq1, off = off, off + T * tiles * 4
+            off += (-off) % 16                                # the table is read 16 bytes at a time
             st.cs, off = off, off + T * hd * 4                # (cos, sin) pairs of hd / 2 angles
             st.tok_page = off
             st.fused, st.mid = 1, int(self.mid)
