@@ -15,6 +15,7 @@
 //   silu            crates/spissa-runtime/src/ops.rs:192-194
 //   argmax          crates/spissa-runtime/src/ops.rs:309-324  (first maximum wins)
 #include "async_copy.cuh"
+#include <type_traits>
 
 SP_API const char* sp_generic_last_error() { return sp_error_text; }
 SP_DEFINE_RANGE_API(generic)
@@ -283,15 +284,19 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 
 // The same product for a few rows of A (a decode step of the 32-bit path): W is streamed once with 16-byte loads,
 // a CTA of four warps owns eight rows of W (two per warp), the rows of A pass through shared memory in slices of
-// 512 columns. Each lane sums its columns k = 4·lane + 128·i in order, the lanes' sums are added by a shuffle tree:
-// the order is fixed and the same for every row of A, whatever M is, but it is another order than the tiled
-// kernel's, so a token's result differs between a decode step and a prompt step by 32-bit rounding.
+// 512 columns. What bounds it is bytes in flight: the next slice of W (and up to 4 rows of A) is asked for before the
+// products of this one, and the kernel may become resident before its predecessor ends. Each lane sums its columns
+// k = 4·lane + 128·i in order, the lanes' sums are added by a shuffle tree: the order is fixed and the same for every row
+// of A, whatever M is, but it is another order than the tiled kernel's, so a token's result differs between a decode step
+// and a prompt step by 32-bit rounding.
 #define GS_KC 512
 #define GS_ROWS 2
 template <int MT>
 __global__ void __launch_bounds__(128)
 gemm_stream_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, void* __restrict__ C, int c_dt,
                        int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
+    constexpr int XV = MT * (GS_KC / 4) / 128;               // 16-byte pieces of a slice of A per thread
+    constexpr bool XAHEAD = MT <= 4;                         // held in registers a slice ahead
     __shared__ __align__(16) float xs[MT][GS_KC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * 4 + warp) * GS_ROWS;
@@ -303,24 +308,36 @@ gemm_stream_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
     const float* wrow[GS_ROWS];
 #pragma unroll
     for (int r = 0; r < GS_ROWS; ++r) wrow[r] = W + (size_t)min(n0 + r, N - 1) * ldw;
-
-    for (int k0 = 0; k0 < K; k0 += GS_KC) {
-        __syncthreads();                                     // the slice before has been used by every warp
-        for (int e = threadIdx.x; e < MT * (GS_KC / 4); e += 128) {
-            const int m = e / (GS_KC / 4), c = (e % (GS_KC / 4)) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m < M && k0 + c < K) v = *(const float4*)(A + (size_t)m * lda + k0 + c);     // K is a multiple of 4
-            *(float4*)&xs[m][c] = v;
-        }
-        __syncthreads();
-        float4 w[GS_ROWS][GS_KC / 128];
+    float4 w[2][GS_ROWS][GS_KC / 128], x_next[XAHEAD ? XV : 1];
+    auto load_w = [&](int k0, float4 (&to)[GS_ROWS][GS_KC / 128]) {
 #pragma unroll
         for (int r = 0; r < GS_ROWS; ++r)
 #pragma unroll
             for (int i = 0; i < GS_KC / 128; ++i) {
                 const int k = k0 + i * 128 + lane * 4;
-                w[r][i] = k < K ? __ldcs((const float4*)(wrow[r] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                to[r][i] = k < K ? __ldcs((const float4*)(wrow[r] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+    };
+    auto load_x = [&](int k0, int v) {
+        const int e = threadIdx.x + 128 * v, m = e / (GS_KC / 4), c = (e % (GS_KC / 4)) * 4;
+        return m < M && k0 + c < K ? *(const float4*)(A + (size_t)m * lda + k0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);     // K is a multiple of 4
+    };
+    auto slice = [&](int k0, auto turn) {
+        constexpr int b = decltype(turn)::value;
+        __syncthreads();                                     // the slice before has been used by every warp
+#pragma unroll
+        for (int v = 0; v < XV; ++v) {
+            const int e = threadIdx.x + 128 * v;
+            *(float4*)&xs[e / (GS_KC / 4)][(e % (GS_KC / 4)) * 4] = XAHEAD ? x_next[XAHEAD ? v : 0] : load_x(k0, v);
+        }
+        __syncthreads();
+        if (k0 + GS_KC < K) {
+            load_w(k0 + GS_KC, w[b ^ 1]);
+            if (XAHEAD) {
+#pragma unroll
+                for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(k0 + GS_KC, v);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < GS_KC / 128; ++i)
 #pragma unroll
@@ -328,12 +345,23 @@ gemm_stream_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
                 const float4 x = *(const float4*)&xs[m][i * 128 + lane * 4];
 #pragma unroll
                 for (int r = 0; r < GS_ROWS; ++r) {
-                    acc[r][m] = fmaf(w[r][i].x, x.x, acc[r][m]);
-                    acc[r][m] = fmaf(w[r][i].y, x.y, acc[r][m]);
-                    acc[r][m] = fmaf(w[r][i].z, x.z, acc[r][m]);
-                    acc[r][m] = fmaf(w[r][i].w, x.w, acc[r][m]);
+                    acc[r][m] = fmaf(w[b][r][i].x, x.x, acc[r][m]);
+                    acc[r][m] = fmaf(w[b][r][i].y, x.y, acc[r][m]);
+                    acc[r][m] = fmaf(w[b][r][i].z, x.z, acc[r][m]);
+                    acc[r][m] = fmaf(w[b][r][i].w, x.w, acc[r][m]);
                 }
             }
+    };
+    sp_allow_dependents();
+    sp_wait_for_predecessor();
+    load_w(0, w[0]);
+    if (XAHEAD) {
+#pragma unroll
+        for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(0, v);
+    }
+    for (int k0 = 0; k0 < K; k0 += 2 * GS_KC) {
+        slice(k0, std::integral_constant<int, 0>());
+        if (k0 + GS_KC < K) slice(k0 + GS_KC, std::integral_constant<int, 1>());
     }
 #pragma unroll
     for (int r = 0; r < GS_ROWS; ++r)
@@ -357,14 +385,14 @@ SP_API int sp_gemm_generic(const void* A, int a_dt, const void* W, int w_dt, voi
         ((((uintptr_t)A) | ((uintptr_t)W)) & 15) == 0) {
         const unsigned blocks = (unsigned)((N + 4 * GS_ROWS - 1) / (4 * GS_ROWS));
 #define GS_LAUNCH(MT) \
-        gemm_stream_f32_kernel<MT><<<blocks, 128, 0, stream>>>((const float*)A, (const float*)W, C, c_dt, M, N, K, lda, ldw, ldc, accumulate)
+        SP_CHECK_CALL("gemm_stream_f32", sp_launch_dependent(gemm_stream_f32_kernel<MT>, dim3(blocks), dim3(128), 0, stream, \
+                                                             (const float*)A, (const float*)W, C, c_dt, M, N, K, lda, ldw, ldc, accumulate))
         if (M <= 1) GS_LAUNCH(1);
         else if (M <= 2) GS_LAUNCH(2);
         else if (M <= 4) GS_LAUNCH(4);
         else if (M <= 8) GS_LAUNCH(8);
         else GS_LAUNCH(16);
 #undef GS_LAUNCH
-        SP_CHECK_LAUNCH("gemm_stream_f32");
         return 0;
     }
     dim3 grid((N + GG_BN - 1) / GG_BN, (M + GG_BM - 1) / GG_BM);
