@@ -54,6 +54,7 @@ MODULES = {
     "decode_layers": "decode_layers.cu",
     "tc_stream": "tc_stream.cu",
     "tc_mid": "tc_mid.cu",
+    "tc_f32": "tc_f32.cu",
     "host_step": "host_step.cu",
     "seqmix": "seqmix_kernels.cu",
     "diff_flash": "diff_flash.cu",

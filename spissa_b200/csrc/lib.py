@@ -166,6 +166,32 @@ def gemm_generic(a, w, out, accumulate=False):
         M, N, K, a.stride(0), w.stride(0), out.stride(0), int(bool(accumulate)), c_void_p(_stream())))
 
 
+def tc_f32_supported(a, w, out) -> bool:
+    """Whether ``tc_f32`` takes these operands (float32, unit strides, rows a multiple of 16 bytes)."""
+    if not (a.dtype == w.dtype == out.dtype == torch.float32) or a.dim() != 2 or w.dim() != 2 or a.shape[1] != w.shape[1]:
+        return False
+    if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
+        return False
+    return load("tc_f32").sp_tc_f32_supported(c_void_p(_ptr(a)), c_void_p(_ptr(w)), a.shape[0], w.shape[0], a.shape[1],
+                                              a.stride(0), w.stride(0)) == 0
+
+
+def tc_f32(a, w, out, accumulate=False):
+    """out[M,N] (+)= a[M,K] · w[N,K]ᵀ, all float32, on the tensor cores: the operands in three bfloat16 parts each, the six
+    largest products of parts, float32 sums rounded to nearest every 64 terms (at least as near to the exact result as the
+    FFMA kernels; infinities and NaN as there)."""
+    lib = load("tc_f32")
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
+        raise KernelError(f"tc_f32: shapes do not match: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if not (a.dtype == w.dtype == out.dtype == torch.float32):
+        raise KernelError("tc_f32 takes float32 operands and writes float32")
+    _check("tc_f32", lib.sp_tc_f32(
+        c_void_p(_ptr(a)), c_void_p(_ptr(w)), c_void_p(_ptr(out)), M, N, K, a.stride(0), w.stride(0), out.stride(0),
+        int(bool(accumulate)), c_void_p(_ptr(status_word(a.device))), c_void_p(_stream())))
+
+
 def rope_kv_write(qkv, q_out, k_pool, v_pool, meta, inv_freq, nh, nkv, hd, rd, write_kv=True):
     """Rotate q and k of ``qkv`` [T, (nh+2·nkv)·hd], store q to ``q_out`` and k, v into the paged cache.
 
@@ -405,6 +431,10 @@ STATUS_TEXT = {101: "the TMA loader waited too long for a free pipeline stage",
                131: "tc_mid: the TMA loader waited too long for a free pipeline stage",
                132: "tc_mid: the MMA issuer waited too long for operands",
                133: "tc_mid: the epilogue warps waited too long for the accumulator",
+               141: "tc_f32: the MMA issuer waited too long for operands",
+               142: "tc_f32: a warp waited too long for an accumulator",
+               143: "tc_f32: a warp waited too long for a free stage",
+               144: "tc_f32: the MMA issuer waited too long for a free accumulator",
                201: "decode layers: the copy warp waited too long for a free stage of the weight ring",
                202: "decode layers: a consumer warp waited too long for a weight tile",
                203: "decode layers: a CTA waited too long at the grid barrier",

@@ -67,7 +67,7 @@ class Model:
         for p in self.parts():
             walk(p)
         if act_dtype != torch.bfloat16:
-            return ["generic"] + own
+            return ["generic", "tc_f32"] + own
         mods = ["generic", "gemv", "tc_gemm", "tc_mid", "tc_stream"] + own
         kinds = {layer.mixer.kind for layer in self.spec.layers}
         if "attention" in kinds:

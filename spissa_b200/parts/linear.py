@@ -3,7 +3,9 @@
 ``Linear`` holds one weight matrix and picks the kernel for a call by the operands'
 storage types and sizes: bfloat16 activations on a bfloat16 weight go to the weight-streaming
 kernel for a few tokens (decoding), to the tcgen05 kernel with the weight's rows as the instruction's M for some dozens
-to some hundreds of tokens, and to the tcgen05 tile kernel otherwise, when the rows are multiples of 16 bytes; everything else, and the whole 32-bit path, goes to the FFMA kernel.
+to some hundreds of tokens, and to the tcgen05 tile kernel otherwise, when the rows are multiples of 16 bytes;
+32-bit products of more than ``GEMV_TOKENS`` rows go to the tcgen05 kernel that multiplies float32 in bfloat16 parts;
+everything else goes to the FFMA kernels.
 """
 from __future__ import annotations
 
@@ -28,6 +30,8 @@ MID_TOKENS = 1023         # from there up to this many tokens the weight's rows 
 #                           100: 53 / 92, 301: 67 / 122, 512: 83 / 108, 1,000: 138 / 201; of the 8B shape 100: 110 / 149,
 #                           301: 171 / 254, 700: 321 / 416, 1,000: 430 / 435. From 1,024 tokens on tc_gemm.cu has enough tiles for
 #                           pairs of CTAs, which read half as much per product
+F32_PARTS_K = 128         # 32-bit products with sums at least so long go to tc_f32.cu. Relative error against 64 bits there / in order
+#                           on FFMA: K = 8 1.0e-7 / 5e-8, 72: 1.2e-7 / 1.5e-7, 128: 1.3e-7 / 2.0e-7, 2,048: 1.6e-7 / 8.1e-7
 STREAM_TOKENS = 64        # what tc_mid.cu does not take (gate and up rows in blocks of 64): tc_stream.cu up to this many tokens
 
 
@@ -71,6 +75,8 @@ class Linear:
             K.tc_stream(x, self.weight, out, mode)
         elif K.tc_gemm_supported(x, self.weight):
             K.tc_gemm(x, self.weight, out, mode, tile_width(x.shape[0], self.out_features, sm_count(x.device)))
+        elif x.shape[0] > GEMV_TOKENS and x.shape[1] >= F32_PARTS_K and K.tc_f32_supported(x, self.weight, out):
+            K.tc_f32(x, self.weight, out, accumulate=accumulate)
         else:
             K.gemm_generic(x, self.weight, out, accumulate=accumulate)
         return out

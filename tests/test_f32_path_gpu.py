@@ -1,0 +1,91 @@
+"""The kernels of 32-bit prompt steps: the product in bfloat16 parts (tc_f32.cu) at the edges of its tiles, its blocks and its
+pieces of K, nearer to 64 bits than the FFMA product; infinities and NaN; the attention by tiles of 64 queries and keys."""
+import math
+
+import pytest
+import torch
+
+import kernel_harness as KH
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def K():
+    from spissa_b200.csrc import lib
+    yield lib
+    lib.check_status(DEV)
+
+
+def operands(M, N, Kd):
+    torch.manual_seed(M + 3 * N + Kd)
+    return torch.randn(M, Kd, device=DEV), torch.randn(N, Kd, device=DEV) * 0.02
+
+
+@pytest.mark.parametrize("M", [1, 17, 32, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("N,Kd", [(1, 8), (130, 128), (127, 136), (128, 2048), (260, 1096)])
+def test_product_against_64_bits(K, M, N, Kd):
+    a, w = operands(M, N, Kd)
+    ref = a.double() @ w.double().t()
+    size = a.double().abs() @ w.double().abs().t()
+    out, ffma = torch.full((M, N), float("nan"), device=DEV), torch.empty(M, N, device=DEV)
+    assert K.tc_f32_supported(a, w, out)
+    K.tc_f32(a, w, out)
+    K.gemm_generic(a, w, ffma)
+    # the three products of parts left out are below 3 · 2^-24 of |a||w|; a block of 64 terms takes 24 additions that truncate
+    # (2^-23 each of what has been added up so far), and K / 64 sums that round
+    bound = (3 * 2.0 ** -24 + 24 * 2.0 ** -23 + (Kd / 64 + 1) * 2.0 ** -24) * size
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    if Kd >= 128 and M * N > 1000:
+        assert float((out.double() - ref).norm()) <= float((ffma.double() - ref).norm())
+    c0 = torch.randn(M, N, device=DEV)
+    acc = c0.clone()
+    K.tc_f32(a, w, acc, accumulate=True)
+    assert torch.equal(acc, c0 + out)                                   # one addition of the same sums
+
+
+def test_rows_apart_and_operands_it_does_not_take(K):
+    a, w = operands(40, 70, 136)
+    wide_a, wide_w, wide_c = (torch.full((t.shape[0], t.shape[1] + 8), 9.0, device=DEV) for t in (a, w, torch.empty(40, 70)))
+    wide_a[:, :136], wide_w[:, :136] = a, w
+    K.tc_f32(wide_a[:, :136], wide_w[:, :136], wide_c[:, 3:73])         # C off a 16-byte boundary
+    out = torch.empty(40, 70, device=DEV)
+    K.tc_f32(a, w, out)
+    assert torch.equal(wide_c[:, 3:73], out) and bool((wide_c[:, :3] == 9.0).all()) and bool((wide_c[:, 73:] == 9.0).all())
+    assert not K.tc_f32_supported(a[:, :132], w[:, :132], out)          # K and the rows' distance in eights
+    assert not K.tc_f32_supported(a[:, 4:132], w[:, 4:132], out)        # operands off a 32-byte boundary
+    assert not K.tc_f32_supported(a.bfloat16(), w, out)
+    with pytest.raises(K.KernelError):
+        K.tc_f32(a[:, :132], w[:, :132], out)
+
+
+@pytest.mark.parametrize("M,N,Kd", [(20, 130, 256), (200, 300, 2048)])
+def test_infinities_nan_and_extremes(K, M, N, Kd):
+    """What a plain float32 sum of products gives: a value that is not finite changes the results it enters and no others."""
+    a, w = operands(M, N, Kd)
+    a[3, 5], a[7, Kd - 1], a[11, 0] = float("inf"), float("-inf"), float("nan")
+    w[9, 17], w[N - 1, 2] = float("inf"), float("nan")
+    a[13, 8], w[20, 8] = 3.0e38, 3.0e38                                 # a product beyond the range of float32
+    out = torch.empty(M, N, device=DEV)
+    K.tc_f32(a, w, out)
+    ref = (a.double() @ w.double().t()).float()
+    assert torch.equal(torch.isnan(out), torch.isnan(ref))
+    assert torch.equal(out[torch.isinf(ref)], ref[torch.isinf(ref)])
+    fine = torch.isfinite(ref)
+    assert float((out[fine] - ref[fine]).abs().max() / ref[fine].abs().max()) <= 1e-5
+    tiny = torch.full((M, Kd), 1e-30, device=DEV)
+    K.tc_f32(tiny, w.nan_to_num(0, 0, 0).clamp(-1, 1), out)
+    ref = tiny.double() @ w.nan_to_num(0, 0, 0).clamp(-1, 1).double().t()
+    assert float((out.double() - ref).norm() / ref.norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd", [(5, 4), (90, 508), (64, 512), (33, 516), (17, 1024), (40, 1540)])
+def test_few_rows_slices_of_k(K, M, N, Kd):
+    a, w = operands(M, N, Kd)
+    out = torch.empty(M, N, device=DEV)
+    K.gemm_generic(a, w, out)
+    size = a.double().abs() @ w.double().abs().t()
+    # a lane adds Kd / 32 terms in order, then five rounds of sums
+    assert bool(((out.double() - a.double() @ w.double().t()).abs() <= (Kd / 32 + 8) * 2.0 ** -24 * size).all())
