@@ -817,6 +817,183 @@ SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, cons
     return 0;
 }
 
+// The same attention in 32 bits for prompts, by tiles: a CTA takes 64 queries of one (sequence, head) and walks the keys 64
+// at a time through shared memory, each of 256 threads 4 x 4 scores and 4 x 4 (per 64 value columns) sums. The kernel
+// above reads every key once per query; here a key is read once per 64 queries (500 tokens, 32 heads of 64 on 8 kv heads:
+// 423 us by the kernel above, 110 us here). Sums, softmax and exponentials are float32 as there; only their order differs.
+#define AT_TILE 64
+#define AT_MAX_D 128
+template <int VC>
+__global__ void __launch_bounds__(256)
+attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__ kpool, const float* __restrict__ vpool,
+                          float* __restrict__ out, KvPlace pl, const int* __restrict__ seq_start, int nh, int nkv, int hd, int vd,
+                          int window, float scale, const float* __restrict__ sink, const float* __restrict__ dist_bias, int dist_cap) {
+    extern __shared__ __align__(16) float at_smem[];
+    const int s = blockIdx.z, h = blockIdx.y, g = h / (nh / nkv);
+    const int tile = gridDim.x - 1 - blockIdx.x;             // the tiles with the most keys first
+    const int t0 = seq_start[s] + tile * AT_TILE, rows = min(AT_TILE, seq_start[s + 1] - t0);
+    if (rows <= 0) return;
+    // rows of four more words: sixteen neighbouring rows fall on different banks
+    const int ks = hd + 4, vs = vd + 4;
+    constexpr int PS = AT_TILE + 4;
+    float* const Q = at_smem;
+    float* const Kt = Q + AT_TILE * ks;
+    float* const V = Kt + AT_TILE * ks;
+    float* const P = V + AT_TILE * vs;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int slot = sp_checked_row(pl.seq_slot[s], pl.rg);
+    const int* pt = pl.page_table + (size_t)slot * pl.max_pages;
+    const int ps = pl.page_size, first = pl.positions[t0], last = first + rows - 1;     // a sequence's tokens stand side by side
+    for (int e = tid; e < AT_TILE * (hd / 4); e += 256) {
+        const int r = e / (hd / 4), c = (e % (hd / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows) v = *(const float4*)(q + (size_t)(t0 + r) * nh * hd + (size_t)h * hd + c);
+        *(float4*)(Q + r * ks + c) = v;
+    }
+    float m[4], l[4], acc[4][4 * VC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4 * VC; ++c) acc[i][c] = 0.0f;
+    }
+    const int lo = window > 0 ? max(0, first - window + 1) : 0;
+    for (int j0 = lo; j0 <= last; j0 += AT_TILE) {
+        __syncthreads();                                     // the tile before has been used
+        const int qd = (hd + vd) / 4;
+        for (int e = tid; e < AT_TILE * qd; e += 256) {
+            const int r = e / qd, c = (e % qd) * 4, j = j0 + r;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j <= last) {
+                const int page = sp_checked_page(pt[sp_checked_entry(j / ps, pl.max_pages, pl.rg)], pl.rg);
+                const size_t at = ((size_t)page * nkv + g) * ps + j % ps;
+                v = c < hd ? *(const float4*)(kpool + at * hd + c) : *(const float4*)(vpool + at * vd + (c - hd));
+            }
+            *(float4*)(c < hd ? Kt + r * ks + c : V + r * vs + (c - hd)) = v;
+        }
+        __syncthreads();
+        float sc[4][4] = {};
+        for (int d = 0; d < hd; d += 4) {
+            float4 a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a[i] = *(const float4*)(Q + (ty + 16 * i) * ks + d);
+                b[i] = *(const float4*)(Kt + (tx + 16 * i) * ks + d);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    sc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, sc[i][j]))));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = first + ty + 16 * i;               // beyond ``rows``: computed on zeros, never stored
+            float top = -INFINITY;
+            bool see[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = j0 + tx + 16 * j;
+                see[j] = key <= p && key <= last && (window <= 0 || key > p - window);
+                sc[i][j] *= scale;
+                if (dist_bias && see[j]) sc[i][j] += dist_bias[(size_t)h * (dist_cap + 1) + min(p - key, dist_cap)];
+                if (see[j]) top = fmaxf(top, sc[i][j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float m_new = fmaxf(m[i], top);
+            const float corr = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_new);
+            float part = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float e = see[j] ? expf(sc[i][j] - m_new) : 0.0f;
+                part += e;
+                P[(ty + 16 * i) * PS + tx + 16 * j] = e;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            l[i] = l[i] * corr + part;
+            m[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < 4 * VC; ++c) acc[i][c] *= corr;
+        }
+        __syncwarp();                                        // a row of P is written and read by the same half warp
+        for (int k = 0; k < AT_TILE; k += 4) {
+            float4 p4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p4[i] = *(const float4*)(P + (ty + 16 * i) * PS + k);
+#pragma unroll
+            for (int c = 0; c < VC; ++c) {
+                if (64 * c + 4 * tx >= vd) continue;
+                float4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = *(const float4*)(V + (k + u) * vs + 64 * c + 4 * tx);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float pu[4] = {p4[i].x, p4[i].y, p4[i].z, p4[i].w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        acc[i][4 * c] = fmaf(pu[u], v[u].x, acc[i][4 * c]);
+                        acc[i][4 * c + 1] = fmaf(pu[u], v[u].y, acc[i][4 * c + 1]);
+                        acc[i][4 * c + 2] = fmaf(pu[u], v[u].z, acc[i][4 * c + 2]);
+                        acc[i][4 * c + 3] = fmaf(pu[u], v[u].w, acc[i][4 * c + 3]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
+        if (r >= rows) continue;
+        float f = 1.0f;
+        if (sink) {
+            const float sk = sink[h], m_all = fmaxf(m[i], sk);
+            f = expf(m[i] - m_all);
+            l[i] = l[i] * f + expf(sk - m_all);
+        }
+#pragma unroll
+        for (int c = 0; c < VC; ++c) {
+            const int d = 64 * c + 4 * tx;
+            if (d < vd)
+                *(float4*)(out + (size_t)(t0 + r) * nh * vd + (size_t)h * vd + d) =
+                    make_float4(acc[i][4 * c] * f / l[i], acc[i][4 * c + 1] * f / l[i], acc[i][4 * c + 2] * f / l[i], acc[i][4 * c + 3] * f / l[i]);
+        }
+    }
+}
+
+// Whether the tiled kernel takes these sizes: rows of whole 16 bytes and at most 128 entries.
+SP_API int sp_attention_tile_f32_supported(int n_seqs, int nh, int nkv, int hd, int vd) {
+    return hd > 0 && vd > 0 && hd % 4 == 0 && vd % 4 == 0 && hd <= AT_MAX_D && vd <= AT_MAX_D && nkv > 0 && nh % nkv == 0 && nh <= 65535 && n_seqs <= 65535;
+}
+
+// ``max_new``: the most tokens that any sequence of the step brings; ``seq_start`` [n_seqs + 1]: where each one's tokens begin.
+SP_API int sp_attention_tile_f32(const float* q, const float* kpool, const float* vpool, float* out, const int* seq_start,
+                                 const int* positions, const int* seq_slot, const int* page_table, int max_pages, int page_size,
+                                 int n_seqs, int max_new, int nh, int nkv, int hd, int vd, int window, float scale, const float* sink,
+                                 const float* dist_bias, int dist_cap, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_new <= 0) return 0;
+    if (!sp_attention_tile_f32_supported(n_seqs, nh, nkv, hd, vd)) SP_FAIL("attention: rows of %d and %d entries, %d heads on %d are not for the tiled kernel", hd, vd, nh, nkv);
+    if (dist_bias && dist_cap < 0) SP_FAIL("attention: a distance-bias table needs at least one entry per head");
+    if (((uintptr_t)q | (uintptr_t)kpool | (uintptr_t)vpool | (uintptr_t)out) & 15) SP_FAIL("attention: the tiled kernel needs tensors on 16-byte boundaries");
+    KvPlace pl{nullptr, positions, seq_slot, page_table, max_pages, page_size, sp_range_host};
+    const dim3 grid((max_new + AT_TILE - 1) / AT_TILE, nh, n_seqs);
+    const int most = (3 * AT_TILE * (AT_MAX_D + 4) + AT_TILE * (AT_TILE + 4)) * 4;
+    const int smem = (2 * AT_TILE * (hd + 4) + AT_TILE * (vd + 4) + AT_TILE * (AT_TILE + 4)) * 4;
+    static SpPerDevice configured;
+    if (!configured.done()) {
+        cudaError_t e = cudaFuncSetAttribute(attention_tile_f32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tile_f32_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) SP_FAIL("attention: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
+        configured.mark();
+    }
+    if (vd <= 64) attention_tile_f32_kernel<1><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap);
+    else attention_tile_f32_kernel<2><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap);
+    SP_CHECK_LAUNCH("attention_tile_f32");
+    return 0;
+}
+
 // ============================================================== act(gate) * up
 // gu row = [gate(0..I) | up(0..I)]; out row = act(gate) ⊙ up · mult (SP_ACT_SILU, SP_ACT_GELU).
 template <typename T>

@@ -243,6 +243,31 @@ def attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, window, scale, 
         c_void_p(_stream())))
 
 
+def attention_tile_f32_supported(q, k_pool, v_pool, n_seqs, nh, nkv, hd, vd) -> bool:
+    """Whether ``attention_tile_f32`` takes a prompt step of these tensors (float32, rows of whole 16 bytes up to 128 entries)."""
+    if not (q.dtype == k_pool.dtype == v_pool.dtype == torch.float32) or not (q.is_contiguous() and k_pool.is_contiguous() and v_pool.is_contiguous()):
+        return False
+    if (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) % 16:
+        return False
+    return bool(load("generic").sp_attention_tile_f32_supported(int(n_seqs), int(nh), int(nkv), int(hd), int(vd)))
+
+
+def attention_tile_f32(q, k_pool, v_pool, out, meta, seq_start, n_seqs, max_new, nh, nkv, hd, window, scale, vd=None, sink=None,
+                       dist_bias=None):
+    """``attention_generic`` for the tokens of a prompt step in float32, by tiles of 64 queries and 64 keys. ``seq_start``
+    [n_seqs + 1] int32 on the device; ``max_new``: the most tokens any sequence brings."""
+    lib = load("generic")
+    bias_ptr, bias_cap = _dist_bias_args(dist_bias, nh)
+    _need_contig(q, out)
+    pt = meta.page_table
+    _declare_bounds("generic", lib, _pool_pages(meta, k_pool), _table_rows(meta, pt), q.device)
+    _check("generic", lib.sp_attention_tile_f32(
+        c_void_p(_ptr(q)), c_void_p(_ptr(k_pool)), c_void_p(_ptr(v_pool)), c_void_p(_ptr(out)), c_void_p(_ptr(seq_start)),
+        c_void_p(_ptr(meta.positions)), c_void_p(_ptr(meta.seq_slot)), c_void_p(_ptr(pt)), pt.shape[1], meta.page_size,
+        int(n_seqs), int(max_new), nh, nkv, hd, int(vd or hd), int(window or 0), c_float(scale), _sink_ptr(sink, nh), bias_ptr,
+        bias_cap, c_void_p(_stream())))
+
+
 def softcap(x, cap: float):
     """x ← cap · tanh(x / cap), element by element, in place (float32)."""
     lib = load("generic")

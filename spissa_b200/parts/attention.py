@@ -42,6 +42,9 @@ def length_bucket(max_len: int, page_size: int) -> int:
     return -(-max_len // step) * step
 
 
+TILED_TOKENS = 32          # 32-bit prompt steps of at least so many tokens take the attention kernel of 64-query tiles
+
+
 @register_part("mixer", "attention")
 class GQAAttention(Mixer):
     graph_safe = True
@@ -166,6 +169,11 @@ def attend_paged(q, step, cache, nh, nkv, hd, window, scale, sink=None, counters
         flash = {}
     elif q.dtype == torch.bfloat16 and K.flash_kv_supported(q, cache.k_pool, nh, nkv, hd, vd or hd, cache.page_size):
         flash = dict(vd=vd or hd)              # sizes of their own, or one that the kernels for one size are not built for
+    elif (not step.all_single and T >= TILED_TOKENS
+          and K.attention_tile_f32_supported(q, cache.k_pool, cache.v_pool, step.n_seqs, nh, nkv, hd, vd or hd)):
+        K.attention_tile_f32(q, cache.k_pool, cache.v_pool, ctx, cache, step.seq_start, step.n_seqs, step.max_new, nh, nkv, hd, window,
+                             scale, vd=vd, sink=sink, dist_bias=dist_bias)
+        return ctx
     else:
         K.attention_generic(q, cache.k_pool, cache.v_pool, ctx, cache, nh, nkv, hd, window, scale, vd=vd, sink=sink,
                             dist_bias=dist_bias)

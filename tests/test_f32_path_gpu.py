@@ -89,3 +89,44 @@ def test_few_rows_slices_of_k(K, M, N, Kd):
     size = a.double().abs() @ w.double().abs().t()
     # a lane adds Kd / 32 terms in order, then five rounds of sums
     assert bool(((out.double() - a.double() @ w.double().t()).abs() <= (Kd / 32 + 8) * 2.0 ** -24 * size).all())
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd", [(4, 2, 64, 64), (3, 1, 32, 32), (2, 2, 20, 20), (4, 1, 128, 128), (2, 1, 96, 36), (2, 2, 4, 128)])
+@pytest.mark.parametrize("window", [None, 1, 63, 100])
+@pytest.mark.parametrize("extra", [False, True])
+def test_attention_tiles(K, nh, nkv, hd, vd, window, extra):
+    new_counts, before = [64, 1, 65, 130, 7], [0, 199, 64, 31, 300]
+    torch.manual_seed(hd + vd + (window or 0))
+    meta = KH.paged_meta(new_counts, before, DEV, seed=hd)
+    qs = [torch.randn(t, nh, hd) for t in meta.total_len]
+    ks = [torch.randn(t, nkv, hd) for t in meta.total_len]
+    vs = [torch.randn(t, nkv, vd) for t in meta.total_len]
+    k_pool, _ = KH.fill_cache(meta, ks, ks, nkv, hd, torch.float32, DEV)
+    v_pool, _ = KH.fill_cache(meta, vs, vs, nkv, vd, torch.float32, DEV)
+    q = torch.cat([qb[-n:] for qb, n in zip(qs, new_counts)], 0).reshape(-1, nh * hd).to(DEV)
+    out = torch.full((q.shape[0], nh * vd), float("nan"), device=DEV)
+    sink = torch.randn(nh, device=DEV) if extra else None
+    bias = torch.randn(nh, 50, device=DEV) if extra else None
+    scale = 1.0 / math.sqrt(hd)
+    assert K.attention_tile_f32_supported(q, k_pool, v_pool, len(new_counts), nh, nkv, hd, vd)
+    K.attention_tile_f32(q, k_pool, v_pool, out, meta, meta.seq_start, len(new_counts), max(new_counts), nh, nkv, hd, window, scale,
+                         vd=vd, sink=sink, dist_bias=bias)
+    rows = []
+    for qb, kb, vb, n in zip(qs, ks, vs, new_counts):
+        L = qb.shape[0]
+        dist = torch.arange(L)[:, None] - torch.arange(L)[None, :]
+        see = (dist >= 0) & (dist < (window or L))
+        heads = []
+        for h in range(nh):
+            s = qb[:, h].double() @ kb[:, h // (nh // nkv)].double().t() * scale
+            if bias is not None:
+                s = s + bias[h].double().cpu()[dist.clamp(0, 49)]
+            s = s.masked_fill(~see, float("-inf"))
+            if sink is not None:
+                s = torch.cat([s, sink[h].double().cpu().expand(L, 1)], dim=1)
+            p = torch.softmax(s, dim=-1)[:, :L]
+            heads.append(p @ vb[:, h // (nh // nkv)].double())
+        rows.append(torch.cat(heads, dim=-1)[-n:])
+    ref = torch.cat(rows)
+    # scores of size sqrt(hd) in float32 sums of hd terms: their error goes into the weights as a factor
+    assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
