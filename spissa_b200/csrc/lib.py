@@ -431,15 +431,25 @@ def sample_scratch_keys(rows: int, V: int) -> int:
     return int(lib.sp_sample_scratch_keys(rows, V))
 
 
+def sample_inline_rows() -> int:
+    """Rows whose uniform numbers ``sample_rows`` takes from host memory."""
+    return int(load("sampling").sp_sample_rows_inline_max())
+
+
 def sample_rows(logits, temperature, top_k, top_p, u, scratch, out):
-    """Temperature / top-k / top-p sampling of each row with the uniform numbers ``u``."""
+    """Temperature / top-k / top-p sampling of each row with the uniform numbers ``u``: a float32 tensor on the device, or a list
+    of at most ``sample_inline_rows()`` numbers, which travel with the launch."""
     lib = load("sampling")
     rows, V = logits.shape
     if logits.dtype != torch.float32 or logits.stride(1) != 1:
         raise KernelError("sampling wants float32 logits with unit column stride")
-    _check("sampling", lib.sp_sample_rows(
+    inline = isinstance(u, list)
+    if inline and len(u) != rows:
+        raise KernelError(f"sampling: {len(u)} uniform numbers for {rows} rows")
+    draws = (c_float * rows)(*u) if inline else c_void_p(_ptr(u))
+    _check("sampling", (lib.sp_sample_rows_inline if inline else lib.sp_sample_rows)(
         c_void_p(_ptr(logits)), logits.stride(0), rows, V, c_float(temperature), int(top_k), c_float(top_p),
-        c_void_p(_ptr(u)), c_void_p(_ptr(scratch)), c_longlong(scratch.numel()), c_void_p(_ptr(out)),
+        draws, c_void_p(_ptr(scratch)), c_longlong(scratch.numel()), c_void_p(_ptr(out)),
         c_void_p(_stream())))
 
 

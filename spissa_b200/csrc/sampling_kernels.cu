@@ -17,6 +17,14 @@
 // so far; once a single token is left it is looked up and the search ends (a peaked distribution is done
 // after a few passes; equal probabilities are told apart by the index bits of the key).
 //
+// Finding the token by that descent alone took some twenty passes of three microseconds (8 rows of 128,256 logits: 80 us).
+// Now one pass adds every token into one of 4,065 buckets, by the upper 14 bits of its probability (sign, exponent and five
+// bits of the mantissa); a bucket's count and the sum of its tokens' lower 18 bits give its exact mass. The buckets' running
+// totals stay in the cluster's shared memory for every question asked of the row; the tokens of the one bucket in which a
+// target is reached are gathered and compared with one another by all CTAs: 41 us (58 with one CTA comparing; what is
+// left are the barriers of the cluster, the softmax and the adding into buckets). Only where more than 1,024 tokens share
+// the bucket (rows of nearly equal probabilities) the descent runs as before.
+//
 // Sums are integers: a probability counts as floor(p · 2^44) and a token as 1 in the high bits of the same
 // 64-bit word, so every total is exact and independent of the order of addition (the same draw always
 // gives the same token), and finer than the 32-bit running sum of a serial walk. Each thread adds into
@@ -189,18 +197,210 @@ __device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned lo
     return false;                                              // not reached: the last digit always ends above
 }
 
+// ---------------------------------------------------------------- the buckets
+constexpr int BK_SHIFT = 18;                       // bits of a probability below its bucket
+constexpr int BK_N = 4096;                         // probabilities are at most 1: bucket 4,064 is the last in use
+constexpr int BK_PER = BK_N / SS_CLUSTER;          // positions (buckets by falling probability) whose totals a CTA keeps
+constexpr int BK_LIST = 1024;                      // tokens of a bucket that are compared with one another
+constexpr unsigned BK_CARRY = 1u << 20;            // in a bucket's count: its sum of lower bits has passed 2^32 (a slice has less than 2^20 tokens)
+
+// In dynamic shared memory, over the descent's words.
+struct Buckets {
+    union { unsigned count[BK_N]; unsigned long long list[BK_LIST]; };         // this CTA's tokens of each bucket; later the gathered keys
+    union { unsigned low[BK_N]; unsigned long long weight[BK_LIST]; };         // their lower bits' contributions; later what the gathered tokens weigh
+    unsigned long long scan[BK_PER];               // running totals (count and mass packed) of this CTA's positions
+    unsigned long long warp_total[32];
+    unsigned long long total;                      // of this CTA's positions
+    unsigned long long key, upto;                  // in CTA 0: the result
+    unsigned long long below, through;             // running totals before and through the bucket
+    int position, n_list[4];                       // (a list's length has a word for each question: none has to be set back)
+};
+
+// What the lower 18 bits of a probability add to its mass, in the bucket's own unit (see bk_mass).
+__device__ __forceinline__ unsigned bk_low(unsigned b) {
+    const int e = (int)(b >> 23), down = 106 - e;                      // mass = mantissa >> down (or << -down)
+    const unsigned l = b & ((1u << BK_SHIFT) - 1u);
+    return e == 0 ? 0u : down <= 0 ? l : down <= BK_SHIFT ? l >> down : 0u;
+}
+// The mass of ``count`` tokens of a bucket whose bk_low add up to ``low``: the sum of ss_weight's masses, exactly. With
+// mantissa = H · 2^18 + L, floor(mantissa / 2^d) is H · 2^(18 - d) + floor(L / 2^d) for d ≤ 18, and floor(H / 2^(d - 18)) beyond.
+__device__ __forceinline__ unsigned long long bk_mass(int bucket, unsigned long long count, unsigned long long low) {
+    const int e = bucket >> 5, down = 106 - e;
+    const unsigned long long H = (unsigned long long)((bucket & 31) | 32);
+    if (e == 0) return 0ull;
+    if (down <= 0) return ((count * H << BK_SHIFT) + low) << -down;
+    if (down <= BK_SHIFT) return (count * H << (BK_SHIFT - down)) + low;
+    return down < 24 ? count * (H >> (down - BK_SHIFT)) : 0ull;
+}
+__device__ __forceinline__ bool bk_reached(unsigned long long total, bool by_mass, unsigned long long target) {
+    return total >= ONE_TOKEN && (by_mass ? (total & MASS_MASK) : (total >> MASS_BITS)) >= target;
+}
+
+// Every CTA: its slice into buckets, then the running totals of its 512 positions of the row's buckets.
+template <int THREADS>
+__device__ void bk_fill(Buckets* bk, const Row& row) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = row.i1 - row.i0;
+    const bool carries = n >= 1 << (32 - BK_SHIFT);                    // a bucket's lower bits could pass 2^32
+    for (int j = tid; j < n; j += THREADS) {
+        const unsigned b = row.bits[j], low = bk_low(b);
+        unsigned one = 1u;
+        if (carries) {
+            if (low && atomicAdd(&bk->low[b >> BK_SHIFT], low) + low < low) one += BK_CARRY;
+        } else if (low) {
+            atomicAdd(&bk->low[b >> BK_SHIFT], low);
+        }
+        atomicAdd(&bk->count[b >> BK_SHIFT], one);
+    }
+    __syncthreads();
+    ss_cluster_sync();
+    constexpr int MINE = BK_PER / (THREADS < BK_PER ? THREADS : BK_PER);          // positions per thread
+    const int rank = (int)ss_cluster_rank();
+    unsigned long long part[MINE], run = 0ull;
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+        part[i] = 0ull;
+        const int pos = rank * BK_PER + tid * MINE + i, bucket = BK_N - 1 - pos;
+        if (tid * MINE < BK_PER) {
+            unsigned long long count = 0ull, low = 0ull;
+#pragma unroll
+            for (unsigned r = 0; r < SS_CLUSTER; ++r) {
+                unsigned c, l;
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c) : "r"(ss_peer_addr(&bk->count[bucket], r)) : "memory");
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(l) : "r"(ss_peer_addr(&bk->low[bucket], r)) : "memory");
+                count += c & (BK_CARRY - 1u);
+                low += l + ((unsigned long long)(c / BK_CARRY) << 32);
+            }
+            part[i] = (count << MASS_BITS) + bk_mass(bucket, count, low);
+        }
+        run += part[i];
+    }
+    // inclusive sums over the threads
+    unsigned long long up = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, up, o);
+        if (lane >= o) up += v;
+    }
+    if (lane == 31) bk->warp_total[warp] = up;
+    __syncthreads();
+    unsigned long long before = up - run;
+    for (int w = 0; w < warp; ++w) before += bk->warp_total[w];
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+        before += part[i];
+        if (tid * MINE < BK_PER) bk->scan[tid * MINE + i] = before;
+    }
+    if (tid == THREADS - 1) bk->total = before;
+    __syncthreads();
+    ss_cluster_sync();                                                 // the counts are not read any more
+}
+
+// The token at which the running count or mass reaches ``target``, among all of the row, as ss_descend gives it. 1: found;
+// 0: even the total does not reach it (``upto``: the total); -1: too many tokens share the bucket. Every CTA alike.
+// ``question``: 0, 1, ... within a row.
+template <int THREADS>
+__device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, unsigned long long target, unsigned long long& key,
+                       unsigned long long& upto) {
+    const int tid = threadIdx.x;
+    unsigned long long base = 0ull, totals[SS_CLUSTER];
+#pragma unroll
+    for (unsigned r = 0; r < SS_CLUSTER; ++r) totals[r] = ss_ld_peer_u64(&bk->total, r);
+    int owner = -1;
+#pragma unroll
+    for (int r = 0; r < SS_CLUSTER; ++r)
+        if (owner < 0) {
+            if (bk_reached(base + totals[r], by_mass, target)) owner = r;
+            else base += totals[r];
+        }
+    if (owner < 0) { upto = base; return 0; }
+    for (int i = tid; i < BK_PER; i += THREADS) {
+        const unsigned long long with = base + ss_ld_peer_u64(&bk->scan[i], (unsigned)owner);
+        const unsigned long long without = base + (i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull);
+        if (bk_reached(with, by_mass, target) && !bk_reached(without, by_mass, target)) {        // one position
+            bk->position = owner * BK_PER + i;
+            bk->below = without;
+            bk->through = with;
+        }
+    }
+    __syncthreads();
+    const unsigned bucket = (unsigned)(BK_N - 1 - bk->position);
+    const unsigned long long below = bk->below;
+    const unsigned long long n_in = (bk->through - below) >> MASS_BITS;
+    if (n_in > BK_LIST) return -1;
+    const unsigned to_list = ss_peer_addr(bk->list, 0u), to_weight = ss_peer_addr(bk->weight, 0u);
+    const unsigned to_n = ss_peer_addr(&bk->n_list[question], 0u);
+    for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
+        const unsigned b = row.bits[i - row.i0];
+        if (b >> BK_SHIFT == bucket) {
+            unsigned at;
+            asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(to_n) : "memory");
+            if (at < BK_LIST) {
+                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(to_list + at * 8u), "l"(ss_key(b, (unsigned)i)) : "memory");
+                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(to_weight + at * 8u), "l"(ss_weight(b)) : "memory");
+            }
+        }
+    }
+    __syncthreads();
+    ss_cluster_sync();
+    // Every CTA compares its share of the tokens with all of them (550 tokens with one another are 300,000 comparisons, a
+    // dozen microseconds for one CTA): eight lanes per token, a lane every eighth of the others.
+    const int m = (int)n_in, rank = (int)ss_cluster_rank();
+    if (rank != 0) {
+        for (int i = tid; i < m; i += THREADS) {
+            bk->list[i] = ss_ld_peer_u64(&bk->list[i], 0u);
+            bk->weight[i] = ss_ld_peer_u64(&bk->weight[i], 0u);
+        }
+    }
+    __syncthreads();
+    const int share = (m + SS_CLUSTER - 1) / SS_CLUSTER, i1 = min(m, (rank + 1) * share);
+    for (int i0 = rank * share; i0 < i1; i0 += THREADS / 8) {          // uniform in the CTA
+        const int i = i0 + (tid >> 3);
+        const unsigned long long mine = i < i1 ? bk->list[i] : 0ull;
+        unsigned long long cum = 0ull;
+        for (int j = tid & 7; j < m; j += 8) cum += bk->list[j] < mine ? bk->weight[j] : 0ull;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) cum += __shfl_xor_sync(0xffffffffu, cum, o);
+        if ((tid & 7) == 0 && i < i1) {
+            const unsigned long long with = below + cum + bk->weight[i];
+            if (bk_reached(with, by_mass, target) && !bk_reached(below + cum, by_mass, target)) {            // one token of the cluster
+                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->key, 0u)), "l"(mine) : "memory");
+                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->upto, 0u)), "l"(with) : "memory");
+            }
+        }
+    }
+    __syncthreads();
+    ss_cluster_sync();
+    key = ss_ld_peer_u64(&bk->key, 0u);                                // (the next result is written behind another barrier of the cluster)
+    upto = ss_ld_peer_u64(&bk->upto, 0u);
+    return 1;
+}
+
+constexpr int INLINE_ROWS = 64;
+struct Draws { float u[INLINE_ROWS]; };            // the rows' uniform numbers, with the launch itself: no copy to the device
+
+template <int THREADS>
+__host__ __device__ constexpr size_t words_bytes() {                   // the descent's words, or the buckets
+    constexpr size_t a = (size_t)SS_SEGS * THREADS * 8, b = (sizeof(Buckets) + 15) / 16 * 16;
+    return a > b ? a : b;
+}
+
 // ``cached`` tokens of a slice fit the dynamic shared memory: the passes then read the probabilities from there,
 // else from the scratch row in global memory (``scratch`` may be null when every slice fits).
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temperature, int top_k, float top_p,
-                   const float* __restrict__ u, unsigned* __restrict__ scratch, int cached, int* __restrict__ out) {
+                   const float* __restrict__ u, const __grid_constant__ Draws draws, unsigned* __restrict__ scratch, int cached,
+                   int* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ Shared sh_;
     Shared* sh = &sh_;
     sh->acc = (unsigned long long*)dyn_smem;                   // every thread writes the same value
-    unsigned* slice_cache = (unsigned*)(dyn_smem + (size_t)SS_SEGS * THREADS * 8);
+    unsigned* slice_cache = (unsigned*)(dyn_smem + words_bytes<THREADS>());
+    Buckets* bk = (Buckets*)dyn_smem;
     const int tid = threadIdx.x;
+    for (int i = tid; i < BK_N; i += THREADS) bk->count[i] = bk->low[i] = 0u;
+    if (tid < 4) bk->n_list[tid] = 0;
     const unsigned rank = ss_cluster_rank();
     const int row_id = blockIdx.x / SS_CLUSTER;
     const float* x = logits + (size_t)row_id * ld;
@@ -214,13 +414,30 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     while (row.idx_digits < 8 && (V - 1) >> (4 * row.idx_digits)) ++row.idx_digits;
     const int n = row.i1 - row.i0;
 
-    // softmax of logits / temperature: exp(x - max) divided by the sum; every thread keeps to its own tokens, so
-    // what it wrote to the slice it reads back itself
+    // softmax of logits / temperature: exp(x - max) divided by the sum; every thread keeps to its own tokens, in registers
+    // where it has few (all of its loads are then in flight together), so what it wrote to the slice it reads back itself
+    constexpr int KEEP = 16;
+    const bool few = n <= KEEP * THREADS;
+    float held[KEEP];
     float mx = -INFINITY;
-    for (int j = tid; j < n; j += THREADS) {
-        const float v = x[row.i0 + j] / temperature;
-        bits[j] = __float_as_uint(v);
-        mx = fmaxf(mx, v);
+    if (few) {
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            const int j = tid + THREADS * i;
+            held[i] = j < n ? x[row.i0 + j] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            held[i] = held[i] / temperature;
+            if (tid + THREADS * i < n) mx = fmaxf(mx, held[i]);
+        }
+    } else {
+#pragma unroll 8
+        for (int j = tid; j < n; j += THREADS) {
+            const float v = x[row.i0 + j] / temperature;
+            bits[j] = __float_as_uint(v);
+            mx = fmaxf(mx, v);
+        }
     }
     mx = sp_block_max(mx, sh->red);
     if (tid == 0) sh->stat[0] = mx;
@@ -229,10 +446,19 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
 #pragma unroll
     for (unsigned r = 0; r < SS_CLUSTER; ++r) mx = fmaxf(mx, ss_ld_peer_f32(&sh->stat[0], r));
     float sum = 0.0f;
-    for (int j = tid; j < n; j += THREADS) {
-        const float e = expf(__uint_as_float(bits[j]) - mx);
-        bits[j] = __float_as_uint(e);
-        sum += e;
+    if (few) {
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            held[i] = expf(held[i] - mx);
+            if (tid + THREADS * i < n) sum += held[i];
+        }
+    } else {
+#pragma unroll 4
+        for (int j = tid; j < n; j += THREADS) {
+            const float e = expf(__uint_as_float(bits[j]) - mx);
+            bits[j] = __float_as_uint(e);
+            sum += e;
+        }
     }
     sum = sp_block_sum(sum, sh->red);
     if (tid == 0) sh->stat[1] = sum;
@@ -240,27 +466,50 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     sum = 0.0f;
 #pragma unroll
     for (unsigned r = 0; r < SS_CLUSTER; ++r) sum += ss_ld_peer_f32(&sh->stat[1], r);       // in rank order, alike in every CTA
-    for (int j = tid; j < n; j += THREADS) {
-        float p = __uint_as_float(bits[j]) / sum;
+    auto probability = [&](float e) {
+        float p = e / sum;
         if (!(p >= 0.0f)) p = 0.0f;                           // NaN logits never win
         if (p > 1.0f) p = 1.0f;
-        bits[j] = __float_as_uint(p);
+        return __float_as_uint(p);
+    };
+    if (few) {
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i)
+            if (tid + THREADS * i < n) bits[tid + THREADS * i] = probability(held[i]);
+    } else {
+#pragma unroll 4
+        for (int j = tid; j < n; j += THREADS) bits[j] = probability(__uint_as_float(bits[j]));
     }
 
+    // By buckets while the tokens in question are few enough to be compared with one another; else by the descent, whose
+    // words lie over the buckets: from then on it answers everything.
+    bk_fill<THREADS>(bk, row);
+    bool buckets = true;
+    int question = 0;
     unsigned parity = 0;
-    unsigned long long limit = ~0ull, key = 0ull, upto = 0ull;
-    if (top_k > 0 && top_k < V) {                              // the first top_k tokens
-        if (ss_descend<THREADS>(sh, row, false, (unsigned long long)top_k, limit, parity, key, upto)) limit = key;
+    auto first_at = [&](bool by_mass, unsigned long long target, unsigned long long& key, unsigned long long& upto) -> bool {
+        if (buckets) {
+            const int got = bk_find<THREADS>(bk, row, question++, by_mass, target, key, upto);
+            if (got >= 0) return got != 0;
+            buckets = false;
+            ss_cluster_sync();                                 // no CTA still reads a peer's buckets
+        }
+        return ss_descend<THREADS>(sh, row, by_mass, target, ~0ull, parity, key, upto);
+    };
+    unsigned long long limit = ~0ull, key = 0ull, upto = 0ull, limit_mass = 0ull;
+    if (top_k > 0 && top_k < V && first_at(false, (unsigned long long)top_k, key, upto)) {      // the first top_k tokens
+        limit = key;
+        limit_mass = upto & MASS_MASK;
     }
     // of those the shortest prefix whose mass reaches top_p; its mass
     unsigned long long kept_mass;
-    if (ss_descend<THREADS>(sh, row, true, __float2ull_rz(top_p * MASS_UNIT), limit, parity, key, upto)) limit = key;
-    kept_mass = upto & MASS_MASK;
-    // the draw: u is a multiple of 2^-24, the target u · mass is taken exactly
-    const unsigned long long n_u = (unsigned long long)(u[row_id] * 16777216.0f);
+    const bool reached = first_at(true, __float2ull_rz(top_p * MASS_UNIT), key, upto);
+    if (limit == ~0ull || (reached && key <= limit)) kept_mass = upto & MASS_MASK;
+    else kept_mass = limit_mass;                               // the first top_k weigh less
+    // the draw: u is a multiple of 2^-24, the target u · mass is taken exactly; it lies among the kept tokens
+    const unsigned long long n_u = (unsigned long long)((u ? u[row_id] : draws.u[row_id]) * 16777216.0f);
     const unsigned long long target = (__umul64hi(kept_mass, n_u) << 40) | ((kept_mass * n_u) >> 24);
-    if (!ss_descend<THREADS>(sh, row, true, target, limit, parity, key, upto))
-        ss_descend<THREADS>(sh, row, true, 0ull, limit, parity, key, upto);                          // the most probable token
+    if (!first_at(true, target, key, upto)) first_at(true, 0ull, key, upto);                    // the most probable token
     if (rank == 0 && tid == 0) out[row_id] = (int)(unsigned)(key & 0xffffffffu);
     ss_cluster_sync();                                         // no CTA leaves while a peer may still read its shared memory
 }
@@ -274,9 +523,28 @@ SP_API long long sp_sample_scratch_keys(int rows, int V) {
     return ((long long)rows * V + 1) / 2;
 }
 
+static int sample_rows_any(const float* logits, int ld, int rows, int V, float temperature, int top_k, float top_p, const float* u,
+                           const Draws& draws, void* scratch, long long scratch_keys, int* out, cudaStream_t stream);
+
 SP_API int sp_sample_rows(const float* logits, int ld, int rows, int V, float temperature, int top_k,
                           float top_p, const float* u, void* scratch, long long scratch_keys, int* out,
                           cudaStream_t stream) {
+    if (!u && rows > 0) SP_FAIL("sample: the rows' uniform numbers are missing");
+    return sample_rows_any(logits, ld, rows, V, temperature, top_k, top_p, u, Draws{}, scratch, scratch_keys, out, stream);
+}
+
+// The same with the uniform numbers in host memory, for up to 64 rows.
+SP_API int sp_sample_rows_inline_max() { return INLINE_ROWS; }
+SP_API int sp_sample_rows_inline(const float* logits, int ld, int rows, int V, float temperature, int top_k, float top_p, const float* u,
+                                 void* scratch, long long scratch_keys, int* out, cudaStream_t stream) {
+    if (rows > INLINE_ROWS) SP_FAIL("sample: %d rows of draws do not go with a launch (%d at most)", rows, INLINE_ROWS);
+    Draws draws{};
+    for (int r = 0; r < rows; ++r) draws.u[r] = u[r];
+    return sample_rows_any(logits, ld, rows, V, temperature, top_k, top_p, nullptr, draws, scratch, scratch_keys, out, stream);
+}
+
+static int sample_rows_any(const float* logits, int ld, int rows, int V, float temperature, int top_k, float top_p, const float* u,
+                           const Draws& draws, void* scratch, long long scratch_keys, int* out, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (V <= 0) SP_FAIL("sample: empty rows");
     if (!(temperature > 0.0f)) SP_FAIL("sample: temperature must be positive here (greedy rows use argmax)");
@@ -292,21 +560,21 @@ SP_API int sp_sample_rows(const float* logits, int ld, int rows, int V, float te
     static SpPerDevice configured;
     if (!configured.done()) {
         cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             SS_CACHE_BYTES + SS_SEGS * 256 * 8);
+                                             SS_CACHE_BYTES + (int)words_bytes<256>());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(sample_rows_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     SS_CACHE_BYTES / 2 + SS_SEGS * 1024 * 8);
+                                     SS_CACHE_BYTES / 2 + (int)words_bytes<1024>());
         if (e != cudaSuccess) SP_FAIL("sample: cannot reserve shared memory: %s", cudaGetErrorString(e));
         configured.mark();
     }
     // few rows: 1,024 threads per CTA (one CTA per SM, a quarter of the tokens per thread); many rows: 256, several CTAs per SM
     if (rows * SS_CLUSTER <= 128 && cache_bytes <= SS_CACHE_BYTES / 2)
         SP_CHECK_CALL("sample_rows", sp_launch_cluster(sample_rows_kernel<1024>, dim3(rows * SS_CLUSTER), dim3(1024),
-                                                       cache_bytes + SS_SEGS * 1024 * 8, stream, SS_CLUSTER, logits, ld, V,
-                                                       temperature, top_k, top_p, u, (unsigned*)scratch, cached, out));
+                                                       cache_bytes + words_bytes<1024>(), stream, SS_CLUSTER, logits, ld, V,
+                                                       temperature, top_k, top_p, u, draws, (unsigned*)scratch, cached, out));
     else
         SP_CHECK_CALL("sample_rows", sp_launch_cluster(sample_rows_kernel<256>, dim3(rows * SS_CLUSTER), dim3(256),
-                                                       cache_bytes + SS_SEGS * 256 * 8, stream, SS_CLUSTER, logits, ld, V,
-                                                       temperature, top_k, top_p, u, (unsigned*)scratch, cached, out));
+                                                       cache_bytes + words_bytes<256>(), stream, SS_CLUSTER, logits, ld, V,
+                                                       temperature, top_k, top_p, u, draws, (unsigned*)scratch, cached, out));
     return 0;
 }

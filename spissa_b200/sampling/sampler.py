@@ -81,7 +81,9 @@ class Sampler:
             need = K.sample_scratch_keys(rows, V)
             if self._scratch is None or self._scratch.numel() < need:
                 self._scratch = torch.empty(need, dtype=torch.int64, device=logits.device)
-            u = torch.tensor(uniforms(params, requests, step), dtype=torch.float32).to(logits.device)
+            u = uniforms(params, requests, step)
+            if rows > K.sample_inline_rows() or len(u) != rows:
+                u = torch.tensor(u, dtype=torch.float32).to(logits.device)
             K.sample_rows(logits, params.temperature, params.top_k, params.top_p, u, self._scratch, out)
         if note is not None:
             self.note(out, note)
