@@ -21,7 +21,7 @@
 // Now one pass adds every token into one of 4,065 buckets, by the upper 14 bits of its probability (sign, exponent and five
 // bits of the mantissa); a bucket's count and the sum of its tokens' lower 18 bits give its exact mass. The buckets' running
 // totals stay in the cluster's shared memory for every question asked of the row; the tokens of the one bucket in which a
-// target is reached are gathered and compared with one another by all CTAs: 41 us (58 with one CTA comparing; what is
+// target is reached are gathered and compared with one another by all CTAs: 39 us (58 with one CTA comparing; what is
 // left are the barriers of the cluster, the softmax and the adding into buckets). Only where more than 1,024 tokens share
 // the bucket (rows of nearly equal probabilities) the descent runs as before.
 //

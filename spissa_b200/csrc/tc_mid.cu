@@ -18,6 +18,10 @@
 // output 10.5 / 17.6, gate/up 26.5 / 59.3, down 19.1 / 27.5; 64 tokens (before: tc_stream.cu) 8.1 / 8.5, 7.3 / 8.0,
 // 18.7 / 20.6, 13.1 / 13.4. The gated tile's activation was half of its time with one warp's 32 values in sequence, a branch
 // on the activation around each (40 us at 301 tokens): it is taken outside now and the values are independent.
+// Grouped (routed experts, sp_tc_mid_grouped): A's rows lie in runs of one expert each, a run's tokens are cut into equal tiles
+// of at most 256 and multiplied with that expert's rows of the stacked weights; the table of the runs is read on the device.
+// 2,048 tokens, 4 of 32 experts of 2,048 x 2,048: 190 us, 237 on tc_gemm.cu's tiles of 128 tokens, of which a fifth is padding.
+// Five waves of CTAs that are alone on their SM: of 36 us each, 18 are the bytes and a dozen the epilogue.
 // Every mbarrier wait is bounded and records a code in ``status``; no load uses cluster multicast.
 #include "tcgen05.cuh"
 #include <string.h>
@@ -69,7 +73,12 @@ struct Args {
     EpiArgs ep;
     SpRange rg;
     SpGate ga;
+    // grouped: per 128 rows of A (expert or -1, first row, rows of them in use); an expert's entries follow one another and
+    // only its last may have less than 128 rows in use
+    const int* tiles;
+    int n_tiles;
 };
+constexpr int GROUP_BOX = 64;               // rows of A per box of a grouped product
 
 __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
     float4 v;
@@ -83,7 +92,7 @@ __device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
 
 // The second part of the epilogue: a warp owns a token at a time (``first``, then every eighth below ``end``), a lane four
 // neighbouring columns of it.
-struct Share { uint32_t smem_base; int tile, tok0, first, end, lane; };
+struct Share { uint32_t smem_base; int tile, tok0, first, end, lane, nt; };
 
 template <bool GATED, int PIECES>
 __device__ __forceinline__ void finish(const Args& a, const Share& sh, const float* rstd_s) {
@@ -152,7 +161,7 @@ __device__ __forceinline__ void finish(const Args& a, const Share& sh, const flo
             for (int sp = 0; sp < PIECES; ++sp) {
                 if (j < j1) {
                     pg[t][sp] = ld_cluster4(peer[sp] + at);
-                    if (two_parts) pu[t][two_parts ? sp : 0] = ld_cluster4(peer[sp] + at + (uint32_t)(a.nt * BW * 4));
+                    if (two_parts) pu[t][two_parts ? sp : 0] = ld_cluster4(peer[sp] + at + (uint32_t)(sh.nt * BW * 4));
                 }
             }
         }
@@ -227,7 +236,7 @@ __device__ __forceinline__ void finish(const Args& a, const Share& sh, const flo
 }
 
 // GATED: two tiles of W per CTA, gate rows and the up rows 128 further on
-template <bool GATED>
+template <bool GATED, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, GATED ? 1 : 2)
 tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const Args a) {
     constexpr int PARTS = GATED ? 2 : 1;
@@ -241,14 +250,30 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.pieces, piece = blockIdx.x % a.pieces;     // the cluster's rank is the piece of K
-    const int tok0 = blockIdx.y * a.nt;
-    const int count = min(a.nt, a.M - tok0);                                   // tokens of this tile
+    int tok0 = blockIdx.y * a.nt, count = min(a.nt, a.M - tok0), nt = a.nt, expert = 0;      // tokens of this tile
+    if (GROUPED) {
+        // entry y of the table is the ``turn``-th 128 rows of its expert's run; the run's first few entries stand for its tiles
+        sp_wait_for_predecessor();
+        const int y = blockIdx.y;
+        expert = a.tiles[3 * y];
+        if (expert < 0) return;
+        int turn = 0, total = a.tiles[3 * y + 2];
+        while (y - turn > 0 && a.tiles[3 * (y - turn - 1)] == expert) total += a.tiles[3 * (y - ++turn) + 2];
+        for (int i = y + 1; i < a.n_tiles && a.tiles[3 * i] == expert; ++i) total += a.tiles[3 * i + 2];
+        const int cut = (total + MAX_NT - 1) / MAX_NT;
+        nt = ((total + cut - 1) / cut + 15) & ~15;
+        if (turn >= cut || turn * nt >= total) return;
+        tok0 = a.tiles[3 * (y - turn) + 1] + turn * nt;
+        count = min(nt, total - turn * nt);
+    }
     const int num_kb = (a.K + BK - 1) / BK;
     const int per = (num_kb + a.pieces - 1) / a.pieces;
     const int kb0 = piece * per, kb1 = min(num_kb, kb0 + per);                 // the host makes every piece non-empty
-    const int row0 = tile * BW * PARTS;
-    const uint32_t stage_bytes = PARTS * W_BYTES + (uint32_t)a.nt * (BK * 2);
-    const int ntp = (a.nt + 31) & ~31;                                         // columns between the two accumulators
+    const int row0 = (GROUPED ? expert * a.N : 0) + tile * BW * PARTS;
+    const int boxes = GROUPED ? (nt + GROUP_BOX - 1) / GROUP_BOX : 1;          // of A, GROUP_BOX rows each
+    const uint32_t stage_bytes = PARTS * W_BYTES + (uint32_t)(GROUPED ? MAX_NT : nt) * (BK * 2);
+    const uint32_t load_bytes = GROUPED ? PARTS * W_BYTES + (uint32_t)boxes * (GROUP_BOX * BK * 2) : stage_bytes;
+    const int ntp = (nt + 31) & ~31;                                         // columns between the two accumulators
 
     if (threadIdx.x == 32) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
@@ -290,16 +315,17 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait(smem_u32(&bar_empty[s]), ph, a.status, 131)) break;
                 const uint32_t dst = smem_base + (uint32_t)s * stage_bytes;
-                mbar_expect_tx(smem_u32(&bar_full[s]), stage_bytes);
+                mbar_expect_tx(smem_u32(&bar_full[s]), load_bytes);
                 tma_load_2d(dst, &map_w, kb * BK, row0, smem_u32(&bar_full[s]));
                 if (GATED) tma_load_2d(dst + W_BYTES, &map_w, kb * BK, row0 + BW, smem_u32(&bar_full[s]));
-                tma_load_2d(dst + PARTS * W_BYTES, &map_a, kb * BK, tok0, smem_u32(&bar_full[s]));
+                for (int b = 0; b < boxes; ++b)
+                    tma_load_2d(dst + PARTS * W_BYTES + (uint32_t)b * (GROUP_BOX * BK * 2), &map_a, kb * BK, tok0 + b * GROUP_BOX, smem_u32(&bar_full[s]));
                 if (++s == a.stages) { s = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16(BW, a.nt);
+            const uint32_t idesc = umma_idesc_bf16(BW, nt);
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; ++kb) {
@@ -366,6 +392,13 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                         const float rs = rstd_s[c0 + j], g = __uint_as_float(rg[j]) * rs, u = __uint_as_float(ru[j]) * rs;
                         rg[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u * a.ga.mult);
                     }
+                } else if (a.ga.kind == SP_ACT_CLAMPED && a.c_dt == SP_DT_BF16) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const float rs = rstd_s[c0 + j], g = fminf(__uint_as_float(rg[j]) * rs, a.ga.limit);
+                        const float u = fminf(fmaxf(__uint_as_float(ru[j]) * rs, -a.ga.limit), a.ga.limit) + 1.0f;
+                        rg[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-a.ga.slope * g)) * u * a.ga.mult);
+                    }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
@@ -380,7 +413,7 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 if (c0 + j < count) {
                     asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)(j * BW * 4)), "r"(rg[j]) : "memory");
                     if (GATED && !act_now)
-                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)((a.nt + j) * BW * 4)), "r"(ru[j]) : "memory");
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)((nt + j) * BW * 4)), "r"(ru[j]) : "memory");
                 }
             }
         }
@@ -391,8 +424,9 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     else __syncthreads();
 
     if (warp >= 2 && healthy) {
-        const Share sh{smem_base, tile, tok0, j0 + ew, j1, lane};
-        switch (a.pieces) {
+        const Share sh{smem_base, tile, tok0, j0 + ew, j1, lane, nt};
+        if (GROUPED) finish<GATED, 1>(a, sh, rstd_s);
+        else switch (a.pieces) {
             case 1: finish<GATED, 1>(a, sh, rstd_s); break;
             case 2: finish<GATED, 2>(a, sh, rstd_s); break;
             case 4: finish<GATED, 4>(a, sh, rstd_s); break;
@@ -494,15 +528,15 @@ Plan plan_of(int mode, int M, int N, int K) {
     return best;
 }
 
-template <bool GATED>
+template <bool GATED, bool GROUPED>
 int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Args& args, const Plan& p, int row_tiles, cudaStream_t stream) {
     static SpPerDevice configured;
     if (!configured.done()) {
-        cudaError_t e = cudaFuncSetAttribute(tc_mid_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+        cudaError_t e = cudaFuncSetAttribute(tc_mid_kernel<GATED, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
         if (e != cudaSuccess) SP_FAIL("tc_mid: cannot reserve %d bytes of shared memory: %s", SMEM_LIMIT, cudaGetErrorString(e));
         configured.mark();
     }
-    SP_CHECK_CALL("tc_mid", sp_launch_cluster(tc_mid_kernel<GATED>, dim3(row_tiles * p.pieces, p.token_tiles), dim3(THREADS),
+    SP_CHECK_CALL("tc_mid", sp_launch_cluster(tc_mid_kernel<GATED, GROUPED>, dim3(row_tiles * p.pieces, p.token_tiles), dim3(THREADS),
                                               (size_t)p.smem, stream, -p.pieces, mw, ma, args));
     return 0;
 }
@@ -557,7 +591,7 @@ SP_API int sp_tc_mid(const void* A, const void* W, void* C, int c_dt, int M, int
     const Plan p = plan_of(mode, M, N, K);
     if (!p.nt) SP_FAIL("tc_mid: no division of %d tokens x %d x %d fits", M, N, K);
     const int parts = parts_of(mode), row_tiles = (N + BW * parts - 1) / (BW * parts);
-    Args args;
+    Args args{};
     args.ep = ep;
     args.rg = sp_range_host;
     args.ga = ga;
@@ -567,6 +601,40 @@ SP_API int sp_tc_mid(const void* A, const void* W, void* C, int c_dt, int M, int
     CUtensorMap mw, ma;
     if (encode_map(&mw, W, N, K, ldw, BW)) return 1;
     if (encode_map(&ma, A, M, K, lda, p.nt)) return 1;
-    if (parts == 2) return launch<true>(mw, ma, args, p, row_tiles, stream);
-    return launch<false>(mw, ma, args, p, row_tiles, stream);
+    if (parts == 2) return launch<true, false>(mw, ma, args, p, row_tiles, stream);
+    return launch<false, false>(mw, ma, args, p, row_tiles, stream);
+}
+
+// Gated products of runs of rows of A [M, K], each with its expert's N rows (gate and up in blocks of 128) of the stacked W
+// [w_rows, K]: C [M, N/2] = act(gate)·up, the clamped unit where ``slope`` is non-zero. ``tiles`` [n_tiles][3] on the device: per
+// 128 rows of A (expert or -1, first row, rows in use), an expert's entries one after another, only its last with less than 128
+// rows in use; rows that no entry names are not written.
+SP_API int sp_tc_mid_grouped(const void* A, const void* W, void* C, int c_dt, int M, int N, int K, int lda, int ldw, int w_rows, int ldc,
+                             const int* tiles, int n_tiles, float limit, float slope, int act, int* status, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || n_tiles <= 0) return 0;
+    const SpGate ga{slope != 0.0f ? (int)SP_ACT_CLAMPED : act, 1.0f, limit, slope};
+    if (!sp_gate_built(ga)) SP_FAIL("tc_mid: activation code %d is not built for gated rows", ga.kind);
+    if (sp_tc_mid_supported(A, W, 1, N, K, lda, ldw, MODE_SILU_MUL, BW)) return 1;
+    if (((uintptr_t)C & 15) || (ldc % 4)) SP_FAIL("tc_mid: C must start on a 16-byte boundary and have rows of a multiple of 4 elements");
+    if (n_tiles > 65535 || !tiles) SP_FAIL("tc_mid: a table of %d runs of rows", n_tiles);
+    constexpr int parts = 2;
+    const int row_tiles = N / (BW * parts);
+    Plan p{n_tiles, MAX_NT, 1, 0, 0, 0};
+    const int stage = parts * BW * BK * 2 + MAX_NT * BK * 2, num_kb = (K + BK - 1) / BK;
+    p.stages = (SMEM_LIMIT - 1024) / stage;
+    if (p.stages > num_kb) p.stages = num_kb;
+    const int held = MAX_NT * BW * 4;
+    p.smem = (p.stages * stage > held ? p.stages * stage : held) + 1024;
+    p.tmem_cols = parts * MAX_NT;
+    Args args{};
+    args.rg = sp_range_host;
+    args.ga = ga;
+    args.C = C; args.status = status;
+    args.c_dt = c_dt; args.M = M; args.N = N; args.K = K; args.ldc = ldc; args.mode = MODE_SILU_MUL;
+    args.nt = p.nt; args.pieces = 1; args.stages = p.stages; args.tmem_cols = p.tmem_cols;
+    args.tiles = tiles; args.n_tiles = n_tiles;
+    CUtensorMap mw, ma;
+    if (encode_map(&mw, W, w_rows, K, ldw, BW)) return 1;
+    if (encode_map(&ma, A, M, K, lda, GROUP_BOX)) return 1;
+    return launch<true, true>(mw, ma, args, p, row_tiles, stream);
 }

@@ -204,7 +204,7 @@ class RoutedExperts(FeedForward):
     expert i's tensors stand under ``expert_prefix`` + i + "." (``e0.gate`` …)."""
     graph_safe = True
     kernel_modules = ("hybrid",)
-    kernel_modules_bf16 = ("tc_gemm",)
+    kernel_modules_bf16 = ("tc_gemm", "tc_mid")
 
     def __init__(self, hidden_size: int, intermediate_size: int, experts: int, top: int, limit: float = 0.0,
                  slope: float = 1.702, groups: int = 1, keep_groups: int = 1, shared=None, prefix: str = "",

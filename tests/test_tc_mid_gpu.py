@@ -150,3 +150,41 @@ def test_qkv_rotates_and_writes_the_cache(K, hd, nh, nkv, new_counts, before):
     for p in pools:                                                     # nothing else was written
         p[page, :, at] = 7.0
         assert bool((p == 7.0).all())
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 128, 129, 256, 257, 513, 600], [0, 0, 0, 1500, 0, 0, 0, 0], [96] * 8])
+@pytest.mark.parametrize("unit", ["clamped", "silu", "relu2"])
+def test_runs_of_an_expert_of_any_length(K, counts, unit):
+    """Grouped products: runs that end at, before and behind the 128 rows of the table and the 256 tokens of a tile."""
+    E, W, F, top = 8, 256, 384, 1
+    T = sum(counts)
+    torch.manual_seed(T)
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)])[torch.randperm(T)].to(DEV).view(T, top)
+    x = torch.randn(T, W, device=DEV).bfloat16()
+    up = (torch.randn(E, F, W, device=DEV) * 0.1).bfloat16()
+    gate = (torch.randn(E, F, W, device=DEV) * 0.1).bfloat16()
+    down = (torch.randn(E, W, F, device=DEV) * 0.1).bfloat16()
+    weights = torch.rand(T, top, device=DEV)
+    y = torch.randn(T, W, device=DEV)
+    before = y.clone()
+    both = torch.stack([gate.view(E, F // 128, 128, W), up.view(E, F // 128, 128, W)], dim=2).reshape(E, 2 * F, W).contiguous()
+    if unit == "relu2":
+        K.moe_experts(x, ids, weights, up, down, y, top, 0.0, 0.0, 0, act=K.ACT_RELU2)
+    else:
+        K.moe_experts(x, ids, weights, both, down, y, top, 7.0 if unit == "clamped" else 0.0, 1.702 if unit == "clamped" else 0.0, 128)
+    ref = before.double()
+    for e in range(E):
+        at = (ids.view(-1) == e).nonzero().view(-1)
+        u, g = x[at].double() @ up[e].double().t(), x[at].double() @ gate[e].double().t()
+        if unit == "relu2":
+            h = u.clamp(min=0.0) ** 2
+        elif unit == "silu":
+            h = P.silu(g) * u
+        else:
+            g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+            h = g * torch.sigmoid(1.702 * g) * (u + 1.0)
+        ref[at] += weights[at].double() * (h @ down[e].double().t())
+    # the hidden rows are rounded to bfloat16 (2^-9 each, independent), everything else is float32
+    assert float((y.double() - ref).abs().max()) <= 2.0 ** -8 * float((ref - before.double()).abs().max()) + 2.0 ** -20 * float(ref.abs().max())
+    rows = (y.double() - before.double()) - (ref - before.double())
+    assert float(rows.norm() / (ref - before.double()).norm()) <= 2.0 ** -8
