@@ -34,6 +34,8 @@ typedef int (*RopeKvWriteFn)(const void*, int, void*, int, void*, void*, int, co
                              int, int, const float*, int, int, int, int, int, int, cudaStream_t);
 typedef int (*FlashPrefillFn)(const void*, void*, const void*, const void*, const int*, const int*, const int*, const int*,
                               int, int, int, int, int, int, int, int, float, cudaStream_t);
+typedef int (*FlashPrefillTcFn)(const void*, void*, const void*, const void*, long long, int, const int*, const int*, const int*, const int*,
+                                int, int, int, int, int, int, int, int, float, int*, cudaStream_t);
 typedef int (*TcStreamFusedFn)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, int*, cudaStream_t);
 typedef int (*RopeTableFn)(const int*, const int*, const int*, const int*, int, int, const float*, int, int, void*, int*, cudaStream_t);
 typedef int (*NormPrepareFn)(const float*, const void*, void*, float*, int, int, cudaStream_t);
@@ -81,12 +83,16 @@ struct HostKernels {
     TcMidFn tc_mid;
     TcStreamSupportedFn tc_mid_supported;
     LastErrorFn err_tc_mid;
+    FlashPrefillTcFn flash_prefill_tc;
+    LastErrorFn err_flash_tc;
     int gemv_tokens;           // up to this many tokens the weight-streaming kernel takes a product
     int stream_tokens;         // up to this many the tensor-core kernel that streams the weight
     int flash_query_tile;      // query rows per CTA of the prompt attention
     int mid_tokens;            // up to this many the one with the tokens as the instruction's N
+    int flash_tc_from;         // from this many on the prompt attention of the tcgen05 tensor cores
+    int pad;
 };
-static_assert(sizeof(HostKernels) == 22 * 8 + 16, "the host packs this layout");
+static_assert(sizeof(HostKernels) == 24 * 8 + 24, "the host packs this layout");
 
 // One layer: a pre-norm block of an RMS norm, a rotary grouped-query attention and a SwiGLU. All pointers are device
 // addresses; weights are bfloat16 [out, in] row-major, the gate/up weight interleaves ``gu_pair`` gate rows and their
@@ -130,8 +136,9 @@ struct HostStep {
     void* cs;
     int* tok_page;
     int T, H, n_seqs, max_pages, page_size, n_q_tiles, fused, mid;     // mid: sp_tc_mid takes the products of the fused sequence
+    int n_tc_tiles, n_pages;   // steps of flash_tc_from tokens or more: 128-query tiles, and the pages of the pools
 };
-static_assert(sizeof(HostStep) == 19 * 8 + 8 * 4, "the host packs this layout");
+static_assert(sizeof(HostStep) == 19 * 8 + 10 * 4, "the host packs this layout");
 
 namespace {
 
@@ -207,9 +214,14 @@ int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, i
     ep.nh = L.nh; ep.nkv = L.nkv; ep.hd = L.hd; ep.page_size = st.page_size;
     if (fused_product(st.xw[0], L.w_qkv, nullptr, DT_BF16, nqkv, st.H, 0, MODE_STREAM_QKV_ROPE, 0, &ep, st, stream)) return 1;
     ++launches;
-    if (k.flash_prefill(st.q, st.ctx, L.k_pool, L.v_pool, st.seq_start, st.positions, st.seq_row, st.page_table, st.max_pages,
-                        st.page_size, st.n_seqs, st.n_q_tiles, L.nh, L.nkv, L.hd, L.window, L.scale, stream))
+    if (st.T >= k.flash_tc_from) {
+        if (k.flash_prefill_tc(st.q, st.ctx, L.k_pool, L.v_pool, st.n_pages, st.T, st.seq_start, st.positions, st.seq_row, st.page_table,
+                               st.max_pages, st.page_size, st.n_seqs, st.n_tc_tiles, L.nh, L.nkv, L.hd, L.window, L.scale, st.status, stream))
+            return fail_from(k.err_flash_tc, "host step");
+    } else if (k.flash_prefill(st.q, st.ctx, L.k_pool, L.v_pool, st.seq_start, st.positions, st.seq_row, st.page_table, st.max_pages,
+                               st.page_size, st.n_seqs, st.n_q_tiles, L.nh, L.nkv, L.hd, L.window, L.scale, stream)) {
         return fail_from(k.err_attention, "host step");
+    }
     // output projection into the residual; the same epilogue writes residual ⊙ second norm weight and its statistics
     memset(&ep, 0, sizeof(ep));
     ep.xw = st.xw[1]; ep.next_w = L.norm2; ep.ssq_out = st.ssq[1];
@@ -234,7 +246,7 @@ SP_API int sp_host_step_bind(const void* table, int bytes) {
     if (bytes != (int)sizeof(HostKernels)) SP_FAIL("host step: the kernel table has %d bytes, %d are expected", bytes, (int)sizeof(HostKernels));
     memcpy(&kernels, table, sizeof(kernels));
     if (!kernels.rmsnorm || !kernels.gemv || !kernels.tc_stream || !kernels.tc_gemm || !kernels.rope_kv_write ||
-        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.rope_table || !kernels.norm_prepare)
+        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.flash_prefill_tc || !kernels.rope_table || !kernels.norm_prepare)
         SP_FAIL("host step: an entry point is missing from the kernel table");
     bound = true;
     return 0;
@@ -245,7 +257,8 @@ SP_API int sp_host_step_kernels_bytes() { return (int)sizeof(HostKernels); }
 // Launches that the last call of sp_host_step_prompt_layers made.
 SP_API int sp_host_step_launches() { return launches; }
 
-// Every layer of a prompt step (several tokens per sequence, at most 128 in all) on the residual ``st->h``, in place:
+// Every layer of a prompt step (several tokens per sequence; at most 128 in all, or 1,023 where sp_tc_mid takes the fused
+// sequence) on the residual ``st->h``, in place:
 // ``layers`` are n_layers descriptors in host memory, run in order. Returns 0, or 1 with the reason as the last error.
 SP_API int sp_host_step_prompt_layers(const void* layers_raw, int n_layers, const void* step_raw, cudaStream_t stream) {
     if (!bound) SP_FAIL("host step: sp_host_step_bind has not been called");

@@ -20,9 +20,10 @@ import torch
 
 from ..csrc import lib as K
 from ..parts import linear as L
+from ..parts.attention import FLASH_TC_TOKENS
 from .fused_decode import collect_fused_fields
 
-MAX_TOKENS = 128
+MAX_TOKENS = 128             # from there up to ``MID_TOKENS`` the fused sequence only
 
 
 class _Kernels(ctypes.Structure):
@@ -30,8 +31,9 @@ class _Kernels(ctypes.Structure):
         "rmsnorm", "gemv", "gemv_supported", "tc_stream", "tc_stream_supported", "tc_gemm", "tc_gemm_supported",
         "gemm_generic", "silu_mul", "rope_kv_write", "flash_prefill", "err_generic", "err_gemv", "err_tc_stream",
         "err_tc_gemm", "err_attention", "tc_stream_fused", "rope_table", "norm_prepare", "tc_mid", "tc_mid_supported",
-        "err_tc_mid")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
-                                            ("flash_query_tile", c_int), ("mid_tokens", c_int)]
+        "err_tc_mid", "flash_prefill_tc", "err_flash_tc")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
+                                            ("flash_query_tile", c_int), ("mid_tokens", c_int),
+                                            ("flash_tc_from", c_int), ("pad", c_int)]
 
 
 class _Layer(ctypes.Structure):
@@ -44,7 +46,7 @@ class _Step(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("h", "x", "qkv", "q", "ctx", "act", "gu", "token_seq", "positions", "seq_row",
                                         "page_table", "seq_start", "status", "xw0", "xw1", "ssq0", "ssq1", "cs",
                                         "tok_page")] + \
-               [(n, c_int) for n in ("T", "H", "n_seqs", "max_pages", "page_size", "n_q_tiles", "fused", "mid")]
+               [(n, c_int) for n in ("T", "H", "n_seqs", "max_pages", "page_size", "n_q_tiles", "fused", "mid", "n_tc_tiles", "n_pages")]
 
 
 def _address(lib, name) -> int:
@@ -80,7 +82,9 @@ def _bind() -> ctypes.CDLL:
     t.tc_mid, t.tc_mid_supported = _address(mid, "sp_tc_mid"), _address(mid, "sp_tc_mid_supported")
     t.err_tc_mid = _address(mid, "sp_tc_mid_last_error")
     t.gemv_tokens, t.stream_tokens, t.mid_tokens = L.GEMV_TOKENS, L.STREAM_TOKENS, L.MID_TOKENS
-    t.flash_query_tile = K.flash_query_tile()
+    flash_tc = K.load("flash_tc")
+    t.flash_prefill_tc, t.err_flash_tc = _address(flash_tc, "sp_flash_prefill_tc"), _address(flash_tc, "sp_flash_tc_last_error")
+    t.flash_query_tile, t.flash_tc_from = K.flash_query_tile(), FLASH_TC_TOKENS
     K._check("host_step", host.sp_host_step_bind(ctypes.byref(t), ctypes.sizeof(t)))
     _bound = True
     return host
@@ -110,11 +114,13 @@ class HostStep:
         runner = cls(model, fields)
         from .fused_prefill import FusedPrefill, mid_layers
         runner.can_fuse = FusedPrefill.plan(model) is not None
+        # (the tcgen05 attention of steps of many tokens takes the fused sequence's head sizes, 64 and 128)
         runner.mid = mid_layers(fields)
         return runner
 
     def takes(self, step, cache) -> bool:
-        if step.all_single or step.n_tokens > MAX_TOKENS or cache.page_size != K.flash_query_tile():
+        most = L.MID_TOKENS if self.can_fuse and self.mid and self.model.fuse_prefill else MAX_TOKENS
+        if step.all_single or step.n_tokens > most or cache.page_size != K.flash_query_tile():
             return False
         if self.cache_id != id(cache):
             self._bind_cache(cache)
@@ -197,8 +203,10 @@ class HostStep:
         st.status = K.status_word(dev).data_ptr()
         st.T, st.H, st.n_seqs, st.max_pages, st.page_size = T, self.H, step.n_seqs, pt.shape[1], cache.page_size
         st.n_q_tiles = K.query_tiles(step.host["new_counts"], K.flash_query_tile())
-        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream", "tc_mid"):       # the debug build's bounds, library by library
+        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream", "tc_mid", "flash_tc"):       # the debug build's bounds, library by library
             K._declare_bounds(module, K.load(module), cache.kv_groups[self.group].n_pages, pt.shape[0], dev)
+        if T >= FLASH_TC_TOKENS:
+            st.n_tc_tiles, st.n_pages = K.query_tiles(step.host["new_counts"], K.flash_tc_query_tile()), cache.kv_groups[self.group].n_pages
         stream = K._stream()
         rc = host.sp_host_step_prompt_layers(self.layers, len(self.fields), ctypes.byref(st), c_void_p(stream))
         K.launches += int(host.sp_host_step_launches()) - 1              # _stream() counted one

@@ -42,6 +42,7 @@ def length_bucket(max_len: int, page_size: int) -> int:
     return -(-max_len // step) * step
 
 
+FLASH_TC_TOKENS = 256      # bfloat16 prompt steps of at least so many tokens take the tcgen05 attention
 TILED_TOKENS = 32          # 32-bit prompt steps of at least so many tokens take the attention kernel of 64-query tiles
 
 
@@ -189,7 +190,7 @@ def attend_paged(q, step, cache, nh, nkv, hd, window, scale, sink=None, counters
                        scale, chunk_tiles, n_chunks, scratch,
                        counters if counters is not None and T * nkv <= counters.numel() else None, sink=sink,
                        dist_bias=dist_bias, **flash)
-    elif T >= 256 and K.flash_tc_supported(q, cache.k_pool, nh, nkv, hd, cache.page_size, window, vd=vd):
+    elif T >= FLASH_TC_TOKENS and K.flash_tc_supported(q, cache.k_pool, nh, nkv, hd, cache.page_size, window, vd=vd):
         # long prompts: 128-token tiles on the tcgen05 tensor cores (S, P and O in tensor memory)
         tiles = K.query_tiles(step.host["new_counts"], K.flash_tc_query_tile())
         K.flash_prefill_tc(q, cache.k_pool, cache.v_pool, ctx, cache, step.seq_start, step.n_seqs, tiles,
