@@ -68,7 +68,8 @@ constexpr int BOX_BYTES = 16 * BOXC * 2;        // one box: 2 halves x 8 rows x 
 constexpr int STAGE_BYTES = (KC / BOXC) * BOX_BYTES;
 constexpr int MAX_STAGES = 12;
 constexpr int MAXT = 16;                        // tokens per step
-constexpr int RED_FLOATS = CWARPS * 2 * 32 * 4; // one buffer of the K-slice sums
+// one buffer of the K-slice sums: a block of eight tokens, or two
+__host__ __device__ constexpr int red_floats(int T) { return CWARPS * (T > 8 ? 2 : 1) * 32 * 4; }
 constexpr int MAX_CHUNKS = 32;                  // key chunks per sequence (a single long sequence still gives most warp groups an item)
 constexpr int MAX_CHUNK_PAGES = 512;            // pages per chunk (their table entries wait in shared memory)
 constexpr int SMEM_LIMIT = 232448;              // per CTA on sm_100
@@ -374,10 +375,10 @@ __device__ __forceinline__ void product(const Params& p, Shared* sh, const Job& 
                 }
             }
             // the warps' K slices, added in warp order
-            float* buf = red + w.red_par * RED_FLOATS;
+            float* buf = red + w.red_par * (CWARPS * NF * 32 * 4);
 #pragma unroll
             for (int i = 0; i < NF; ++i)
-                *(float4*)(buf + ((warp * 2 + i) * 32 + lane) * 4) =
+                *(float4*)(buf + ((warp * NF + i) * 32 + lane) * 4) =
                     make_float4(acc[i][0][0] + acc[i][1][0], acc[i][0][1] + acc[i][1][1], acc[i][0][2] + acc[i][1][2],
                                 acc[i][0][3] + acc[i][1][3]);
             bar_sync(1, CTHREADS);
@@ -387,8 +388,8 @@ __device__ __forceinline__ void product(const Params& p, Shared* sh, const Job& 
                 float a = 0.0f, b = 0.0f;
 #pragma unroll
                 for (int ww = 0; ww < CWARPS; ++ww) {
-                    a += buf[((ww * 2 + i) * 32 + lp) * 4 + v];
-                    b += buf[((ww * 2 + i) * 32 + lp) * 4 + v + 2];
+                    a += buf[((ww * NF + i) * 32 + lp) * 4 + v];
+                    b += buf[((ww * NF + i) * 32 + lp) * 4 + v + 2];
                 }
                 epi(rb, e_m, e_c, a, b, rowA, rowB, nA, nB, held);
             }
@@ -1073,7 +1074,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
     Shared* sh = &sh_;
     const uint32_t ring = smem_u32(smem);
     float* red = (float*)(smem + (size_t)p.n_stages * STAGE_BYTES);
-    uint8_t* uni = (uint8_t*)(red + 2 * RED_FLOATS);               // normalised residual, or attention tiles
+    uint8_t* uni = (uint8_t*)(red + 2 * red_floats(p.T));            // normalised residual, or attention tiles
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = gridDim.x, cta = blockIdx.x;
 
@@ -1092,8 +1093,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
     if (p.trace && (cta == 0 || cta == 77) && tid == 0) p.trace[cta ? 401 : 1] = global_ns();
     if (warp == CWARPS) {
         copy_warp<HD>(p, sh, ring, lane);
-    } else if (p.T > 8) {
-        consumers<HD, ST, AG, true, PAIRS>(p, sh, ring, red, uni);
+    } else if (ST < 3 && p.T > 8) {
+        consumers<HD, ST < 3 ? ST : 2, AG, true, PAIRS>(p, sh, ring, red, uni);
     } else {
         consumers<HD, ST, AG, false, PAIRS>(p, sh, ring, red, uni);
     }
@@ -1150,7 +1151,12 @@ template <int HD>
 constexpr int attention_bytes(int st, int groups) {
     return groups * (16 * Tile<HD>::ROW + 2 * st * Tile<HD>::BYTES + MAX_CHUNK_PAGES * 4);
 }
-constexpr int ATT_BYTES_64 = attention_bytes<64>(2, 2), ATT_BYTES_128 = attention_bytes<128>(2, 1);
+// Key and value stages of the attention: three for head size 64 and up to eight tokens (a group has two pages on their way
+// while it works on one; with two stages a page took a whole round trip), two where the products of more tokens or larger
+// heads leave no room beside the weights' ring. The room comes from half of the sums' buffer and one stage of that ring.
+// Eight sequences of 2,048 keys, sixteen layers of the 1B configuration: 936 us a step before, 900 after; one: 824 and 806.
+int attention_stages(int hd, int T) { return hd == 64 && T <= 8 ? 3 : 2; }
+int attention_room(int hd, int T) { return hd == 64 ? attention_bytes<64>(attention_stages(hd, T), 2) : attention_bytes<128>(2, 1); }
 
 int sm_count() { return sp_sm_count(); }
 
@@ -1259,9 +1265,9 @@ SP_API int sp_decode_layers_supported(int T, int H, int hd, int page_size, int m
     if (H % 8) { snprintf(sp_error_text, sizeof(sp_error_text), "decode_layers: width %d is no multiple of 8", H); return 0; }
     if (max_heads_per_kv > 16) { snprintf(sp_error_text, sizeof(sp_error_text), "decode_layers: %d query heads per kv head, at most 16 fit one tile", max_heads_per_kv); return 0; }
     const int xn = T * (((H * 2 + 127) / 128) * 128 + 64);
-    const int att = hd == 64 ? ATT_BYTES_64 : ATT_BYTES_128;
+    const int att = attention_room(hd, T);
     const int uni = xn > att ? xn : att;
-    if ((SMEM_LIMIT - STATIC_SMEM - 2 * RED_FLOATS * 4 - uni) / STAGE_BYTES < 2) {
+    if ((SMEM_LIMIT - STATIC_SMEM - 2 * red_floats(T) * 4 - uni) / STAGE_BYTES < 2) {
         snprintf(sp_error_text, sizeof(sp_error_text), "decode_layers: width %d with %d tokens leaves no room for the weight ring", H, T);
         return 0;
     }
@@ -1326,9 +1332,9 @@ SP_API int sp_decode_layers(const void* layers, const void* maps, int n_layers, 
     p.n_layers = n_layers; p.T = T; p.H = H; p.max_pages = max_pages;
     p.xn_row = ((H * 2 + 127) / 128) * 128 + 64;
     const int xn = T * p.xn_row;
-    const int att = hd == 64 ? ATT_BYTES_64 : ATT_BYTES_128;
+    const int att = attention_room(hd, T);
     const int uni = xn > att ? xn : att;
-    int stages = (SMEM_LIMIT - STATIC_SMEM - 2 * RED_FLOATS * 4 - uni) / STAGE_BYTES;
+    int stages = (SMEM_LIMIT - STATIC_SMEM - 2 * red_floats(T) * 4 - uni) / STAGE_BYTES;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.n_stages = stages;
     p.plan = plan;
@@ -1354,13 +1360,15 @@ SP_API int sp_decode_layers(const void* layers, const void* maps, int n_layers, 
     next_greedy = GreedyArgs{nullptr, nullptr, 0, nullptr, nullptr};
     p.rg = sp_range_host;
     if (plan_split(G, T, hd, len_pages, max_nkv, &p.chunk_pages, &p.n_chunks)) return 1;
-    const int smem = stages * STAGE_BYTES + 2 * RED_FLOATS * 4 + uni;
+    const int smem = stages * STAGE_BYTES + 2 * red_floats(T) * 4 + uni;
 
     void* args[] = {(void*)&p};
-    const void* fn = hd == 64 ? (p.pairs ? (const void*)decode_layers_kernel<64, 2, 2, true> : (const void*)decode_layers_kernel<64, 2, 2, false>)
-                              : (const void*)decode_layers_kernel<128, 2, 1, false>;
-    static SpPerDevice configured[3];
-    const int which = hd == 64 ? (p.pairs ? 2 : 0) : 1;
+    const bool three = attention_stages(hd, T) == 3;
+    const void* fn = hd != 64 ? (const void*)decode_layers_kernel<128, 2, 1, false>
+                     : three ? (p.pairs ? (const void*)decode_layers_kernel<64, 3, 2, true> : (const void*)decode_layers_kernel<64, 3, 2, false>)
+                             : (p.pairs ? (const void*)decode_layers_kernel<64, 2, 2, true> : (const void*)decode_layers_kernel<64, 2, 2, false>);
+    static SpPerDevice configured[5];
+    const int which = hd != 64 ? 0 : 1 + (three ? 2 : 0) + (p.pairs ? 1 : 0);
     if (!configured[which].done()) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT - STATIC_SMEM);
         if (e != cudaSuccess) SP_FAIL("decode_layers: cannot reserve shared memory: %s", cudaGetErrorString(e));

@@ -239,3 +239,23 @@ def test_real_layer_sizes_repeat_bit_for_bit():
     again = decode_rows(engine, seqs, lens, 60)
     assert torch.isfinite(first).all()
     assert torch.equal(first, again)
+
+
+@pytest.mark.parametrize("n_seqs", [1, 8, 9])
+def test_chunks_of_several_pages(tmp_path, n_seqs):
+    """Sixteen kv heads leave a sequence few chunks of the keys, so a group walks one, two, three and more pages in
+    turn: with eight sequences or fewer it keeps three pages' stages, with nine two. Lengths end on both sides of a page."""
+    cfg = dict(tiny.TINY_E, num_attention_heads=16, num_key_value_heads=16, num_hidden_layers=2)
+    folder = tiny.make_folder(cfg, tiny.TINY_E_INIT, tmp_path / "pages")
+    pcfg, w = P.read_model_folder(folder)
+    V = cfg["vocab_size"]
+    lens = [700, 62, 63, 64, 190, 317, 447, 1, 520][:n_seqs]
+    steps = 4
+    seqs = [tiny.random_prompt(V, n + steps, 5 * n + n_seqs) for n in lens]
+    engine = Engine.from_folder(str(folder), dtype="bfloat16", max_tokens=64 * 64, use_graphs=False)
+    rows = decode_rows(engine, seqs, lens, steps)
+    assert engine.model._fused.runs == steps
+    for b, (q, n) in enumerate(zip(seqs, lens)):
+        ref = P.model_logits(pcfg, w, q, torch.float64)
+        err = float((rows[:, b].double() - ref[n:n + steps]).abs().max()) / float(ref.abs().max())
+        assert err <= TOL, f"{n_seqs} sequences, sequence {b}: {err:.3e}"
