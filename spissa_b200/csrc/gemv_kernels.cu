@@ -284,9 +284,7 @@ gemv_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int tile = blockIdx.x * 4 + warp;
-    // launched as a programmatic dependent: x is what the kernel before wrote
     sp_allow_dependents();
-    sp_wait_for_predecessor();
     if (tile >= tiles) return;
     constexpr int HALF = RT / 2 > 0 ? RT / 2 : 1;
     int row_base[RT];
@@ -429,6 +427,22 @@ SP_API int sp_gemv_supported(const void* x, const void* W, int M, int K, int ldx
 
 namespace {
 
+// The streaming kernel holds no shared memory, and its loads on the way to registers are held by the level-1 cache. Behind a
+// kernel that took most of an SM's memory as shared memory (the tcgen05 products do) the cache stays at a few tens of KB
+// unless a launch asks for another split, and the loads in flight with it: the head of the 1B configuration (525 MB) took
+// 121 to 151 us at the end of a prompt step, 82 behind kernels without shared memory, and 85 to 90 with this request.
+// Not launched as a programmatic dependent: blocks that arrive while the products' last blocks are there keep the old split
+// on their SM (prompt steps of 40, 301 and 2,048 tokens: 1216 and 1211, 1649 and 1634, 5486 and 5454 us without).
+template <int RT, int U, typename... Args>
+void launch_stream(int ctas, cudaStream_t stream, Args... args) {
+    static SpPerDevice configured;
+    if (!configured.done()) {
+        cudaFuncSetAttribute((const void*)gemv_stream_kernel<RT, U>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+        configured.mark();
+    }
+    gemv_stream_kernel<RT, U><<<dim3(ctas), dim3(128), 0, stream>>>(args...);
+}
+
 int launch_gemv(const void* x, const void* W, void* out, int out_dt, int M, int N, int K, int ldx, int ldw, int ldo,
                 int mode, int pair, const RopeOut& rope, cudaStream_t stream, SpGate ga = SpGate{}) {
     const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
@@ -437,11 +451,9 @@ int launch_gemv(const void* x, const void* W, void* out, int out_dt, int M, int 
     if (M <= 16 && stream_tiles >= 148 * 16 && mode != MODE_ROPE_KV) {
         // enough rows (the output head) to give every warp rows of its own and still fill every SM sixteen warps deep
         if (mode == MODE_SILU_MUL)
-            sp_launch_dependent(gemv_stream_kernel<2, 4>, dim3((stream_tiles + 3) / 4), dim3(128), 0, stream, xp, wp, out, out_dt, M,
-                                N, K, ldx, ldw, ldo, mode, pair, stream_tiles, ga);
+            launch_stream<2, 4>((stream_tiles + 3) / 4, stream, xp, wp, out, out_dt, M, N, K, ldx, ldw, ldo, mode, pair, stream_tiles, ga);
         else
-            sp_launch_dependent(gemv_stream_kernel<1, 8>, dim3((stream_tiles + 3) / 4), dim3(128), 0, stream, xp, wp, out, out_dt, M,
-                                N, K, ldx, ldw, ldo, mode, pair, stream_tiles, ga);
+            launch_stream<1, 8>((stream_tiles + 3) / 4, stream, xp, wp, out, out_dt, M, N, K, ldx, ldw, ldo, mode, pair, stream_tiles, ga);
         SP_CHECK_LAUNCH("gemv_stream");
         return 0;
     }
@@ -517,8 +529,8 @@ SP_API int sp_gemv_argmax(const void* x, const void* W, void* cand, int M, int N
     if (sp_gemv_supported(x, W, M, K, ldx, ldw)) return 1;
     const int tiles = sp_gemv_argmax_candidates(N);
     if (ld_cand < tiles) SP_FAIL("gemv (argmax): the candidate table has %d columns, %d are needed", ld_cand, tiles);
-    sp_launch_dependent(gemv_stream_kernel<1, 8>, dim3((tiles + 3) / 4), dim3(128), 0, stream, (const __nv_bfloat16*)x,
-                        (const __nv_bfloat16*)W, cand, (int)SP_DT_F32, M, N, K, ldx, ldw, ld_cand, (int)MODE_ARGMAX, 0, tiles, SpGate{});
+    launch_stream<1, 8>((tiles + 3) / 4, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, cand, (int)SP_DT_F32, M, N, K,
+                        ldx, ldw, ld_cand, (int)MODE_ARGMAX, 0, tiles, SpGate{});
     SP_CHECK_LAUNCH("gemv_argmax");
     return 0;
 }
