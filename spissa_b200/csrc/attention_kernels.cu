@@ -108,8 +108,8 @@ int launch_flash_decode_as(dim3 grid, cudaStream_t stream, const __nv_bfloat16* 
                            int nh, int window, float sl, int chunk_tiles, float* part_o, float* part_ml, int* counters,
                            void* out, int out_dt) {
     static SpPerDevice ok;            // the opt-in holds for one device: asked for on each device's first launch
-    if (!ok.done()) { if (opt_in_smem(flash_decode_kernel<HD, NH>, decode_smem<HD>(), "flash_decode")) return 1; ok.mark(); }
-    sp_launch_dependent(flash_decode_kernel<HD, NH>, grid, dim3(128), (size_t)decode_smem<HD>(), stream, q, kv, seq_len, nh, window, sl,
+    if (!ok.done()) { if (opt_in_smem(flash_decode_kernel<HD, NH>, decode_smem<HD, NH>(), "flash_decode")) return 1; ok.mark(); }
+    sp_launch_dependent(flash_decode_kernel<HD, NH>, grid, dim3(128), (size_t)decode_smem<HD, NH>(), stream, q, kv, seq_len, nh, window, sl,
                         chunk_tiles, part_o, part_ml, counters, out, out_dt, HD, HD);
     return 0;
 }

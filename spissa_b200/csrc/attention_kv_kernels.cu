@@ -36,8 +36,8 @@ template <int HD, int VD, int NH>
 int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, const PagedKV& kv, const int* seq_len, int nh, int window,
                   float sl, int chunk_tiles, float* part_o, float* part_ml, int* counters, void* out, int out_dt, int d, int vd) {
     static SpPerDevice ok;
-    if (!ok.done()) { if (opt_in_smem(flash_decode_kernel<HD, NH, VD, true>, decode_smem<HD, VD>(), "flash_decode")) return 1; ok.mark(); }
-    SP_CHECK_CALL("flash_decode (kv)", sp_launch_dependent(flash_decode_kernel<HD, NH, VD, true>, grid, dim3(128), (size_t)decode_smem<HD, VD>(), stream,
+    if (!ok.done()) { if (opt_in_smem(flash_decode_kernel<HD, NH, VD, true>, decode_smem<HD, NH, VD>(), "flash_decode")) return 1; ok.mark(); }
+    SP_CHECK_CALL("flash_decode (kv)", sp_launch_dependent(flash_decode_kernel<HD, NH, VD, true>, grid, dim3(128), (size_t)decode_smem<HD, NH, VD>(), stream,
                                                            q, kv, seq_len, nh, window, sl, chunk_tiles, part_o, part_ml, counters, out, out_dt, d, vd));
     return 0;
 }

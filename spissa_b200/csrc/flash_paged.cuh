@@ -173,6 +173,10 @@ __device__ __forceinline__ void combine_if_last(const float* part_o, const float
 
 // ------------------------------------------------------------------ decode
 // grid (chunks, kv heads, sequences). part_o [B][nh][chunks][HD], part_ml [B][nh][chunks][2] (m in log2 units).
+// Bytes in flight bound it, so what counts is how many CTAs an SM holds: the merge buffer lies over the used tiles and the
+// query tile has a row per head only, which makes room for four CTAs instead of three (head size 64) or two instead of one
+// (128). 2,048 keys, 8 kv heads: 64 sequences of head size 64 55.7 -> 54.1 us (50.9 with one chunk of the keys instead of
+// two), of 128 133 -> 99 (92 with one chunk); 16 sequences of 128 45 -> 33.
 template <int HD, int NH, int VD = HD, bool PAD = false>
 __global__ void __launch_bounds__(128)
 flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* __restrict__ seq_len, int nh,
@@ -183,10 +187,12 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
     using TV = Tile<VD>;
     const int d = PAD ? d_ : HD, vd = PAD ? vd_ : VD;
     extern __shared__ __align__(128) uint8_t smem[];
-    const uint32_t q_tile = smem_u32(smem);                       // 16 rows used
-    const uint32_t k_tiles = q_tile + 16 * T::ROW;
+    constexpr int QR = NH * 8;                                    // rows of the query tile: one per head of the kv head
+    const uint32_t q_tile = smem_u32(smem);
+    const uint32_t k_tiles = q_tile + QR * T::ROW;
     const uint32_t v_tiles = k_tiles + DEC_STAGES * T::BYTES;
-    float* merge = (float*)(smem + 16 * T::ROW + DEC_STAGES * (T::BYTES + TV::BYTES));    // [4 warps][16 rows][VD + 2]
+    float* merge = (float*)(smem + QR * T::ROW);                  // [4 warps][QR rows][VD + 2], over the tiles once they are used up
+    static_assert(4 * QR * (VD + 2) * 4 <= DEC_STAGES * (T::BYTES + TV::BYTES), "the merge buffer fits over the tiles");
     sp_allow_dependents();
     sp_wait_for_predecessor();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -210,11 +216,11 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
     const int* pt = kv.page_table + (size_t)sp_checked_row(kv.seq_row[b], kv.rg) * kv.max_pages;
 
     if (PAD && d < HD) {
-        zero_columns(q_tile, 16 + DEC_STAGES * KT, T::ROW, d, HD, tid, 128);      // the queries and all stages of keys
+        zero_columns(q_tile, QR + DEC_STAGES * KT, T::ROW, d, HD, tid, 128);      // the queries and all stages of keys
         __syncthreads();
     }
-    // the G heads of this kv head as rows 0..G-1 of a 16-row tile
-    for (int c = tid; c < 16 * T::CHUNKS; c += 128) {
+    // the G heads of this kv head as rows 0..G-1 of the tile
+    for (int c = tid; c < QR * T::CHUNKS; c += 128) {
         const int r = c / T::CHUNKS, k = c % T::CHUNKS;
         const uint32_t to = q_tile + r * T::ROW + k * 16;
         if (PAD && k * 8 >= d) continue;
@@ -291,6 +297,7 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
         __syncwarp();                                              // the stage is free for this warp's next fetch
     }
     cp_async_wait<0>();
+    __syncthreads();                                               // every warp is done with the tiles: they become the merge buffer
 
     // merge the four warps' (m, l, o): each covered other keys of the same rows
     constexpr int MS = VD + 2;
@@ -302,7 +309,7 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
             l[i][c] += __shfl_xor_sync(0xffffffffu, l[i][c], 4);   // the lanes that share lt hold the head's other keys
             l[i][c] += __shfl_xor_sync(0xffffffffu, l[i][c], 8);
             l[i][c] += __shfl_xor_sync(0xffffffffu, l[i][c], 16);
-            float* dst = merge + ((size_t)warp * 16 + i * 8 + 2 * lt + c) * MS;
+            float* dst = merge + ((size_t)warp * QR + i * 8 + 2 * lt + c) * MS;
 #pragma unroll
             for (int dt = 0; dt < VD / 16; ++dt) {
                 dst[dt * 16 + lg] = o[dt][i][c];
@@ -315,12 +322,12 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
         const int row = e / vd, c = e % vd;
         float mm = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, merge[((size_t)w * 16 + row) * MS + VD]);
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, merge[((size_t)w * QR + row) * MS + VD]);
         const float msafe = (mm == -INFINITY) ? 0.0f : mm;
         float acc = 0.0f, ll = 0.0f;
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const float* src = merge + ((size_t)w * 16 + row) * MS;
+            const float* src = merge + ((size_t)w * QR + row) * MS;
             const float f = exp2f(src[VD] - msafe);
             acc += src[c] * f;
             ll += src[VD + 1] * f;
@@ -358,8 +365,8 @@ __global__ void decode_combine_kernel(const float* __restrict__ part_o, const fl
 
 template <int HD, int VD = HD>
 constexpr int prefill_smem() { return 3 * Tile<HD>::BYTES + 2 * Tile<VD>::BYTES; }
-template <int HD, int VD = HD>
-constexpr int decode_smem() { return 16 * Tile<HD>::ROW + DEC_STAGES * (Tile<HD>::BYTES + Tile<VD>::BYTES) + 4 * 16 * (VD + 2) * 4; }
+template <int HD, int NH, int VD = HD>
+constexpr int decode_smem() { return NH * 8 * Tile<HD>::ROW + DEC_STAGES * (Tile<HD>::BYTES + Tile<VD>::BYTES); }
 
 template <typename Kern>
 int opt_in_smem(Kern kern, int bytes, const char* name) {
