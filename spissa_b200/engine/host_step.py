@@ -3,7 +3,7 @@
 A prompt of a few dozen tokens is bound by the host, not the GPU: part by part a layer is eight launches of a few
 microseconds each, and from Python each costs ten microseconds or more. When every layer's parts describe themselves
 through ``fused_fields()`` (the description the one-kernel decode path and the fused prompt path read), a prompt step
-of at most 128 tokens hands the whole sequence to ``csrc/host_step.cu``: a table of layer descriptors built once per
+of at most 1,023 tokens (128 where ``tc_mid`` does not take the layers) hands the whole sequence to ``csrc/host_step.cu``: a table of layer descriptors built once per
 cache, the step's arrays and its activation buffers. Up to 16 tokens the kernels are the same as part by part, chosen
 by the same thresholds (``parts/linear.py``), so the results are bit-identical to the Python path. From 17 tokens on
 (head sizes 64 and 128) a layer is five launches instead of eight: the norms, the rotation and the cache write ride in

@@ -151,7 +151,7 @@ class Model:
                 return done                                # the kernel ran the final norm and the head as well
             h = self._fused.last_h
         elif self.host_steps and not profiling() and self._host_runner(step, cache):
-            self._host_step.run(h, step, cache)            # a prompt step of up to 128 tokens: launched from C++
+            self._host_step.run(h, step, cache)            # a prompt step of up to 1,023 tokens: launched from C++
         elif self.fuse_prefill and self._fused_prefill is not None and self._fused_prefill.takes(step, cache):
             self._fused_prefill.run(h, step, cache)
         else:
