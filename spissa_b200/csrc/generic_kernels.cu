@@ -862,6 +862,7 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
     for (int j0 = lo; j0 <= last; j0 += AT_TILE) {
         __syncthreads();                                     // the tile before has been used
         const int qd = (hd + vd) / 4;
+        int odd = 0;                                         // an infinity or NaN among this thread's pieces of the values
         for (int e = tid; e < AT_TILE * qd; e += 256) {
             const int r = e / qd, c = (e % qd) * 4, j = j0 + r;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -871,8 +872,10 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
                 v = c < hd ? *(const float4*)(kpool + at * hd + c) : *(const float4*)(vpool + at * vd + (c - hd));
             }
             *(float4*)(c < hd ? Kt + r * ks + c : V + r * vs + (c - hd)) = v;
+            // x - x is NaN for what is not finite, else zero
+            if (c >= hd) odd |= (v.x - v.x) + (v.y - v.y) + (v.z - v.z) + (v.w - v.w) != 0.0f;
         }
-        __syncthreads();
+        odd = __syncthreads_or(odd);
         float sc[4][4] = {};
         for (int d = 0; d < hd; d += 4) {
             float4 a[4], b[4];
@@ -902,12 +905,12 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            const float m_new = fmaxf(m[i], top);
+            const float m_new = fmaxf(m[i], top), base = m_new == -INFINITY ? 0.0f : m_new;     // scores may be -inf (a bias)
             const float corr = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_new);
             float part = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float e = see[j] ? expf(sc[i][j] - m_new) : 0.0f;
+                const float e = see[j] ? expf(sc[i][j] - base) : 0.0f;
                 part += e;
                 P[(ty + 16 * i) * PS + tx + 16 * j] = e;
             }
@@ -929,6 +932,25 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
                 float4 v[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) v[u] = *(const float4*)(V + (k + u) * vs + 64 * c + 4 * tx);
+                if (odd) {
+                    // a value that is not finite reaches the queries that see its key and no others: zero weights of
+                    // hidden keys would make it NaN for all
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float pu[4] = {p4[i].x, p4[i].y, p4[i].z, p4[i].w};
+                        const int p = first + ty + 16 * i;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int key = j0 + k + u;
+                            if (!(key <= p && key <= last && (window <= 0 || key > p - window))) continue;
+                            acc[i][4 * c] = fmaf(pu[u], v[u].x, acc[i][4 * c]);
+                            acc[i][4 * c + 1] = fmaf(pu[u], v[u].y, acc[i][4 * c + 1]);
+                            acc[i][4 * c + 2] = fmaf(pu[u], v[u].z, acc[i][4 * c + 2]);
+                            acc[i][4 * c + 3] = fmaf(pu[u], v[u].w, acc[i][4 * c + 3]);
+                        }
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float pu[4] = {p4[i].x, p4[i].y, p4[i].z, p4[i].w};

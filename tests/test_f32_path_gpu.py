@@ -130,3 +130,64 @@ def test_attention_tiles(K, nh, nkv, hd, vd, window, extra):
     ref = torch.cat(rows)
     # scores of size sqrt(hd) in float32 sums of hd terms: their error goes into the weights as a factor
     assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
+
+
+def visible(L, window):
+    dist = torch.arange(L)[:, None] - torch.arange(L)[None, :]
+    return (dist >= 0) & (dist < (window or L))
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd", [(4, 2, 64, 64), (2, 1, 96, 36), (2, 2, 4, 128)])
+@pytest.mark.parametrize("window", [None, 1, 20, 100])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_values_that_are_not_finite_reach_who_sees_them(K, nh, nkv, hd, vd, window, bad):
+    """A token's value row with an infinity or NaN in it: the tokens that may not see it (earlier ones, and later ones whose
+    window has left it behind) keep their results, the others get what a sum over the visible keys gives."""
+    new_counts, before = [150, 70], [0, 130]
+    torch.manual_seed(hd + (window or 0))
+    meta = KH.paged_meta(new_counts, before, DEV, seed=hd)
+    qs, ks, vs = ([torch.randn(t, n, d) for t in meta.total_len] for n, d in ((nh, hd), (nkv, hd), (nkv, vd)))
+    for b, at in ((0, 40), (0, 127), (1, 100), (1, 150)):               # in front of, within and at the end of tiles of 64
+        vs[b][at, 0, vd // 2] = bad
+    k_pool, _ = KH.fill_cache(meta, ks, ks, nkv, hd, torch.float32, DEV)
+    v_pool, _ = KH.fill_cache(meta, vs, vs, nkv, vd, torch.float32, DEV)
+    q = torch.cat([qb[-n:] for qb, n in zip(qs, new_counts)], 0).reshape(-1, nh * hd).to(DEV)
+    out = torch.full((q.shape[0], nh * vd), 7.0, device=DEV)
+    K.attention_tile_f32(q, k_pool, v_pool, out, meta, meta.seq_start, len(new_counts), max(new_counts), nh, nkv, hd, window,
+                         1.0 / math.sqrt(hd), vd=vd)
+    rows = []
+    for qb, kb, vb, n in zip(qs, ks, vs, new_counts):
+        see, heads = visible(qb.shape[0], window), []
+        for h in range(nh):
+            g = h // (nh // nkv)
+            s = (qb[:, h].double() @ kb[:, g].double().t() / math.sqrt(hd)).masked_fill(~see, float("-inf"))
+            terms = torch.softmax(s, dim=-1)[:, :, None] * vb[None, :, g].double()
+            heads.append(terms.masked_fill(~see[:, :, None], 0.0).sum(1))
+        rows.append(torch.cat(heads, dim=-1)[-n:])
+    ref, got = torch.cat(rows), out.double().cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref))
+    assert torch.equal(got[torch.isinf(ref)], ref[torch.isinf(ref)])
+    fine = torch.isfinite(ref)
+    assert bool((~fine).any()) and float((got[fine] - ref[fine]).abs().max()) <= 3e-6 * float(ref[fine].abs().max())
+
+
+@pytest.mark.parametrize("window", [None, 33, 64, 100])
+def test_distances_that_a_bias_rules_out(K, window):
+    """A bias of -inf from a distance on: a tile whose visible keys are all ruled out for a query leaves its sums alone."""
+    nh, nkv, hd, L, near = 2, 1, 32, 200, 30
+    torch.manual_seed(window or 0)
+    meta = KH.paged_meta([L], [0], DEV, seed=3)
+    q, k, v = torch.randn(L, nh, hd), torch.randn(L, nkv, hd), torch.randn(L, nkv, hd)
+    k_pool, v_pool = KH.fill_cache(meta, [k], [v], nkv, hd, torch.float32, DEV)
+    bias = torch.randn(nh, 41)
+    bias[:, near:] = float("-inf")
+    out = torch.empty(L, nh * hd, device=DEV)
+    K.attention_tile_f32(q.reshape(L, -1).to(DEV), k_pool, v_pool, out, meta, meta.seq_start, 1, L, nh, nkv, hd, window, 0.2,
+                         dist_bias=bias.to(DEV))
+    dist = (torch.arange(L)[:, None] - torch.arange(L)[None, :]).clamp(0, 40)
+    heads = []
+    for h in range(nh):
+        s = (q[:, h].double() @ k[:, 0].double().t() * 0.2 + bias[h].double()[dist]).masked_fill(~visible(L, window), float("-inf"))
+        heads.append(torch.softmax(s, dim=-1) @ v[:, 0].double())
+    ref = torch.cat(heads, dim=-1)
+    assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
