@@ -92,7 +92,7 @@ __device__ __forceinline__ float4 ld_peer_f4(const void* local, uint32_t rank) {
 // MODE_SILU_MUL: the first RT/2 row groups are gate rows, the others the up rows ``pair`` rows further on.
 template <int MT, int RT, int UNROLL>
 __global__ void __launch_bounds__(MAX_KS * 32)
-gemv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
+gemv_kernel(const __nv_bfloat16* x, const __nv_bfloat16* W, void* out,
             int out_dt, int M, int N, int K, int ldx, int ldw, int ldo, int mode, int pair, int ks, int cs,
             RopeOut rope, SpGate ga) {
     __shared__ __align__(16) float red[MAX_KS][MT][RT][32][4];

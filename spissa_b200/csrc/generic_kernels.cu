@@ -285,7 +285,8 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 // The same product for a few rows of A (a decode step of the 32-bit path): W is streamed once with 16-byte loads,
 // a CTA of four warps owns eight rows of W (two per warp), the rows of A pass through shared memory in slices of
 // 512 columns. What bounds it is bytes in flight: the next slice of W (and up to 4 rows of A) is asked for before the
-// products of this one, and the kernel may become resident before its predecessor ends. Each lane sums its columns
+// products of this one, and the kernel may become resident before its predecessor ends (so A, which that one writes, is not
+// read by read-only loads). Each lane sums its columns
 // k = 4·lane + 128·i in order, the lanes' sums are added by a shuffle tree: the order is fixed and the same for every row
 // of A, whatever M is, but it is another order than the tiled kernel's, so a token's result differs between a decode step
 // and a prompt step by 32-bit rounding.
@@ -293,7 +294,7 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 #define GS_ROWS 2
 template <int MT>
 __global__ void __launch_bounds__(128)
-gemm_stream_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, void* __restrict__ C, int c_dt,
+gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
                        int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
     constexpr int XV = MT * (GS_KC / 4) / 128;               // 16-byte pieces of a slice of A per thread
     constexpr bool XAHEAD = MT <= 4;                         // held in registers a slice ahead
@@ -315,12 +316,15 @@ gemm_stream_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
 #pragma unroll
             for (int i = 0; i < GS_KC / 128; ++i) {
                 const int k = k0 + i * 128 + lane * 4;
-                to[r][i] = k < K ? __ldcs((const float4*)(wrow[r] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                to[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k < K)
+                    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(to[r][i].x), "=f"(to[r][i].y), "=f"(to[r][i].z), "=f"(to[r][i].w) : "l"(wrow[r] + k) : "memory");
             }
     };
     auto load_x = [&](int k0, int v) {
         const int e = threadIdx.x + 128 * v, m = e / (GS_KC / 4), c = (e % (GS_KC / 4)) * 4;
-        return m < M && k0 + c < K ? *(const float4*)(A + (size_t)m * lda + k0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);     // K is a multiple of 4
+        return m < M && k0 + c < K ? sp_ld_written((const float4*)(A + (size_t)m * lda + k0 + c)) : make_float4(0.f, 0.f, 0.f, 0.f);     // K is a multiple of 4
     };
     auto slice = [&](int k0, auto turn) {
         constexpr int b = decltype(turn)::value;

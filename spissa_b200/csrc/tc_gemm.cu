@@ -323,7 +323,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // microsecond under load; a tile has up to eight chunks.)
             float ssq_sum = 0.0f;                                   // the row's partial sums of squares, in tile order
             if (ep.row_ssq && row < M)
-                for (int i = 0; i < ep.n_ssq; ++i) ssq_sum += __ldg(ep.row_ssq + (size_t)row * ep.n_ssq + i);
+                for (int i = 0; i < ep.n_ssq; ++i) ssq_sum += sp_ld_written(ep.row_ssq + (size_t)row * ep.n_ssq + i);
             // The accumulating epilogue that also prepares the next norm regroups each 32 x 32 chunk so that eight
             // lanes cover the 128 bytes of one row (a lane: 4 columns of rows sub, sub + 4, ... sub + 28): a warp's
             // load or store of the residual then touches 4 whole lines instead of a piece of 32 lines.
@@ -348,11 +348,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             float4 cs_reg[16];                                      // (cos, sin) of 32 dims of this thread's token
             int pos = 0, page = 0;
             if (mode == MODE_QKV_ROPE && row < M) {
-                pos = __ldg(ep.positions + row);
-                page = __ldg(ep.tok_page + row);
+                pos = sp_ld_written(ep.positions + row);
+                page = sp_ld_written(ep.tok_page + row);
                 const float4* t4 = (const float4*)(ep.cs + (size_t)row * (ep.hd >> 1));
 #pragma unroll
-                for (int j = 0; j < 16; ++j) cs_reg[j] = __ldg(t4 + j);
+                for (int j = 0; j < 16; ++j) cs_reg[j] = sp_ld_written(t4 + j);
             }
             const bool ok = mbar_wait(smem_u32(&bar_acc_full[buf]), use & 1u, status, 103);
             tc_fence_after();
@@ -388,7 +388,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             // head size 128: the table's other half (one half per head otherwise: loaded once per tile)
                             const float4* t4 = (const float4*)(ep.cs + (size_t)row * half + c);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) cs_reg[j] = __ldg(t4 + j);
+                            for (int j = 0; j < 16; ++j) cs_reg[j] = sp_ld_written(t4 + j);
                         }
                         tc_ld_32x32(taddr + (uint32_t)(hh * hd + c), ra);
                         tc_ld_32x32(taddr + (uint32_t)(hh * hd + half + c), rb);

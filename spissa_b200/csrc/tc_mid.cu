@@ -143,12 +143,12 @@ __device__ __forceinline__ void finish(const Args& a, const Share& sh, const flo
             if (rope_mode) {
                 if (r_q || r_k) {
                     const float4* src = (const float4*)(ep.cs + m * r_half + (r_d < r_half ? r_d : r_d - r_half));
-                    ea[t] = __ldg(src);
-                    eb[t] = __ldg(src + 1);
+                    ea[t] = sp_ld_written(src);
+                    eb[t] = sp_ld_written(src + 1);
                 }
                 if (!r_q) {
-                    page[t] = __ldg(ep.tok_page + m);
-                    pos[t] = __ldg(ep.positions + m);
+                    page[t] = sp_ld_written(ep.tok_page + m);
+                    pos[t] = sp_ld_written(ep.positions + m);
                 }
             }
         }
@@ -356,7 +356,7 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 const int j = jb + t * EPI_WARPS;
                 sum[t] = 0.0f;
                 if (ep.row_ssq && j < count)
-                    for (int i = lane; i < ep.n_ssq; i += 32) sum[t] += __ldg(ep.row_ssq + (size_t)(tok0 + j) * ep.n_ssq + i);
+                    for (int i = lane; i < ep.n_ssq; i += 32) sum[t] += sp_ld_written(ep.row_ssq + (size_t)(tok0 + j) * ep.n_ssq + i);
             }
 #pragma unroll
             for (int t = 0; t < 4; ++t) {

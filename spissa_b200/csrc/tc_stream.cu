@@ -182,10 +182,10 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (j >= j_end || !col_ok || GATED) continue;
             if (a.mode == MODE_ACCUMULATE) pre.oldc[t] = ((const float*)a.C)[(size_t)j * a.ldc + col];
             if (rope_mode) {
-                if (r_rot) pre.cs[t] = __ldg(ep.cs + (size_t)j * r_half + (r_d < r_half ? r_d : r_d - r_half));
+                if (r_rot) pre.cs[t] = sp_ld_written(ep.cs + (size_t)j * r_half + (r_d < r_half ? r_d : r_d - r_half));
                 if (!r_q) {
-                    pre.page[t] = __ldg(ep.tok_page + j);
-                    pre.pos[t] = __ldg(ep.positions + j);
+                    pre.page[t] = sp_ld_written(ep.tok_page + j);
+                    pre.pos[t] = sp_ld_written(ep.positions + j);
                 }
             }
         }
@@ -303,7 +303,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 float r = 1.0f;
                 if (ep.row_ssq && e < a.M) {
                     float sum = 0.0f;
-                    for (int i = 0; i < ep.n_ssq; ++i) sum += __ldg(ep.row_ssq + (size_t)e * ep.n_ssq + i);
+                    for (int i = 0; i < ep.n_ssq; ++i) sum += sp_ld_written(ep.row_ssq + (size_t)e * ep.n_ssq + i);
                     r = 1.0f / sqrtf(sum / (float)ep.norm_width + ep.eps);
                 }
                 rstd_s[e] = r;
