@@ -15,9 +15,8 @@
 //              a load, and global memory is touched in whole lines (tc_stream.cu's thread-per-column epilogue costs a
 //              microsecond per four tokens, which is what keeps that kernel to a few dozen).
 // Measured back to back on weights from HBM (us, this kernel / the one that ran before), 1B shape: 301 tokens QKV 11.0 / 17.2,
-// output 10.5 / 17.6, gate/up 26.5 / 59.3, down 19.1 / 27.5; 64 tokens (before: tc_stream.cu) 8.1 / 8.5, 7.3 / 8.0,
-// 18.7 / 20.6, 13.1 / 13.4. The gated tile's activation was half of its time with one warp's 32 values in sequence, a branch
-// on the activation around each (40 us at 301 tokens): it is taken outside now and the values are independent.
+// output 10.5 / 17.6, gate/up 27.3 / 59.3, down 19.1 / 27.5; 64 tokens (before: tc_stream.cu) 8.1 / 8.5, 7.3 / 8.0,
+// 18.7 / 20.6, 13.1 / 13.4.
 // Grouped (routed experts, sp_tc_mid_grouped): A's rows lie in runs of one expert each, a run's tokens are cut into equal tiles
 // of at most 256 and multiplied with that expert's rows of the stacked weights; the table of the runs is read on the device.
 // 2,048 tokens, 4 of 32 experts of 2,048 x 2,048: 190 us, 237 on tc_gemm.cu's tiles of 128 tokens, of which a fifth is padding.
@@ -88,6 +87,50 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
 __device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
     const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
     return make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+}
+
+// x / d for 1 <= d <= 2^100 and finite x: the remainder of a quotient by an approximate reciprocal (two units at most off)
+// corrects it to within half a unit and 2^-20 of one (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990). No branch, unlike the general quotient.
+__device__ __forceinline__ float quotient(float x, float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = x * r;
+    return fmaf(fmaf(-d, q, x), r, q);
+}
+// act(gate)·up of 32 tokens of a row of W (the first ``n`` are tokens), in place of the gate: sp_gated, as where pieces of K are added first. Gates of
+// ordinary size (all of them, in earnest) go through without a branch on one value, so that the 32 overlap. 301 tokens x
+// 16,384 x 2,048: 27.3 us, 32.0 with the general quotient, 40 with a branch on the activation around each value.
+template <int KIND>
+__device__ __forceinline__ void activate(uint32_t (&rg)[32], const uint32_t (&ru)[32], const float* rstd, int n, SpGate ga) {
+    ga.kind = KIND;
+    const float slope = KIND == SP_ACT_CLAMPED ? ga.slope : 1.0f;
+    float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};                     // (NaN is left out: the quotient is NaN either way)
+    if (KIND != SP_ACT_GELU) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            float g = __uint_as_float(rg[j]) * rstd[j];
+            if (KIND == SP_ACT_CLAMPED) g = fminf(g, ga.limit);
+            top[j & 3] = fmaxf(top[j & 3], j < n ? fabsf(slope * g) : 0.0f);
+        }
+    }
+    if (KIND != SP_ACT_GELU && __all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= 60.0f)) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            float g = __uint_as_float(rg[j]) * rstd[j], u = __uint_as_float(ru[j]) * rstd[j];
+            if (KIND == SP_ACT_CLAMPED) {
+                g = fminf(g, ga.limit);
+                u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
+            }
+            rg[j] = __float_as_uint(quotient(g, 1.0f + expf(-slope * g)) * u * ga.mult);
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const float rs = rstd[j];
+        rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]) * rs, __uint_as_float(ru[j]) * rs, ga));
+    }
 }
 
 // The second part of the epilogue: a warp owns a token at a time (``first``, then every eighth below ``end``), a lane four
@@ -384,28 +427,10 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             if (GATED) tc_ld_32x32(lane_base + (uint32_t)(ntp + c0), ru);
             tc_ld_wait();
             if (GATED && act_now) {
-                if (a.ga.kind == SP_ACT_SILU && a.c_dt == SP_DT_BF16) {
-                    // the quick quotient and exponential are good to some 1e-6 of the result, which is then rounded to a
-                    // bfloat16 (4e-3); they have no branch, so the 32 values overlap
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float rs = rstd_s[c0 + j], g = __uint_as_float(rg[j]) * rs, u = __uint_as_float(ru[j]) * rs;
-                        rg[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u * a.ga.mult);
-                    }
-                } else if (a.ga.kind == SP_ACT_CLAMPED && a.c_dt == SP_DT_BF16) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float rs = rstd_s[c0 + j], g = fminf(__uint_as_float(rg[j]) * rs, a.ga.limit);
-                        const float u = fminf(fmaxf(__uint_as_float(ru[j]) * rs, -a.ga.limit), a.ga.limit) + 1.0f;
-                        rg[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-a.ga.slope * g)) * u * a.ga.mult);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float rs = rstd_s[c0 + j];
-                        rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]) * rs, __uint_as_float(ru[j]) * rs, a.ga));
-                    }
-                }
+                // (the kind is a constant to each loop, so that the 32 values are independent of one another)
+                if (a.ga.kind == SP_ACT_SILU) activate<SP_ACT_SILU>(rg, ru, rstd_s + c0, count - c0, a.ga);
+                else if (a.ga.kind == SP_ACT_CLAMPED) activate<SP_ACT_CLAMPED>(rg, ru, rstd_s + c0, count - c0, a.ga);
+                else activate<SP_ACT_GELU>(rg, ru, rstd_s + c0, count - c0, a.ga);
             }
             const uint32_t dst = smem_base + (uint32_t)((c0 * BW + row) * 4);
 #pragma unroll

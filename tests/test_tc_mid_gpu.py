@@ -188,3 +188,39 @@ def test_runs_of_an_expert_of_any_length(K, counts, unit):
     assert float((y.double() - ref).abs().max()) <= 2.0 ** -8 * float((ref - before.double()).abs().max()) + 2.0 ** -20 * float(ref.abs().max())
     rows = (y.double() - before.double()) - (ref - before.double())
     assert float(rows.norm() / (ref - before.double()).norm()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu", "clamped"])
+def test_gated_rows_keep_the_bits_of_32_bit_arithmetic(K, act):
+    """Gates that are one bfloat16 each, exactly: of ordinary size, tiny, beyond the exponential's range, infinite and NaN. A
+    float32 result is as near to 64 bits as float32 arithmetic is, and a bfloat16 one is that result rounded."""
+    M, I, H = 1000, 128, 64
+    g = torch.Generator().manual_seed(1)
+    x = (torch.randn(M, H, generator=g) * torch.logspace(-6, 1.7, H)).bfloat16()
+    x[5, :10] = torch.tensor([-87.0, -87.5, -88.0, -88.5, -90.0, 90.0, 3e38, -100.0, 1e-38, -1e-38]).bfloat16()
+    x[6, 0], x[7, 1], x[8, 2] = float("inf"), float("-inf"), float("nan")
+    x[:, H - 1] = 1.0
+    w = torch.zeros(2, 128, H)
+    w[0, torch.arange(128), torch.arange(128) % (H - 1)] = 1.0          # a gate row is one column of x
+    w[1, :, H - 1] = 1.0
+    w = w.reshape(256, H).bfloat16()
+    keep = torch.isfinite(x).all(1)                                     # (0 times an infinity is NaN in the other columns)
+    kw = dict(silu={}, gelu=dict(act=K.ACT_GELU), clamped=dict(act=K.ACT_CLAMPED, limit=7.0, slope=1.702))[act]
+    assert K.tc_mid_plan(K.TC_SILU_MUL, M, 2 * I, H)[2] == 1
+    full, short = (torch.full((M, I), 7.0, dtype=dt, device=DEV) for dt in (torch.float32, torch.bfloat16))
+    for out in (full, short):
+        K.tc_mid(x.to(DEV), w.to(DEV), out, K.TC_SILU_MUL, 128, **kw)
+    assert torch.equal(full.bfloat16().view(torch.int16)[keep.to(DEV)], short.view(torch.int16)[keep.to(DEV)])
+    assert torch.equal(torch.isnan(full), torch.isnan(short)) and bool(torch.isnan(full[~keep.to(DEV)]).any())
+    gate = x[keep][:, torch.arange(128) % (H - 1)].double()
+    if act == "clamped":
+        gate = gate.clamp(max=7.0)
+        ref = gate * torch.sigmoid(1.702 * gate) * 2.0
+    else:
+        ref = torch.nn.functional.gelu(gate, approximate="tanh") if act == "gelu" else P.silu(gate)
+    got = full[keep.to(DEV)].double().cpu()
+    # the exponential is off by one unit (2^-23), the sum and the quotient by half of one each, the slope's product turns into
+    # |slope · gate| halves; from where the exponential overflows (88) the quotient is 0, and below 2^-126 units are absolute
+    bound = (4.0 + (1.702 * gate.abs().clamp(max=90.0) if act == "clamped" else 0.0)) * 2.0 ** -23 * ref.abs() + 2.0 ** -118
+    if act != "gelu":
+        assert bool(((got - ref).abs() <= bound).all())
