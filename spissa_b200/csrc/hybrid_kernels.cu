@@ -1194,10 +1194,12 @@ __global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int* 
 __global__ void __launch_bounds__(1024)
 moe_place_kernel(const int* __restrict__ ids, int n_pairs, const int* __restrict__ counts, int E, int* __restrict__ sorted,
                  int* __restrict__ tiles /* [max_tiles][3] */, int max_tiles, int tm, int padded, int* __restrict__ pos,
-                 int* __restrict__ tab_up, int* __restrict__ tab_down, int up_rows, int down_rows) {
+                 int* __restrict__ tab_up, int* __restrict__ tab_down, int up_rows, int down_rows, int run) {
     // ``padded``: every expert's rows begin at a tile's first row (the sorted list then has holes, which say -1, and
     // ``pos`` gives every pair its row); ``tab_up`` / ``tab_down``: per tile the row at which the expert's matrices begin
-    // in the stacked weights (-1: the tile is not in use), for products that take whole tiles of one expert.
+    // in the stacked weights (-1: the tile is not in use), for products that take whole tiles of one expert. ``tiles`` then
+    // holds, for products that take up to ``run`` rows of an expert at once, its rows in equal parts of a multiple of 16: there
+    // are never more of them than tiles, the entries left over say -1.
     __shared__ int start, tile0, mine, wsum[32], running;     // blocks of up to 1,024 threads: a pass of the list per 1,024 pairs
     const int e = blockIdx.x;
     if (threadIdx.x == 0) {
@@ -1229,12 +1231,13 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, const int* __restrict
         }
         __syncthreads();
     }
-    const int n_mine = (mine + tm - 1) / tm;
+    const int n_mine = (mine + tm - 1) / tm, n_parts = (mine + run - 1) / run;
+    const int part = padded && n_parts > 0 ? ((mine + n_parts - 1) / n_parts + 15) & ~15 : tm;
     for (int i = threadIdx.x; i < n_mine; i += blockDim.x) {
         if (tile0 + i >= max_tiles) break;
-        tiles[(tile0 + i) * 3 + 0] = e;
-        tiles[(tile0 + i) * 3 + 1] = (padded ? tile0 * tm : start) + i * tm;
-        tiles[(tile0 + i) * 3 + 2] = min(tm, mine - i * tm);
+        tiles[(tile0 + i) * 3 + 0] = i * part < mine ? e : -1;
+        tiles[(tile0 + i) * 3 + 1] = (padded ? tile0 * tm : start) + i * part;
+        tiles[(tile0 + i) * 3 + 2] = min(part, mine - i * part);
         if (tab_up) { tab_up[tile0 + i] = e * up_rows; tab_down[tile0 + i] = e * down_rows; }
     }
     if (e == E - 1)
@@ -1250,7 +1253,7 @@ static int moe_plan(const int* ids, int n_pairs, int E, int* counts, int* sorted
                     cudaStream_t stream) {
     moe_count_kernel<<<E, 256, 0, stream>>>(ids, n_pairs, counts);
     SP_CHECK_LAUNCH("moe_count");
-    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, 0, stream>>>(ids, n_pairs, counts, E, sorted, tiles, max_tiles, tm, 0, nullptr, nullptr, nullptr, 0, 0);
+    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, 0, stream>>>(ids, n_pairs, counts, E, sorted, tiles, max_tiles, tm, 0, nullptr, nullptr, nullptr, 0, 0, tm);
     SP_CHECK_LAUNCH("moe_place");
     return 0;
 }
@@ -1268,16 +1271,17 @@ __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, cons
 }
 
 SP_API int sp_moe_plan_tiles(const void* x, const int* ids, int T, int top, int W, int E, int up_rows, int down_rows, int* counts,
-                             int* sorted, int* pos, int* tiles, int* tab_up, int* tab_down, int max_tiles, void* xs,
+                             int* sorted, int* pos, int* tiles, int* tab_up, int* tab_down, int max_tiles, int run, void* xs,
                              cudaStream_t stream) {
     const int n_pairs = T * top;
     if (n_pairs <= 0) return 0;
     if (W % 8 || (((uintptr_t)x | (uintptr_t)xs) & 15)) SP_FAIL("moe_plan_tiles: rows of %d do not move in 16-byte pieces", W);
     if ((n_pairs + 127) / 128 + E > max_tiles) SP_FAIL("moe_plan_tiles: the tile table is too short");
+    if (run < 128 || run % 16) SP_FAIL("moe_plan_tiles: parts of %d rows", run);
     SP_CHECK_CALL("moe_plan_tiles", cudaMemsetAsync(sorted, 0xff, (size_t)max_tiles * 128 * sizeof(int), stream));
     moe_count_kernel<<<E, 256, 0, stream>>>(ids, n_pairs, counts);
     SP_CHECK_LAUNCH("moe_count");
-    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, 0, stream>>>(ids, n_pairs, counts, E, sorted, tiles, max_tiles, 128, 1, pos, tab_up, tab_down, up_rows, down_rows);
+    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, 0, stream>>>(ids, n_pairs, counts, E, sorted, tiles, max_tiles, 128, 1, pos, tab_up, tab_down, up_rows, down_rows, run);
     SP_CHECK_LAUNCH("moe_place");
     const size_t n = (size_t)max_tiles * 128 * (W / 8);
     const size_t want = (n + 255) / 256;

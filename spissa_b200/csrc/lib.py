@@ -1414,6 +1414,12 @@ def moe_tile_rows() -> int:
     return int(load("hybrid").sp_moe_tile_rows())
 
 
+MID_EXPERT_TOKENS = 4096     # up to so many pairs an expert gated rows in blocks of 128 run as parts of up to 256 tokens (tc_mid.cu), else on
+#                              tc_gemm.cu's tiles of 128, whose pairs of CTAs read less of W. The whole call in us, tc_mid / tc_gemm:
+#                              32 experts of 2,048 x 2,048 16 tokens each 201 / 241, 256 each 353 / 426, 1,024 each 1,025 / 1,089;
+#                              128 of 2,048 x 768, 8 to 512 each 315 / 407 to 1,149 / 1,312; 8 of 4,096 x 2,048, 64 each 123 / 145,
+#                              1,024 each 481 / 500, 2,048 each 900 / 925, 8,192 each 3,343 / 3,281 (all on two of them 3,589 / 3,499).
+#                              The down product, whose columns fill pairs of CTAs, is the faster one on tc_gemm.cu (94 / 133)
 TC_EXPERT_PAIRS = 512        # from this many (token, expert) pairs on, and 8 per expert, whole 128-row tiles pay off
 
 
@@ -1451,15 +1457,14 @@ def moe_experts(x, ids, weights, w_gate_up, w_down, y, top, limit, slope=1.702, 
         hidden = torch.empty(rows, F, dtype=torch.bfloat16, device=dev)
         out_rows = torch.empty(rows, W, dtype=torch.float32, device=dev)
         launches += 6
+        runs = glu and glu_block == 128 and (slope == 0.0 or limit > 0.0) and n_pairs < MID_EXPERT_TOKENS * E and max_tiles <= 65535
         _check("hybrid", lib.sp_moe_plan_tiles(
             c_void_p(_ptr(x)), c_void_p(_ptr(ids)), T, int(top), W, E, F2, W, c_void_p(_ptr(counts)), c_void_p(_ptr(order)),
             c_void_p(_ptr(pos)), c_void_p(_ptr(tiles)), c_void_p(_ptr(tab_up)), c_void_p(_ptr(tab_down)), max_tiles,
-            c_void_p(_ptr(xs)), c_void_p(_stream())))
+            int(load("tc_mid").sp_tc_mid_run()) if runs else 256, c_void_p(_ptr(xs)), c_void_p(_stream())))
         status = c_void_p(_ptr(status_word(dev)))
 
-        if glu and glu_block == 128 and (slope == 0.0 or limit > 0.0):
-            # gated rows in blocks of 128: runs of up to 256 tokens on tc_mid (2,048 tokens, 4 of 32 experts of 2,048: 190 us,
-            # 237 on tc_gemm's tiles of 128 tokens; its plain tiles are the faster ones for the down product, 94 us / 133)
+        if runs:
             _check("tc_mid", load("tc_mid").sp_tc_mid_grouped(
                 c_void_p(_ptr(xs)), c_void_p(_ptr(w_gate_up)), c_void_p(_ptr(hidden)), dt_code(hidden), rows, F2, W, W, W, E * F2, F,
                 c_void_p(_ptr(tiles)), max_tiles, c_float(limit), c_float(slope), int(act), status, c_void_p(_stream())))

@@ -17,10 +17,12 @@
 // Measured back to back on weights from HBM (us, this kernel / the one that ran before), 1B shape: 301 tokens QKV 11.0 / 17.2,
 // output 10.5 / 17.6, gate/up 27.3 / 59.3, down 19.1 / 27.5; 64 tokens (before: tc_stream.cu) 8.1 / 8.5, 7.3 / 8.0,
 // 18.7 / 20.6, 13.1 / 13.4.
-// Grouped (routed experts, sp_tc_mid_grouped): A's rows lie in runs of one expert each, a run's tokens are cut into equal tiles
-// of at most 256 and multiplied with that expert's rows of the stacked weights; the table of the runs is read on the device.
-// 2,048 tokens, 4 of 32 experts of 2,048 x 2,048: 190 us, 237 on tc_gemm.cu's tiles of 128 tokens, of which a fifth is padding.
-// Five waves of CTAs that are alone on their SM: of 36 us each, 18 are the bytes and a dozen the epilogue.
+// Grouped (routed experts, sp_tc_mid_grouped): A's rows lie in runs of one expert each, in equal tiles of at most 256 rows
+// (moe_place_kernel cuts them), each multiplied with that expert's rows of the stacked weights; a CTA reads its tile's entry
+// of the table on the device.
+// 2,048 tokens, 4 of 32 experts of 2,048 x 2,048: 353 us the whole layer, 426 on tc_gemm.cu's tiles of 128 tokens, of which a
+// fifth is padding. Five waves of CTAs that are alone on their SM, about half of each its bytes. (Where each CTA found its
+// tile by walking its expert's entries of the table, an expert of 65,536 tokens took twice as long as on tc_gemm.cu.)
 // Every mbarrier wait is bounded and records a code in ``status``; no load uses cluster multicast.
 #include "tcgen05.cuh"
 #include <string.h>
@@ -72,10 +74,7 @@ struct Args {
     EpiArgs ep;
     SpRange rg;
     SpGate ga;
-    // grouped: per 128 rows of A (expert or -1, first row, rows of them in use); an expert's entries follow one another and
-    // only its last may have less than 128 rows in use
-    const int* tiles;
-    int n_tiles;
+    const int* tiles;       // grouped: per token tile (expert or -1, first row of A, rows: 1 to MAX_NT)
 };
 constexpr int GROUP_BOX = 64;               // rows of A per box of a grouped product
 
@@ -295,19 +294,12 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const int tile = blockIdx.x / a.pieces, piece = blockIdx.x % a.pieces;     // the cluster's rank is the piece of K
     int tok0 = blockIdx.y * a.nt, count = min(a.nt, a.M - tok0), nt = a.nt, expert = 0;      // tokens of this tile
     if (GROUPED) {
-        // entry y of the table is the ``turn``-th 128 rows of its expert's run; the run's first few entries stand for its tiles
         sp_wait_for_predecessor();
-        const int y = blockIdx.y;
-        expert = a.tiles[3 * y];
+        expert = a.tiles[3 * blockIdx.y];
         if (expert < 0) return;
-        int turn = 0, total = a.tiles[3 * y + 2];
-        while (y - turn > 0 && a.tiles[3 * (y - turn - 1)] == expert) total += a.tiles[3 * (y - ++turn) + 2];
-        for (int i = y + 1; i < a.n_tiles && a.tiles[3 * i] == expert; ++i) total += a.tiles[3 * i + 2];
-        const int cut = (total + MAX_NT - 1) / MAX_NT;
-        nt = ((total + cut - 1) / cut + 15) & ~15;
-        if (turn >= cut || turn * nt >= total) return;
-        tok0 = a.tiles[3 * (y - turn) + 1] + turn * nt;
-        count = min(nt, total - turn * nt);
+        tok0 = a.tiles[3 * blockIdx.y + 1];
+        count = a.tiles[3 * blockIdx.y + 2];
+        nt = (count + 15) & ~15;
     }
     const int num_kb = (a.K + BK - 1) / BK;
     const int per = (num_kb + a.pieces - 1) / a.pieces;
@@ -631,9 +623,9 @@ SP_API int sp_tc_mid(const void* A, const void* W, void* C, int c_dt, int M, int
 }
 
 // Gated products of runs of rows of A [M, K], each with its expert's N rows (gate and up in blocks of 128) of the stacked W
-// [w_rows, K]: C [M, N/2] = act(gate)·up, the clamped unit where ``slope`` is non-zero. ``tiles`` [n_tiles][3] on the device: per
-// 128 rows of A (expert or -1, first row, rows in use), an expert's entries one after another, only its last with less than 128
-// rows in use; rows that no entry names are not written.
+// [w_rows, K]: C [M, N/2] = act(gate)·up, the clamped unit where ``slope`` is non-zero. ``tiles`` [n_tiles][3] on the device:
+// (expert or -1, first row of A, rows: 1 to sp_tc_mid_run()); rows that no entry names are not written.
+SP_API int sp_tc_mid_run() { return MAX_NT; }
 SP_API int sp_tc_mid_grouped(const void* A, const void* W, void* C, int c_dt, int M, int N, int K, int lda, int ldw, int w_rows, int ldc,
                              const int* tiles, int n_tiles, float limit, float slope, int act, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || n_tiles <= 0) return 0;
@@ -657,7 +649,7 @@ SP_API int sp_tc_mid_grouped(const void* A, const void* W, void* C, int c_dt, in
     args.C = C; args.status = status;
     args.c_dt = c_dt; args.M = M; args.N = N; args.K = K; args.ldc = ldc; args.mode = MODE_SILU_MUL;
     args.nt = p.nt; args.pieces = 1; args.stages = p.stages; args.tmem_cols = p.tmem_cols;
-    args.tiles = tiles; args.n_tiles = n_tiles;
+    args.tiles = tiles;
     CUtensorMap mw, ma;
     if (encode_map(&mw, W, w_rows, K, ldw, BW)) return 1;
     if (encode_map(&ma, A, M, K, lda, GROUP_BOX)) return 1;

@@ -224,3 +224,54 @@ def test_gated_rows_keep_the_bits_of_32_bit_arithmetic(K, act):
     bound = (4.0 + (1.702 * gate.abs().clamp(max=90.0) if act == "clamped" else 0.0)) * 2.0 ** -23 * ref.abs() + 2.0 ** -118
     if act != "gelu":
         assert bool(((got - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 128, 129, 256, 257, 513, 600], [0, 3000, 0, 5], [16, 17, 15]])
+def test_parts_of_an_experts_rows(K, counts):
+    """The table that the grouped products read: an expert's rows in equal parts of a multiple of 16, at most 256 each, and
+    nothing that a product has to look for among its neighbours."""
+    import ctypes as C
+    E, W, T = len(counts), 64, sum(counts)
+    g = torch.Generator().manual_seed(T)
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)])[torch.randperm(T, generator=g)].to(DEV)
+    x = torch.randn(T, W, device=DEV).bfloat16()
+    most = -(-T // 128) + E
+    ints = lambda n: torch.full((n,), -7, dtype=torch.int32, device=DEV)       # noqa: E731
+    per, order, pos, tiles, up, down = ints(E), ints(most * 128), ints(T), ints(most * 3), ints(most), ints(most)
+    xs = torch.empty(most * 128, W, dtype=torch.bfloat16, device=DEV)
+    run = int(K.load("tc_mid").sp_tc_mid_run())
+    ptr = lambda t: C.c_void_p(t.data_ptr())                            # noqa: E731
+    assert K.load("hybrid").sp_moe_plan_tiles(ptr(x), ptr(ids), T, 1, W, E, 3, 5, ptr(per), ptr(order), ptr(pos), ptr(tiles), ptr(up),
+                                              ptr(down), most, run, ptr(xs), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want, first = [], 0
+    for e, n in enumerate(counts):
+        cut = -(-n // run)
+        part = -(-(-(-n // cut)) // 16) * 16 if n else 1
+        entries = [(e, first + i, min(part, n - i)) for i in range(0, n, part)]
+        assert len(entries) <= -(-n // 128) and all(0 < c <= run for _, _, c in entries)
+        want += entries
+        first += -(-n // 128) * 128
+    got = tiles.view(-1, 3).tolist()
+    assert [tuple(t) for t in got if t[0] >= 0] == want and len(got) == most
+    for e, at, c in want:
+        assert torch.equal(ids[order[at:at + c].long()], torch.full((c,), e, dtype=torch.int32, device=DEV))
+        assert torch.equal(xs[at:at + c], x[order[at:at + c].long()])
+
+
+def test_experts_of_many_tokens_take_the_tiles_of_128(K, monkeypatch):
+    E, W, F, T = 2, 128, 256, 700
+    torch.manual_seed(5)
+    ids = (torch.rand(T, 1, device=DEV) < 0.9).int()
+    x, y = torch.randn(T, W, device=DEV).bfloat16(), torch.zeros(T, W, device=DEV)
+    both, down = (torch.randn(E, 2 * F, W, device=DEV) * 0.1).bfloat16(), (torch.randn(E, W, F, device=DEV) * 0.1).bfloat16()
+    weights = torch.rand(T, 1, device=DEV)
+    rows = []
+    for most in (K.MID_EXPERT_TOKENS, 1):
+        monkeypatch.setattr(K, "MID_EXPERT_TOKENS", most)
+        y.zero_()
+        K.moe_experts(x, ids, weights, both, down, y, 1, 7.0, 1.702, 128)
+        rows.append(y.clone())
+    # the hidden rows are bfloat16 of the same 32-bit sums in another order
+    assert float((rows[0] - rows[1]).norm() / rows[0].norm()) <= 2.0 ** -8
+    with pytest.raises(K.KernelError):
+        K._check("hybrid", K.load("hybrid").sp_moe_plan_tiles(None, None, 8, 1, 64, 1, 1, 1, None, None, None, None, None, None, 4, 100, None, None))
