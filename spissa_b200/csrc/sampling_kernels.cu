@@ -10,7 +10,7 @@
 // Every step of that walk asks the same question: which is the first token, in that order, at which a
 // running total (a count for top-k, a mass for top-p and for the draw) reaches a target? The order is the
 // rising order of a 64-bit key (inverted probability bits, then index), keys are unique, and the total up
-// to a key is a plain sum over the tokens with smaller or equal keys. So the token is found by descending
+// to a key is a plain sum over the tokens with smaller or equal keys. So the token can be found by descending
 // the key four bits at a time: one pass over the row adds every token that is still in question into one
 // of 16 sums by its next four key bits, the sums are added up in rising order until the target is
 // reached, and the search goes on inside that one. A pass touches only tokens that share the bits chosen
@@ -23,7 +23,7 @@
 // totals stay in the cluster's shared memory for every question asked of the row; the tokens of the one bucket in which a
 // target is reached are gathered and compared with one another by all CTAs: 39 us (58 with one CTA comparing; what is
 // left are the barriers of the cluster, the softmax and the adding into buckets). Only where more than 1,024 tokens share
-// the bucket (rows of nearly equal probabilities) the descent runs as before.
+// the bucket (rows of nearly equal probabilities) the descent runs, from the three digits of the key that the bucket fixes.
 //
 // Sums are integers: a probability counts as floor(p · 2^44) and a token as 1 in the high bits of the same
 // 64-bit word, so every total is exact and independent of the order of addition (the same draw always
@@ -96,39 +96,37 @@ struct Row {
     int idx_digits;            // four-bit digits that hold an index
 };
 
-// The first key (rising) among those ≤ ``limit`` at which the running count (by_mass false) or mass reaches
-// ``target``. Returns false when even the total does not; ``upto`` is then that total. Else ``key`` is the
-// token's key and ``upto`` the packed total up to and including it. Every thread of the cluster runs this alike.
+constexpr int SS_KNOWN = 3;                        // digits of the key that are known from the buckets
+
+// The first key (rising) at which the running count (by_mass false) or mass reaches ``target``, where it begins with the
+// SS_KNOWN digits of ``prefix`` and the tokens before those come to ``below``. ``upto``: the packed total up to and
+// including it. Every thread of the cluster runs this alike.
 template <int THREADS>
-__device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned long long target, unsigned long long limit,
-                           unsigned& parity, unsigned long long& key, unsigned long long& upto) {
+__device__ void ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned long long target, unsigned long long prefix,
+                           unsigned long long below, unsigned& parity, unsigned long long& key, unsigned long long& upto) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned long long* acc = sh->acc;
-    unsigned long long prefix = 0, below = 0;
     const int n_digits = 8 + row.idx_digits;
-    for (int d = 0; d < n_digits; ++d) {
+    for (int d = SS_KNOWN; d < n_digits; ++d) {
         const int shift = d < 8 ? 60 - 4 * d : 4 * (n_digits - 1 - d);
-        // bits above this digit that a token must share with the prefix (all of them; none in the first pass)
-        const unsigned long long above = d == 0 ? 0ull : ~0ull << (shift + 4 > 63 ? 63 : shift + 4);
+        const unsigned long long above = ~0ull << (shift + 4);          // bits above this digit: a token must share them with the prefix
 #pragma unroll
         for (int s = 0; s < SS_SEGS; ++s) acc[s * THREADS + tid] = 0ull;
         if (d < 8) {
-            // a digit of the probability: 32-bit arithmetic on the key's upper half; the index only settles
-            // whether a token with the limit's own probability is still inside
-            const unsigned lim_hi = (unsigned)(limit >> 32), lim_lo = (unsigned)limit;
+            // a digit of the probability: 32-bit arithmetic on the key's upper half
             const unsigned pre_hi = (unsigned)(prefix >> 32), above_hi = (unsigned)(above >> 32);
             const int sh_hi = shift - 32;
             for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
                 const unsigned b = row.bits[i - row.i0];
                 const unsigned kb = ~b;
-                if (((kb ^ pre_hi) & above_hi) == 0u && (kb < lim_hi || (kb == lim_hi && (unsigned)i <= lim_lo)))
+                if (((kb ^ pre_hi) & above_hi) == 0u)
                     acc[((kb >> sh_hi) & 15u) * THREADS + tid] += ss_weight(b);
             }
         } else {
             for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
                 const unsigned b = row.bits[i - row.i0];
                 const unsigned long long k = ss_key(b, (unsigned)i);
-                if (k <= limit && ((k ^ prefix) & above) == 0ull) acc[((k >> shift) & 15u) * THREADS + tid] += ss_weight(b);
+                if (((k ^ prefix) & above) == 0ull) acc[((k >> shift) & 15u) * THREADS + tid] += ss_weight(b);
             }
         }
         __syncthreads();
@@ -155,7 +153,7 @@ __device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned lo
         }
         parity ^= 1u;
         __syncthreads();
-        int chosen = -1;
+        int chosen = SS_SEGS - 1;
         unsigned long long cum = below;
         for (int s = 0; s < SS_SEGS; ++s) {
             const unsigned long long t = sh->total[s];
@@ -164,11 +162,6 @@ __device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned lo
                 if ((by_mass ? (with & MASS_MASK) : (with >> MASS_BITS)) >= target) { chosen = s; break; }
                 cum = with;
             }
-        }
-        if (chosen < 0) {                                      // only the first pass can fail: later ones search a segment that reached
-            upto = cum;
-            __syncthreads();
-            return false;
         }
         below = cum;
         prefix |= (unsigned long long)chosen << shift;
@@ -181,7 +174,7 @@ __device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned lo
             __syncthreads();
             for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
                 const unsigned long long k = ss_key(row.bits[i - row.i0], (unsigned)i);
-                if (k <= limit && ((k ^ prefix) & fixed) == 0ull) sh->loc = k + 1ull;       // at most one thread of the cluster
+                if (((k ^ prefix) & fixed) == 0ull) sh->loc = k + 1ull;       // at most one thread of the cluster
             }
             __syncthreads();
             ss_cluster_sync();
@@ -191,10 +184,9 @@ __device__ bool ss_descend(Shared* sh, const Row& row, bool by_mass, unsigned lo
             ss_cluster_sync();                                 // all have read before anyone's loc is reset
             key = found - 1ull;
             upto = below + in_segment;
-            return true;
+            return;
         }
     }
-    return false;                                              // not reached: the last digit always ends above
 }
 
 // ---------------------------------------------------------------- the buckets
@@ -204,10 +196,12 @@ constexpr int BK_PER = BK_N / SS_CLUSTER;          // positions (buckets by fall
 constexpr int BK_LIST = 1024;                      // tokens of a bucket that are compared with one another
 constexpr unsigned BK_CARRY = 1u << 20;            // in a bucket's count: its sum of lower bits has passed 2^32 (a slice has less than 2^20 tokens)
 
-// In dynamic shared memory, over the descent's words.
-struct Buckets {
+// In dynamic shared memory, in the place of the descent's words.
+struct Lists {
     union { unsigned count[BK_N]; unsigned long long list[BK_LIST]; };         // this CTA's tokens of each bucket; later the gathered keys
     union { unsigned low[BK_N]; unsigned long long weight[BK_LIST]; };         // their lower bits' contributions; later what the gathered tokens weigh
+};
+struct Buckets {
     unsigned long long scan[BK_PER];               // running totals (count and mass packed) of this CTA's positions
     unsigned long long warp_total[32];
     unsigned long long total;                      // of this CTA's positions
@@ -238,19 +232,28 @@ __device__ __forceinline__ bool bk_reached(unsigned long long total, bool by_mas
 
 // Every CTA: its slice into buckets, then the running totals of its 512 positions of the row's buckets.
 template <int THREADS>
-__device__ void bk_fill(Buckets* bk, const Row& row) {
+__device__ void bk_fill(Buckets* bk, Lists* li, const Row& row) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = row.i1 - row.i0;
     const bool carries = n >= 1 << (32 - BK_SHIFT);                    // a bucket's lower bits could pass 2^32
-    for (int j = tid; j < n; j += THREADS) {
-        const unsigned b = row.bits[j], low = bk_low(b);
-        unsigned one = 1u;
-        if (carries) {
-            if (low && atomicAdd(&bk->low[b >> BK_SHIFT], low) + low < low) one += BK_CARRY;
-        } else if (low) {
-            atomicAdd(&bk->low[b >> BK_SHIFT], low);
+    for (int j0 = warp * 32; j0 < n; j0 += THREADS) {
+        const int j = j0 + lane;
+        const unsigned b = j < n ? row.bits[j] : ~0u, bucket = b >> BK_SHIFT;
+        unsigned low = j < n ? bk_low(b) : 0u, one = 1u;
+        int alike;                                                     // a warp of one bucket (probabilities of zero, equal tokens) adds once
+        __match_all_sync(0xffffffffu, bucket, &alike);
+        if (alike) {
+            low = __reduce_add_sync(0xffffffffu, low);
+            one = 32u;
         }
-        atomicAdd(&bk->count[b >> BK_SHIFT], one);
+        if (j < n && (!alike || lane == 0)) {
+            if (carries) {
+                if (low && atomicAdd(&li->low[bucket], low) + low < low) one += BK_CARRY;
+            } else if (low) {
+                atomicAdd(&li->low[bucket], low);
+            }
+            atomicAdd(&li->count[bucket], one);
+        }
     }
     __syncthreads();
     ss_cluster_sync();
@@ -266,8 +269,8 @@ __device__ void bk_fill(Buckets* bk, const Row& row) {
 #pragma unroll
             for (unsigned r = 0; r < SS_CLUSTER; ++r) {
                 unsigned c, l;
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c) : "r"(ss_peer_addr(&bk->count[bucket], r)) : "memory");
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(l) : "r"(ss_peer_addr(&bk->low[bucket], r)) : "memory");
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c) : "r"(ss_peer_addr(&li->count[bucket], r)) : "memory");
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(l) : "r"(ss_peer_addr(&li->low[bucket], r)) : "memory");
                 count += c & (BK_CARRY - 1u);
                 low += l + ((unsigned long long)(c / BK_CARRY) << 32);
             }
@@ -296,12 +299,12 @@ __device__ void bk_fill(Buckets* bk, const Row& row) {
     ss_cluster_sync();                                                 // the counts are not read any more
 }
 
-// The token at which the running count or mass reaches ``target``, among all of the row, as ss_descend gives it. 1: found;
-// 0: even the total does not reach it (``upto``: the total); -1: too many tokens share the bucket. Every CTA alike.
-// ``question``: 0, 1, ... within a row.
+// The token at which the running count or mass reaches ``target``, among all of the row: its key, and the packed total up to
+// and including it. False when even the total does not (``upto``: the total). Every CTA alike. ``question``: 0, 1, ... within
+// a row.
 template <int THREADS>
-__device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, unsigned long long target, unsigned long long& key,
-                       unsigned long long& upto) {
+__device__ bool bk_find(Shared* sh, Buckets* bk, Lists* li, const Row& row, int question, bool by_mass, unsigned long long target,
+                        unsigned& parity, unsigned long long& key, unsigned long long& upto) {
     const int tid = threadIdx.x;
     unsigned long long base = 0ull, totals[SS_CLUSTER];
 #pragma unroll
@@ -313,7 +316,7 @@ __device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, 
             if (bk_reached(base + totals[r], by_mass, target)) owner = r;
             else base += totals[r];
         }
-    if (owner < 0) { upto = base; return 0; }
+    if (owner < 0) { upto = base; return false; }
     for (int i = tid; i < BK_PER; i += THREADS) {
         const unsigned long long with = base + ss_ld_peer_u64(&bk->scan[i], (unsigned)owner);
         const unsigned long long without = base + (i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull);
@@ -327,8 +330,15 @@ __device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, 
     const unsigned bucket = (unsigned)(BK_N - 1 - bk->position);
     const unsigned long long below = bk->below;
     const unsigned long long n_in = (bk->through - below) >> MASS_BITS;
-    if (n_in > BK_LIST) return -1;
-    const unsigned to_list = ss_peer_addr(bk->list, 0u), to_weight = ss_peer_addr(bk->weight, 0u);
+    if (n_in > BK_LIST) {
+        // from the first of the four buckets that share the key's first SS_KNOWN digits
+        const int first = bk->position & ~3, i = first - owner * BK_PER;
+        const unsigned long long before = base + (i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull);
+        const unsigned long long prefix = (unsigned long long)((16383u - (unsigned)(BK_N - 1 - first)) >> 2) << 52;
+        ss_descend<THREADS>(sh, row, by_mass, target, prefix, before, parity, key, upto);
+        return true;
+    }
+    const unsigned to_list = ss_peer_addr(li->list, 0u), to_weight = ss_peer_addr(li->weight, 0u);
     const unsigned to_n = ss_peer_addr(&bk->n_list[question], 0u);
     for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
         const unsigned b = row.bits[i - row.i0];
@@ -348,21 +358,21 @@ __device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, 
     const int m = (int)n_in, rank = (int)ss_cluster_rank();
     if (rank != 0) {
         for (int i = tid; i < m; i += THREADS) {
-            bk->list[i] = ss_ld_peer_u64(&bk->list[i], 0u);
-            bk->weight[i] = ss_ld_peer_u64(&bk->weight[i], 0u);
+            li->list[i] = ss_ld_peer_u64(&li->list[i], 0u);
+            li->weight[i] = ss_ld_peer_u64(&li->weight[i], 0u);
         }
     }
     __syncthreads();
     const int share = (m + SS_CLUSTER - 1) / SS_CLUSTER, i1 = min(m, (rank + 1) * share);
     for (int i0 = rank * share; i0 < i1; i0 += THREADS / 8) {          // uniform in the CTA
         const int i = i0 + (tid >> 3);
-        const unsigned long long mine = i < i1 ? bk->list[i] : 0ull;
+        const unsigned long long mine = i < i1 ? li->list[i] : 0ull;
         unsigned long long cum = 0ull;
-        for (int j = tid & 7; j < m; j += 8) cum += bk->list[j] < mine ? bk->weight[j] : 0ull;
+        for (int j = tid & 7; j < m; j += 8) cum += li->list[j] < mine ? li->weight[j] : 0ull;
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) cum += __shfl_xor_sync(0xffffffffu, cum, o);
         if ((tid & 7) == 0 && i < i1) {
-            const unsigned long long with = below + cum + bk->weight[i];
+            const unsigned long long with = below + cum + li->weight[i];
             if (bk_reached(with, by_mass, target) && !bk_reached(below + cum, by_mass, target)) {            // one token of the cluster
                 asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->key, 0u)), "l"(mine) : "memory");
                 asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->upto, 0u)), "l"(with) : "memory");
@@ -373,15 +383,15 @@ __device__ int bk_find(Buckets* bk, const Row& row, int question, bool by_mass, 
     ss_cluster_sync();
     key = ss_ld_peer_u64(&bk->key, 0u);                                // (the next result is written behind another barrier of the cluster)
     upto = ss_ld_peer_u64(&bk->upto, 0u);
-    return 1;
+    return true;
 }
 
 constexpr int INLINE_ROWS = 64;
 struct Draws { float u[INLINE_ROWS]; };            // the rows' uniform numbers, with the launch itself: no copy to the device
 
 template <int THREADS>
-__host__ __device__ constexpr size_t words_bytes() {                   // the descent's words, or the buckets
-    constexpr size_t a = (size_t)SS_SEGS * THREADS * 8, b = (sizeof(Buckets) + 15) / 16 * 16;
+__host__ __device__ constexpr size_t words_bytes() {                   // the descent's words, or the lists
+    constexpr size_t a = (size_t)SS_SEGS * THREADS * 8, b = (sizeof(Lists) + 15) / 16 * 16;
     return a > b ? a : b;
 }
 
@@ -397,9 +407,11 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     Shared* sh = &sh_;
     sh->acc = (unsigned long long*)dyn_smem;                   // every thread writes the same value
     unsigned* slice_cache = (unsigned*)(dyn_smem + words_bytes<THREADS>());
-    Buckets* bk = (Buckets*)dyn_smem;
+    Lists* li = (Lists*)dyn_smem;
+    __shared__ Buckets bk_;
+    Buckets* bk = &bk_;
     const int tid = threadIdx.x;
-    for (int i = tid; i < BK_N; i += THREADS) bk->count[i] = bk->low[i] = 0u;
+    for (int i = tid; i < BK_N; i += THREADS) li->count[i] = li->low[i] = 0u;
     if (tid < 4) bk->n_list[tid] = 0;
     const unsigned rank = ss_cluster_rank();
     const int row_id = blockIdx.x / SS_CLUSTER;
@@ -481,31 +493,22 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
         for (int j = tid; j < n; j += THREADS) bits[j] = probability(__uint_as_float(bits[j]));
     }
 
-    // By buckets while the tokens in question are few enough to be compared with one another; else by the descent, whose
-    // words lie over the buckets: from then on it answers everything.
-    bk_fill<THREADS>(bk, row);
-    bool buckets = true;
+    bk_fill<THREADS>(bk, li, row);
     int question = 0;
     unsigned parity = 0;
     auto first_at = [&](bool by_mass, unsigned long long target, unsigned long long& key, unsigned long long& upto) -> bool {
-        if (buckets) {
-            const int got = bk_find<THREADS>(bk, row, question++, by_mass, target, key, upto);
-            if (got >= 0) return got != 0;
-            buckets = false;
-            ss_cluster_sync();                                 // no CTA still reads a peer's buckets
-        }
-        return ss_descend<THREADS>(sh, row, by_mass, target, ~0ull, parity, key, upto);
+        return bk_find<THREADS>(sh, bk, li, row, question++, by_mass, target, parity, key, upto);
     };
-    unsigned long long limit = ~0ull, key = 0ull, upto = 0ull, limit_mass = 0ull;
-    if (top_k > 0 && top_k < V && first_at(false, (unsigned long long)top_k, key, upto)) {      // the first top_k tokens
-        limit = key;
-        limit_mass = upto & MASS_MASK;
-    }
+    unsigned long long key = 0ull, upto = 0ull, limit_mass = 0ull;
+    const bool limited = top_k > 0 && top_k < V && first_at(false, (unsigned long long)top_k, key, upto);       // the first top_k tokens
+    if (limited) limit_mass = upto & MASS_MASK;
     // of those the shortest prefix whose mass reaches top_p; its mass
-    unsigned long long kept_mass;
-    const bool reached = first_at(true, __float2ull_rz(top_p * MASS_UNIT), key, upto);
-    if (limit == ~0ull || (reached && key <= limit)) kept_mass = upto & MASS_MASK;
-    else kept_mass = limit_mass;                               // the first top_k weigh less
+    const unsigned long long enough = __float2ull_rz(top_p * MASS_UNIT);
+    unsigned long long kept_mass = limit_mass;                 // the first top_k weigh less
+    if (!limited || limit_mass >= enough) {
+        first_at(true, enough, key, upto);
+        kept_mass = upto & MASS_MASK;
+    }
     // the draw: u is a multiple of 2^-24, the target u · mass is taken exactly; it lies among the kept tokens
     const unsigned long long n_u = (unsigned long long)((u ? u[row_id] : draws.u[row_id]) * 16777216.0f);
     const unsigned long long target = (__umul64hi(kept_mass, n_u) << 40) | ((kept_mass * n_u) >> 24);

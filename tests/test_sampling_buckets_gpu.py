@@ -52,3 +52,36 @@ def test_draws_that_do_not_fit(K):
         K.sample_rows(logits, 1.0, 0, 1.0, [0.5] * 3, scratch, out)
     K.sample_rows(logits, 1.0, 0, 1.0, torch.full((65,), 0.5, device=DEV), scratch, out)
     assert out.tolist() == [49] * 65
+
+
+@pytest.mark.parametrize("V,equal", [(270001, 266310), (32000, 31999), (128256, 128256), (2000, 2000)])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.5), (50, 0.9), (1500, 0.3), (1500, 1.0)])
+def test_many_equal_tokens(K, V, equal, top_k, top_p):
+    """All of the mass in one bucket: its sums pass 32 bits in every slice (266,310 tokens), and the search goes on from it."""
+    if equal == 266310:
+        low = int(np.float32(1.0 / 266310).view(np.uint32)) & ((1 << 18) - 1)
+        assert low * (equal // 8) > 2 * 2 ** 32
+    test_equal_tokens_are_walked_in_whole_numbers(K, V, equal, top_k, top_p)
+
+
+@pytest.mark.parametrize("rows", [3, 20])
+@pytest.mark.parametrize("std", [0.02, 0.5])
+@pytest.mark.parametrize("top_k,top_p", [(0, 0.95), (50, 0.9), (9000, 0.4), (9000, 1.0)])
+def test_nearly_equal_tokens(K, rows, std, top_k, top_p):
+    """More than 1,024 tokens in the bucket of an answer. The walk in 64 bits says between which tokens it lies: a float32
+    probability is off by some 2^-22, which moves a running total by as much of itself."""
+    V = 32000
+    g = torch.Generator().manual_seed(rows)
+    logits = torch.randn(rows, V, generator=g) * std
+    us = [(i + 0.5) / rows for i in range(rows)]
+    us = [int(u * 2 ** 24) / 2 ** 24 for u in us]
+    scratch = torch.empty(K.sample_scratch_keys(rows, V), dtype=torch.int64, device=DEV)
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    K.sample_rows(logits.to(DEV), 1.0, top_k, top_p, us, scratch, out)
+    p, order = torch.softmax(logits.double(), dim=-1).sort(dim=-1, descending=True, stable=True)
+    run = p.cumsum(dim=-1)
+    for r, (u, token) in enumerate(zip(us, out.tolist())):
+        at = int((order[r] == token).nonzero())
+        kept = min(float(run[r, top_k - 1]) if top_k else 1.0, max(top_p, float(run[r, 0])))
+        slack = 2.0 ** -19 + 2 * float(p[r, 0])                        # the kept mass ends behind the token that reaches top_p
+        assert float(run[r, at]) >= u * kept - slack and float(run[r, at] - p[r, at]) <= u * kept + slack
