@@ -38,6 +38,24 @@ def mid_layers(fields: list) -> bool:
     return all(f["ffn"]["pair"] == 128 and f["mixer"]["hidden_size"] % 8 == 0 for f in fields)
 
 
+def fusable(fields: list) -> bool:
+    """Whether the fused sequence is built for these layers: a tile of the gate/up product holds both halves."""
+    return fields[0]["mixer"]["head_dim"] in (64, 128) and all(f["ffn"]["pair"] in (64, 128) for f in fields)
+
+
+def rope_ids(fields: list) -> list:
+    """Per layer the number of its frequency table among the different ones, compared on the host's copies."""
+    tables, ids = [], []
+    for f in fields:
+        t = f["mixer"].get("inv_freq_host")
+        t = (f["mixer"]["inv_freq"].detach() if t is None else t).float().cpu()
+        at = next((i for i, have in enumerate(tables) if have.shape == t.shape and torch.equal(have, t)), len(tables))
+        if at == len(tables):
+            tables.append(t)
+        ids.append(at)
+    return ids
+
+
 def fuses(n_tokens: int, mid: bool) -> bool:
     return MIN_TOKENS <= n_tokens <= (MID_TOKENS if mid else STREAM_TOKENS) or n_tokens >= TILE_TOKENS
 
@@ -52,31 +70,13 @@ class FusedPrefill:
         self.runs = 0
         self.layer_bytes = max(sum(w.numel() * w.element_size() for w in (f["mixer"]["qkv"], f["mixer"]["o"], f["ffn"]["gate_up"],
                                                                      f["ffn"]["down"])) for f in fields)
-        # layers whose frequency tables are equal share one table of angles per step
-        tables, self.rope_id = [], []
-        for f in fields:
-            t = f["mixer"]["inv_freq"].detach().float().cpu()
-            for i, have in enumerate(tables):
-                if have.shape == t.shape and torch.equal(have, t):
-                    self.rope_id.append(i)
-                    break
-            else:
-                self.rope_id.append(len(tables))
-                tables.append(t)
+        self.rope_id = rope_ids(fields)        # layers whose frequency tables are equal share one table of angles per step
 
     @classmethod
     def plan(cls, model):
         """A runner for ``model`` or None when some layer has to run part by part."""
         fields = collect_fused_fields(model)
-        if fields is None:
-            return None
-        hd = fields[0]["mixer"]["head_dim"]
-        if hd not in (64, 128):
-            return None
-        for f in fields:
-            if f["ffn"]["pair"] not in (64, 128):          # a tile of the gate/up product holds both halves
-                return None
-        return cls(model, fields)
+        return cls(model, fields) if fields is not None and fusable(fields) else None
 
     def takes(self, step, cache) -> bool:
         # (a decode step of up to 16 sequences comes here too where large layers make this the faster way)

@@ -112,8 +112,9 @@ class HostStep:
             if hd % 16 or not 16 <= hd <= 128 or m["num_heads"] // m["num_kv_heads"] > 16:
                 return None                              # the prompt attention kernel's sizes
         runner = cls(model, fields)
-        from .fused_prefill import FusedPrefill, mid_layers
-        runner.can_fuse = FusedPrefill.plan(model) is not None
+        from .fused_prefill import fusable, mid_layers, rope_ids
+        runner.can_fuse = fusable(fields)
+        runner.rope_id = model._fused_prefill.rope_id if model._fused_prefill else rope_ids(fields)
         # (the tcgen05 attention of steps of many tokens takes the fused sequence's head sizes, 64 and 128)
         runner.mid = mid_layers(fields)
         return runner
@@ -128,21 +129,17 @@ class HostStep:
 
     def _bind_cache(self, cache) -> None:
         self.cache_id, self.layers = id(cache), None
-        rows, keep, tables = [], [], []
-        for e, f in zip(self.model.spec.schedule, self.fields):
+        rows, keep, tables = [], [], {}
+        for e, f, rope in zip(self.model.spec.schedule, self.fields, self.rope_id):
             g = cache.kv_groups.get(cache.cache_group.get(e.cache))
             if g is None or g.request.window or g.k.dtype != torch.bfloat16:
                 return
             m, ff = f["mixer"], f["ffn"]
             i = g.index[e.cache]
             k_pool, v_pool = g.k[i], g.v[i]
-            inv = m["inv_freq"].to(device=k_pool.device, dtype=torch.float32).contiguous()
-            for have in tables:                          # equal tables share one tensor: the runner compares addresses
-                if have.shape == inv.shape and torch.equal(have, inv):
-                    inv = have
-                    break
-            else:
-                tables.append(inv)
+            if rope not in tables:                       # equal tables share one tensor: the runner compares addresses
+                tables[rope] = m["inv_freq"].to(device=k_pool.device, dtype=torch.float32).contiguous()
+            inv = tables[rope]
             keep += [inv, k_pool, v_pool]
             r = _Layer()
             r.w_qkv, r.w_o, r.w_gu, r.w_down = (t.data_ptr() for t in (m["qkv"], m["o"], ff["gate_up"], ff["down"]))

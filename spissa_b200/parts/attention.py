@@ -103,6 +103,7 @@ class GQAAttention(Mixer):
         if rd != self.head_dim or self.qkv.weight.dtype != torch.bfloat16 or self.o.weight.dtype != torch.bfloat16:
             return None
         return dict(kind="gqa_rotary", qkv=self.qkv.weight, o=self.o.weight, inv_freq=inv_freq, scale=self.scale,
+                    inv_freq_host=getattr(self.position, "inv_freq_host", None),
                     hidden_size=self.hidden_size, num_heads=self.num_heads, num_kv_heads=self.num_kv_heads,
                     head_dim=self.head_dim)
 
