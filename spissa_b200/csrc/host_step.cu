@@ -215,6 +215,7 @@ int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, i
     if (fused_product(st.xw[0], L.w_qkv, nullptr, DT_BF16, nqkv, st.H, 0, MODE_STREAM_QKV_ROPE, 0, &ep, st, stream)) return 1;
     ++launches;
     if (st.T >= k.flash_tc_from) {
+        if (!k.flash_prefill_tc) SP_FAIL("host step: the attention of steps of %d tokens or more has not been bound", k.flash_tc_from);
         if (k.flash_prefill_tc(st.q, st.ctx, L.k_pool, L.v_pool, st.n_pages, st.T, st.seq_start, st.positions, st.seq_row, st.page_table,
                                st.max_pages, st.page_size, st.n_seqs, st.n_tc_tiles, L.nh, L.nkv, L.hd, L.window, L.scale, st.status, stream))
             return fail_from(k.err_flash_tc, "host step");
@@ -244,9 +245,12 @@ int fused_layer(const HostLayer& L, const HostLayer* next, const HostStep& st, i
 
 SP_API int sp_host_step_bind(const void* table, int bytes) {
     if (bytes != (int)sizeof(HostKernels)) SP_FAIL("host step: the kernel table has %d bytes, %d are expected", bytes, (int)sizeof(HostKernels));
+    const FlashPrefillTcFn tc = kernels.flash_prefill_tc;             // comes with the first step that needs it, and stays
+    const LastErrorFn tc_err = kernels.err_flash_tc;
     memcpy(&kernels, table, sizeof(kernels));
+    if (!kernels.flash_prefill_tc) { kernels.flash_prefill_tc = tc; kernels.err_flash_tc = tc_err; }
     if (!kernels.rmsnorm || !kernels.gemv || !kernels.tc_stream || !kernels.tc_gemm || !kernels.rope_kv_write ||
-        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.flash_prefill_tc || !kernels.rope_table || !kernels.norm_prepare)
+        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.rope_table || !kernels.norm_prepare)
         SP_FAIL("host step: an entry point is missing from the kernel table");
     bound = true;
     return 0;

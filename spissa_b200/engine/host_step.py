@@ -53,14 +53,15 @@ def _address(lib, name) -> int:
     return ctypes.cast(getattr(lib, name), c_void_p).value
 
 
-_bound = False
+_bound = 0             # 1: handed over; 2: with the attention of steps of ``FLASH_TC_TOKENS`` tokens or more
 
 
-def _bind() -> ctypes.CDLL:
-    """Hand the other libraries' entry points to the C++ runner, once per process."""
+def _bind(flash_tc: bool) -> ctypes.CDLL:
+    """Hand the other libraries' entry points to the C++ runner, once per process (and once more for the first step of
+    ``FLASH_TC_TOKENS`` tokens, whose attention is a library that only these need)."""
     global _bound
     host = K.load("host_step")
-    if _bound:
+    if _bound > int(flash_tc):
         return host
     for struct, size in ((_Kernels, "kernels"), (_Layer, "layer"), (_Step, "step")):
         want = int(getattr(host, f"sp_host_step_{size}_bytes")())
@@ -82,11 +83,12 @@ def _bind() -> ctypes.CDLL:
     t.tc_mid, t.tc_mid_supported = _address(mid, "sp_tc_mid"), _address(mid, "sp_tc_mid_supported")
     t.err_tc_mid = _address(mid, "sp_tc_mid_last_error")
     t.gemv_tokens, t.stream_tokens, t.mid_tokens = L.GEMV_TOKENS, L.STREAM_TOKENS, L.MID_TOKENS
-    flash_tc = K.load("flash_tc")
-    t.flash_prefill_tc, t.err_flash_tc = _address(flash_tc, "sp_flash_prefill_tc"), _address(flash_tc, "sp_flash_tc_last_error")
+    if flash_tc:
+        tc = K.load("flash_tc")
+        t.flash_prefill_tc, t.err_flash_tc = _address(tc, "sp_flash_prefill_tc"), _address(tc, "sp_flash_tc_last_error")
     t.flash_query_tile, t.flash_tc_from = K.flash_query_tile(), FLASH_TC_TOKENS
     K._check("host_step", host.sp_host_step_bind(ctypes.byref(t), ctypes.sizeof(t)))
-    _bound = True
+    _bound = max(_bound, 1 + int(flash_tc))
     return host
 
 
@@ -161,9 +163,10 @@ class HostStep:
 
     def run(self, h: torch.Tensor, step, cache) -> None:
         """All layers on the residual stream ``h`` [T, H] (float32), in place."""
-        host = _bind()
         self.runs += 1
         T, dev, bf = step.n_tokens, h.device, torch.bfloat16
+        flash_tc = T >= FLASH_TC_TOKENS
+        host = _bind(flash_tc)
         # one buffer for the step's activations (bfloat16 except the unrounded QKV products)
         n_bf = T * (self.H + 2 * self.max_q + self.max_I)
         work = torch.empty(n_bf * 2 + T * self.max_qkv * 4 + 64, dtype=torch.uint8, device=dev)
@@ -200,9 +203,9 @@ class HostStep:
         st.status = K.status_word(dev).data_ptr()
         st.T, st.H, st.n_seqs, st.max_pages, st.page_size = T, self.H, step.n_seqs, pt.shape[1], cache.page_size
         st.n_q_tiles = K.query_tiles(step.host["new_counts"], K.flash_query_tile())
-        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream", "tc_mid", "flash_tc"):       # the debug build's bounds, library by library
+        for module in ("generic", "attention", "gemv", "tc_gemm", "tc_stream", "tc_mid") + (("flash_tc",) if flash_tc else ()):       # the debug build's bounds, library by library
             K._declare_bounds(module, K.load(module), cache.kv_groups[self.group].n_pages, pt.shape[0], dev)
-        if T >= FLASH_TC_TOKENS:
+        if flash_tc:
             st.n_tc_tiles, st.n_pages = K.query_tiles(step.host["new_counts"], K.flash_tc_query_tile()), cache.kv_groups[self.group].n_pages
         stream = K._stream()
         rc = host.sp_host_step_prompt_layers(self.layers, len(self.fields), ctypes.byref(st), c_void_p(stream))

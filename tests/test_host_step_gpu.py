@@ -5,7 +5,8 @@ import torch
 
 import tiny
 from spissa_b200 import Engine
-from spissa_b200.engine import pack_step
+from spissa_b200.csrc import lib as K
+from spissa_b200.engine import host_step, pack_step
 
 pytestmark = pytest.mark.gpu
 # gate and up rows in blocks of 128, head sizes 64 and 128
@@ -67,3 +68,16 @@ def test_the_first_step_does_not_wait_for_the_device(folders):
         torch.cuda.set_sync_debug_mode("default")
     tables = {r.inv_freq for r in engine.model._host_step.layers}
     assert len(tables) == 1                                                     # equal frequency tables are one
+
+
+
+def test_short_steps_ask_for_no_attention_of_long_ones(folders, monkeypatch):
+    asked, load = [], K.load
+    monkeypatch.setattr(K, "load", lambda m, *a, **k: (asked.append(m), load(m, *a, **k))[1])
+    monkeypatch.setattr(host_step, "_bound", 0)
+    engine = Engine.from_folder(folders[64], dtype="bfloat16", max_tokens=64 * 16)
+    s = engine.acquire()
+    engine.step([(s, tiny.random_prompt(777, 255, 1), [254])])
+    assert engine.model._host_step.runs == 1 and "flash_tc" not in asked
+    engine.step([(s, tiny.random_prompt(777, 256, 2), [255])])
+    assert engine.model._host_step.runs == 2 and "flash_tc" in asked
