@@ -14,6 +14,7 @@ step) runs as before.
 from __future__ import annotations
 
 import ctypes
+import weakref
 from ctypes import c_float, c_int, c_void_p
 
 import torch
@@ -98,7 +99,7 @@ class HostStep:
         self.fields = fields
         self.H = fields[0]["mixer"]["hidden_size"]
         self.runs = 0
-        self.cache_id = None
+        self.cache = lambda: None                        # (a weak reference to) the cache that ``layers`` describes
         self.layers = None
         self.keep = None
 
@@ -125,12 +126,12 @@ class HostStep:
         most = L.MID_TOKENS if self.can_fuse and self.mid and self.model.fuse_prefill else MAX_TOKENS
         if step.all_single or step.n_tokens > most or cache.page_size != K.flash_query_tile():
             return False
-        if self.cache_id != id(cache):
+        if self.cache() is not cache:
             self._bind_cache(cache)
         return self.layers is not None
 
     def _bind_cache(self, cache) -> None:
-        self.cache_id, self.layers = id(cache), None
+        self.cache, self.layers = weakref.ref(cache), None
         rows, keep, tables = [], [], {}
         for e, f, rope in zip(self.model.spec.schedule, self.fields, self.rope_id):
             g = cache.kv_groups.get(cache.cache_group.get(e.cache))

@@ -70,6 +70,15 @@ def test_the_first_step_does_not_wait_for_the_device(folders):
     assert len(tables) == 1                                                     # equal frequency tables are one
 
 
+def test_records_of_another_cache_are_made_anew(folders):
+    one, two = (Engine.from_folder(folders[64], dtype="bfloat16", max_tokens=64 * 8) for _ in range(2))
+    _, step = first_step(one, 100)
+    runner = one.model._host_step or (one.model._host_runner(step, one.cache) and one.model._host_step)
+    pools = [r.k_pool for r in runner.layers]
+    assert runner.takes(step, two.cache) and [r.k_pool for r in runner.layers] != pools
+    assert runner.takes(step, one.cache) and [r.k_pool for r in runner.layers] == pools
+    assert runner.cache() is one.cache                                          # the cache itself, not a number that another may get
+
 
 def test_short_steps_ask_for_no_attention_of_long_ones(folders, monkeypatch):
     asked, load = [], K.load
