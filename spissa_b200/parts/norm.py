@@ -41,6 +41,8 @@ class RMSNorm(Norm):
     def bind(self, tensors, rt):
         super().bind(tensors, rt)
         self.weight = tensors[self.weight_name].contiguous()
+        if self.weight.data_ptr() % 16:                                # a part of a larger buffer: kernels read it in whole pieces
+            self.weight = self.weight.clone()
         if self.around_zero:
             self.weight = (1.0 + self.weight.float()).contiguous()     # 32-bit: 1 + w rounded to 16 bits would lose w
         if self.weight_scale != 1.0:

@@ -90,3 +90,34 @@ def test_short_steps_ask_for_no_attention_of_long_ones(folders, monkeypatch):
     assert engine.model._host_step.runs == 1 and "flash_tc" not in asked
     engine.step([(s, tiny.random_prompt(777, 256, 2), [255])])
     assert engine.model._host_step.runs == 2 and "flash_tc" in asked
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_norm_weights_at_any_address(folders, hd):
+    """Weights that a program hands over as parts of one buffer, at odd places."""
+    import json
+    from pathlib import Path
+
+    from spissa_b200 import LlamaConfig
+    cfg = LlamaConfig.from_dict(json.loads((Path(folders[hd]) / "config.json").read_text()))
+    H = MODELS[hd][0]["hidden_size"]
+    g = torch.Generator(device="cuda:0").manual_seed(1)
+
+    def tensors():
+        probe = Engine.from_folder(folders[hd], dtype="bfloat16", max_tokens=64)
+        return {w.name: torch.empty(w.shape, device="cuda:0").normal_(0, 0.02, generator=g).bfloat16() for w in probe.model.weight_specs()}
+    plain = tensors()
+    odd = {}
+    for name, t in plain.items():
+        if t.dim() == 1:
+            room = torch.empty(H + 1, dtype=t.dtype, device=t.device)
+            room[1:] = t
+            t = room[1:]
+            assert t.data_ptr() % 4 == 2
+        odd[name] = t
+    rows = []
+    for weights in (plain, odd):
+        engine = Engine(cfg, weights, "bfloat16", 64 * 8, 2, "cuda:0")
+        s = engine.acquire()
+        rows.append([engine.step([(s, tiny.random_prompt(500, n, n), [n - 1])]).cpu() for n in (40, 200, 1)])
+    assert all(torch.isfinite(a).all() and torch.equal(a, b) for a, b in zip(*rows))
