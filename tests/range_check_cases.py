@@ -123,6 +123,36 @@ def main() -> int:
     assert code == 401 and bool((kp[bad] == 9.0).all())
     assert any(bool((kp[p] != 9.0).any()) for p in other)
 
+    # and of the one for steps of 17 to 1,023 tokens
+    assert K.range_checked("tc_mid")
+
+    def mid(declared):
+        kp = torch.full((wmeta.n_pages, nkv, 64, hd), 9.0, dtype=torch.bfloat16, device=DEV)
+        vp = torch.full_like(kp, -9.0)
+        rope = dict(cs=cs, tok_page=tok_page, positions=wmeta.positions, q_out=qo, k_pool=kp, v_pool=vp, nh=nh, nkv=nkv,
+                    hd=hd, page_size=64)
+        if declared is not None:
+            rope["declared_pages"] = declared
+        return code_of(lambda: K.tc_mid_fused(xw, w, None, K.TC_QKV_ROPE, 0, rope=rope)), kp
+    code, kp = mid(None)
+    assert code == 0
+    code, kp = mid(bad)
+    assert code == 401 and bool((kp[bad] == 9.0).all())
+    assert any(bool((kp[p] != 9.0).any()) for p in other)
+
+    # the 32-bit attention of prompts, by tiles
+    kp32, vp32 = (torch.ones(wmeta.n_pages, nkv, 64, hd, device=DEV) for _ in range(2))
+    q32, out32 = torch.randn(T, nh * hd, device=DEV), torch.empty(T, nh * hd, device=DEV)
+
+    def tiles():
+        K.attention_tile_f32(q32, kp32, vp32, out32, wmeta, wmeta.seq_start, len(new_counts), max(new_counts), nh, nkv, hd, None, scale)
+    assert code_of(tiles) == 0
+    wmeta.declared_pages = bad
+    assert code_of(tiles) == 401
+    wmeta.declared_pages, wmeta.declared_rows = None, 1
+    assert code_of(tiles) == 402
+    wmeta.declared_rows = None
+
     # key and value rows of two sizes: the decode attention's table, and the kernels that place q, k and v head by head
     d, vd = 40, 24
     assert K.range_checked("attention_kv") and K.range_checked("sandwich")
