@@ -167,7 +167,7 @@ def gemm_generic(a, w, out, accumulate=False):
 
 
 def tc_f32_supported(a, w, out) -> bool:
-    """Whether ``tc_f32`` takes these operands (float32, unit strides, rows a multiple of 16 bytes)."""
+    """Whether ``tc_f32`` takes these operands (float32, unit strides, rows a multiple of 32 bytes and on such boundaries)."""
     if not (a.dtype == w.dtype == out.dtype == torch.float32) or a.dim() != 2 or w.dim() != 2 or a.shape[1] != w.shape[1]:
         return False
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:

@@ -5,10 +5,14 @@
 // itself (74 TFLOP/s) is a twentieth of the bfloat16 rate. A float32 has 24 significant bits, a bfloat16 8 and the same
 // exponents, so x = x1 + x2 + x3 exactly, each part the leading 8 bits of what the parts before leave (cut off, not rounded:
 // the differences are exact). Of the nine products of parts the six largest are computed, a1w1, a1w2, a2w1, a1w3, a2w2,
-// a3w1; the three left out are together below 2^-23 of |a||w| in the worst case and 2^-25 on average, what one float32
-// rounding of the product would cost. Products of 8-bit parts are exact; the tensor core adds them into a float32 accumulator
-// and truncates, so an accumulator holds 64 terms of K only: then it is added to a float32 sum in registers, rounded to
-// nearest. Against 64 bits the result is nearer than a float32 sum in order (tests/test_tc_f32_gpu.py measures both).
+// a3w1; the three left out have the product's own sign and are together below 2^-21 of |a||w| (|a2| < 2^-7 |a|, |a3| <
+// 2^-15 |a|) and 2^-24.5 of it on average. Products of 8-bit parts are exact; the tensor core adds them into a float32
+// accumulator and truncates, so an accumulator holds 64 terms of K only: then it is added to a float32 sum in registers,
+// rounded to nearest. Both losses are toward zero, so they add up where all terms have one sign: 1.2e-7 of the result, for
+// any K. Even so the result is nearer to 64 bits than a float32 sum in order (relative error, this / in order, operands of one
+// sign: K = 128 1.27e-7 / 1.64e-7, 2,048 1.28e-7 / 6.6e-7; of both signs 1.28e-7 / 2.0e-7 and 1.4e-7 / 8.1e-7;
+// tests/test_f32_path_gpu.py holds it to that). Parts below 2^-126 have fewer bits: a term loses up to 2^-133 times its other
+// factor, which is beyond the 24th bit of values from 2^-109 on.
 // A value that is not finite has no such parts: a CTA that meets one computes its tile again with plain FFMA.
 //
 //   warps 0-15  split, block of 64 of K by block, 128 x 64 of W and tokens x 64 of A (fetched a block ahead into registers, 32

@@ -33,9 +33,9 @@ def test_product_against_64_bits(K, M, N, Kd):
     assert K.tc_f32_supported(a, w, out)
     K.tc_f32(a, w, out)
     K.gemm_generic(a, w, ffma)
-    # the three products of parts left out are below 3 · 2^-24 of |a||w|; a block of 64 terms takes 24 additions that truncate
+    # the three products of parts left out are below 2^-21 of |a||w|; a block of 64 terms takes 24 additions that truncate
     # (2^-23 each of what has been added up so far), and K / 64 sums that round
-    bound = (3 * 2.0 ** -24 + 24 * 2.0 ** -23 + (Kd / 64 + 1) * 2.0 ** -24) * size
+    bound = (2.0 ** -21 + 24 * 2.0 ** -23 + (Kd / 64 + 1) * 2.0 ** -24) * size
     assert bool(((out.double() - ref).abs() <= bound).all())
     if Kd >= 128 and M * N > 1000:
         assert float((out.double() - ref).norm()) <= float((ffma.double() - ref).norm())
@@ -191,3 +191,36 @@ def test_distances_that_a_bias_rules_out(K, window):
         heads.append(torch.softmax(s, dim=-1) @ v[:, 0].double())
     ref = torch.cat(heads, dim=-1)
     assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("M", [24, 500])
+@pytest.mark.parametrize("Kd", [128, 192, 512, 2048])
+@pytest.mark.parametrize("kind", ["uniform", "exponential", "all bits"])
+def test_product_of_one_sign_is_as_near_as_ffma(K, M, Kd, kind):
+    """What the parts leave out and what the accumulator cuts off goes toward zero: operands of one sign add it all up."""
+    torch.manual_seed(Kd + M)
+    if kind == "uniform":
+        a, w = torch.rand(M, Kd, device=DEV), torch.rand(520, Kd, device=DEV)
+    elif kind == "exponential":
+        a, w = torch.empty(M, Kd, device=DEV).exponential_(), torch.empty(520, Kd, device=DEV).exponential_()
+    else:                                                               # every part as large as it can be: 2^-21 is left out
+        a, w = (torch.full((n, Kd), 1 + 2.0 ** -7 - 2.0 ** -23, device=DEV) for n in (M, 520))
+    out, ffma = (torch.empty(M, 520, device=DEV) for _ in range(2))
+    K.tc_f32(a, w, out)
+    K.gemm_generic(a, w, ffma)
+    ref = a.double() @ w.double().t()
+    err = (out.double() - ref).abs()
+    assert bool((err <= (2.0 ** -21 + 24 * 2.0 ** -23 + (Kd / 64 + 1) * 2.0 ** -24) * ref).all())
+    if kind != "all bits":
+        assert float(err.norm()) <= float((ffma.double() - ref).norm())
+
+
+@pytest.mark.parametrize("size", [1e-33, 1e-36, 1e-38])
+def test_values_whose_parts_run_out_of_exponents(K, size):
+    a, w = operands(40, 130, 256)
+    a *= size
+    out = torch.empty(40, 130, device=DEV)
+    K.tc_f32(a, w, out)
+    ref, terms = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = (2.0 ** -21 + 24 * 2.0 ** -23 + 5 * 2.0 ** -24) * terms + 2.0 ** -133 * w.double().abs().sum(1) + 2.0 ** -145
+    assert bool(((out.double() - ref).abs() <= bound).all())
