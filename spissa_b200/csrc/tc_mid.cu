@@ -101,35 +101,30 @@ __device__ __forceinline__ float quotient(float x, float d) {
 // ordinary size (all of them, in earnest) go through without a branch on one value, so that the 32 overlap. 301 tokens x
 // 16,384 x 2,048: 27.3 us, 32.0 with the general quotient, 40 with a branch on the activation around each value.
 template <int KIND>
-__device__ __forceinline__ void activate(uint32_t (&rg)[32], const uint32_t (&ru)[32], const float* rstd, int n, SpGate ga) {
+__device__ __forceinline__ void activate(uint32_t (&rg)[32], uint32_t (&ru)[32], const float* rstd, int n, SpGate ga) {
     ga.kind = KIND;
     const float slope = KIND == SP_ACT_CLAMPED ? ga.slope : 1.0f;
     float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};                     // (NaN is left out: the quotient is NaN either way)
-    if (KIND != SP_ACT_GELU) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            float g = __uint_as_float(rg[j]) * rstd[j];
-            if (KIND == SP_ACT_CLAMPED) g = fminf(g, ga.limit);
-            top[j & 3] = fmaxf(top[j & 3], j < n ? fabsf(slope * g) : 0.0f);
-        }
+    for (int j = 0; j < 32; ++j) {
+        float g = __uint_as_float(rg[j]) * rstd[j];
+        if (KIND == SP_ACT_CLAMPED) g = fminf(g, ga.limit);
+        top[j & 3] = fmaxf(top[j & 3], j < n ? fabsf(slope * g) : 0.0f);
+        rg[j] = __float_as_uint(g);
+        ru[j] = __float_as_uint(__uint_as_float(ru[j]) * rstd[j]);
     }
     if (KIND != SP_ACT_GELU && __all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= 60.0f)) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-            float g = __uint_as_float(rg[j]) * rstd[j], u = __uint_as_float(ru[j]) * rstd[j];
-            if (KIND == SP_ACT_CLAMPED) {
-                g = fminf(g, ga.limit);
-                u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
-            }
+            const float g = __uint_as_float(rg[j]);
+            float u = __uint_as_float(ru[j]);
+            if (KIND == SP_ACT_CLAMPED) u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
             rg[j] = __float_as_uint(quotient(g, 1.0f + expf(-slope * g)) * u * ga.mult);
         }
         return;
     }
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        const float rs = rstd[j];
-        rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]) * rs, __uint_as_float(ru[j]) * rs, ga));
-    }
+    for (int j = 0; j < 32; ++j) rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]), __uint_as_float(ru[j]), ga));
 }
 
 // The second part of the epilogue: a warp owns a token at a time (``first``, then every eighth below ``end``), a lane four
