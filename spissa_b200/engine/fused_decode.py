@@ -20,16 +20,18 @@ MAX_TOKENS = 16
 
 
 def five_launch_from(layer_bytes: float) -> int:
-    """The number of sequences from which a decode step is faster as the five-launch sequence of the weight-streaming
-    tcgen05 product (``engine/fused_prefill.py``) than in this kernel, by the bytes of a layer's weights. Measured on a
-    B200, decode step in ms, this kernel / five launches:
+    """The number of sequences from which a decode step runs as the five-launch sequence of the tcgen05 products
+    (``engine/fused_prefill.py``) and not in this kernel, by the bytes of a layer's weights. Measured on a B200 with some
+    1,000 keys a sequence, a decode step in us, this kernel / five launches of ``tc_mid`` / five of ``tc_stream``:
 
-        1B layers, 122 MB (width 2048, head 64):   8 sequences 0.95 / 1.14,  16: 1.09 / 1.37
-        3B layers, 201 MB (width 3072, head 128):  2: 2.21 / 2.08,  4: 2.32 / 2.26,  6: 2.44 / 2.35,  8: 2.57 / 2.38,
-                                                   12: 2.87 / 2.73,  16: 3.06 / 2.87
-        8B layers, 436 MB (width 4096, head 128):  4: 3.93 / 4.01,  6: 4.11 / 4.15,  7: 4.30 / 4.39,  8: 4.7 / 4.21,
-                                                   9: 4.54 / 4.45,  12: 5.17 / 4.84,  16: 6.4 / 5.06
+        8 1B layers, 122 MB each (width 2048, head 64):   2 sequences 373 / 458 / 465,  8: 399 / 480 / 496,  16: 455 / 539 / 555
+        8 3B layers, 201 MB (width 3072, head 128):       2: 601 / 579 / 580,  4: 641 / 583 / 590,  8: 697 / 600 / 607,
+                                                          12: 785 / 635 / 646,  16: 836 / 667 / 686
+        4 8B layers, 436 MB (width 4096, head 128):       2: 468 / 458 / 470,  4: 489 / 467 / 486,  7: 517 / 479 / 502,
+                                                          8: 525 / 475 / 498,  12: 601 / 510 / 519,  16: 672 / 529 / 548
 
+    The 8B line was drawn on ``tc_stream`` and 32 layers (7 sequences 4.30 ms / 4.39, 8: 4.7 / 4.21); ``tc_mid`` is the
+    faster one there from 2 sequences on, by 2 to 7 % below the line.
     The kernel's products walk blocks of 16 rows dealt to 148 CTAs; the 3B widths leave many CTAs a round short (192
     blocks: two rounds for 44 of them), and with more than 8 tokens it keeps 16 rows of normed activations in shared
     memory (128 KB at width 4096: two ring stages are left of four) and one tile's fragments in flight instead of two.

@@ -77,7 +77,7 @@ def test_short_prompts_run_from_cpp_and_other_models_part_by_part(folders):
 
 @pytest.mark.parametrize("name", ["E", "F"])
 def test_short_prompt_steps_through_the_host_runner_equal_the_parts_bit_for_bit(folders, name):
-    """Up to 128 tokens the layers' launch sequence runs as one call into C++ (csrc/host_step.cu): the same kernels
+    """The layers' launch sequence as one call into C++ (csrc/host_step.cu; from 129 tokens on in test_host_step_gpu): the same kernels
     with the same arguments as from Python (part by part up to 16 tokens, the fused sequence from 17), so not a bit
     may differ; ragged batches and prompts that continue."""
     folder, pcfg, w = folders[name]
