@@ -158,24 +158,25 @@ __device__ __forceinline__ void sp_wait_for_predecessor() { asm volatile("gridde
 // What a predecessor writes is loaded behind the wait by an ordinary load that stays there. A read-only load (__ldg, .nc, or
 // what the compiler makes of a ``const __restrict__`` parameter) is for memory that nothing writes while the kernel is
 // resident, which a dependent kernel is from before its predecessor's end; and the compiler may move it ahead of the wait.
+// (Volatile, so that it stays behind the wait; no memory clobber, so that several are under way while others are stored.)
 __device__ __forceinline__ float sp_ld_written(const float* p) {
     float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ int sp_ld_written(const int* p) {
     int v;
-    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float2 sp_ld_written(const float2* p) {
     float2 v;
-    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float4 sp_ld_written(const float4* p) {
     float4 v;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
 

@@ -286,18 +286,27 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 // a CTA of four warps owns eight rows of W (two per warp), the rows of A pass through shared memory in slices of
 // 512 columns. What bounds it is bytes in flight: the next slice of W (and up to 4 rows of A) is asked for before the
 // products of this one, and the kernel may become resident before its predecessor ends (so A, which that one writes, is not
-// read by read-only loads). Each lane sums its columns
+// read by read-only loads). For 9 to 16 rows the second slice took the registers that five CTAs on an SM need instead: four
+// layers of the 1B shape, a step of 12 / 16 sequences 1,492 / 1,581 us with it, 1,243 / 1,336 without (6 / 8: 684 / 706 with
+// it, 749 / 771 without). Each lane sums its columns
 // k = 4·lane + 128·i in order, the lanes' sums are added by a shuffle tree: the order is fixed and the same for every row
 // of A, whatever M is, but it is another order than the tiled kernel's, so a token's result differs between a decode step
 // and a prompt step by 32-bit rounding.
 #define GS_KC 512
 #define GS_ROWS 2
+// 16 bytes, or zeros where not ``ok``; under a predicate, so that the loads of a slice go out side by side.
+__device__ __forceinline__ float4 gs_load(const float* p, bool ok) {
+    float4 v;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                 "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}" : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(p), "r"((int)ok));
+    return v;
+}
 template <int MT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, MT == 16 ? 5 : MT == 8 ? 3 : 4)
 gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
                        int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
     constexpr int XV = MT * (GS_KC / 4) / 128;               // 16-byte pieces of a slice of A per thread
-    constexpr bool XAHEAD = MT <= 4;                         // held in registers a slice ahead
+    constexpr bool XAHEAD = MT <= 4, WAHEAD = MT <= 8, PRED = MT == 16;      // AHEAD: held in registers a slice ahead
     __shared__ __align__(16) float xs[MT][GS_KC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * 4 + warp) * GS_ROWS;
@@ -309,7 +318,7 @@ gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
     const float* wrow[GS_ROWS];
 #pragma unroll
     for (int r = 0; r < GS_ROWS; ++r) wrow[r] = W + (size_t)min(n0 + r, N - 1) * ldw;
-    float4 w[2][GS_ROWS][GS_KC / 128], x_next[XAHEAD ? XV : 1];
+    float4 w[WAHEAD ? 2 : 1][GS_ROWS][GS_KC / 128], x_next[XAHEAD ? XV : 1];
     auto load_w = [&](int k0, float4 (&to)[GS_ROWS][GS_KC / 128]) {
 #pragma unroll
         for (int r = 0; r < GS_ROWS; ++r)
@@ -319,24 +328,28 @@ gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
                 to[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (k < K)
                     asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                 : "=f"(to[r][i].x), "=f"(to[r][i].y), "=f"(to[r][i].z), "=f"(to[r][i].w) : "l"(wrow[r] + k) : "memory");
+                                 : "=f"(to[r][i].x), "=f"(to[r][i].y), "=f"(to[r][i].z), "=f"(to[r][i].w) : "l"(wrow[r] + k));
             }
     };
     auto load_x = [&](int k0, int v) {
         const int e = threadIdx.x + 128 * v, m = e / (GS_KC / 4), c = (e % (GS_KC / 4)) * 4;
-        return m < M && k0 + c < K ? sp_ld_written((const float4*)(A + (size_t)m * lda + k0 + c)) : make_float4(0.f, 0.f, 0.f, 0.f);     // K is a multiple of 4
+        const float* p = A + (size_t)m * lda + k0 + c;
+        const bool ok = m < M && k0 + c < K;                 // K is a multiple of 4
+        if constexpr (PRED) return gs_load(p, ok);
+        else return ok ? sp_ld_written((const float4*)p) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     auto slice = [&](int k0, auto turn) {
-        constexpr int b = decltype(turn)::value;
+        constexpr int b = WAHEAD ? decltype(turn)::value : 0;
         __syncthreads();                                     // the slice before has been used by every warp
-#pragma unroll
+#pragma unroll(MT == 16 ? 4 : XV)
         for (int v = 0; v < XV; ++v) {
             const int e = threadIdx.x + 128 * v;
             *(float4*)&xs[e / (GS_KC / 4)][(e % (GS_KC / 4)) * 4] = XAHEAD ? x_next[XAHEAD ? v : 0] : load_x(k0, v);
         }
         __syncthreads();
-        if (k0 + GS_KC < K) {
-            load_w(k0 + GS_KC, w[b ^ 1]);
+        if (!WAHEAD) load_w(k0, w[0]);
+        if (WAHEAD && k0 + GS_KC < K) {
+            load_w(k0 + GS_KC, w[WAHEAD ? b ^ 1 : 0]);
             if (XAHEAD) {
 #pragma unroll
                 for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(k0 + GS_KC, v);
@@ -358,7 +371,7 @@ gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
     };
     sp_allow_dependents();
     sp_wait_for_predecessor();
-    load_w(0, w[0]);
+    if (WAHEAD) load_w(0, w[0]);
     if (XAHEAD) {
 #pragma unroll
         for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(0, v);
