@@ -287,7 +287,7 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 // 512 columns. What bounds it is bytes in flight: the next slice of W (and up to 4 rows of A) is asked for before the
 // products of this one, and the kernel may become resident before its predecessor ends (so A, which that one writes, is not
 // read by read-only loads). For 9 to 16 rows the second slice took the registers that five CTAs on an SM need instead: four
-// layers of the 1B shape, a step of 12 / 16 sequences 1,492 / 1,581 us with it, 1,243 / 1,336 without (6 / 8: 684 / 706 with
+// layers of the 1B shape, a step of 12 / 16 sequences 1,492 / 1,581 us with it, 1,243 / 1,336 without (6 / 8: 696 / 718 with
 // it, 749 / 771 without). Each lane sums its columns
 // k = 4·lane + 128·i in order, the lanes' sums are added by a shuffle tree: the order is fixed and the same for every row
 // of A, whatever M is, but it is another order than the tiled kernel's, so a token's result differs between a decode step
