@@ -20,11 +20,14 @@
 // Finding the token by that descent alone took some twenty passes of three microseconds (8 rows of 128,256 logits: 80 us).
 // Now one pass adds every token into one of 4,065 buckets, by the upper 14 bits of its probability (sign, exponent and five
 // bits of the mantissa); a bucket's count and the sum of its tokens' lower 18 bits give its exact mass. The buckets' running
-// totals stay in the cluster's shared memory for every question asked of the row; the tokens of the one bucket in which a
-// target is reached are gathered and compared with one another by all CTAs: 39 us (58 with one CTA comparing; what is
-// left are the barriers of the cluster, the softmax and the adding into buckets). Only where more than 1,024 tokens share
+// totals stay in the cluster's shared memory for every question asked of the row, and each group of sixteen's in every CTA's:
+// a question finds its bucket with one look at another CTA, the bucket's tokens go to all CTAs at once, each at a place that
+// the counts have set aside, and behind that one barrier of the cluster every CTA finds the token among them for itself,
+// by bins of the next ten bits. 8 rows 25 us (38 with the tokens gathered in one CTA and compared with one another by all,
+// which took three trips between the CTAs and two barriers a question), 64 rows 101 (129), 64 of 32,000 37 (41). What is
+// left are five barriers of the cluster, the softmax and the adding into buckets. Only where more than 1,024 tokens share
 // the bucket (rows of nearly equal probabilities) the descent runs, from the three digits of the key that the bucket fixes
-// (8 rows, top_k 50: logits N(0, 0.5) 27 us, by the descent from its first digit 55; all tokens equal 131 and 129:
+// (8 rows, top_k 50: logits N(0, 0.5) 23 us, by the descent from its first digit 55; all tokens equal 131 and 129:
 // there a vote in front of the adding saves 12 us, which costs every other row 2).
 //
 // Sums are integers: a probability counts as floor(p · 2^44) and a token as 1 in the high bits of the same
@@ -65,10 +68,8 @@ __device__ __forceinline__ unsigned long long ss_ld_peer_u64(const void* local, 
     asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(ss_peer_addr(local, rank)) : "memory");
     return v;
 }
-__device__ __forceinline__ float ss_ld_peer_f32(const void* local, unsigned rank) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ss_peer_addr(local, rank)) : "memory");
-    return v;
+__device__ __forceinline__ void ss_st_peer_f32(const void* local, unsigned rank, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ss_peer_addr(local, rank)), "f"(v) : "memory");
 }
 
 __device__ __forceinline__ unsigned long long ss_key(unsigned prob_bits, unsigned idx) {
@@ -88,7 +89,7 @@ struct Shared {
     unsigned long long seg[2][SS_SEGS];            // this CTA's sums of a pass (two buffers: peers read one while the next fills)
     unsigned long long total[SS_SEGS];             // the cluster's sums
     unsigned long long loc;                        // this CTA's find of a lookup (0: none)
-    float stat[2];                                 // this CTA's maximum / sum of exponentials
+    float stat[2][SS_CLUSTER];                     // the CTAs' maxima / sums of exponentials
     float red[32];
 };
 
@@ -198,18 +199,26 @@ constexpr int BK_PER = BK_N / SS_CLUSTER;          // positions (buckets by fall
 constexpr int BK_LIST = 1024;                      // tokens of a bucket that are compared with one another
 constexpr unsigned BK_CARRY = 1u << 20;            // in a bucket's count: its sum of lower bits has passed 2^32 (a slice has less than 2^20 tokens)
 
-// In dynamic shared memory, in the place of the descent's words.
+constexpr int BK_GROUP = 16;                       // positions (buckets by falling probability) whose total every CTA knows
+constexpr int BK_GROUPS = BK_N / BK_GROUP;
+constexpr int RF_BINS = 1024;                      // bins by which a list is searched
+// In dynamic shared memory, in the place of the descent's words (which spoils them for the questions that follow).
+struct Search {
+    unsigned long long list[BK_LIST];              // a bucket's keys
+    unsigned bin_count[RF_BINS], bin_low[RF_BINS];
+};
 struct Lists {
-    union { unsigned count[BK_N]; unsigned long long list[BK_LIST]; };         // this CTA's tokens of each bucket; later the gathered keys
-    union { unsigned low[BK_N]; unsigned long long weight[BK_LIST]; };         // their lower bits' contributions; later what the gathered tokens weigh
+    unsigned count[BK_N];                          // this CTA's tokens of each bucket; later the place of the first of them in the bucket's list
+    union { unsigned low[BK_N]; Search find; };    // their lower bits' contributions; later what a question needs
 };
 struct Buckets {
     unsigned long long scan[BK_PER];               // running totals (count and mass packed) of this CTA's positions
+    unsigned long long groups[BK_GROUPS];          // running totals at the end of each group, from the first position of its CTA on
     unsigned long long warp_total[32];
-    unsigned long long total;                      // of this CTA's positions
-    unsigned long long key, upto;                  // in CTA 0: the result
-    unsigned long long below, through;             // running totals before and through the bucket
-    int position, n_list[4];                       // (a list's length has a word for each question: none has to be set back)
+    unsigned long long below, through;             // running totals before and through what was chosen
+    unsigned long long key;
+    int chosen, alone;
+    int n_list[4], n_spoilt[4];                    // (a list's length has a word for each question: none has to be set back)
 };
 
 // What the lower 18 bits of a probability add to its mass, in the bucket's own unit (see bk_mass).
@@ -228,11 +237,15 @@ __device__ __forceinline__ unsigned long long bk_mass(int bucket, unsigned long 
     if (down <= BK_SHIFT) return (count * H << (BK_SHIFT - down)) + low;
     return down < 24 ? count * (H >> (down - BK_SHIFT)) : 0ull;
 }
+__device__ __forceinline__ unsigned long long bk_total(int bucket, unsigned long long count, unsigned long long low) {
+    return (count << MASS_BITS) + bk_mass(bucket, count, low);
+}
 __device__ __forceinline__ bool bk_reached(unsigned long long total, bool by_mass, unsigned long long target) {
     return total >= ONE_TOKEN && (by_mass ? (total & MASS_MASK) : (total >> MASS_BITS)) >= target;
 }
 
-// Every CTA: its slice into buckets, then the running totals of its 512 positions of the row's buckets.
+// Every CTA: its slice into buckets, then the running totals of its 512 positions of the row's buckets. What the questions
+// need of them goes to every CTA at once: the groups' totals, and where in a bucket's list each CTA's own tokens begin.
 template <int THREADS>
 __device__ void bk_fill(Buckets* bk, Lists* li, const Row& row) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -258,16 +271,21 @@ __device__ void bk_fill(Buckets* bk, Lists* li, const Row& row) {
         part[i] = 0ull;
         const int pos = rank * BK_PER + tid * MINE + i, bucket = BK_N - 1 - pos;
         if (tid * MINE < BK_PER) {
-            unsigned long long count = 0ull, low = 0ull;
+            unsigned c[SS_CLUSTER], l[SS_CLUSTER];
 #pragma unroll
             for (unsigned r = 0; r < SS_CLUSTER; ++r) {
-                unsigned c, l;
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c) : "r"(ss_peer_addr(&li->count[bucket], r)) : "memory");
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(l) : "r"(ss_peer_addr(&li->low[bucket], r)) : "memory");
-                count += c & (BK_CARRY - 1u);
-                low += l + ((unsigned long long)(c / BK_CARRY) << 32);
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c[r]) : "r"(ss_peer_addr(&li->count[bucket], r)) : "memory");
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(l[r]) : "r"(ss_peer_addr(&li->low[bucket], r)) : "memory");
             }
-            part[i] = (count << MASS_BITS) + bk_mass(bucket, count, low);
+            unsigned count = 0u;
+            unsigned long long low = 0ull;
+#pragma unroll
+            for (unsigned r = 0; r < SS_CLUSTER; ++r) {                // nobody else reads or writes this bucket's words here
+                if (c[r]) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ss_peer_addr(&li->count[bucket], r)), "r"(count) : "memory");
+                count += c[r] & (BK_CARRY - 1u);
+                low += l[r] + ((unsigned long long)(c[r] / BK_CARRY) << 32);
+            }
+            part[i] = bk_total(bucket, count, low);
         }
         run += part[i];
     }
@@ -281,101 +299,184 @@ __device__ void bk_fill(Buckets* bk, Lists* li, const Row& row) {
     if (lane == 31) bk->warp_total[warp] = up;
     __syncthreads();
     unsigned long long before = up - run;
-    for (int w = 0; w < warp; ++w) before += bk->warp_total[w];
+    for (int w = 0; w < warp && w < BK_PER / MINE / 32; ++w) before += bk->warp_total[w];
 #pragma unroll
     for (int i = 0; i < MINE; ++i) {
         before += part[i];
-        if (tid * MINE < BK_PER) bk->scan[tid * MINE + i] = before;
+        const int p = tid * MINE + i;
+        if (p < BK_PER) {
+            bk->scan[p] = before;
+            if ((p & (BK_GROUP - 1)) == BK_GROUP - 1) {
+#pragma unroll
+                for (unsigned r = 0; r < SS_CLUSTER; ++r)
+                    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->groups[(rank * BK_PER + p) / BK_GROUP], r)), "l"(before) : "memory");
+            }
+        }
     }
-    if (tid == THREADS - 1) bk->total = before;
     __syncthreads();
     ss_cluster_sync();                                                 // the counts are not read any more
 }
 
+// The first key (rising) among the ``m`` keys of a list, all of ``bucket``, at which the running total from ``below`` on reaches
+// the target, and the total up to and including it. A CTA searches for itself: the keys fall into bins by the next bits of the
+// key, the bins' running totals tell which one holds the boundary, and its keys go on to the next bits until one is left (for
+// most lists that is the first or the second pass; equal probabilities go on to the bits of their index). Arrives at the
+// cluster's barrier as soon as the keys are in registers: the next list may then be written.
+template <int THREADS>
+__device__ void bk_refine(Buckets* bk, Search* se, int m, int bucket, bool by_mass, unsigned long long target,
+                          unsigned long long below, unsigned long long& key, unsigned long long& upto) {
+    constexpr int PER = BK_LIST / THREADS, BINS = RF_BINS / THREADS;   // keys and bins of a thread
+    static_assert(PER >= 1 && BINS >= 1, "at most 1,024 threads");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long mine[PER];
+    bool in[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        in[i] = tid + THREADS * i < m;
+        mine[i] = in[i] ? se->list[tid + THREADS * i] : 0ull;
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // digits of a key below its bucket: 10 and 8 bits of the probability, 10 and 9 of the index
+#pragma unroll 1
+    for (int d = 0; d < 4; ++d) {
+        const int shift = d == 0 ? 40 : d == 1 ? 32 : d == 2 ? 9 : 0;
+        const unsigned mask = d == 0 || d == 2 ? 1023u : d == 1 ? 255u : 511u;
+#pragma unroll
+        for (int i = 0; i < BINS; ++i) se->bin_count[tid * BINS + i] = se->bin_low[tid * BINS + i] = 0u;
+        __syncthreads();
+        unsigned bin[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            bin[i] = (unsigned)(mine[i] >> shift) & mask;
+            if (in[i]) {
+                atomicAdd(&se->bin_count[bin[i]], 1u);
+                const unsigned low = bk_low(~(unsigned)(mine[i] >> 32));
+                if (low) atomicAdd(&se->bin_low[bin[i]], low);
+            }
+        }
+        __syncthreads();
+        // running counts and sums (1,024 keys of 18 bits: both fit 32 bits; scanned as one word)
+        unsigned long long part[BINS], run = 0ull;
+#pragma unroll
+        for (int i = 0; i < BINS; ++i) {
+            part[i] = ((unsigned long long)se->bin_count[tid * BINS + i] << 32) | se->bin_low[tid * BINS + i];
+            run += part[i];
+        }
+        unsigned long long up = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long v = __shfl_up_sync(0xffffffffu, up, o);
+            if (lane >= o) up += v;
+        }
+        if (lane == 31) bk->warp_total[warp] = up;
+        __syncthreads();
+        unsigned long long before = up - run, t = lane < THREADS / 32 && lane < warp ? bk->warp_total[lane] : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        before += t;
+#pragma unroll
+        for (int i = 0; i < BINS; ++i) {
+            const unsigned long long after = before + part[i];
+            if (part[i] >> 32) {
+                const unsigned long long with = below + bk_total(bucket, after >> 32, after & 0xffffffffull);
+                const unsigned long long without = below + bk_total(bucket, before >> 32, before & 0xffffffffull);
+                if (bk_reached(with, by_mass, target) && !bk_reached(without, by_mass, target)) {
+                    bk->chosen = tid * BINS + i;                       // one bin
+                    bk->alone = part[i] >> 32 == 1ull;
+                    bk->below = without;
+                    bk->through = with;
+                }
+            }
+            before = after;
+        }
+        __syncthreads();
+        const unsigned chosen = (unsigned)bk->chosen;
+        const bool last = bk->alone || d == 3;
+        below = bk->below;
+        upto = bk->through;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            in[i] = in[i] && bin[i] == chosen;
+            if (last && in[i]) bk->key = mine[i];                      // keys are unique: one thread
+        }
+        if (last) break;
+    }
+    __syncthreads();
+    key = bk->key;
+}
+
 // The token at which the running count or mass reaches ``target``, among all of the row: its key, and the packed total up to
 // and including it. False when even the total does not (``upto``: the total). Every CTA alike. ``question``: 0, 1, ... within
-// a row.
+// a row. ``spoilt``: a descent has overwritten where the CTAs' tokens begin in a list. ``arrived``: at the cluster's barrier, for
+// which is waited before it is used again.
 template <int THREADS>
 __device__ bool bk_find(Shared* sh, Buckets* bk, Lists* li, const Row& row, int question, bool by_mass, unsigned long long target,
-                        unsigned& parity, unsigned long long& key, unsigned long long& upto) {
-    const int tid = threadIdx.x;
-    unsigned long long base = 0ull, totals[SS_CLUSTER];
+                        unsigned& parity, bool& spoilt, bool& arrived, unsigned long long& key, unsigned long long& upto) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER_CTA = BK_GROUPS / SS_CLUSTER;                    // groups of a CTA: one for each lane of a warp
+    static_assert(PER_CTA == 32 && THREADS >= BK_GROUPS, "a warp looks at the groups of one CTA");
+    unsigned long long total = 0ull;
 #pragma unroll
-    for (unsigned r = 0; r < SS_CLUSTER; ++r) totals[r] = ss_ld_peer_u64(&bk->total, r);
-    int owner = -1;
-#pragma unroll
-    for (int r = 0; r < SS_CLUSTER; ++r)
-        if (owner < 0) {
-            if (bk_reached(base + totals[r], by_mass, target)) owner = r;
-            else base += totals[r];
-        }
-    if (owner < 0) { upto = base; return false; }
-    for (int i = tid; i < BK_PER; i += THREADS) {
-        const unsigned long long with = base + ss_ld_peer_u64(&bk->scan[i], (unsigned)owner);
-        const unsigned long long without = base + (i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull);
-        if (bk_reached(with, by_mass, target) && !bk_reached(without, by_mass, target)) {        // one position
-            bk->position = owner * BK_PER + i;
-            bk->below = without;
-            bk->through = with;
+    for (int r = 0; r < SS_CLUSTER; ++r) total += bk->groups[r * PER_CTA + PER_CTA - 1];
+    if (!bk_reached(total, by_mass, target)) { upto = total; return false; }
+    if (warp < SS_CLUSTER) {
+        unsigned long long base = 0ull;
+        for (int r = 0; r < warp; ++r) base += bk->groups[r * PER_CTA + PER_CTA - 1];
+        const unsigned long long with = base + bk->groups[tid];
+        const unsigned long long without = base + (lane ? bk->groups[tid - 1] : 0ull);
+        const unsigned here = __ballot_sync(0xffffffffu, bk_reached(with, by_mass, target) && !bk_reached(without, by_mass, target));
+        if (here) {                                                    // one warp: the group's positions, from the CTA that has them
+            const int group = warp * PER_CTA + __ffs(here) - 1;
+            const unsigned long long before = __shfl_sync(0xffffffffu, without, __ffs(here) - 1);
+            const int pos = group * BK_GROUP + lane;
+            unsigned long long w = lane < BK_GROUP ? base + ss_ld_peer_u64(&bk->scan[pos % BK_PER], (unsigned)warp) : 0ull;
+            unsigned long long wo = __shfl_up_sync(0xffffffffu, w, 1);
+            if (lane == 0) wo = before;
+            if (lane < BK_GROUP && bk_reached(w, by_mass, target) && !bk_reached(wo, by_mass, target)) {         // one lane
+                bk->chosen = pos;
+                bk->below = wo;
+                bk->through = w;
+            }
         }
     }
     __syncthreads();
-    const unsigned bucket = (unsigned)(BK_N - 1 - bk->position);
+    const int position = bk->chosen;
+    const unsigned bucket = (unsigned)(BK_N - 1 - position);
     const unsigned long long below = bk->below;
     const unsigned long long n_in = (bk->through - below) >> MASS_BITS;
+    if (arrived) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    arrived = false;
     if (n_in > BK_LIST) {
         // from the first of the four buckets that share the key's first SS_KNOWN digits
-        const int first = bk->position & ~3, i = first - owner * BK_PER;
-        const unsigned long long before = base + (i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull);
+        const int first = position & ~3, owner = first / BK_PER, i = first % BK_PER;
+        unsigned long long before = i ? ss_ld_peer_u64(&bk->scan[i - 1], (unsigned)owner) : 0ull;
+        for (int r = 0; r < owner; ++r) before += bk->groups[r * PER_CTA + PER_CTA - 1];
         const unsigned long long prefix = (unsigned long long)((16383u - (unsigned)(BK_N - 1 - first)) >> 2) << 52;
+        __syncthreads();                                               // what was chosen is read by all
         ss_descend<THREADS>(sh, row, by_mass, target, prefix, before, parity, key, upto);
+        spoilt = true;
         return true;
     }
-    const unsigned to_list = ss_peer_addr(li->list, 0u), to_weight = ss_peer_addr(li->weight, 0u);
-    const unsigned to_n = ss_peer_addr(&bk->n_list[question], 0u);
+    // the bucket's tokens, to every CTA: a place of its own for each, in the order of the CTAs (within a CTA any order will do)
+    const unsigned start = spoilt ? 0u : li->count[bucket];
     for (int i = row.i0 + tid; i < row.i1; i += THREADS) {
         const unsigned b = row.bits[i - row.i0];
         if (b >> BK_SHIFT == bucket) {
             unsigned at;
-            asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(to_n) : "memory");
+            if (spoilt) asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(ss_peer_addr(&bk->n_spoilt[question], 0u)) : "memory");
+            else at = start + (unsigned)atomicAdd(&bk->n_list[question], 1);
             if (at < BK_LIST) {
-                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(to_list + at * 8u), "l"(ss_key(b, (unsigned)i)) : "memory");
-                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(to_weight + at * 8u), "l"(ss_weight(b)) : "memory");
-            }
-        }
-    }
-    __syncthreads();
-    ss_cluster_sync();
-    // Every CTA compares its share of the tokens with all of them (550 tokens with one another are 300,000 comparisons, a
-    // dozen microseconds for one CTA): eight lanes per token, a lane every eighth of the others.
-    const int m = (int)n_in, rank = (int)ss_cluster_rank();
-    if (rank != 0) {
-        for (int i = tid; i < m; i += THREADS) {
-            li->list[i] = ss_ld_peer_u64(&li->list[i], 0u);
-            li->weight[i] = ss_ld_peer_u64(&li->weight[i], 0u);
-        }
-    }
-    __syncthreads();
-    const int share = (m + SS_CLUSTER - 1) / SS_CLUSTER, i1 = min(m, (rank + 1) * share);
-    for (int i0 = rank * share; i0 < i1; i0 += THREADS / 8) {          // uniform in the CTA
-        const int i = i0 + (tid >> 3);
-        const unsigned long long mine = i < i1 ? li->list[i] : 0ull;
-        unsigned long long cum = 0ull;
-        for (int j = tid & 7; j < m; j += 8) cum += li->list[j] < mine ? li->weight[j] : 0ull;
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) cum += __shfl_xor_sync(0xffffffffu, cum, o);
-        if ((tid & 7) == 0 && i < i1) {
-            const unsigned long long with = below + cum + li->weight[i];
-            if (bk_reached(with, by_mass, target) && !bk_reached(below + cum, by_mass, target)) {            // one token of the cluster
-                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->key, 0u)), "l"(mine) : "memory");
-                asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&bk->upto, 0u)), "l"(with) : "memory");
+                for (unsigned r = 0; r < SS_CLUSTER; ++r)
+                    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ss_peer_addr(&li->find.list[at], r)), "l"(ss_key(b, (unsigned)i)) : "memory");
             }
         }
     }
     __syncthreads();
     ss_cluster_sync();
-    key = ss_ld_peer_u64(&bk->key, 0u);                                // (the next result is written behind another barrier of the cluster)
-    upto = ss_ld_peer_u64(&bk->upto, 0u);
+    bk_refine<THREADS>(bk, &li->find, (int)n_in, (int)bucket, by_mass, target, below, key, upto);
+    arrived = true;
     return true;
 }
 
@@ -405,7 +506,8 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     Buckets* bk = &bk_;
     const int tid = threadIdx.x;
     for (int i = tid; i < BK_N; i += THREADS) li->count[i] = li->low[i] = 0u;
-    if (tid < 4) bk->n_list[tid] = 0;
+    if (tid < 4) bk->n_list[tid] = bk->n_spoilt[tid] = 0;
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");          // this CTA's shared memory may be written to
     const unsigned rank = ss_cluster_rank();
     const int row_id = blockIdx.x / SS_CLUSTER;
     const float* x = logits + (size_t)row_id * ld;
@@ -445,11 +547,13 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
         }
     }
     mx = sp_block_max(mx, sh->red);
-    if (tid == 0) sh->stat[0] = mx;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < SS_CLUSTER) ss_st_peer_f32(&sh->stat[0][rank], (unsigned)tid, mx);
+    __syncwarp();
     ss_cluster_sync();
     mx = -INFINITY;
 #pragma unroll
-    for (unsigned r = 0; r < SS_CLUSTER; ++r) mx = fmaxf(mx, ss_ld_peer_f32(&sh->stat[0], r));
+    for (unsigned r = 0; r < SS_CLUSTER; ++r) mx = fmaxf(mx, sh->stat[0][r]);
     float sum = 0.0f;
     if (few) {
 #pragma unroll
@@ -466,11 +570,12 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
         }
     }
     sum = sp_block_sum(sum, sh->red);
-    if (tid == 0) sh->stat[1] = sum;
+    if (tid < SS_CLUSTER) ss_st_peer_f32(&sh->stat[1][rank], (unsigned)tid, sum);
+    __syncwarp();
     ss_cluster_sync();
     sum = 0.0f;
 #pragma unroll
-    for (unsigned r = 0; r < SS_CLUSTER; ++r) sum += ss_ld_peer_f32(&sh->stat[1], r);       // in rank order, alike in every CTA
+    for (unsigned r = 0; r < SS_CLUSTER; ++r) sum += sh->stat[1][r];       // in rank order, alike in every CTA
     auto probability = [&](float e) {
         float p = e / sum;
         if (!(p >= 0.0f)) p = 0.0f;                           // NaN logits never win
@@ -489,8 +594,9 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     bk_fill<THREADS>(bk, li, row);
     int question = 0;
     unsigned parity = 0;
+    bool spoilt = false, arrived = false;
     auto first_at = [&](bool by_mass, unsigned long long target, unsigned long long& key, unsigned long long& upto) -> bool {
-        return bk_find<THREADS>(sh, bk, li, row, question++, by_mass, target, parity, key, upto);
+        return bk_find<THREADS>(sh, bk, li, row, question++, by_mass, target, parity, spoilt, arrived, key, upto);
     };
     unsigned long long key = 0ull, upto = 0ull, limit_mass = 0ull;
     const bool limited = top_k > 0 && top_k < V && first_at(false, (unsigned long long)top_k, key, upto);       // the first top_k tokens
@@ -506,8 +612,9 @@ sample_rows_kernel(const float* __restrict__ logits, int ld, int V, float temper
     const unsigned long long n_u = (unsigned long long)((u ? u[row_id] : draws.u[row_id]) * 16777216.0f);
     const unsigned long long target = (__umul64hi(kept_mass, n_u) << 40) | ((kept_mass * n_u) >> 24);
     if (!first_at(true, target, key, upto)) first_at(true, 0ull, key, upto);                    // the most probable token
+    if (arrived) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // (behind the last question's barrier of the cluster nobody reads or writes a peer's shared memory: all may leave)
     if (rank == 0 && tid == 0) out[row_id] = (int)(unsigned)(key & 0xffffffffu);
-    ss_cluster_sync();                                         // no CTA leaves while a peer may still read its shared memory
 }
 
 }  // namespace

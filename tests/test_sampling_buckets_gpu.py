@@ -85,3 +85,26 @@ def test_nearly_equal_tokens(K, rows, std, top_k, top_p):
         kept = min(float(run[r, top_k - 1]) if top_k else 1.0, max(top_p, float(run[r, 0])))
         slack = 2.0 ** -19 + 2 * float(p[r, 0])                        # the kept mass ends behind the token that reaches top_p
         assert float(run[r, at]) >= u * kept - slack and float(run[r, at] - p[r, at]) <= u * kept + slack
+
+
+@pytest.mark.parametrize("rows", [6, 18])
+@pytest.mark.parametrize("head", [40, 900])
+def test_answers_of_few_and_of_many_tokens_in_one_row(K, rows, head):
+    """The top_k boundary lies among 2,000 equal tokens (the descent), the draw among tokens of their own probabilities (by bins)
+    or among the equal ones. Every draw is aimed at the middle of a token's mass: 1e-4 of the total, a thousand times what the
+    32-bit probabilities are off by."""
+    V, top_k = 5003, 1500
+    g = torch.Generator().manual_seed(head)
+    at = torch.randperm(V, generator=g)
+    logits = torch.full((V,), -200.0)
+    logits[at[:head]] = 1.0 + torch.arange(head, 0, -1) * (0.5 / head)
+    logits[at[head:head + 2000]] = 0.0
+    p, order = torch.softmax(logits.double(), dim=-1).sort(descending=True, stable=True)
+    run = p.cumsum(dim=-1)
+    kept = float(run[top_k - 1])
+    want = [0, 5, head - 1, head, (head + top_k) // 2, top_k - 1] * (rows // 6)
+    us = [int((float(run[j]) - float(p[j]) / 2) / kept * 2 ** 24) / 2 ** 24 for j in want]
+    scratch = torch.empty(K.sample_scratch_keys(rows, V), dtype=torch.int64, device=DEV)
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    K.sample_rows(logits.repeat(rows, 1).to(DEV), 1.0, top_k, 1.0, us, scratch, out)
+    assert out.tolist() == [int(order[j]) for j in want]
