@@ -294,6 +294,7 @@ gemm_generic_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* __
 // and a prompt step by 32-bit rounding.
 #define GS_KC 512
 #define GS_ROWS 2
+#define GS_PIECES 4                                          // most CTAs of a cluster that share the columns of W
 // 16 bytes, or zeros where not ``ok``; under a predicate, so that the loads of a slice go out side by side.
 __device__ __forceinline__ float4 gs_load(const float* p, bool ok) {
     float4 v;
@@ -301,15 +302,26 @@ __device__ __forceinline__ float4 gs_load(const float* p, bool ok) {
                  "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}" : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(p), "r"((int)ok));
     return v;
 }
-template <int MT>
+// SPLIT: a cluster's CTAs share the columns, where there are too few rows of W to fill the chip (a product of 2,048 rows has
+// 256 CTAs, which keep half of the bytes in flight that the memory takes): the first adds the others' sums in their order.
+// 4 rows, 2,048 x 8,192: 18.5 us with one CTA for all of K, 16.5 with two. For 1 to 4 rows: beyond them
+// fewer CTAs fit an SM and the rows of a layer's products fill it.
+template <int MT, bool SPLIT>
 __global__ void __launch_bounds__(128, MT == 16 ? 5 : MT == 8 ? 3 : 4)
 gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
-                       int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
+                       int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int n_pieces) {
     constexpr int XV = MT * (GS_KC / 4) / 128;               // 16-byte pieces of a slice of A per thread
     constexpr bool XAHEAD = MT <= 4, WAHEAD = MT <= 8, PRED = MT == 16;      // AHEAD: held in registers a slice ahead
     __shared__ __align__(16) float xs[MT][GS_KC];
+    __shared__ float parts[SPLIT ? GS_PIECES - 1 : 1][SPLIT ? 4 : 1][GS_ROWS][MT];     // of the first CTA of a cluster: the others' sums
+    const int pieces = SPLIT ? n_pieces : 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (blockIdx.x * 4 + warp) * GS_ROWS;
+    const int piece = SPLIT ? blockIdx.x % pieces : 0;       // the CTA's rank in its cluster
+    const int n0 = ((SPLIT ? blockIdx.x / pieces : blockIdx.x) * 4 + warp) * GS_ROWS;
+    const int per = SPLIT ? ((K + GS_KC - 1) / GS_KC + pieces - 1) / pieces * GS_KC : 0;
+    const int k_from = SPLIT ? piece * per : 0;
+    if (SPLIT) K = min(K, k_from + per);                     // this CTA's columns (none: its sums are zero)
+    if (SPLIT) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // its shared memory may be written to
     float acc[GS_ROWS][MT];
 #pragma unroll
     for (int r = 0; r < GS_ROWS; ++r)
@@ -371,20 +383,43 @@ gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
     };
     sp_allow_dependents();
     sp_wait_for_predecessor();
-    if (WAHEAD) load_w(0, w[0]);
+    if (WAHEAD) load_w(k_from, w[0]);
     if (XAHEAD) {
 #pragma unroll
-        for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(0, v);
+        for (int v = 0; v < (XAHEAD ? XV : 1); ++v) x_next[v] = load_x(k_from, v);
     }
-    for (int k0 = 0; k0 < K; k0 += 2 * GS_KC) {
+    for (int k0 = k_from; k0 < K; k0 += 2 * GS_KC) {
         slice(k0, std::integral_constant<int, 0>());
         if (k0 + GS_KC < K) slice(k0 + GS_KC, std::integral_constant<int, 1>());
+    }
+    if constexpr (SPLIT) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (piece > 0) {
+#pragma unroll
+            for (int r = 0; r < GS_ROWS; ++r)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float v = sp_warp_sum(acc[r][m]);
+                    if (lane == 0) {
+                        uint32_t at;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&parts[piece - 1][warp][r][m])));
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+                    }
+                }
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (piece > 0) return;
     }
 #pragma unroll
     for (int r = 0; r < GS_ROWS; ++r)
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            const float v = sp_warp_sum(acc[r][m]);
+            float v = sp_warp_sum(acc[r][m]);
+            if constexpr (SPLIT) {
+                for (int i = 0; i + 1 < pieces; ++i) v += parts[i][warp][r][m];
+            }
             if (lane == 0 && m < M && n0 + r < N) {
                 const size_t o = (size_t)m * ldc + n0 + r;
                 sp_st_dt(C, c_dt, o, accumulate ? v + ((float*)C)[o] : v);
@@ -401,14 +436,20 @@ SP_API int sp_gemm_generic(const void* A, int a_dt, const void* W, int w_dt, voi
     if (M <= 16 && a_dt == SP_DT_F32 && w_dt == SP_DT_F32 && ((K | lda | ldw) & 3) == 0 &&
         ((((uintptr_t)A) | ((uintptr_t)W)) & 15) == 0) {
         const unsigned blocks = (unsigned)((N + 4 * GS_ROWS - 1) / (4 * GS_ROWS));
-#define GS_LAUNCH(MT) \
-        SP_CHECK_CALL("gemm_stream_f32", sp_launch_dependent(gemm_stream_f32_kernel<MT>, dim3(blocks), dim3(128), 0, stream, \
-                                                             (const float*)A, (const float*)W, C, c_dt, M, N, K, lda, ldw, ldc, accumulate))
-        if (M <= 1) GS_LAUNCH(1);
-        else if (M <= 2) GS_LAUNCH(2);
-        else if (M <= 4) GS_LAUNCH(4);
-        else if (M <= 8) GS_LAUNCH(8);
-        else GS_LAUNCH(16);
+        unsigned pieces = 1;
+        while (M <= 4 && pieces < GS_PIECES && blocks * pieces * 2 <= (unsigned)sp_sm_count() * 4 && (unsigned)K >= pieces * 2 * GS_KC) pieces *= 2;
+#define GS_LAUNCH(MT, SPLIT) \
+        SP_CHECK_CALL("gemm_stream_f32", sp_launch_cluster(gemm_stream_f32_kernel<MT, SPLIT>, dim3(blocks * pieces), dim3(128), 0, stream, -(int)pieces, \
+                                                           (const float*)A, (const float*)W, C, c_dt, M, N, K, lda, ldw, ldc, accumulate, (int)pieces))
+        if (pieces > 1) {
+            if (M <= 1) GS_LAUNCH(1, true);
+            else if (M <= 2) GS_LAUNCH(2, true);
+            else GS_LAUNCH(4, true);
+        } else if (M <= 1) GS_LAUNCH(1, false);
+        else if (M <= 2) GS_LAUNCH(2, false);
+        else if (M <= 4) GS_LAUNCH(4, false);
+        else if (M <= 8) GS_LAUNCH(8, false);
+        else GS_LAUNCH(16, false);
 #undef GS_LAUNCH
         return 0;
     }
@@ -454,10 +495,12 @@ __device__ __forceinline__ bool kv_page_of(const KvPlace& pl, int t, int pos, in
 }
 
 template <typename TIN, typename TQ, typename TC>
-__global__ void rope_kv_write_kernel(const TIN* __restrict__ qkv, TQ* __restrict__ q_out,
+__global__ void rope_kv_write_kernel(const TIN* qkv, TQ* __restrict__ q_out,
                                      TC* __restrict__ kpool, TC* __restrict__ vpool, KvPlace pl,
                                      const float* __restrict__ inv_freq, int T, int nh, int nkv, int hd,
                                      int rd, int write_kv) {
+    sp_allow_dependents();
+    sp_wait_for_predecessor();
     const int t = blockIdx.x;
     if (t >= T) return;
     const int pos = pl.positions[t];
@@ -618,7 +661,7 @@ SP_API int sp_rope_kv_write(const void* qkv, int in_dt, void* q_out, int q_dt, v
     }
     const int threads = 256;
 #define RK_LAUNCH(TIN, TQ, TC)                                                                                  \
-    SP_CHECK_CALL("rope_kv_write", sp_launch_cluster(rope_kv_write_kernel<TIN, TQ, TC>, dim3(T), dim3(threads), 0, stream, 1, \
+    SP_CHECK_CALL("rope_kv_write", sp_launch_cluster(rope_kv_write_kernel<TIN, TQ, TC>, dim3(T), dim3(threads), 0, stream, -1, \
                                                 (const TIN*)qkv, (TQ*)q_out, (TC*)kpool, (TC*)vpool, pl, inv_freq, T, nh, \
                                                 nkv, hd, rd, write_kv))
     const int key = in_dt * 4 + q_dt * 2 + cache_dt;
@@ -798,6 +841,155 @@ attention_generic_kernel(const TQ* __restrict__ q, const TC* __restrict__ kpool,
     }
 }
 
+// The same attention in 32 bits where there are few (token, head) pairs (a decode step): a cluster of eight CTAs per (token,
+// kv head), whose 32 warps take turns at batches of keys, each batch for all query heads of the group. A key or value row is
+// read once per group instead of once per head, in whole lines (16 or 32 lanes a row), the loads of a batch's rows of K
+// and V all in flight together: what bounds the step is the latency of three trips (table, rows, the cluster's
+// barrier). Each warp keeps its own running maximum and sum; the warps of a CTA, then the CTAs, are merged in their order
+// (every CTA an eighth of the results, the parts pushed into its shared memory behind one barrier of the cluster).
+// 4 sequences of 500 keys, 32 heads of 64 on 8 kv heads: 27 us by the kernel above, 7.9 us here (batches of
+// eight rows per lane took registers that a fourth CTA on an SM needs: 8 sequences of 60 keys 10.8 us against 8.3).
+#define AD_CLUSTER 8
+template <int LPR, int REP>
+__global__ void __launch_bounds__(128)
+attention_decode_f32_kernel(const float* q, const float* kpool, const float* vpool, float* out, KvPlace pl, int nh, int nkv,
+                            int hd, int vd, int window, float scale, const float* sink, const float* dist_bias, int dist_cap) {
+    constexpr int WARPS = 4, SUBS = 32 / LPR, AD_LOADS = 4, BATCH = AD_LOADS * SUBS, OWN = REP * LPR / AD_CLUSTER;
+    __shared__ __align__(16) float4 part_acc[WARPS][REP][LPR];
+    __shared__ float2 part_ml[WARPS][REP];
+    __shared__ __align__(16) float4 in_acc[AD_CLUSTER][OWN];
+    __shared__ float2 in_ml[AD_CLUSTER][REP];
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");        // this CTA's shared memory may be written to
+    sp_wait_for_predecessor();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane / LPR, c = (lane % LPR) * 4;
+    const int rank = blockIdx.x, g = blockIdx.y, t = blockIdx.z, rep = nh / nkv;
+    const int p = sp_ld_written(pl.positions + t), seq = sp_ld_written(pl.token_seq + t);      // one trip
+    const int slot = sp_checked_row(pl.seq_slot[seq], pl.rg);
+    const int* pt = pl.page_table + (size_t)slot * pl.max_pages;
+    const int ps = pl.page_size;
+    float4 qv[REP], acc[REP];
+    float m[REP], l[REP];
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+        qv[r] = gs_load(q + (size_t)t * nh * hd + (size_t)(g * rep + r) * hd + c, r < rep && c < hd);
+        acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        m[r] = -INFINITY;
+        l[r] = 0.0f;
+    }
+    const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+    for (int j0 = lo + (rank * WARPS + warp) * BATCH; j0 <= p; j0 += AD_CLUSTER * WARPS * BATCH) {
+        float4 k[AD_LOADS], v[AD_LOADS];
+        int page[AD_LOADS];
+#pragma unroll
+        for (int i = 0; i < AD_LOADS; ++i) {
+            const int j = min(j0 + i * SUBS + sub, p);
+            page[i] = sp_checked_page(pt[sp_checked_entry(j / ps, pl.max_pages, pl.rg)], pl.rg);
+        }
+#pragma unroll
+        for (int i = 0; i < AD_LOADS; ++i) {
+            const int j = j0 + i * SUBS + sub;
+            const size_t row = ((size_t)page[i] * nkv + g) * ps + min(j, p) % ps;
+            k[i] = gs_load(kpool + row * hd + c, j <= p && c < hd);
+            v[i] = gs_load(vpool + row * vd + c, j <= p && c < vd);
+        }
+        float s[REP][AD_LOADS];
+#pragma unroll
+        for (int i = 0; i < AD_LOADS; ++i) {
+#pragma unroll
+            for (int r = 0; r < REP; ++r) {
+                float d = qv[r].x * k[i].x;
+                d = fmaf(qv[r].y, k[i].y, d); d = fmaf(qv[r].z, k[i].z, d); d = fmaf(qv[r].w, k[i].w, d);
+#pragma unroll
+                for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                const int j = j0 + i * SUBS + sub;
+                d *= scale;
+                if (dist_bias && r < rep) d += dist_bias[(size_t)(g * rep + r) * (dist_cap + 1) + min(max(p - j, 0), dist_cap)];
+                s[r][i] = j <= p ? d : -INFINITY;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < REP; ++r) {
+            float m_new = m[r];
+#pragma unroll
+            for (int i = 0; i < AD_LOADS; ++i) m_new = fmaxf(m_new, s[r][i]);
+            if (SUBS == 2) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 16));
+            const float at = m_new == -INFINITY ? 0.0f : m_new;                  // (scores of -inf only: nothing is added)
+            const float corr = expf(m[r] - at);
+            l[r] *= corr;
+            acc[r].x *= corr; acc[r].y *= corr; acc[r].z *= corr; acc[r].w *= corr;
+#pragma unroll
+            for (int i = 0; i < AD_LOADS; ++i) {
+                const float e = expf(s[r][i] - at);
+                l[r] += e;
+                acc[r].x = fmaf(e, v[i].x, acc[r].x); acc[r].y = fmaf(e, v[i].y, acc[r].y);
+                acc[r].z = fmaf(e, v[i].z, acc[r].z); acc[r].w = fmaf(e, v[i].w, acc[r].w);
+            }
+            m[r] = m_new;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+        if (SUBS == 2) {
+            l[r] += __shfl_xor_sync(0xffffffffu, l[r], 16);
+            acc[r].x += __shfl_xor_sync(0xffffffffu, acc[r].x, 16);
+            acc[r].y += __shfl_xor_sync(0xffffffffu, acc[r].y, 16);
+            acc[r].z += __shfl_xor_sync(0xffffffffu, acc[r].z, 16);
+            acc[r].w += __shfl_xor_sync(0xffffffffu, acc[r].w, 16);
+        }
+        if (sub == 0) part_acc[warp][r][lane] = acc[r];
+        if (lane == 0) part_ml[warp][r] = make_float2(m[r], l[r]);
+    }
+    sp_allow_dependents();                                   // (not before: the product's CTAs would crowd on a few SMs)
+    __syncthreads();
+    // parts whose sum is 0 saw no key; a sum that is not a number goes on as it is
+    auto merge = [&](auto ml_of, auto acc_of, int n, float4& a, float2& ml) {
+        ml = make_float2(-INFINITY, 0.0f);
+        a = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int w = 0; w < n; ++w) ml.x = fmaxf(ml.x, ml_of(w).x);
+        for (int w = 0; w < n; ++w) {
+            const float2 o = ml_of(w);
+            if (o.y <= 0.0f) continue;
+            const float f = expf(o.x - ml.x);
+            const float4 b = acc_of(w);
+            ml.y = fmaf(o.y, f, ml.y);
+            a.x = fmaf(b.x, f, a.x); a.y = fmaf(b.y, f, a.y); a.z = fmaf(b.z, f, a.z); a.w = fmaf(b.w, f, a.w);
+        }
+    };
+    auto peer = [](const void* at, int of) {
+        uint32_t a;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(of));
+        return a;
+    };
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int e = tid; e < REP * LPR; e += 32 * WARPS) {
+        const int r = e / LPR;
+        float4 a;
+        float2 ml;
+        merge([&](int w) { return part_ml[w][r]; }, [&](int w) { return part_acc[w][r][e % LPR]; }, WARPS, a, ml);
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(peer(&in_acc[rank][e / AD_CLUSTER], e % AD_CLUSTER)),
+                     "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w) : "memory");
+        if (e % LPR < AD_CLUSTER)
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer(&in_ml[rank][r], e % LPR)), "f"(ml.x), "f"(ml.y) : "memory");
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = tid; i < OWN; i += 32 * WARPS) {
+        const int e = i * AD_CLUSTER + rank, r = e / LPR, d = (e % LPR) * 4;
+        if (r >= rep || d >= vd) continue;
+        float4 a;
+        float2 ml;
+        merge([&](int w) { return in_ml[w][r]; }, [&](int w) { return in_acc[w][i]; }, AD_CLUSTER, a, ml);
+        const int h = g * rep + r;
+        if (sink) {
+            const float all = fmaxf(ml.x, sink[h]), f = expf(ml.x - all);
+            ml.y = ml.y * f + expf(sink[h] - all);
+            a.x *= f; a.y *= f; a.z *= f; a.w *= f;
+        }
+        *(float4*)(out + (size_t)t * nh * vd + (size_t)h * vd + d) = make_float4(a.x / ml.y, a.y / ml.y, a.z / ml.y, a.w / ml.y);
+    }
+}
+
 SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, const void* vpool, int cache_dt,
                                 void* out, const int* token_seq, const int* positions, const int* seq_slot,
                                 const int* page_table, int max_pages, int page_size, int T, int nh, int nkv,
@@ -813,6 +1005,24 @@ SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, cons
     const long long warps = (long long)T * nh;
     // few (token, head) pairs (a decode step): a CTA per pair, its warps share the keys
     const bool split = warps <= 4096;
+    const int rep = nh / nkv;
+    if (split && q_dt == SP_DT_F32 && cache_dt == SP_DT_F32 && rep <= 8 && hd <= 128 && vd <= 128 && ((hd | vd) & 3) == 0 &&
+        (((uintptr_t)q | (uintptr_t)kpool | (uintptr_t)vpool | (uintptr_t)out) & 15) == 0) {
+#define AD_LAUNCH(LPR, REP)                                                                                            \
+    SP_CHECK_CALL("attention_decode_f32", sp_launch_cluster(attention_decode_f32_kernel<LPR, REP>, dim3(AD_CLUSTER, nkv, T), dim3(128), 0, stream, \
+                                                            -AD_CLUSTER, (const float*)q, (const float*)kpool, (const float*)vpool, (float*)out, pl, \
+                                                            nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap))
+#define AD_BY_REP(LPR)                                                                                                 \
+    if (rep == 1) AD_LAUNCH(LPR, 1);                                                                                   \
+    else if (rep == 2) AD_LAUNCH(LPR, 2);                                                                              \
+    else if (rep <= 4) AD_LAUNCH(LPR, 4);                                                                              \
+    else AD_LAUNCH(LPR, 8)
+        if (hd <= 64 && vd <= 64) { AD_BY_REP(16); }
+        else { AD_BY_REP(32); }
+#undef AD_BY_REP
+#undef AD_LAUNCH
+        return 0;
+    }
     const long long blocks = split ? warps : (warps + AG_WARPS - 1) / AG_WARPS;
     if (blocks > 2147483647LL) SP_FAIL("attention: too many (token, head) pairs for one launch");
 #define AG_ARGS(TQ, TC) (const TQ*)q, (const TC*)kpool, (const TC*)vpool, (TQ*)out, pl, T, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap
@@ -1036,7 +1246,8 @@ SP_API int sp_attention_tile_f32(const float* q, const float* kpool, const float
 // ============================================================== act(gate) * up
 // gu row = [gate(0..I) | up(0..I)]; out row = act(gate) ⊙ up · mult (SP_ACT_SILU, SP_ACT_GELU).
 template <typename T>
-__global__ void gated_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, size_t rows, int I, int act, float mult) {
+__global__ void gated_mul_kernel(const T* gu, T* __restrict__ out, size_t rows, int I, int act, float mult) {
+    sp_wait_for_predecessor();
     const size_t n = rows * (size_t)I;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
         const size_t r = e / I;
@@ -1045,6 +1256,8 @@ __global__ void gated_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, 
         const float u = sp_ld(gu, r * 2 * I + I + c);
         sp_st(out, e, sp_gated(g, u, SpGate{act, mult, 0.0f, 0.0f}));
     }
+    // not before: the next product's CTAs would crowd on the SMs that are free so far (8 rows, down product 26 -> 33 us)
+    sp_allow_dependents();
 }
 
 SP_API int sp_gated_mul(const void* gu, void* out, int dt, int rows, int I, int act, float mult, cudaStream_t stream) {
@@ -1052,8 +1265,8 @@ SP_API int sp_gated_mul(const void* gu, void* out, int dt, int rows, int I, int 
     if (act != SP_ACT_SILU && act != SP_ACT_GELU) SP_FAIL("gated_mul: activation code %d is not built", act);
     const size_t n = (size_t)rows * I;
     const int blocks = (int)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
-    if (dt == SP_DT_F32) gated_mul_kernel<float><<<blocks, 256, 0, stream>>>((const float*)gu, (float*)out, rows, I, act, mult);
-    else if (dt == SP_DT_BF16) gated_mul_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, I, act, mult);
+    if (dt == SP_DT_F32) sp_launch_dependent(gated_mul_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)gu, (float*)out, rows, I, act, mult);
+    else if (dt == SP_DT_BF16) sp_launch_dependent(gated_mul_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, I, act, mult);
     else SP_FAIL("gated_mul: unsupported dtype code %d", dt);
     SP_CHECK_LAUNCH("gated_mul");
     return 0;

@@ -21,7 +21,8 @@ def function(text: str, name: str) -> str:
     raise AssertionError(f"{name} has no end")
 
 
-@pytest.mark.parametrize("source,kernel", [("generic_kernels.cu", "gemm_stream_f32_kernel"), ("gemv_kernels.cu", "gemv_kernel")])
+@pytest.mark.parametrize("source,kernel", [("generic_kernels.cu", "gemm_stream_f32_kernel"),
+                                           ("generic_kernels.cu", "attention_decode_f32_kernel"), ("gemv_kernels.cu", "gemv_kernel")])
 def test_parameters_and_loads_of_a_dependent_kernel(source, kernel):
     text = (CSRC / source).read_text()
     body = function(text, kernel)

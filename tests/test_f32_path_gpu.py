@@ -91,6 +91,73 @@ def test_few_rows_slices_of_k(K, M, N, Kd):
     assert bool(((out.double() - a.double() @ w.double().t()).abs() <= (Kd / 32 + 8) * 2.0 ** -24 * size).all())
 
 
+@pytest.mark.parametrize("M", [1, 4, 5, 16])
+@pytest.mark.parametrize("N,Kd", [(9, 1024), (24, 2048), (17, 2564), (3, 5000), (2048, 8192)])
+def test_few_rows_columns_shared_by_ctas(K, M, N, Kd):
+    a, w = operands(M, N, Kd)
+    c0 = torch.randn(M, N, device=DEV)
+    out, acc = torch.empty(M, N, device=DEV), c0.clone()
+    K.gemm_generic(a, w, out)
+    K.gemm_generic(a, w, acc, accumulate=True)
+    size = a.double().abs() @ w.double().abs().t()
+    # a lane adds Kd / 32 terms or fewer in order, five rounds of sums, at most three sums of pieces
+    assert bool(((out.double() - a.double() @ w.double().t()).abs() <= (Kd / 32 + 11) * 2.0 ** -24 * size).all())
+    assert torch.equal(acc, out + c0)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd", [(4, 2, 64, 64), (3, 1, 32, 32), (2, 2, 20, 20), (8, 2, 128, 128), (8, 1, 96, 36), (10, 2, 4, 128)])
+@pytest.mark.parametrize("window", [None, 1, 100])
+@pytest.mark.parametrize("extra", [False, True])
+def test_attention_of_a_decode_step(K, nh, nkv, hd, vd, window, extra):
+    before = [0, 1, 63, 64, 511, 512, 700, 2100]
+    torch.manual_seed(hd + vd + (window or 0))
+    meta = KH.paged_meta([1] * len(before), before, DEV, seed=hd)
+    qs = [torch.randn(nh, hd) for _ in before]
+    ks = [torch.randn(t, nkv, hd) for t in meta.total_len]
+    vs = [torch.randn(t, nkv, vd) for t in meta.total_len]
+    k_pool, _ = KH.fill_cache(meta, ks, ks, nkv, hd, torch.float32, DEV)
+    v_pool, _ = KH.fill_cache(meta, vs, vs, nkv, vd, torch.float32, DEV)
+    q = torch.stack(qs).reshape(-1, nh * hd).to(DEV)
+    out = torch.full((len(before), nh * vd), float("nan"), device=DEV)
+    sink = torch.randn(nh, device=DEV) if extra else None
+    bias = torch.randn(nh, 50, device=DEV) if extra else None
+    if extra:
+        bias[0, 7:] = float("-inf")                                     # whole batches of keys that a head does not see
+    scale = 1.0 / math.sqrt(hd)
+    K.attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, window, scale, vd=vd, sink=sink, dist_bias=bias)
+    rows = []
+    for qb, kb, vb in zip(qs, ks, vs):
+        L = kb.shape[0]
+        dist = L - 1 - torch.arange(L)
+        for h in range(nh):
+            s = kb[:, h // (nh // nkv)].double() @ qb[h].double() * scale
+            if bias is not None:
+                s = s + bias[h].double().cpu()[dist.clamp(0, 49)]
+            s = s.masked_fill(dist >= (window or L), float("-inf"))
+            if sink is not None:
+                s = torch.cat([s, sink[h:h + 1].double().cpu()])
+            rows.append(torch.softmax(s, dim=-1)[:L] @ vb[:, h // (nh // nkv)].double())
+    ref = torch.cat(rows).view(len(before), nh * vd)
+    # as for the tiles below: the error of scores of size sqrt(hd) goes into the weights as a factor
+    assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
+
+
+def test_a_value_that_is_not_finite_stays_with_its_group(K):
+    """A decode step's NaN key and infinite value reach the heads and the sequence that see them, and no others."""
+    nh, nkv, hd, before = 4, 2, 64, [600, 600]
+    torch.manual_seed(5)
+    meta = KH.paged_meta([1, 1], before, DEV, seed=3)
+    ks = [torch.randn(t, nkv, hd) for t in meta.total_len]
+    vs = [torch.randn(t, nkv, hd) for t in meta.total_len]
+    ks[0][17, 0, 3], vs[0][599, 1, 5] = float("nan"), float("inf")
+    k_pool, v_pool = KH.fill_cache(meta, ks, vs, nkv, hd, torch.float32, DEV)
+    out = torch.zeros(2, nh * hd, device=DEV)
+    K.attention_generic(torch.randn(2, nh * hd, device=DEV), k_pool, v_pool, out, meta, nh, nkv, hd, None, 0.125)
+    out = out.view(2, nh, hd).cpu()
+    assert bool(out[0, :2].isnan().all()) and bool(out[1].isfinite().all())
+    assert bool((out[0, 2:, 5] == float("inf")).all()) and bool(out[0, 2:, [i for i in range(hd) if i != 5]].isfinite().all())
+
+
 @pytest.mark.parametrize("nh,nkv,hd,vd", [(4, 2, 64, 64), (3, 1, 32, 32), (2, 2, 20, 20), (4, 1, 128, 128), (2, 1, 96, 36), (2, 2, 4, 128)])
 @pytest.mark.parametrize("window", [None, 1, 63, 100])
 @pytest.mark.parametrize("extra", [False, True])
