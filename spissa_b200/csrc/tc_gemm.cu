@@ -517,10 +517,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     uint32_t u[32];
                     tc_ld_32x32(taddr + (uint32_t)(c0 + BN / 2), u);
                     tc_ld_wait();
+                    auto scale = [&](int) { return rstd; };
+                    if (ga.kind == SP_ACT_SILU) tc_activate<SP_ACT_SILU>(r, u, scale, 32, ga);
+                    else if (ga.kind == SP_ACT_CLAMPED) tc_activate<SP_ACT_CLAMPED>(r, u, scale, 32, ga);
+                    else tc_activate<SP_ACT_GELU>(r, u, scale, 32, ga);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        v[j] = sp_gated(__uint_as_float(r[j]) * rstd, __uint_as_float(u[j]) * rstd, ga);
-                    }
+                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
                 } else {
                     tc_ld_wait();
 #pragma unroll

@@ -88,45 +88,6 @@ __device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
     return make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
 }
 
-// x / d for 1 <= d <= 2^100 and finite x: the remainder of a quotient by an approximate reciprocal (two units at most off)
-// corrects it to within half a unit and 2^-20 of one (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990). No branch, unlike the general quotient.
-__device__ __forceinline__ float quotient(float x, float d) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-    const float q = x * r;
-    return fmaf(fmaf(-d, q, x), r, q);
-}
-// act(gate)·up of 32 tokens of a row of W (the first ``n`` are tokens), in place of the gate: sp_gated, as where pieces of K are added first. Gates of
-// ordinary size (all of them, in earnest) go through without a branch on one value, so that the 32 overlap. 301 tokens x
-// 16,384 x 2,048: 27.3 us, 32.0 with the general quotient, 40 with a branch on the activation around each value.
-template <int KIND>
-__device__ __forceinline__ void activate(uint32_t (&rg)[32], uint32_t (&ru)[32], const float* rstd, int n, SpGate ga) {
-    ga.kind = KIND;
-    const float slope = KIND == SP_ACT_CLAMPED ? ga.slope : 1.0f;
-    float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};                     // (NaN is left out: the quotient is NaN either way)
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        float g = __uint_as_float(rg[j]) * rstd[j];
-        if (KIND == SP_ACT_CLAMPED) g = fminf(g, ga.limit);
-        top[j & 3] = fmaxf(top[j & 3], j < n ? fabsf(slope * g) : 0.0f);
-        rg[j] = __float_as_uint(g);
-        ru[j] = __float_as_uint(__uint_as_float(ru[j]) * rstd[j]);
-    }
-    if (KIND != SP_ACT_GELU && __all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= 60.0f)) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const float g = __uint_as_float(rg[j]);
-            float u = __uint_as_float(ru[j]);
-            if (KIND == SP_ACT_CLAMPED) u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
-            rg[j] = __float_as_uint(quotient(g, 1.0f + expf(-slope * g)) * u * ga.mult);
-        }
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]), __uint_as_float(ru[j]), ga));
-}
-
 // The second part of the epilogue: a warp owns a token at a time (``first``, then every eighth below ``end``), a lane four
 // neighbouring columns of it.
 struct Share { uint32_t smem_base; int tile, tok0, first, end, lane, nt; };
@@ -415,9 +376,9 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             tc_ld_wait();
             if (GATED && act_now) {
                 // (the kind is a constant to each loop, so that the 32 values are independent of one another)
-                if (a.ga.kind == SP_ACT_SILU) activate<SP_ACT_SILU>(rg, ru, rstd_s + c0, count - c0, a.ga);
-                else if (a.ga.kind == SP_ACT_CLAMPED) activate<SP_ACT_CLAMPED>(rg, ru, rstd_s + c0, count - c0, a.ga);
-                else activate<SP_ACT_GELU>(rg, ru, rstd_s + c0, count - c0, a.ga);
+                if (a.ga.kind == SP_ACT_SILU) tc_activate<SP_ACT_SILU>(rg, ru, [&](int j) { return rstd_s[c0 + j]; }, count - c0, a.ga);
+                else if (a.ga.kind == SP_ACT_CLAMPED) tc_activate<SP_ACT_CLAMPED>(rg, ru, [&](int j) { return rstd_s[c0 + j]; }, count - c0, a.ga);
+                else tc_activate<SP_ACT_GELU>(rg, ru, [&](int j) { return rstd_s[c0 + j]; }, count - c0, a.ga);
             }
             const uint32_t dst = smem_base + (uint32_t)((c0 * BW + row) * 4);
 #pragma unroll

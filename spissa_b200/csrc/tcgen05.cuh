@@ -108,4 +108,46 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_bmn(int m, int n) {
     return umma_idesc_bf16(m, n) | (1u << 16);
 }
 
+// x / d for 1 <= d <= 2^100 and finite x: the remainder of a quotient by an approximate reciprocal (two units at most off)
+// corrects it to within half a unit and 2^-20 of one (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990). No branch, unlike the general quotient.
+__device__ __forceinline__ float tc_quotient(float x, float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = x * r;
+    return fmaf(fmaf(-d, q, x), r, q);
+}
+// act(gate)·up of 32 pairs of an epilogue's thread (the first ``n`` exist), each times its ``scale``, in place of the gate:
+// sp_gated. Gates of ordinary size (all of them, in earnest) go through without a branch on one value, so that the 32 overlap:
+// tc_mid.cu, 301 tokens x 16,384 x 2,048: 27.3 us, 32.0 with the general quotient, 40 with a branch on the activation around
+// each value. In tc_gemm.cu the general quotient's way for a numerator of zero, which the rows behind the last token all take,
+// held up the tiles behind them: 16,384 x 2,048 on weights from HBM, 1,408 tokens 130 us, 82 here (2,048 tokens, without
+// such rows, 123 and 102; of the 8B shape, 28,672 x 4,096, 6,000 tokens 1,180 and 1,098).
+template <int KIND, typename Scale>
+__device__ __forceinline__ void tc_activate(uint32_t (&rg)[32], uint32_t (&ru)[32], Scale scale, int n, SpGate ga) {
+    ga.kind = KIND;
+    const float slope = KIND == SP_ACT_CLAMPED ? ga.slope : 1.0f;
+    float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};                     // (NaN is left out: the quotient is NaN either way)
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        float g = __uint_as_float(rg[j]) * scale(j);
+        if (KIND == SP_ACT_CLAMPED) g = fminf(g, ga.limit);
+        top[j & 3] = fmaxf(top[j & 3], j < n ? fabsf(slope * g) : 0.0f);
+        rg[j] = __float_as_uint(g);
+        ru[j] = __float_as_uint(__uint_as_float(ru[j]) * scale(j));
+    }
+    if (KIND != SP_ACT_GELU && __all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= 60.0f)) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float g = __uint_as_float(rg[j]);
+            float u = __uint_as_float(ru[j]);
+            if (KIND == SP_ACT_CLAMPED) u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
+            rg[j] = __float_as_uint(tc_quotient(g, 1.0f + expf(-slope * g)) * u * ga.mult);
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) rg[j] = __float_as_uint(sp_gated(__uint_as_float(rg[j]), __uint_as_float(ru[j]), ga));
+}
+
 }  // namespace
