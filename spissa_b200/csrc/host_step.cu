@@ -41,6 +41,7 @@ typedef int (*RopeTableFn)(const int*, const int*, const int*, const int*, int, 
 typedef int (*NormPrepareFn)(const float*, const void*, void*, float*, int, int, cudaStream_t);
 typedef int (*TcMidFn)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, int, float, float,
                        float, int*, cudaStream_t);
+typedef int (*MidOrPairsFn)(int, int, int, int, int);
 typedef const char* (*LastErrorFn)();
 }
 
@@ -85,6 +86,8 @@ struct HostKernels {
     LastErrorFn err_tc_mid;
     FlashPrefillTcFn flash_prefill_tc;
     LastErrorFn err_flash_tc;
+    TcStreamFusedFn tc_gemm_fused;
+    MidOrPairsFn mid_or_pairs;
     int gemv_tokens;           // up to this many tokens the weight-streaming kernel takes a product
     int stream_tokens;         // up to this many the tensor-core kernel that streams the weight
     int flash_query_tile;      // query rows per CTA of the prompt attention
@@ -92,7 +95,7 @@ struct HostKernels {
     int flash_tc_from;         // from this many on the prompt attention of the tcgen05 tensor cores
     int pad;
 };
-static_assert(sizeof(HostKernels) == 24 * 8 + 24, "the host packs this layout");
+static_assert(sizeof(HostKernels) == 26 * 8 + 24, "the host packs this layout");
 
 // One layer: a pre-norm block of an RMS norm, a rotary grouped-query attention and a SwiGLU. All pointers are device
 // addresses; weights are bfloat16 [out, in] row-major, the gate/up weight interleaves ``gu_pair`` gate rows and their
@@ -191,6 +194,13 @@ int fused_product(const void* x, const void* W, void* out, int out_dt, int N, in
     const HostKernels& k = kernels;
     ++launches;
     if (st.mid) {
+        const int width = k.mid_or_pairs(mode, st.T, N, K, mode == MODE_STREAM_QKV_ROPE ? ep->hd : 1);
+        if (width) {
+            // (the rotating epilogue has another number in tc_gemm.cu)
+            if (k.tc_gemm_fused(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode == MODE_STREAM_QKV_ROPE ? 3 : mode, width, ep, st.status, stream))
+                return fail_from(k.err_tc_gemm, "host step");
+            return 0;
+        }
         if (k.tc_mid(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode, pair, ep, SP_ACT_SILU, 1.0f, 0.0f, 0.0f, st.status, stream))
             return fail_from(k.err_tc_mid, "host step");
         return 0;
@@ -250,7 +260,7 @@ SP_API int sp_host_step_bind(const void* table, int bytes) {
     memcpy(&kernels, table, sizeof(kernels));
     if (!kernels.flash_prefill_tc) { kernels.flash_prefill_tc = tc; kernels.err_flash_tc = tc_err; }
     if (!kernels.rmsnorm || !kernels.gemv || !kernels.tc_stream || !kernels.tc_gemm || !kernels.rope_kv_write ||
-        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.rope_table || !kernels.norm_prepare)
+        !kernels.flash_prefill || !kernels.tc_stream_fused || !kernels.tc_mid || !kernels.tc_mid_supported || !kernels.tc_gemm_fused || !kernels.mid_or_pairs || !kernels.rope_table || !kernels.norm_prepare)
         SP_FAIL("host step: an entry point is missing from the kernel table");
     bound = true;
     return 0;

@@ -7,6 +7,7 @@ size that a kernel refuses raises ``KernelError`` with the kernel's own words.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_void_p, c_int, c_float, c_longlong
 
 import torch
@@ -1087,6 +1088,13 @@ def tc_mid_plan(mode, M: int, N: int, K: int) -> tuple:
     if load("tc_mid").sp_tc_mid_plan(int(mode), int(M), int(N), int(K), out):
         raise KernelError(f"tc_mid: no division of {M} tokens x {N} x {K}")
     return tuple(out)
+
+
+@functools.lru_cache(maxsize=4096)
+def tc_mid_or_pairs(mode, M: int, N: int, K: int, multiple: int = 1) -> int:
+    """For a product that ``tc_mid`` and ``tc_gemm``'s tiles by pairs of CTAs could both take: the faster one by its sizes, as the
+    width of those tiles (a multiple of ``multiple``) or 0 for ``tc_mid``."""
+    return int(load("tc_mid").sp_tc_mid_or_pairs(int(mode), int(M), int(N), int(K), int(multiple)))
 
 
 # ------------------------------------------------------------------ seqmix: other mixers, their norm and activation

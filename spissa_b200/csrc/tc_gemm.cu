@@ -987,8 +987,9 @@ static int tc_gemm_any(const void* A, const void* W, void* C, int c_dt, int M, i
     if (mode == MODE_SILU_MUL && (N % bn)) SP_FAIL("tc_gemm: the fused silu epilogue needs N (%d) to be a multiple of the tile width %d", N, bn);
     CUtensorMap ma, mw;
     if (make_map(&ma, A, M, K, lda, BM)) return 1;
-    // a prompt's worth of rows: pairs of CTAs on tiles of 256 rows, each fetching half of the W tile
-    if (pairs_from > 0 && M >= pairs_from) {
+    // a prompt's worth of rows: pairs of CTAs on tiles of 256 rows, each fetching half of the W tile. 256-wide tiles of gated
+    // products, of which there are the most, from two row tiles on (800 tokens x 16,384 x 2,048: 83 us singly, 56 by pairs)
+    if (pairs_from > 0 && (M >= pairs_from || (mode == MODE_SILU_MUL && bn == 256 && M > BM))) {
         if (make_map(&mw, W, N, K, ldw, bn / 2)) return 1;
         if (bn == 128) return launch_pair<128, 8>(ma, mw, C, c_dt, M, N, K, ldc, mode, status, stream, ep, ga);
         if (bn == 192) return launch_pair<192, 7>(ma, mw, C, c_dt, M, N, K, ldc, mode, status, stream, ep, ga);

@@ -475,12 +475,12 @@ bool fill_plan(Plan& p, int parts, int M, int num_kb) {
     return p.stages >= 1 && p.tmem_cols <= 512;
 }
 
-// The division of a product, by an estimate of its time in nanoseconds that was fitted to 1,276 measured divisions of the
+// The division of a product (``estimate``: its time), by an estimate of its time in nanoseconds that was fitted to 1,276 measured divisions of the
 // products of the 1B and 8B layer sizes at 17 to 1,000 tokens (its choices are 1.5 % slower than the best of them on
 // average, 11 % at worst). A CTA takes in its blocks of K at about 115 bytes a nanosecond, two on one SM together at 136;
 // every wave adds the epilogue: 42 ns a token of the tile, 12 per token of the share, a microsecond for the exchange of
 // pieces and 170 ns per piece. Clusters of 4 and 8 do not find room on every SM: 136 and 128 CTAs at a time.
-Plan plan_of(int mode, int M, int N, int K) {
+Plan plan_of(int mode, int M, int N, int K, double* estimate = nullptr) {
     const int parts = parts_of(mode);
     const int row_tiles = (N + BW * parts - 1) / (BW * parts), num_kb = (K + BK - 1) / BK;
     const int sms = sp_sm_count() > 0 ? sp_sm_count() : 148;
@@ -498,6 +498,7 @@ Plan plan_of(int mode, int M, int N, int K) {
                              + waves * (42.0 * p.nt + 12.0 * p.nt / pieces + (pieces > 1 ? 1000.0 : 0.0) + 170.0 * pieces);
             if (best.nt == 0 || t < best_t) { best = p; best_t = t; }
         }
+    if (estimate) *estimate = best_t;
     return best;
 }
 
@@ -521,6 +522,30 @@ SP_API int sp_tc_mid_plan(int mode, int M, int N, int K, int* out) {
     const Plan p = plan_of(mode, M, N, K);
     out[0] = p.token_tiles; out[1] = p.nt; out[2] = p.pieces; out[3] = p.stages;
     return p.nt ? 0 : 1;
+}
+
+// Which kernel takes a product of more than 128 tokens that both this one and the tiles by pairs of CTAs of tc_gemm.cu (256
+// rows, 74 pairs on 148 SMs) could: the width of those tiles, a multiple of ``multiple``, or 0 for this kernel. By the two
+// estimates of time: a round of pair tiles takes 0.36 us per 64 of K at 256 columns, 0.335 at 192 and 0.31 at 128, and the
+// launch with its last epilogue 10 us (measured at 128 to 6,000 tokens of the 1B and 8B layer sizes: within 15 %).
+// Gated products are worth pairs as soon as their rounds come out full, for they have the most rows of W (us, this kernel /
+// pairs: 1B 200 tokens 24.8 / 21.1, 301: 27.7 / 31.6, 512: 37.4 / 32.6, 1,023: 71.8 / 58.2; 8B 512: 122 / 103, 768: 206 / 138); the
+// others from 1,024 tokens on, this kernel still where their pair tiles fill few SMs (1B, 1,280 tokens: output 16.1 / 20.2,
+// down 40.5 / 51.7, 1,700 QKV 22.6 / 30.3; 8B 1,280 down 125 / 168).
+SP_API int sp_tc_mid_or_pairs(int mode, int M, int N, int K, int multiple) {
+    const bool gated = mode == MODE_SILU_MUL;
+    if (M <= 128 || (!gated && M < 1024)) return 0;
+    const int walkers = (sp_sm_count() > 0 ? sp_sm_count() : 148) / 2, row_tiles = (M + 255) / 256, num_kb = (K + BK - 1) / BK;
+    int best = 0;
+    double best_t = 0;
+    for (const int bn : {256, 192, 128}) {
+        if ((gated && bn != 256) || (multiple > 1 && bn % multiple)) continue;
+        const int rounds = (row_tiles * ((N + bn - 1) / bn) + walkers - 1) / walkers;
+        const double t = 10000.0 + (double)rounds * num_kb * (bn == 256 ? 360.0 : bn == 192 ? 335.0 : 310.0);
+        if (!best || t < best_t) { best = bn; best_t = t; }
+    }
+    double mine = 0;
+    return M <= 2048 && plan_of(mode, M, N, K, &mine).nt && mine < best_t ? 0 : best;
 }
 
 // Whether this kernel takes the product (0) or another has to (1, the reason as the last error).

@@ -4,7 +4,8 @@ Part by part a layer is eight launches: norm, QKV, rotate-and-store, attention, 
 down. When every layer's parts describe themselves through ``fused_fields()`` (the same pre-norm / RMS norm / rotary
 grouped-query attention / SwiGLU, bfloat16 description that the one-kernel decode path reads) a step of 17 tokens
 or more runs each layer as five: up to ``MID_TOKENS`` on ``tc_mid`` (a prompt, or a decode step of that many sequences),
-beyond on the tile kernel, ``tc_gemm``. Where gate and up rows lie in blocks of 64 ``tc_mid`` does not take the layer:
+beyond on the tile kernel, ``tc_gemm``; the gated product, and beyond ``MID_TOKENS`` every product, on whichever of the two
+is the faster at its sizes. Where gate and up rows lie in blocks of 64 ``tc_mid`` does not take the layer:
 ``tc_stream`` does up to 64 tokens and ``tc_gemm`` from 129 on, and between them the step runs part by part (the tile
 kernel then splits K over a cluster, which has no such epilogues):
 
@@ -25,7 +26,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import lib as K
-from ..parts.linear import MID_TOKENS, STREAM_TOKENS, sm_count, tile_width
+from ..parts.linear import MID_TOKENS, PAIR_TOKENS, STREAM_TOKENS, sm_count, tile_width
 from .fused_decode import collect_fused_fields, five_launch_from
 from ..phases import phase
 
@@ -110,8 +111,16 @@ class FusedPrefill:
         stream = not mid and T <= STREAM_TOKENS        # the kernel that streams the weights takes these few tokens
         schedule = self.model.spec.schedule
 
+        paired = self.mid and T >= PAIR_TOKENS         # each product by pairs of CTAs, or on tc_mid where that is the faster one
+
+        def width_of(mode, w, bn, multiple=1):
+            """The width of tc_gemm's tiles; 0 where tc_mid takes the product."""
+            if mid or paired:
+                return K.tc_mid_or_pairs(mode, T, w.shape[0], w.shape[1], multiple)
+            return bn
+
         def product(a, w, out, mode, bn, pair=0, **kw):
-            if mid:
+            if (mid or paired) and not bn:
                 K.tc_mid_fused(a, w, out, mode, pair, **kw)
             elif stream:
                 K.tc_stream_fused(a, w, out, mode, pair, **kw)
@@ -119,13 +128,13 @@ class FusedPrefill:
                 K.tc_gemm_fused(a, w, out, mode, bn, **kw)
 
         def res_tiles(bn):
-            return K.tc_stream_n_tiles(H) if mid or stream else K.tc_gemm_n_tiles(H, bn)
+            return K.tc_stream_n_tiles(H) if stream or not bn else K.tc_gemm_n_tiles(H, bn)
 
         def into_residual(a, w, next_w):
             """h += a·wᵀ, and the next norm's input: (residual ⊙ next_w in bfloat16, the rows' sums of squares)."""
-            bn = tile_width(T, H, sms)
+            bn = width_of(K.TC_ACCUMULATE, w, 0 if mid or paired else tile_width(T, H, sms))
             xw = torch.empty(T, H, dtype=bf, device=dev)
-            if not (mid or stream) and K.tc_gemm_splits(T, H, a.shape[1], bn) > 1:
+            if not (mid or paired or stream) and K.tc_gemm_splits(T, H, a.shape[1], bn) > 1:
                 # few tiles and a long K (the down projection of a few hundred tokens): the kernel that splits K over a
                 # cluster has the plain epilogues only, so the norm's input is a small kernel of its own behind it
                 ssq = torch.empty(T, 1, dtype=torch.float32, device=dev)
@@ -150,7 +159,7 @@ class FusedPrefill:
                 cs, tok_page = self._tables(step, view, m["inv_freq"], self.rope_id[i])
             q = torch.empty(T, nh * hd, dtype=bf, device=dev)
             n_qkv = m["qkv"].shape[0]
-            bn = tile_width(T, n_qkv, sms)
+            bn = width_of(K.TC_QKV_ROPE, m["qkv"], 0 if mid or paired else tile_width(T, n_qkv, sms), hd)
             if bn % hd:
                 bn = 256
             with phase("attention_norm+qkv_projection+rotary+kv_append_ms"):
@@ -165,15 +174,15 @@ class FusedPrefill:
             # ---- gate/up with silu(gate)·up on the normed residual
             act = torch.empty(T, ff["intermediate_size"], dtype=bf, device=dev)
             with phase("mlp_norm+gate_projection+up_projection+activation_multiply_ms"):
-                product(xw, ff["gate_up"], act, K.TC_SILU_MUL, 2 * ff["pair"], ff["pair"], row_ssq=ssq, norm_width=H,
-                        eps=f["ffn_norm"]["eps"])
+                product(xw, ff["gate_up"], act, K.TC_SILU_MUL, width_of(K.TC_SILU_MUL, ff["gate_up"], 2 * ff["pair"]), ff["pair"],
+                        row_ssq=ssq, norm_width=H, eps=f["ffn_norm"]["eps"])
             # ---- down projection into the residual, preparing the next layer's first norm
             with phase("down_projection+mlp_residual_ms"):
                 if i + 1 < len(self.fields):
                     xw, ssq = into_residual(act, ff["down"], self.fields[i + 1]["mixer_norm"]["weight"])
-                elif mid:
+                elif mid or (paired and not width_of(K.TC_ACCUMULATE, ff["down"], 0)):
                     K.tc_mid(act, ff["down"], h, K.TC_ACCUMULATE)
                 elif stream:
                     K.tc_stream(act, ff["down"], h, K.TC_ACCUMULATE)
                 else:
-                    K.tc_gemm(act, ff["down"], h, K.TC_ACCUMULATE, tile_width(T, H, sms))
+                    K.tc_gemm(act, ff["down"], h, K.TC_ACCUMULATE, width_of(K.TC_ACCUMULATE, ff["down"], 0) or tile_width(T, H, sms))

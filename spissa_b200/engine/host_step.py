@@ -32,7 +32,7 @@ class _Kernels(ctypes.Structure):
         "rmsnorm", "gemv", "gemv_supported", "tc_stream", "tc_stream_supported", "tc_gemm", "tc_gemm_supported",
         "gemm_generic", "silu_mul", "rope_kv_write", "flash_prefill", "err_generic", "err_gemv", "err_tc_stream",
         "err_tc_gemm", "err_attention", "tc_stream_fused", "rope_table", "norm_prepare", "tc_mid", "tc_mid_supported",
-        "err_tc_mid", "flash_prefill_tc", "err_flash_tc")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
+        "err_tc_mid", "flash_prefill_tc", "err_flash_tc", "tc_gemm_fused", "mid_or_pairs")] + [("gemv_tokens", c_int), ("stream_tokens", c_int),
                                             ("flash_query_tile", c_int), ("mid_tokens", c_int),
                                             ("flash_tc_from", c_int), ("pad", c_int)]
 
@@ -83,6 +83,7 @@ def _bind(flash_tc: bool) -> ctypes.CDLL:
     t.err_attention = _address(att, "sp_attention_last_error")
     t.tc_mid, t.tc_mid_supported = _address(mid, "sp_tc_mid"), _address(mid, "sp_tc_mid_supported")
     t.err_tc_mid = _address(mid, "sp_tc_mid_last_error")
+    t.tc_gemm_fused, t.mid_or_pairs = _address(gemm, "sp_tc_gemm_fused"), _address(mid, "sp_tc_mid_or_pairs")
     t.gemv_tokens, t.stream_tokens, t.mid_tokens = L.GEMV_TOKENS, L.STREAM_TOKENS, L.MID_TOKENS
     if flash_tc:
         tc = K.load("flash_tc")

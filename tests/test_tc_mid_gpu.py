@@ -275,3 +275,47 @@ def test_experts_of_many_tokens_take_the_tiles_of_128(K, monkeypatch):
     assert float((rows[0] - rows[1]).norm() / rows[0].norm()) <= 2.0 ** -8
     with pytest.raises(K.KernelError):
         K._check("hybrid", K.load("hybrid").sp_moe_plan_tiles(None, None, 8, 1, 64, 1, 1, 1, None, None, None, None, None, None, 4, 100, None, None))
+
+
+@pytest.mark.parametrize("act", ["ACT_SILU", "ACT_GELU", "ACT_CLAMPED"])
+@pytest.mark.parametrize("M", [129, 255, 256, 257, 400, 513, 1025, 1152, 1300])
+def test_gated_products_by_pairs_of_ctas(K, M, act):
+    """The tiles of 256 rows that gated products take from 129 tokens on: rows behind the last token, gates of all sizes."""
+    act = getattr(K, act)
+    limit, slope = (7.0, 1.7) if act == K.ACT_CLAMPED else (0.0, 0.0)
+    a, w = operands(M, 768, 200)
+    a[0], a[M - 1] = 0.0, a[M - 1] * 60.0                               # gates of zero, and some beyond the branch-free range
+    out = torch.full((M + 3, 384), 9.0, device=DEV)
+    K.tc_gemm(a, w, out[:M], K.TC_SILU_MUL, 256, act=act, limit=limit, slope=slope)
+    y = (a.double() @ w.double().t()).view(M, 3, 2, 128)
+    g, u = y[:, :, 0].reshape(M, 384), y[:, :, 1].reshape(M, 384)
+    if act == K.ACT_CLAMPED:
+        g, u = g.clamp(max=limit), u.clamp(-limit, limit) + 1.0
+    ref = torch.nn.functional.gelu(g, approximate="tanh") * u if act == K.ACT_GELU else g * torch.sigmoid((slope or 1.0) * g) * u
+    # the sums' error (200 terms of at most 0.1 · 60 · 4 in 2^-23 each) through an activation of slope 1.1 and the other factor
+    bound = 1.2 * 200 * 2.0 ** -23 * (a.double().abs() @ w.double().abs().t()).amax(1, keepdim=True) * (1.0 + g.abs() + u.abs())
+    assert bool(((out[:M].double() - ref).abs() <= bound).all())
+    assert bool((out[M:] == 9.0).all())
+
+
+def test_the_choice_between_the_two_kernels(K):
+    for N, Kd in ((3072, 2048), (16384, 2048), (28672, 4096), (4096, 14336), (40, 64)):
+        for M in (1, 128, 129, 300, 1023, 1024, 1500, 2048, 2049, 6000):
+            for mode in (K.TC_STORE, K.TC_SILU_MUL):
+                width = K.tc_mid_or_pairs(mode, M, N, Kd, 128)
+                assert width in (0, 128, 256) and not (width and M <= 128) and (width or M <= 2048)
+                assert mode == K.TC_SILU_MUL or not width or M >= 1024
+                assert mode != K.TC_SILU_MUL or width in (0, 256)
+    assert K.tc_mid_or_pairs(K.TC_ACCUMULATE, 1280, 2048, 8192) == 0 and K.tc_mid_or_pairs(K.TC_ACCUMULATE, 2048, 2048, 8192) == 256
+    assert K.tc_mid_or_pairs(K.TC_SILU_MUL, 301, 16384, 2048) == 0 and K.tc_mid_or_pairs(K.TC_SILU_MUL, 512, 16384, 2048) == 256
+
+
+@pytest.mark.parametrize("M", [1024, 1279, 1537, 2048])
+@pytest.mark.parametrize("N,Kd", [(2048, 512), (520, 1096)])
+def test_linear_of_more_tokens(K, M, N, Kd):
+    from spissa_b200.parts.linear import Linear
+    a, w = operands(M, N, Kd)
+    c0 = torch.randn(M, N, device=DEV)
+    acc = c0.clone()
+    Linear(w)(a, out=acc, accumulate=True)
+    within(acc, a, w, extra=c0)
