@@ -7,6 +7,7 @@ they stand. The arrays travel to the device as ONE int32 buffer and one copy.
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -64,19 +65,16 @@ def pack_step(entries, lengths_before, kv_tables: dict, device, pinned: bool = T
     widths = {g: max(1, max(len(p) for p in rows)) for g, rows in kv_tables.items()}
     sizes = [T, T, T, B + 1, B, B, B, W] + [B * widths[g] for g in kv_tables]
     total = sum(sizes)
-    flat = torch.empty(total, dtype=torch.int32, pin_memory=pinned and torch.cuda.is_available())
+    on_gpu = torch.device(device).type == "cuda"
+    flat = torch.empty(total, dtype=torch.int32, pin_memory=pinned and (on_gpu or torch.cuda.is_available()))
     small = seq_start + seq_slot + list(range(B)) + seq_len + want_rows
     for g, rows in kv_tables.items():
         w = widths[g]
         for r in rows:
             small.extend(r)
             small.extend([0] * (w - len(r)))
-    torch.cat(tok_parts + pos_parts + seq_parts + [torch.tensor(small, dtype=torch.int32)], out=flat)
-    dev = flat.to(device, non_blocking=True)
-    views, off = [], 0
-    for s in sizes:
-        views.append(dev[off:off + s])
-        off += s
+    torch.cat(tok_parts + pos_parts + seq_parts + [torch.frombuffer(array("i", small), dtype=torch.int32)], out=flat)
+    views = flat.to(device, non_blocking=True).split(sizes)
     page_tables = {}
     for i, g in enumerate(kv_tables):
         page_tables[g] = views[8 + i].view(B, widths[g])

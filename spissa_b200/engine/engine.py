@@ -9,6 +9,7 @@ final norm, last row, head; position offset = cached length, :326).
 """
 from __future__ import annotations
 
+from array import array
 import json
 import sys
 from dataclasses import dataclass
@@ -183,16 +184,7 @@ class Engine:
             if not toks:
                 raise StepError(f"slot {slot}: a sequence of a step brings at least one token")
             if len(toks) > 32:
-                # a prompt: checked as a tensor (which the packing below takes as it is)
-                try:
-                    as_tensor = torch.tensor(toks, dtype=torch.int64)
-                except (TypeError, ValueError, RuntimeError, OverflowError):
-                    raise StepError(f"slot {slot}: token ids must be integers") from None
-                bad = (as_tensor < 0) | (as_tensor >= self.vocab_size)
-                if bool(bad.any()):
-                    t = int(as_tensor[bad][0])
-                    raise StepError(f"slot {slot}: token id {t} is outside the vocabulary of {self.vocab_size}")
-                packed[len(lengths)] = as_tensor.to(torch.int32)
+                packed[len(lengths)] = self._prompt_tensor(slot, toks)
             else:
                 for t in toks:
                     if not (0 <= int(t) < self.vocab_size):
@@ -204,6 +196,26 @@ class Engine:
             self._check_position(slot, before, len(toks))
             lengths.append(before)
         return lengths, packed
+
+    def _prompt_tensor(self, slot: int, toks) -> torch.Tensor:
+        """A prompt's tokens as an int32 tensor, which the packing takes as it is; refused where one is out of range."""
+        try:
+            # a quarter of what torch.tensor takes for a list (2,048 tokens: 24 us, 92 there)
+            as_tensor = torch.frombuffer(array("i", toks), dtype=torch.int32)
+            low, high = torch.aminmax(as_tensor)
+            if int(low) >= 0 and int(high) < self.vocab_size:
+                return as_tensor
+        except (TypeError, OverflowError):
+            pass                                         # not all of them integers of 32 bits: below
+        try:
+            as_tensor = torch.tensor(toks, dtype=torch.int64)
+        except (TypeError, ValueError, RuntimeError, OverflowError):
+            raise StepError(f"slot {slot}: token ids must be integers") from None
+        bad = (as_tensor < 0) | (as_tensor >= self.vocab_size)
+        if bool(bad.any()):
+            t = int(as_tensor[bad][0])
+            raise StepError(f"slot {slot}: token id {t} is outside the vocabulary of {self.vocab_size}")
+        return as_tensor.to(torch.int32)
 
     def _check_position(self, slot: int, before: int, new: int) -> None:
         # the reference refuses a turn that would pass max_seq_len before anything runs
@@ -310,8 +322,11 @@ class Engine:
         never been asked for. ``check=False`` returns without waiting; such steps are settled by the next checked
         step, by ``check()`` or ``settle()``, and until then ``length`` counts them.
         """
-        ents = [(e.slot, list(e.tokens), list(e.want)) if isinstance(e, StepEntry)
-                else (e[0], list(e[1]), list(e[2])) for e in entries]
+        def as_list(x):                                  # (nothing below changes the caller's lists)
+            return x if type(x) is list else list(x)
+
+        ents = [(e.slot, as_list(e.tokens), as_list(e.want)) if isinstance(e, StepEntry)
+                else (e[0], as_list(e[1]), as_list(e[2])) for e in entries]
         lengths, packed = self._validate(ents)
         counts = [(slot, len(toks)) for slot, toks, _ in ents]
         with torch.cuda.device(self.device):
