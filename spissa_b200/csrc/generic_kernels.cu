@@ -1046,27 +1046,35 @@ SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, cons
 
 // The same attention in 32 bits for prompts, by tiles: a CTA takes 64 queries of one (sequence, head) and walks the keys 64
 // at a time through shared memory, each of 256 threads 4 x 4 scores and 4 x 4 (per 64 value columns) sums. The kernel
-// above reads every key once per query; here a key is read once per 64 queries (500 tokens, 32 heads of 64 on 8 kv heads:
-// 423 us by the kernel above, 110 us here). Sums, softmax and exponentials are float32 as there; only their order differs.
+// above reads every key once per query; here a key is read once per 64 queries, and the next tile's rows are copied into a
+// second buffer under this one's products (500 tokens, 32 heads of 64 on 8 kv heads: 423 us by the kernel above, 114 us with a
+// tile's rows fetched in front of its products one piece after another, 66 us here; the products' FFMAs alone are 17).
+// Sums, softmax and exponentials are float32 as there; only their order differs.
 #define AT_TILE 64
 #define AT_MAX_D 128
 template <int VC>
 __global__ void __launch_bounds__(256)
 attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__ kpool, const float* __restrict__ vpool,
                           float* __restrict__ out, KvPlace pl, const int* __restrict__ seq_start, int nh, int nkv, int hd, int vd,
-                          int window, float scale, const float* __restrict__ sink, const float* __restrict__ dist_bias, int dist_cap) {
+                          int window, float scale, const float* __restrict__ sink, const float* __restrict__ dist_bias, int dist_cap,
+                          int n_seqs, int sms) {
     extern __shared__ __align__(16) float at_smem[];
-    const int s = blockIdx.z, h = blockIdx.y, g = h / (nh / nkv);
-    const int tile = gridDim.x - 1 - blockIdx.x;             // the tiles with the most keys first
+    // The tiles with the most keys first, all heads of them side by side; every second round of CTAs over the SMs goes backwards,
+    // so that an SM's two CTAs are one of many keys and one of few (500 tokens: 8 tiles of keys on every SM; tile by tile of a
+    // head it was 12 on some and 5 on others: 94 us, and 66 so).
+    int at_cta = blockIdx.x;
+    const int turn_of = at_cta / sms, turn_from = turn_of * sms, turn_to = min((int)gridDim.x, turn_from + sms);
+    if (turn_of & 1) at_cta = turn_from + turn_to - 1 - at_cta;
+    const int side_by_side = nh * n_seqs, s = at_cta % side_by_side / nh, h = at_cta % nh, g = h / (nh / nkv);
+    const int tile = (int)gridDim.x / side_by_side - 1 - at_cta / side_by_side;
     const int t0 = seq_start[s] + tile * AT_TILE, rows = min(AT_TILE, seq_start[s + 1] - t0);
     if (rows <= 0) return;
     // rows of four more words: sixteen neighbouring rows fall on different banks
     const int ks = hd + 4, vs = vd + 4;
     constexpr int PS = AT_TILE + 4;
     float* const Q = at_smem;
-    float* const Kt = Q + AT_TILE * ks;
-    float* const V = Kt + AT_TILE * ks;
-    float* const P = V + AT_TILE * vs;
+    float* const P = Q + AT_TILE * ks;
+    float* const KV = P + AT_TILE * PS;                      // two tiles of keys and values
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int slot = sp_checked_row(pl.seq_slot[s], pl.rg);
     const int* pt = pl.page_table + (size_t)slot * pl.max_pages;
@@ -1086,21 +1094,39 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
         for (int c = 0; c < 4 * VC; ++c) acc[i][c] = 0.0f;
     }
     const int lo = window > 0 ? max(0, first - window + 1) : 0;
-    for (int j0 = lo; j0 <= last; j0 += AT_TILE) {
+    const int mine = tid >> 2, c_mine = (tid & 3) * 4;       // four threads copy a row: every fourth 16 bytes each
+    auto fetch = [&](int j0, float* to) {
+        const int j = j0 + mine;
+        const bool there = j <= last;
+        size_t at = 0;
+        if (there) {
+            const int page = sp_checked_page(pt[sp_checked_entry(j / ps, pl.max_pages, pl.rg)], pl.rg);
+            at = ((size_t)page * nkv + g) * ps + j % ps;
+        }
+        auto copy = [&](float* dst, const float* src) {      // zeros where there is no such key
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+        };
+        for (int c = c_mine; c < hd; c += 16) copy(to + mine * ks + c, kpool + at * hd + c);
+        for (int c = c_mine; c < vd; c += 16) copy(to + AT_TILE * ks + mine * vs + c, vpool + at * vd + c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int turn = 0;
+    fetch(lo, KV);
+    for (int j0 = lo; j0 <= last; j0 += AT_TILE, turn ^= 1) {
+        float* const Kt = KV + turn * (AT_TILE * (ks + vs));
+        float* const V = Kt + AT_TILE * ks;
         __syncthreads();                                     // the tile before has been used
-        const int qd = (hd + vd) / 4;
+        if (j0 + AT_TILE <= last) {
+            fetch(j0 + AT_TILE, KV + (turn ^ 1) * (AT_TILE * (ks + vs)));
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
         int odd = 0;                                         // an infinity or NaN among this thread's pieces of the values
-        for (int e = tid; e < AT_TILE * qd; e += 256) {
-            const int r = e / qd, c = (e % qd) * 4, j = j0 + r;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j <= last) {
-                const int page = sp_checked_page(pt[sp_checked_entry(j / ps, pl.max_pages, pl.rg)], pl.rg);
-                const size_t at = ((size_t)page * nkv + g) * ps + j % ps;
-                v = c < hd ? *(const float4*)(kpool + at * hd + c) : *(const float4*)(vpool + at * vd + (c - hd));
-            }
-            *(float4*)(c < hd ? Kt + r * ks + c : V + r * vs + (c - hd)) = v;
+        for (int c = c_mine; c < vd; c += 16) {
+            const float4 v = *(const float4*)(V + mine * vs + c);
             // x - x is NaN for what is not finite, else zero
-            if (c >= hd) odd |= (v.x - v.x) + (v.y - v.y) + (v.z - v.z) + (v.w - v.w) != 0.0f;
+            odd |= (v.x - v.x) + (v.y - v.y) + (v.z - v.z) + (v.w - v.w) != 0.0f;
         }
         odd = __syncthreads_or(odd);
         float sc[4][4] = {};
@@ -1227,9 +1253,12 @@ SP_API int sp_attention_tile_f32(const float* q, const float* kpool, const float
     if (dist_bias && dist_cap < 0) SP_FAIL("attention: a distance-bias table needs at least one entry per head");
     if (((uintptr_t)q | (uintptr_t)kpool | (uintptr_t)vpool | (uintptr_t)out) & 15) SP_FAIL("attention: the tiled kernel needs tensors on 16-byte boundaries");
     KvPlace pl{nullptr, positions, seq_slot, page_table, max_pages, page_size, sp_range_host};
-    const dim3 grid((max_new + AT_TILE - 1) / AT_TILE, nh, n_seqs);
-    const int most = (3 * AT_TILE * (AT_MAX_D + 4) + AT_TILE * (AT_TILE + 4)) * 4;
-    const int smem = (2 * AT_TILE * (hd + 4) + AT_TILE * (vd + 4) + AT_TILE * (AT_TILE + 4)) * 4;
+    const long long ctas = (long long)((max_new + AT_TILE - 1) / AT_TILE) * nh * n_seqs;
+    if (ctas > 2147483647LL) SP_FAIL("attention: too many tiles of queries for one launch");
+    const unsigned grid = (unsigned)ctas;
+    const int sms = sp_sm_count() > 0 ? sp_sm_count() : 148;
+    const int most = (5 * AT_TILE * (AT_MAX_D + 4) + AT_TILE * (AT_TILE + 4)) * 4;
+    const int smem = (3 * AT_TILE * (hd + 4) + 2 * AT_TILE * (vd + 4) + AT_TILE * (AT_TILE + 4)) * 4;
     static SpPerDevice configured;
     if (!configured.done()) {
         cudaError_t e = cudaFuncSetAttribute(attention_tile_f32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -1237,8 +1266,8 @@ SP_API int sp_attention_tile_f32(const float* q, const float* kpool, const float
         if (e != cudaSuccess) SP_FAIL("attention: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
         configured.mark();
     }
-    if (vd <= 64) attention_tile_f32_kernel<1><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap);
-    else attention_tile_f32_kernel<2><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap);
+    if (vd <= 64) attention_tile_f32_kernel<1><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap, n_seqs, sms);
+    else attention_tile_f32_kernel<2><<<grid, 256, smem, stream>>>(q, kpool, vpool, out, pl, seq_start, nh, nkv, hd, vd, window, scale, sink, dist_bias, dist_cap, n_seqs, sms);
     SP_CHECK_LAUNCH("attention_tile_f32");
     return 0;
 }
