@@ -16,14 +16,17 @@
 // A value that is not finite has no such parts: a CTA that meets one computes its tile again with plain FFMA.
 //
 //   warps 0-15  split, block of 64 of K by block, 128 x 64 of W and tokens x 64 of A (fetched a block ahead into registers, 32
-//               bytes a load) into three tiles each in the swizzled layout of the instruction's operands, and add the finished
-//               accumulator of the block before (two in tensor memory, in turn) to their sums in registers: a thread has a
-//               row of W and 32 tokens;
-//   warp 16     issues tcgen05.mma: M 128 rows of W, N tokens, K 16, small products first.
-// What bounds it is the path to shared memory: of a block's 2.0 us at 128 tokens some 1.5 are its 128 bytes a cycle (split
-// tiles in 768 cycles, the loads 512, the instructions' operands 1,536). 500 tokens x 16,384 x 2,048: 272 us = 123 TFLOP/s
-// (1,640 us on FFMA tiles; 345 with 16-byte loads and all warps in step; adding an accumulator only every 256 terms of K is
-// 3 % faster and ten times as far from the exact result: the small products are cut off against a large sum).
+//               bytes a load) into three tiles each in the swizzled layout of the instruction's operands;
+//   warps 16-19 add the finished accumulator of the block before (two in tensor memory, in turn) to the sums, which stand behind
+//               them in tensor memory: 128 rows of W x tokens;
+//   warp 20     issues tcgen05.mma: M 128 rows of W, N tokens, K 16, small products first.
+// What bounds it is the path to shared memory: of a block's 1.65 us at 128 tokens 1.45 are its 128 bytes a cycle (split
+// tiles in 768 cycles, the loads 512, the instructions' operands 1,536). 500 tokens x 16,384 x 2,048: 239 us = 140 TFLOP/s
+// (1,640 us on FFMA tiles; 345 with 16-byte loads and all warps in step; 262 with the sums in the splitting warps' registers,
+// which read every accumulator between two blocks; 219 by pairs of CTAs, M 256 and N 256 in two halves, but its other products
+// 62 / 62 / 204 for 60 / 38 / 114 here: an accumulator's way through both CTAs' barriers takes longer than a block).
+// Adding an accumulator only every 256 terms of K is 3 % faster and ten times as far from the exact result: the small products
+// are cut off against a large sum.
 // K is cut over the CTAs of a cluster where the tiles alone leave SMs idle; the pieces are added in order through
 // distributed shared memory. Every wait is bounded and records a code in ``status``.
 #include "tcgen05.cuh"
@@ -37,9 +40,9 @@ constexpr int BW = 128;                     // rows of W per CTA
 constexpr int BK = 64;                      // K per stage: 64 bf16 of a part = 128 bytes = one swizzle span
 constexpr int MAX_NT = 128;                 // tokens per CTA
 constexpr int STAGES = 2;                   // of split operands, and accumulators
-constexpr int WARPS = 16;
-constexpr int THREADS = 32 * (WARPS + 1);
-constexpr int GROUP = 1;                    // blocks of K whose products one accumulator takes before it is added to the sums
+constexpr int WARPS = 16;                   // that split operands; four that add accumulators to the sums and one that issues the products
+constexpr int ISSUER = WARPS + 4;
+constexpr int THREADS = 32 * (ISSUER + 1);
 constexpr int PART_W = BW * BK * 2;
 constexpr int MAX_PIECES = 8;
 
@@ -117,7 +120,7 @@ tc_f32_kernel(const Args a) {
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_done[b]), 1);
-            mbar_init(smem_u32(&bar_free[b]), WARPS);
+            mbar_init(smem_u32(&bar_free[b]), 4);
         }
         odd = 0;
         failed = 0;
@@ -125,20 +128,17 @@ tc_f32_kernel(const Args a) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
-    if (warp == WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(256u) : "memory");
+    if (warp == ISSUER) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(4u * MAX_NT) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
-    const int row = (warp & 3) * 32 + lane, j32 = (warp >> 2) * 32;      // a thread's row of W and its 32 tokens
-    uint64_t sum[16];                                             // in pairs
-#pragma unroll
-    for (int j = 0; j < 16; ++j) sum[j] = 0ull;
-
-    const int groups = (blocks + GROUP - 1) / GROUP;
+    const int row = (warp & 3) * 32 + lane;                       // a thread's row of W
+    const uint32_t lanes = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    // tensor memory: two accumulators, which take the blocks of K in turn, and the sums behind them
     if (warp < WARPS) {
         // eight lanes take the 64 values of a row, a warp four rows at a time; the 16-byte stores of eight lanes fall on the
         // eight swizzled places of one row: no bank conflicts
@@ -164,30 +164,10 @@ tc_f32_kernel(const Args a) {
             fetch(w_at, a.ldw, w_ok[t], t, kb0, wl[t], wh[t]);
             fetch(a_at, a.lda, a_ok[t], t, kb0, al[t], ah[t]);
         }
-        auto add_group = [&](int g) -> bool {
-            const int b = g & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait_flag(smem_u32(&bar_done[b]), ((uint32_t)g >> 1) & 1u, a.status, 142, &failed))) return false;
-            tc_fence_after();
-            if (j32 < a.nt) {                                     // uniform in the warp
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    uint32_t r[8];
-                    tc_ld_32x8(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * MAX_NT + j32 + 8 * h), r);
-                    tc_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) sum[4 * h + j] = add2(sum[4 * h + j], pair(r[2 * j], r[2 * j + 1]));
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_free[b]));
-            return true;
-        };
         uint64_t check = 0;
-        bool going = true;
         for (int i = 0; i < blocks; ++i) {
             const int s = i & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait_flag(smem_u32(&bar_empty[s]), (((uint32_t)i >> 1) & 1u) ^ 1u, a.status, 143, &failed))) { going = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait_flag(smem_u32(&bar_empty[s]), (((uint32_t)i >> 1) & 1u) ^ 1u, a.status, 143, &failed))) break;
             const uint32_t dst = smem_base + (uint32_t)s * stage_bytes;
             const bool more = i + 1 < blocks;
 #pragma unroll
@@ -211,21 +191,42 @@ tc_f32_kernel(const Args a) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_full[s]));
-            // the group before is finished when this one's second block has been split
-            if (i >= GROUP && i % GROUP == (GROUP > 1 ? 1 : 0) && !(going = add_group(i / GROUP - 1))) break;
-        }
-        if (going) {
-            if (GROUP > 1 && groups > 1 && (blocks - 1) % GROUP == 0) going = add_group(groups - 2);       // the last group has one block only
-            if (going) add_group(groups - 1);
         }
         uint32_t c_lo, c_hi;
         unpair(check, c_lo, c_hi);
         if ((c_lo | c_hi) & 0x7fffffffu) odd = 1;
+    } else if (warp < ISSUER) {
+        // an accumulator's 32-bit values into the sums, rounded to nearest
+        for (int i = 0; i < blocks; ++i) {
+            const int b = i & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait_flag(smem_u32(&bar_done[b]), ((uint32_t)i >> 1) & 1u, a.status, 142, &failed))) break;
+            tc_fence_after();
+            const uint32_t from = lanes + (uint32_t)(b * MAX_NT), to = lanes + (uint32_t)(2 * MAX_NT);
+            for (int c = 0; c < a.nt; c += 16) {
+                uint32_t r[16], t[16];
+                tc_ld_32x8(from + c, r);
+                tc_ld_32x8(from + c + 8, r + 8);
+                if (i > 0) {
+                    tc_ld_32x8(to + c, t);
+                    tc_ld_32x8(to + c + 8, t + 8);
+                }
+                tc_ld_wait();
+                if (i > 0) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) unpair(add2(pair(t[j], t[j + 1]), pair(r[j], r[j + 1])), r[j], r[j + 1]);
+                }
+                tc_st_32x16(to + c, r);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bar_free[b]));
+            tc_st_wait();
+        }
     } else if (lane == 0) {
         const uint32_t idesc = umma_idesc_bf16(BW, a.nt);
         for (int i = 0; i < blocks; ++i) {
-            const int s = i & 1, g = i / GROUP, b = g & 1;
-            if (i % GROUP == 0 && !mbar_wait_flag(smem_u32(&bar_free[b]), (((uint32_t)g >> 1) & 1u) ^ 1u, a.status, 144, &failed)) break;
+            const int s = i & 1, b = i & 1;
+            if (!mbar_wait_flag(smem_u32(&bar_free[b]), (((uint32_t)i >> 1) & 1u) ^ 1u, a.status, 144, &failed)) break;
             if (!mbar_wait_flag(smem_u32(&bar_full[s]), ((uint32_t)i >> 1) & 1u, a.status, 141, &failed)) break;
             tc_fence_after();
             const uint32_t src = smem_base + (uint32_t)s * stage_bytes;
@@ -237,40 +238,38 @@ tc_f32_kernel(const Args a) {
                 const uint64_t da = umma_desc_sw128(src + 3 * PART_W + PA[p] * part_a);
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    tc_mma_bf16(tmem_base + (uint32_t)(b * MAX_NT), dw + 2 * k, da + 2 * k, idesc, (i % GROUP | p | k) != 0 ? 1u : 0u);
+                    tc_mma_bf16(tmem_base + (uint32_t)(b * MAX_NT), dw + 2 * k, da + 2 * k, idesc, (p | k) != 0 ? 1u : 0u);
             }
             tc_commit(smem_u32(&bar_empty[s]));
-            if (i % GROUP == GROUP - 1 || i + 1 == blocks) tc_commit(smem_u32(&bar_done[b]));
+            tc_commit(smem_u32(&bar_done[b]));
         }
     }
+    tc_fence_before();
     __syncwarp();
-    __syncthreads();                                              // all products are done (or a wait was given up), ``odd`` is known
+    // all products are done (or a wait was given up), ``odd`` is known
+    __syncthreads();
+    tc_fence_after();
     if (warp < WARPS) {
-        if (odd) {
-            // infinities or NaN among the operands: this piece again, term by term
-            const int k0 = kb0 * BK, k1 = min(a.K, (kb0 + blocks) * BK);
-            const float* w = a.W + (size_t)min(row0 + row, a.N - 1) * a.ldw;
+        // the sums, [token][row of W], into shared memory, whose stages are free
+        for (int c = (warp >> 2) * 8; c < a.nt; c += 32) {
+            uint32_t r[8];
+            tc_ld_32x8(lanes + (uint32_t)(2 * MAX_NT + c), r);
+            tc_ld_wait();
+            if (odd) {
+                // infinities or NaN among the operands: this piece again, term by term
+                const int k1 = min(a.K, (kb0 + blocks) * BK);
+                const float* w = a.W + (size_t)min(row0 + row, a.N - 1) * a.ldw;
+                float again[8] = {};
+                for (int k = kb0 * BK; k < k1; ++k)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sum[j] = 0ull;
-            for (int k = k0; k < k1; ++k) {
-                const uint32_t x = __float_as_uint(__ldg(w + k));
+                    for (int j = 0; j < 8; ++j) again[j] = fmaf(__ldg(w + k), __ldg(a.A + (size_t)(tok0 + min(c + j, count - 1)) * a.lda + k), again[j]);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float y0 = __ldg(a.A + (size_t)(tok0 + min(j32 + 2 * j, count - 1)) * a.lda + k);
-                    const float y1 = __ldg(a.A + (size_t)(tok0 + min(j32 + 2 * j + 1, count - 1)) * a.lda + k);
-                    sum[j] = fma2(pair(x, x), pair(__float_as_uint(y0), __float_as_uint(y1)), sum[j]);
-                }
+                for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(again[j]);
             }
-        }
-        // [token][row of W] into shared memory, whose stages are free
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t v[2];
-            unpair(sum[j], v[0], v[1]);
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                if (j32 + 2 * j + e < count)
-                    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_base + (uint32_t)(((j32 + 2 * j + e) * BW + row) * 4)), "r"(v[e]) : "memory");
+            for (int j = 0; j < 8; ++j) {
+                if (c + j < count) asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_base + (uint32_t)(((c + j) * BW + row) * 4)), "r"(r[j]) : "memory");
+            }
         }
     }
     if (a.pieces > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -305,22 +304,22 @@ tc_f32_kernel(const Args a) {
     }
     __syncwarp();
     // nobody leaves (and frees its shared memory) before every CTA has read what it needs
-    if (a.pieces > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_before();
-    __syncthreads();
-    if (warp == WARPS) {
+    if (a.pieces > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+    if (warp == ISSUER) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(256u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4u * MAX_NT) : "memory");
     }
 }
 
-int smem_bytes(int nt) {
-    const int ring = STAGES * 3 * (PART_W + nt * BK * 2), held = nt * BW * 4;
-    return (ring > held ? ring : held) + 1024;
-}
+// What a CTA asks for, more than it needs at fewer tokens: it takes all of an SM's tensor memory, so nothing that takes some
+// may share the SM with it (clusters that wait for one another's tensor memory on two SMs would wait for good).
+constexpr int SMEM = 224 * 1024;
+static_assert(2 * 3 * (PART_W + MAX_NT * BK * 2) + 1024 <= SMEM && MAX_NT * BW * 4 + 1024 <= SMEM, "two stages, or the sums");
 
 // Tokens in equal tiles of at most 128; as many pieces of K (a power of two) as shorten the longest SM's work: a block of K
-// takes about 1.55 us and 3 ns a token, a CTA 6 us around them; clusters leave SMs over.
+// takes about 1.3 us and 2.7 ns a token, a CTA 6 us around them; clusters leave SMs over.
 void plan(int M, int N, int K, int* nt, int* token_tiles, int* pieces) {
     const int num_kb = (K + BK - 1) / BK, sms = sp_sm_count() > 0 ? sp_sm_count() : 148;
     const int tt = (M + MAX_NT - 1) / MAX_NT;
@@ -333,7 +332,7 @@ void plan(int M, int N, int K, int* nt, int* token_tiles, int* pieces) {
         if ((p - 1) * mine >= num_kb) continue;                    // no empty piece
         const int room = p <= 2 ? sms : p == 4 ? sms * 132 / 148 : sms * 112 / 148;
         const int ctas = (N + BW - 1) / BW * *token_tiles * p;
-        const double t = (double)((ctas + room - 1) / room) * (mine * (1.55 + 0.0032 * *nt) + 6.0 + (p > 1 ? 1.5 : 0.0));
+        const double t = (double)((ctas + room - 1) / room) * (mine * (1.3 + 0.0027 * *nt) + 6.0 + (p > 1 ? 1.5 : 0.0));
         if (p == 1 || t < best) { best = t; *pieces = p; }
     }
 }
@@ -356,14 +355,14 @@ SP_API int sp_tc_f32(const void* A, const void* W, void* C, int M, int N, int K,
     if (sp_tc_f32_supported(A, W, M, N, K, lda, ldw)) return 1;
     static SpPerDevice configured;
     if (!configured.done()) {
-        cudaError_t e = cudaFuncSetAttribute(tc_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MAX_NT));
-        if (e != cudaSuccess) SP_FAIL("tc_f32: cannot reserve %d bytes of shared memory: %s", smem_bytes(MAX_NT), cudaGetErrorString(e));
+        cudaError_t e = cudaFuncSetAttribute(tc_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) SP_FAIL("tc_f32: cannot reserve %d bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
         configured.mark();
     }
     Args args{(const float*)A, (const float*)W, (float*)C, status, M, N, K, lda, ldw, ldc, accumulate, 0, 0};
     int token_tiles = 1;
     plan(M, N, K, &args.nt, &token_tiles, &args.pieces);
-    SP_CHECK_CALL("tc_f32", sp_launch_cluster(tc_f32_kernel, dim3((N + BW - 1) / BW * args.pieces, token_tiles), dim3(THREADS),
-                                              (size_t)smem_bytes(args.nt), stream, args.pieces, args));
+    SP_CHECK_CALL("tc_f32", sp_launch_cluster(tc_f32_kernel, dim3((N + BW - 1) / BW * args.pieces, token_tiles), dim3(THREADS), (size_t)SMEM, stream,
+                                              args.pieces, args));
     return 0;
 }
