@@ -50,7 +50,7 @@ struct EpiArgs {
     const float* row_ssq;
     int n_ssq, norm_width;
     float eps;
-    int pad0;
+    int w_settled;
     void* xw;
     const void* next_w;
     float* ssq_out;
@@ -189,9 +189,10 @@ int linear(const void* x, const void* W, void* out, int out_dt, int M, int N, in
 }
 
 // A product of the fused sequence with its epilogue's arguments.
-int fused_product(const void* x, const void* W, void* out, int out_dt, int N, int K, int ldo, int mode, int pair, const EpiArgs* ep,
+int fused_product(const void* x, const void* W, void* out, int out_dt, int N, int K, int ldo, int mode, int pair, EpiArgs* ep,
                   const HostStep& st, cudaStream_t stream) {
     const HostKernels& k = kernels;
+    ep->w_settled = 1;                                   // a model's weights: complete before the step's first kernel
     ++launches;
     if (st.mid) {
         const int width = k.mid_or_pairs(mode, st.T, N, K, mode == MODE_STREAM_QKV_ROPE ? ep->hd : 1);

@@ -561,7 +561,7 @@ def tc_gemm(a, w, out, mode=TC_STORE, bn=128, act=ACT_SILU, mult: float = 1.0, l
 
 class _EpiArgs(ctypes.Structure):
     """Mirror of ``EpiArgs`` in tc_gemm.cu."""
-    _fields_ = [("row_ssq", c_void_p), ("n_ssq", c_int), ("norm_width", c_int), ("eps", c_float), ("pad0", c_int),
+    _fields_ = [("row_ssq", c_void_p), ("n_ssq", c_int), ("norm_width", c_int), ("eps", c_float), ("w_settled", c_int),
                 ("xw", c_void_p), ("next_w", c_void_p), ("ssq_out", c_void_p),
                 ("cs", c_void_p), ("tok_page", c_void_p), ("positions", c_void_p),
                 ("q_out", c_void_p), ("kpool", c_void_p), ("vpool", c_void_p),
@@ -613,11 +613,13 @@ def tc_stream_fused(a, w, out, mode, pair=0, row_ssq=None, norm_width=0, eps=0.0
                    next_w, ssq_out, rope)
 
 
-def _fused_product(module, a, w, out, mode, width, n_tiles, row_ssq, norm_width, eps, xw, next_w, ssq_out, rope):
+def _fused_product(module, a, w, out, mode, width, n_tiles, row_ssq, norm_width, eps, xw, next_w, ssq_out, rope,
+                   w_settled=False):
     lib = load(module)
     M, K = a.shape
     N = w.shape[0]
     ep = _EpiArgs()
+    ep.w_settled = int(bool(w_settled))
     if row_ssq is not None:
         if row_ssq.dtype != torch.float32 or row_ssq.dim() != 2 or row_ssq.shape[0] < M or not row_ssq.is_contiguous():
             raise KernelError(f"{module}_fused: the row statistics are a contiguous float32 [M, n] tensor")
@@ -1076,10 +1078,12 @@ def tc_mid(x, w, out, mode=TC_STORE, pair=0, act=ACT_SILU, mult: float = 1.0, li
 
 
 def tc_mid_fused(a, w, out, mode, pair=0, row_ssq=None, norm_width=0, eps=0.0, xw=None, next_w=None, ssq_out=None,
-                 rope=None):
-    """``tc_mid`` with the epilogues of ``tc_stream_fused``; ``ssq_out`` is [M, tc_stream_n_tiles(N)] as there."""
+                 rope=None, w_settled=False):
+    """``tc_mid`` with the epilogues of ``tc_stream_fused``; ``ssq_out`` is [M, tc_stream_n_tiles(N)] as there.
+    ``w_settled``: ``w`` was complete before the kernel in front of this one began (a model's weights within a step), so
+    that it may be read before that one has finished."""
     _fused_product("tc_mid", a, w, out, mode, int(pair), tc_stream_n_tiles(w.shape[0]), row_ssq, norm_width, eps, xw,
-                   next_w, ssq_out, rope)
+                   next_w, ssq_out, rope, w_settled)
 
 
 def tc_mid_plan(mode, M: int, N: int, K: int) -> tuple:

@@ -51,7 +51,7 @@ struct EpiArgs {
     const float* row_ssq;          // [M][n_ssq] partial sums of squares of the residual rows (null: no scaling)
     int n_ssq, norm_width;         // 1/rms = 1/sqrt(sum/norm_width + eps)
     float eps;
-    int pad0;
+    int w_settled;                 // W may be read before the kernel in front of this one has finished: see the loader
     __nv_bfloat16* xw;             // MODE_ACCUMULATE: [M][N] new C ⊙ next_w (null: plain accumulation)
     const __nv_bfloat16* next_w;   // [N]
     float* ssq_out;                // [M][tiles of 128 columns]
@@ -290,7 +290,7 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
-    sp_allow_dependents();                                        // what touches global memory below waits for the predecessor first
+    // what touches global memory below waits for the predecessor first, but for W where the caller says that it is settled
 
     const EpiArgs& ep = a.ep;
     const int ew = warp - 2;                                      // epilogue warp 0..7
@@ -300,15 +300,28 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 
     if (warp == 0) {
         if (lane == 0) {
-            sp_wait_for_predecessor();
-            int s = 0;
-            uint32_t ph = 1;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(smem_u32(&bar_empty[s]), ph, a.status, 131)) break;
+            auto load_w = [&](int kb, int s) {
                 const uint32_t dst = smem_base + (uint32_t)s * stage_bytes;
                 mbar_expect_tx(smem_u32(&bar_full[s]), load_bytes);
                 tma_load_2d(dst, &map_w, kb * BK, row0, smem_u32(&bar_full[s]));
                 if (GATED) tma_load_2d(dst + W_BYTES, &map_w, kb * BK, row0 + BW, smem_u32(&bar_full[s]));
+            };
+            // The ring's first tiles of W are asked for while the predecessor's epilogue runs. That is for weights which were
+            // complete before the predecessor began, as in a step's layers (a kernel without a signal of its own, torch's for
+            // instance, lets this one in when its CTAs have left, before their writes need be visible): the caller says so.
+            // A step of 40 tokens of the 1B shape 1,184 -> 1,147 us, 64: 1,236 -> 1,174, 301: 1,600 -> 1,564; a decode step of
+            // 64 sequences 960 -> 945. (With the signal at the kernels' start it was 1,255 -> 1,272 for 40 tokens.)
+            const int ahead = GROUPED || !ep.w_settled ? 0 : min(a.stages, kb1 - kb0);
+            for (int i = 0; i < ahead; ++i) load_w(kb0 + i, i);
+            sp_wait_for_predecessor();
+            int s = 0;
+            uint32_t ph = 1;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (kb - kb0 >= ahead) {
+                    if (!mbar_wait(smem_u32(&bar_empty[s]), ph, a.status, 131)) break;
+                    load_w(kb, s);
+                }
+                const uint32_t dst = smem_base + (uint32_t)s * stage_bytes;
                 for (int b = 0; b < boxes; ++b)
                     tma_load_2d(dst + PARTS * W_BYTES + (uint32_t)b * (GROUP_BOX * BK * 2), &map_a, kb * BK, tok0 + b * GROUP_BOX, smem_u32(&bar_full[s]));
                 if (++s == a.stages) { s = 0; ph ^= 1u; }
@@ -359,6 +372,9 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         }
         const bool ok = mbar_wait(smem_u32(&bar_acc), 0, a.status, 133);
         tc_fence_after();
+        // The next kernel's CTAs may come now: what they ask for ahead then falls into this one's epilogue. (Allowed from the
+        // start, they sat beside its products and crowded on the SMs that were free first.)
+        sp_allow_dependents();
         // the epilogue threads act together from here on: one verdict for all of them
         if (!(ok && !(a.status && *(volatile int*)a.status != 0))) unhealthy = 1;
         asm volatile("bar.sync 1, 256;" ::: "memory");

@@ -121,7 +121,7 @@ class FusedPrefill:
 
         def product(a, w, out, mode, bn, pair=0, **kw):
             if (mid or paired) and not bn:
-                K.tc_mid_fused(a, w, out, mode, pair, **kw)
+                K.tc_mid_fused(a, w, out, mode, pair, w_settled=True, **kw)
             elif stream:
                 K.tc_stream_fused(a, w, out, mode, pair, **kw)
             else:
@@ -181,7 +181,7 @@ class FusedPrefill:
                 if i + 1 < len(self.fields):
                     xw, ssq = into_residual(act, ff["down"], self.fields[i + 1]["mixer_norm"]["weight"])
                 elif mid or (paired and not width_of(K.TC_ACCUMULATE, ff["down"], 0)):
-                    K.tc_mid(act, ff["down"], h, K.TC_ACCUMULATE)
+                    K.tc_mid_fused(act, ff["down"], h, K.TC_ACCUMULATE, w_settled=True)
                 elif stream:
                     K.tc_stream(act, ff["down"], h, K.TC_ACCUMULATE)
                 else:
