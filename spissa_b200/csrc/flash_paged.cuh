@@ -193,7 +193,6 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
     const uint32_t v_tiles = k_tiles + DEC_STAGES * T::BYTES;
     float* merge = (float*)(smem + QR * T::ROW);                  // [4 warps][QR rows][VD + 2], over the tiles once they are used up
     static_assert(4 * QR * (VD + 2) * 4 <= DEC_STAGES * (T::BYTES + TV::BYTES), "the merge buffer fits over the tiles");
-    sp_allow_dependents();
     sp_wait_for_predecessor();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int chunk = blockIdx.x, n_chunks = gridDim.x, g = blockIdx.y, b = blockIdx.z;
@@ -297,6 +296,8 @@ flash_decode_kernel(const __nv_bfloat16* __restrict__ q, PagedKV kv, const int* 
         __syncwarp();                                              // the stage is free for this warp's next fetch
     }
     cp_async_wait<0>();
+    // (not before: the next product's CTAs would crowd on the SMs that are free first, 17 sequences of 500 keys 574 -> 559 us a step)
+    sp_allow_dependents();
     __syncthreads();                                               // every warp is done with the tiles: they become the merge buffer
 
     // merge the four warps' (m, l, o): each covered other keys of the same rows
