@@ -46,6 +46,37 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// The softmax warps wait for tensor memory and for one another more than they compute (the exponential unit is busy for 46 % of
+// the time), so fewer instructions between two waits is what helps: maxima of three, products and sums of two values at a time.
+// 2,048 tokens, 32 heads of 64: 39.3 -> 38.0 us, 6,000 of 128: 349 -> 336. (Four CTAs on an SM for head size 64, with one score
+// buffer and the scores read twice in halves instead of held: 68 us. Tensor memory gives a warp 64 columns in about 500 cycles.)
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+// two 32-bit values side by side
+__device__ __forceinline__ uint64_t both(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ float2 apart(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+
 // Operands lie in shared memory as boxes of 64 columns (one 128-byte swizzle span): a query tile is HD / 64 boxes of
 // 128 rows, a K page HD / 64 boxes of 64 rows, a V page HDV / 64 (value rows may be shorter than key rows).
 template <int HD, int HDV = HD>
@@ -257,12 +288,9 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             // than the exponentials
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int i = 0; i < KB; i += 4) {
-                mx4[0] = fmaxf(mx4[0], __uint_as_float(r[i]));
-                mx4[1] = fmaxf(mx4[1], __uint_as_float(r[i + 1]));
-                mx4[2] = fmaxf(mx4[2], __uint_as_float(r[i + 2]));
-                mx4[3] = fmaxf(mx4[3], __uint_as_float(r[i + 3]));
-            }
+            for (int i = 0; i < KB; i += 8)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) mx4[u] = max3(mx4[u], __uint_as_float(r[i + 2 * u]), __uint_as_float(r[i + 2 * u + 1]));
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl;
             // move the reference only when it is far behind (or not set yet)
             const bool move = mx > m + RESCALE_STEP || (m == -INFINITY && mx > -INFINITY);
@@ -288,17 +316,19 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 m = m_new;
             }
             const float m_safe = (m == -INFINITY) ? 0.0f : m;
-            float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const uint64_t sl2 = both(sl, sl), minus_m = both(-m_safe, -m_safe);
+            uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};
             uint32_t pk[KB / 2];
 #pragma unroll
             for (int i = 0; i < KB; i += 2) {
-                const float p0 = ex2(fmaf(__uint_as_float(r[i]), sl, -m_safe));
-                const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), sl, -m_safe));
-                sum4[(i >> 1) & 3] += p0 + p1;
+                const float2 x = apart(fma2(both(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2, minus_m));
+                const float p0 = ex2(x.x), p1 = ex2(x.y);
+                sum4[(i >> 1) & 3] = add2(sum4[(i >> 1) & 3], both(p0, p1));
                 __nv_bfloat162 pr = __floats2bfloat162_rn(p0, p1);
                 pk[i >> 1] = *(uint32_t*)&pr;
             }
-            l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            const float2 sum = apart(add2(add2(sum4[0], sum4[1]), add2(sum4[2], sum4[3])));
+            l += sum.x + sum.y;
             tc_st_32x32(s_addr, pk);                              // P over the first half of the scores it came from
             tc_st_wait();
             tc_fence_before();
