@@ -150,6 +150,25 @@ def test_dynamic_tanh_and_polynorm_kernels(out_dtype):
     assert worst(rows32, x.double() + bias.double()) <= 1e-6
 
 
+@pytest.mark.parametrize("width", [4, 201, 1028, 8192, 8196])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_dynamic_tanh_and_polynorm_by_sixteen_bytes_and_by_elements(width, dtype):
+    """Widths in fours and not, rows longer than what a block of PolyNorm holds."""
+    from spissa_b200.csrc import lib as K
+    g = torch.Generator().manual_seed(width)
+    x = 2 * torch.randn(5, width, generator=g)
+    w, b, alpha = (torch.randn(n, generator=g).to(dtype) for n in (width, width, 1))
+    out, act = torch.empty(5, width, dtype=dtype, device=DEV), torch.empty(5, width, dtype=dtype, device=DEV)
+    K.dyt_norm(x.to(DEV), w.to(DEV), b.to(DEV), alpha.to(DEV), out)
+    ref = torch.tanh(alpha.double() * x.double()) * w.double() + b.double()
+    assert worst(out, ref) <= (2e-6 if dtype == torch.float32 else 5e-3)
+    coef = torch.tensor([0.7, -1.3, 0.45, 0.2]).to(dtype)
+    K.polynorm(x.to(DEV), coef.to(DEV), act, 1e-4)
+    z, c = x.double(), coef.double()
+    ref = c[0] * D.unit_rms(z, 1e-4) + c[1] * D.unit_rms(z ** 2, 1e-4) + c[2] * D.unit_rms(z ** 3, 1e-4) + c[3]
+    assert worst(act, ref) <= (5e-6 if dtype == torch.float32 else 5e-3)
+
+
 def test_token_shift_kernel_carries_the_last_row_in_the_state():
     from spissa_b200.csrc import lib as K
     g = torch.Generator().manual_seed(2)
@@ -184,7 +203,7 @@ def test_token_shift_kernel_carries_the_last_row_in_the_state():
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(3, 8, 16), (1, 40, 24), (2, 16, 70), (2, 128, 130), (1, 72, 256), (1, 130, 8),
-                                             (2, 100, 40), (2, 32, 32)])
+                                             (2, 100, 40), (2, 32, 32), (1, 20, 644)])
 def test_retention_kernel(heads, dim, vdim):
     """Sequences of 50 and 39 tokens run in chunks (where the key size allows), the single token and the portions
     below token by token; a chunk boundary lies inside nothing here, the next test crosses several."""
