@@ -1464,13 +1464,11 @@ def moe_experts(x, ids, weights, w_gate_up, w_down, y, top, limit, slope=1.702, 
         max_tiles = (n_pairs + 127) // 128 + E
         rows = max_tiles * 128
         book = torch.empty(E + rows + n_pairs + 5 * max_tiles, dtype=torch.int32, device=dev)
-        counts, order, pos = book[:E], book[E:E + rows], book[E + rows:E + rows + n_pairs]
-        rest = book[E + rows + n_pairs:]
-        tiles, tab_up, tab_down = rest[:3 * max_tiles], rest[3 * max_tiles:4 * max_tiles], rest[4 * max_tiles:]
+        counts, order, pos, tiles, tab_up, tab_down = book.split([E, rows, n_pairs, 3 * max_tiles, max_tiles, max_tiles])
         xs = torch.empty(rows, W, dtype=torch.bfloat16, device=dev)
         hidden = torch.empty(rows, F, dtype=torch.bfloat16, device=dev)
         out_rows = torch.empty(rows, W, dtype=torch.float32, device=dev)
-        launches += 6
+        launches += 4
         runs = glu and glu_block == 128 and (slope == 0.0 or limit > 0.0) and n_pairs < MID_EXPERT_TOKENS * E and max_tiles <= 65535
         _check("hybrid", lib.sp_moe_plan_tiles(
             c_void_p(_ptr(x)), c_void_p(_ptr(ids)), T, int(top), W, E, F2, W, c_void_p(_ptr(counts)), c_void_p(_ptr(order)),
@@ -1497,14 +1495,14 @@ def moe_experts(x, ids, weights, w_gate_up, w_down, y, top, limit, slope=1.702, 
         return
     tm = moe_tile_rows()
     max_tiles = (n_pairs + tm - 1) // tm + E
-    book = torch.empty(E + n_pairs + 3 * max_tiles, dtype=torch.int32, device=dev)
-    counts, order, tiles = book[:E], book[E:E + n_pairs], book[E + n_pairs:]
+    book = torch.empty(n_pairs + 3 * max_tiles, dtype=torch.int32, device=dev)
+    order, tiles = book[:n_pairs], book[n_pairs:]
     hidden = torch.empty(n_pairs, F, dtype=x.dtype, device=dev)
     out_pairs = torch.empty(n_pairs, W, dtype=torch.float32, device=dev)
-    launches += 4
+    launches += 3
     _check("hybrid", lib.sp_moe_experts(
         c_void_p(_ptr(x)), dt_code(x), c_void_p(_ptr(ids)), c_void_p(_ptr(w_gate_up)), c_void_p(_ptr(w_down)),
-        _w_dt(w_gate_up, w_down), E, c_void_p(_ptr(counts)), c_void_p(_ptr(order)), c_void_p(_ptr(tiles)), max_tiles,
+        _w_dt(w_gate_up, w_down), E, c_void_p(_ptr(order)), c_void_p(_ptr(tiles)), max_tiles,
         c_void_p(_ptr(weights)), c_void_p(_ptr(hidden)), c_void_p(_ptr(out_pairs)), c_void_p(_ptr(y)), T, int(top), W, F,
         c_float(limit), c_float(slope), int(glu_block), int(act), int(bool(identities)), c_void_p(_stream())))
 
