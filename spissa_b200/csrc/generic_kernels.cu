@@ -1289,9 +1289,29 @@ __global__ void gated_mul_kernel(const T* gu, T* __restrict__ out, size_t rows, 
     sp_allow_dependents();
 }
 
+// The same for float32 rows in fours on 16-byte boundaries: a block per row and 1,024 columns, no division per element. 500 rows of
+// 8,192: 15.4 -> 9.0 us.
+__global__ void __launch_bounds__(256)
+gated_mul_vec_kernel(const float* gu, float* __restrict__ out, int rows, int I, int act, float mult) {
+    sp_wait_for_predecessor();
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+    for (int r = blockIdx.y; r < rows && c < I; r += gridDim.y) {
+        const float* row = gu + (size_t)r * 2 * I;
+        const float4 g = sp_ld_written((const float4*)(row + c)), u = sp_ld_written((const float4*)(row + I + c));
+        const SpGate ga{act, mult, 0.0f, 0.0f};
+        *(float4*)(out + (size_t)r * I + c) = make_float4(sp_gated(g.x, u.x, ga), sp_gated(g.y, u.y, ga), sp_gated(g.z, u.z, ga), sp_gated(g.w, u.w, ga));
+    }
+    sp_allow_dependents();                                   // (as above)
+}
+
 SP_API int sp_gated_mul(const void* gu, void* out, int dt, int rows, int I, int act, float mult, cudaStream_t stream) {
     if (rows <= 0 || I <= 0) return 0;
     if (act != SP_ACT_SILU && act != SP_ACT_GELU) SP_FAIL("gated_mul: activation code %d is not built", act);
+    if (dt == SP_DT_F32 && (I & 3) == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
+        SP_CHECK_CALL("gated_mul", sp_launch_dependent(gated_mul_vec_kernel, dim3((I / 4 + 255) / 256, rows < 65535 ? rows : 65535), dim3(256), 0, stream,
+                                                       (const float*)gu, (float*)out, rows, I, act, mult));
+        return 0;
+    }
     const size_t n = (size_t)rows * I;
     const int blocks = (int)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
     if (dt == SP_DT_F32) sp_launch_dependent(gated_mul_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)gu, (float*)out, rows, I, act, mult);

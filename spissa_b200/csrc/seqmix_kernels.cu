@@ -253,7 +253,15 @@ __global__ void diff_qkv_store_kernel(const float* __restrict__ qkv, const void*
     if (t >= T) return;
     // the output projection's bias goes into the token's row of the residual stream here, ahead of the product that
     // accumulates into it: one launch less than adding it behind
-    if (stream)
+    if (stream && (width & 3) == 0 && (((uintptr_t)stream | (uintptr_t)stream_bias) & 15) == 0) {
+        for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
+            float4* at = (float4*)(stream + (size_t)t * width + c);
+            const float4 b = sm_ld4_dt(stream_bias, b_dt, c);
+            float4 v = *at;
+            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+            *at = v;
+        }
+    } else if (stream)
         for (int c = threadIdx.x; c < width; c += blockDim.x) stream[(size_t)t * width + c] += sp_ld_dt(stream_bias, b_dt, c);
     const int pos = pl.positions[t];
     const int half = rd >> 1;
@@ -331,7 +339,7 @@ SP_API int sp_diff_qkv_store(const float* qkv, const void* bias, int b_dt, void*
     KvPlace pl{token_seq, positions, seq_slot, page_table, max_pages, page_size, sp_range_host};
     const size_t smem = (size_t)rd * sizeof(float);
 #define QS_LAUNCH(TO, TC)                                                                                          \
-    diff_qkv_store_kernel<TO, TC><<<T, 128, smem, stream>>>(qkv, bias, b_dt, (TO*)q_out, (TC*)kpool, (TC*)vpool, pl, \
+    diff_qkv_store_kernel<TO, TC><<<T, 256, smem, stream>>>(qkv, bias, b_dt, (TO*)q_out, (TC*)kpool, (TC*)vpool, pl, \
                                                            inv_freq, T, nq, nk, G, d, vd, rd, residual, residual_bias, width)
     if (q_dt == SP_DT_F32 && cache_dt == SP_DT_F32) QS_LAUNCH(float, float);
     else if (q_dt == SP_DT_BF16 && cache_dt == SP_DT_BF16) QS_LAUNCH(__nv_bfloat16, __nv_bfloat16);
