@@ -1178,30 +1178,37 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// The split of the keys: about one (sequence, kv head, chunk) item per warp group of the grid. Where 1, 2 or 4 chunks
-// keep at least three quarters of the groups busy (and the CTAs can be launched as pairs) that split is taken, even if
-// the last chunks of a short sequence are empty: the pair-wise combination then saves a phase and a grid barrier.
-// chunks per (sequence, kv head) for the pair-wise combination with T sequences, or 0 where it does not pay
+// The most chunks of a (sequence, kv head) that T sequences can have combined within a CTA or a CTA pair, or 0. Fewer than eight
+// (sequence, kv head) in all would leave nearly every SM without keys: these keep the finer split, whatever the length.
 int pair_chunks(int G, int T, int hd, int max_nkv) {
-    if (hd != 64 || (G % 2) != 0) return 0;
-    const int groups = G * 2, items = T * (max_nkv > 0 ? max_nkv : 1);
-    const int want = groups / items;
-    const int c = want >= 4 ? 4 : (want >= 2 ? 2 : (want >= 1 ? 1 : 0));
-    return (c > 0 && 4 * items * c >= 3 * groups) ? c : 0;
+    const int items = T * (max_nkv > 0 ? max_nkv : 1);
+    if (hd != 64 || (G % 2) != 0 || items < 8) return 0;
+    const int want = G * 2 / items;
+    return want >= 4 ? 4 : (want >= 2 ? 2 : (want >= 1 ? 1 : 0));
 }
 
+// The split of the keys. Either about one (sequence, kv head, chunk) item per warp group of the grid, whose results a phase of its
+// own behind one more grid barrier combines; or 1, 2 or 4 chunks of longer, combined within a CTA (two) or a CTA pair (four). By
+// an estimate in microseconds: a page costs a group 0.6 (0.9 with two stages), the phase and its barrier 5.4, the exchange
+// between the CTAs of a pair 1.5. Measured with 8 layers of the 1B shape, us a step by the first / by the estimate: 1 sequence of
+// 100 keys SPLIT_A, 600 SPLIT_B, 2,048 SPLIT_C; 4 of 1,000 SPLIT_D; 10 of 500 SPLIT_E, of 2,048 SPLIT_F; 13 of 600 SPLIT_G.
 int plan_split(int G, int T, int hd, int len_pages, int max_nkv, int* chunk_pages, int* n_chunks) {
     if (len_pages < 1) len_pages = 1;
     const int groups = G * (hd == 64 ? 2 : 1);
     int want = groups / (T * (max_nkv > 0 ? max_nkv : 1));
     if (want < 1) want = 1;
-    if (const int c = pair_chunks(G, T, hd, max_nkv)) {
+    const double page = attention_stages(hd, T) == 3 ? 0.6 : 0.9;
+    double best = 5.4 + page * ((len_pages + want - 1) / want);
+    int pages = 0, chunks = 0;
+    for (int c = 1; c <= pair_chunks(G, T, hd, max_nkv); c *= 2) {
         const int per = (len_pages + c - 1) / c;
-        if (per <= 64) {
-            *chunk_pages = per;
-            *n_chunks = c;
-            return 0;
-        }
+        const double t = page * per + (c == 4 ? 1.5 : c == 2 ? 0.3 : 0.0);
+        if (per <= 64 && t < best) { best = t; pages = per; chunks = c; }
+    }
+    if (chunks) {
+        *chunk_pages = pages;
+        *n_chunks = chunks;
+        return 0;
     }
     if (want > MAX_CHUNKS) want = MAX_CHUNKS;
     if (want > len_pages) want = len_pages;
