@@ -322,11 +322,9 @@ class Engine:
         never been asked for. ``check=False`` returns without waiting; such steps are settled by the next checked
         step, by ``check()`` or ``settle()``, and until then ``length`` counts them.
         """
-        def as_list(x):                                  # (nothing below changes the caller's lists)
-            return x if type(x) is list else list(x)
-
-        ents = [(e.slot, as_list(e.tokens), as_list(e.want)) if isinstance(e, StepEntry)
-                else (e[0], as_list(e[1]), as_list(e[2])) for e in entries]
+        # (copies: what has been checked is what runs, whatever the caller's other threads do with their lists meanwhile)
+        ents = [(e.slot, list(e.tokens), list(e.want)) if isinstance(e, StepEntry)
+                else (e[0], list(e[1]), list(e[2])) for e in entries]
         lengths, packed = self._validate(ents)
         counts = [(slot, len(toks)) for slot, toks, _ in ents]
         with torch.cuda.device(self.device):

@@ -208,6 +208,25 @@ def test_step_refusals_leave_the_cache_alone(folders):
     assert out.shape == (1, 256) and engine.length(s) == 4
 
 
+@pytest.mark.parametrize("n", [3, 40])
+def test_a_callers_lists_may_change_once_their_step_is_checked(folders, n):
+    """What has been checked is what runs, whatever another thread does with the lists meanwhile."""
+    folder, _, _ = folders["A"]
+    engine = Engine.from_folder(folder, dtype="float32", max_tokens=256, max_seqs=2)
+    prompt = [(7 * i + 3) % 256 for i in range(n)]
+    plain = engine.step([(engine.acquire(), prompt, [0, n - 1])])
+    tokens, want, check = list(prompt), [0, n - 1], engine._validate
+
+    def check_and_change(entries):
+        got = check(entries)
+        tokens[:] = [9] * n
+        want[:] = [1]
+        return got
+
+    engine._validate = check_and_change
+    assert torch.equal(engine.step([(engine.acquire(), tokens, want)]), plain)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["A", "B", "E"])
 def test_graph_replay_equals_kernel_by_kernel(folders, name, dtype):
