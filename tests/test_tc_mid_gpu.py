@@ -319,3 +319,48 @@ def test_linear_of_more_tokens(K, M, N, Kd):
     acc = c0.clone()
     Linear(w)(a, out=acc, accumulate=True)
     within(acc, a, w, extra=c0)
+
+
+@pytest.mark.parametrize("act", ["ACT_SILU", "ACT_CLAMPED"])
+@pytest.mark.parametrize("kernel,width", [("tc_mid", 128), ("tc_gemm", 256), ("tc_gemm", 128)])
+def test_a_tokens_gated_values_do_not_depend_on_its_neighbours(K, act, kernel, width):
+    """Gates beyond the branch-free range in every sixteenth token leave the others' bits as they are."""
+    kw = dict(act=getattr(K, act))
+    if act == "ACT_CLAMPED":
+        kw.update(limit=100.0, slope=1.702)
+    a, w = operands(2048, 16384, 64)
+    b = a.clone()
+    b[::16] *= 1000.0
+    plain, beside = torch.empty(2048, 8192, device=DEV), torch.empty(2048, 8192, device=DEV)
+    getattr(K, kernel)(a, w, plain, K.TC_SILU_MUL, width, **kw)
+    getattr(K, kernel)(b, w, beside, K.TC_SILU_MUL, width, **kw)
+    rest = torch.arange(2048, device=DEV) % 16 != 0
+    assert torch.equal(plain[rest], beside[rest])
+
+
+@pytest.mark.parametrize("kernel,width", [("tc_mid", 128), ("tc_gemm", 256), ("tc_gemm", 128)])
+@pytest.mark.parametrize("slope,gate", [(0.2526956572140501, 0.020345522090792656), (0.5680828327219911, 0.007325529120862484),
+                                        (0.7441885108658084, 0.0013069163542240858), (0.7441885108658084, 0.10660775750875473),
+                                        (0.974886949234209, 0.012287044897675514), (2.8710412953340563, 0.0016809902153909206),
+                                        (4.926993966922774, 0.005847701337188482)])
+def test_clamped_units_whose_quotient_lies_near_the_middle_of_two_floats(K, kernel, width, slope, gate):
+    """Gates whose quotient by an unrefined reciprocal is a last bit off: the same value alone and beside a large gate."""
+    parts, left = [], torch.tensor(gate)
+    for _ in range(3):                                                  # the gate as an exact sum of three bfloat16 numbers
+        parts.append(left.bfloat16())
+        left = left - parts[-1].float()
+    assert float(left) == 0.0
+    half = width if kernel == "tc_mid" else width // 2
+    w = torch.zeros(512, 64, dtype=torch.bfloat16, device=DEV)
+    w.view(-1, 2, half, 64)[:, 0, :, :3] = 1.0                          # gate rows; the up rows are zero, so up + 1 is 1
+    a = torch.zeros(130, 64, dtype=torch.bfloat16, device=DEV)
+    a[:, :3] = torch.stack(parts).to(DEV)
+    b = a.clone()
+    b[1::2, 0] = 512.0
+    outs = [torch.empty(130, 256, device=DEV) for _ in range(2)]
+    for x, out in zip((a, b), outs):
+        getattr(K, kernel)(x, w, out, K.TC_SILU_MUL, width, act=K.ACT_CLAMPED, limit=1000.0, slope=slope)
+    assert torch.equal(outs[0][::2], outs[1][::2])
+    want = gate / (1.0 + float(torch.exp(torch.tensor(-slope * gate, dtype=torch.float64))))
+    # half a unit, and an expf that is two units of 2^-24 off below 1
+    assert float((outs[0][::2].double() - want).abs().max()) <= 4 * 2.0 ** -24 * want
