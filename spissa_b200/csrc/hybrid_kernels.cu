@@ -12,7 +12,7 @@
 //                     channel from a low-rank projection, rms norm with a weight per head, gate silu(g)
 //   gelu_tanh, clamped_glu     activations of feed-forwards
 //   moe_select        sigmoid router: choice among the best groups of experts with a correction, weights without it
-//   moe_plan / moe_up / moe_down / moe_combine      the chosen experts' products over token lists sorted by expert
+//   moe_place / moe_up / moe_down / moe_combine      the chosen experts' products over token lists sorted by expert
 //
 // Everything but the experts' products is computed in 32-bit (FFMA, expf / tanhf / sqrtf / division without
 // fast-math); stores round to the activation type. States are 32-bit. Every output row is reduced in an order that
@@ -1169,7 +1169,7 @@ SP_API int sp_moe_select(const float* z, const void* corr, int corr_dt, int* ids
 }
 
 // ============================================================== the chosen experts' products
-// A pair p = token · top + k names one chosen expert of one token. ``moe_plan`` sorts the pairs by expert (pairs of
+// A pair p = token · top + k names one chosen expert of one token. ``moe_place`` sorts the pairs by expert (pairs of
 // one expert in ascending order) and cuts every expert's list into tiles of ME_TM rows: (expert, first place in the
 // sorted list, rows); unused entries of the tile table (it is sized for the worst case) say expert −1. An id of E or
 // more names an identity expert, whose output is the token's input: such a pair is in no list and no product, the
@@ -1177,9 +1177,16 @@ SP_API int sp_moe_select(const float* z, const void* corr, int corr_dt, int* ids
 #define ME_TM 32
 // A block per expert, which counts all experts' pairs for itself (integers: any order gives the same) and then sets its own in
 // order, each thread a piece of the list. 8,192 pairs, 32 experts: 8 us; with the counts from a kernel of their own and
-// the list in passes of 1,024 pairs 27, and 4 for clearing the list.
+// the list in passes of 1,024 pairs 27, and 4 for clearing the list. (More experts than PLACE_COUNTS: the counts are
+// ``given``, in global memory.)
+#define PLACE_COUNTS 12000                                   // 48 KB, what a block has without asking for more
+__global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ counts, int E) {
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += gridDim.x * blockDim.x)
+        if (ids[p] >= 0 && ids[p] < E) atomicAdd(&counts[ids[p]], 1);
+}
+
 __global__ void __launch_bounds__(1024)
-moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ counts_out, int E, int* __restrict__ sorted,
+moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* counts_out, const int* given, int E, int* __restrict__ sorted,
                  int* __restrict__ tiles /* [max_tiles][3] */, int max_tiles, int tm, int padded, int* __restrict__ pos,
                  int* __restrict__ tab_up, int* __restrict__ tab_down, int up_rows, int down_rows, int run) {
     // ``padded``: every expert's rows begin at a tile's first row (the sorted list then has holes, which say -1, and
@@ -1187,17 +1194,20 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ cou
     // in the stacked weights (-1: the tile is not in use), for products that take whole tiles of one expert. ``tiles`` then
     // holds, for products that take up to ``run`` rows of an expert at once, its rows in equal parts of a multiple of 16: there
     // are never more of them than tiles, the entries left over say -1.
-    extern __shared__ int counts[];                          // [E]
+    extern __shared__ int counted[];                         // [E]
     __shared__ int wsum[32], before[2];
     const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int x = threadIdx.x; x < E; x += blockDim.x) counts[x] = 0;
     if (threadIdx.x < 2) before[threadIdx.x] = 0;
-    __syncthreads();
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const int id = ids[p];
-        if (id >= 0 && id < E) atomicAdd(&counts[id], 1);
+    if (!given) {
+        for (int x = threadIdx.x; x < E; x += blockDim.x) counted[x] = 0;
+        __syncthreads();
+        for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+            const int id = ids[p];
+            if (id >= 0 && id < E) atomicAdd(&counted[id], 1);
+        }
     }
     __syncthreads();
+    const int* const counts = given ? given : counted;
     int s = 0, t = 0;
     for (int x = threadIdx.x; x < e; x += blockDim.x) { s += counts[x]; t += (counts[x] + tm - 1) / tm; }
 #pragma unroll
@@ -1224,7 +1234,7 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ cou
             if (pos) pos[p] = at;
             ++at;
         }
-    if (counts_out && threadIdx.x == 0) counts_out[e] = mine;
+    if (!given && threadIdx.x == 0) counts_out[e] = mine;
     if (padded)                                              // the holes behind its rows; the last expert's reach to the end
         for (int i = from + mine + (int)threadIdx.x; i < (e == E - 1 ? max_tiles : tile0 + (mine + tm - 1) / tm) * tm; i += blockDim.x) sorted[i] = -1;
     const int n_mine = (mine + tm - 1) / tm, n_parts = (mine + run - 1) / run;
@@ -1245,9 +1255,17 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ cou
 
 SP_API int sp_moe_tile_rows() { return ME_TM; }          // the smallest tile any path uses: sizes the tile table
 
-static int moe_plan(const int* ids, int n_pairs, int E, int* sorted, int* tiles, int max_tiles, int tm, cudaStream_t stream) {
-    if (E > 12000) SP_FAIL("moe_plan: %d experts, this kernel takes up to 12000", E);
-    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, (size_t)E * sizeof(int), stream>>>(ids, n_pairs, nullptr, E, sorted, tiles, max_tiles, tm, 0, nullptr, nullptr, nullptr, 0, 0, tm);
+// moe_place_kernel behind the counts where they do not fit it; counts [E].
+static int place(const int* ids, int n_pairs, int E, int* counts, int* sorted, int* tiles, int max_tiles, int tm, int padded, int* pos,
+                 int* tab_up, int* tab_down, int up_rows, int down_rows, int run, cudaStream_t stream) {
+    const bool many = E > PLACE_COUNTS;
+    if (many) {
+        SP_CHECK_CALL("moe_count", cudaMemsetAsync(counts, 0, (size_t)E * sizeof(int), stream));
+        moe_count_kernel<<<(n_pairs + 255) / 256 > 148 * 8 ? 148 * 8 : (n_pairs + 255) / 256, 256, 0, stream>>>(ids, n_pairs, counts, E);
+        SP_CHECK_LAUNCH("moe_count");
+    }
+    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, many ? 0 : (size_t)E * sizeof(int), stream>>>(
+        ids, n_pairs, counts, many ? counts : nullptr, E, sorted, tiles, max_tiles, tm, padded, pos, tab_up, tab_down, up_rows, down_rows, run);
     SP_CHECK_LAUNCH("moe_place");
     return 0;
 }
@@ -1272,9 +1290,7 @@ SP_API int sp_moe_plan_tiles(const void* x, const int* ids, int T, int top, int 
     if (W % 8 || (((uintptr_t)x | (uintptr_t)xs) & 15)) SP_FAIL("moe_plan_tiles: rows of %d do not move in 16-byte pieces", W);
     if ((n_pairs + 127) / 128 + E > max_tiles) SP_FAIL("moe_plan_tiles: the tile table is too short");
     if (run < 128 || run % 16) SP_FAIL("moe_plan_tiles: parts of %d rows", run);
-    if (E > 12000) SP_FAIL("moe_plan_tiles: %d experts, this kernel takes up to 12000", E);
-    moe_place_kernel<<<E, n_pairs >= 2048 ? 1024 : 256, (size_t)E * sizeof(int), stream>>>(ids, n_pairs, counts, E, sorted, tiles, max_tiles, 128, 1, pos, tab_up, tab_down, up_rows, down_rows, run);
-    SP_CHECK_LAUNCH("moe_place");
+    if (place(ids, n_pairs, E, counts, sorted, tiles, max_tiles, 128, 1, pos, tab_up, tab_down, up_rows, down_rows, run, stream)) return 1;
     const size_t n = (size_t)max_tiles * 128 * (W / 8);
     const size_t want = (n + 255) / 256;
     moe_gather_rows_kernel<<<(unsigned)(want > 148 * 16 ? 148 * 16 : want), 256, 0, stream>>>(
@@ -1628,7 +1644,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ out, float* __restr
 }
 
 SP_API int sp_moe_experts(const void* x, int x_dt, const int* ids, const void* wgu, const void* wd, int w_dt, int E,
-                          int* sorted, int* tiles, int max_tiles, const float* wts, void* act, float* out_pairs,
+                          int* counts, int* sorted, int* tiles, int max_tiles, const float* wts, void* act, float* out_pairs,
                           float* y, int T, int top, int W, int F, float limit, float slope, int glu_block, int act_kind,
                           int identities, cudaStream_t stream) {
     // ``act_kind`` SP_ACT_RELU2: ``wgu`` holds up rows alone, F per expert; ``identities``: ids of E and more are in use
@@ -1644,7 +1660,7 @@ SP_API int sp_moe_experts(const void* x, int x_dt, const int* ids, const void* w
         SP_FAIL("moe_experts: operands beyond 2^31 elements");
     const int tm = mma ? MM_TM : ME_TM;
     if ((n_pairs + tm - 1) / tm + E > max_tiles) SP_FAIL("moe_experts: the tile table is too short");
-    if (moe_plan(ids, n_pairs, E, sorted, tiles, max_tiles, tm, stream)) return 1;
+    if (place(ids, n_pairs, E, counts, sorted, tiles, max_tiles, tm, 0, nullptr, nullptr, nullptr, 0, 0, tm, stream)) return 1;
     if (mma) {
         const int used = (n_pairs + tm - 1) / tm + E;           // entries beyond the tiles in use say expert -1
         static SpPerDevice mma_ready;

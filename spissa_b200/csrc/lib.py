@@ -1495,14 +1495,14 @@ def moe_experts(x, ids, weights, w_gate_up, w_down, y, top, limit, slope=1.702, 
         return
     tm = moe_tile_rows()
     max_tiles = (n_pairs + tm - 1) // tm + E
-    book = torch.empty(n_pairs + 3 * max_tiles, dtype=torch.int32, device=dev)
-    order, tiles = book[:n_pairs], book[n_pairs:]
+    book = torch.empty(E + n_pairs + 3 * max_tiles, dtype=torch.int32, device=dev)
+    counts, order, tiles = book.split([E, n_pairs, 3 * max_tiles])
     hidden = torch.empty(n_pairs, F, dtype=x.dtype, device=dev)
     out_pairs = torch.empty(n_pairs, W, dtype=torch.float32, device=dev)
     launches += 3
     _check("hybrid", lib.sp_moe_experts(
         c_void_p(_ptr(x)), dt_code(x), c_void_p(_ptr(ids)), c_void_p(_ptr(w_gate_up)), c_void_p(_ptr(w_down)),
-        _w_dt(w_gate_up, w_down), E, c_void_p(_ptr(order)), c_void_p(_ptr(tiles)), max_tiles,
+        _w_dt(w_gate_up, w_down), E, c_void_p(_ptr(counts)), c_void_p(_ptr(order)), c_void_p(_ptr(tiles)), max_tiles,
         c_void_p(_ptr(weights)), c_void_p(_ptr(hidden)), c_void_p(_ptr(out_pairs)), c_void_p(_ptr(y)), T, int(top), W, F,
         c_float(limit), c_float(slope), int(glu_block), int(act), int(bool(identities)), c_void_p(_stream())))
 

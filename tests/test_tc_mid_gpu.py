@@ -226,7 +226,8 @@ def test_gated_rows_keep_the_bits_of_32_bit_arithmetic(K, act):
         assert bool(((got - ref).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("counts", [[0, 1, 128, 129, 256, 257, 513, 600], [0, 3000, 0, 5], [16, 17, 15]])
+@pytest.mark.parametrize("counts", [[0, 1, 128, 129, 256, 257, 513, 600], [0, 3000, 0, 5], [16, 17, 15], [5] + 11998 * [0] + [7],
+                                    [3] + 11999 * [0] + [200]])
 def test_parts_of_an_experts_rows(K, counts):
     """The table that the grouped products read: an expert's rows in equal parts of a multiple of 16, at most 256 each, and
     nothing that a product has to look for among its neighbours."""
@@ -256,6 +257,21 @@ def test_parts_of_an_experts_rows(K, counts):
     for e, at, c in want:
         assert torch.equal(ids[order[at:at + c].long()], torch.full((c,), e, dtype=torch.int32, device=DEV))
         assert torch.equal(xs[at:at + c], x[order[at:at + c].long()])
+    assert per.tolist() == counts
+
+
+def test_more_experts_than_a_block_counts(K):
+    E, W, F, T, top = 12001, 16, 8, 5, 2
+    g = torch.Generator().manual_seed(1)
+    x, up, down = (torch.randn(*s, generator=g) for s in ((T, W), (E, F, W), (E, W, F)))
+    ids = torch.tensor([[0, 12000], [12000, 7], [11999, 3], [7, 0], [5000, 12000]], dtype=torch.int32)
+    weights = torch.rand(T, top, generator=g)
+    y = torch.zeros(T, W, device=DEV)
+    K.moe_experts(x.to(DEV), ids.to(DEV), weights.to(DEV), up.to(DEV), down.to(DEV), y, top, 0.0, 0.0, act=K.ACT_RELU2)
+    h = torch.relu(torch.einsum("tkfw,tw->tkf", up[ids.long()].double(), x.double())) ** 2
+    ref = torch.einsum("tk,tkwf,tkf->tw", weights.double(), down[ids.long()].double(), h)
+    # sums of 16 and 8 terms, a square: some twenty roundings of 2^-24 on sums of absolute values a few times the result
+    assert float((y.double().cpu() - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
 
 
 def test_experts_of_many_tokens_take_the_tiles_of_128(K, monkeypatch):
