@@ -1176,8 +1176,9 @@ SP_API int sp_moe_select(const float* z, const void* corr, int corr_dt, int* ids
 // combining kernel adds the input times the pair's weight.
 #define ME_TM 32
 // A block per expert, which counts all experts' pairs for itself (integers: any order gives the same) and then sets its own in
-// order, each thread a piece of the list. 8,192 pairs, 32 experts: 8 us; with the counts from a kernel of their own and
-// the list in passes of 1,024 pairs 27, and 4 for clearing the list. (More experts than PLACE_COUNTS: the counts are
+// order, each thread a piece of the list. 8,192 pairs, 32 experts, gather included: 8.1 us; with the counts from a kernel of their
+// own, the list in passes of 1,024 pairs and a copy that clears it 22. 65,536 pairs, 256 experts: 57 (158 with a pair a load, 150
+// by passes); what is left is mostly the counting, 77 us where half of 65,536 pairs name one of eight experts. (More experts than PLACE_COUNTS: the counts are
 // ``given``, in global memory.)
 #define PLACE_COUNTS 12000                                   // 48 KB, what a block has without asking for more
 __global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ counts, int E) {
@@ -1213,10 +1214,23 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* counts_out, cons
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); t += __shfl_xor_sync(0xffffffffu, t, o); }
     if (lane == 0 && (s | t)) { atomicAdd(&before[0], s); atomicAdd(&before[1], t); }
-    // this thread's piece of the list
-    const int per = (n_pairs + (int)blockDim.x - 1) / (int)blockDim.x, p0 = min(n_pairs, (int)threadIdx.x * per), p1 = min(n_pairs, p0 + per);
+    // this thread's piece of the list, in fours (the lanes' pieces lie apart: a load of a warp costs 32 lines however wide it is)
+    const int fours = (n_pairs + 3) / 4, per = (fours + (int)blockDim.x - 1) / (int)blockDim.x * 4;
+    const int p0 = min(n_pairs, (int)threadIdx.x * per), p1 = min(n_pairs, p0 + per);
+    const bool vec = ((uintptr_t)ids & 15) == 0;
+    auto four = [&](int p, int (&id)[4]) {                   // -1 behind the end: no expert's
+        if (vec && p + 4 <= n_pairs) { const int4 v = *(const int4*)(ids + p); id[0] = v.x; id[1] = v.y; id[2] = v.z; id[3] = v.w; }
+        else
+#pragma unroll
+            for (int i = 0; i < 4; ++i) id[i] = p + i < n_pairs ? ids[p + i] : -1;
+    };
     int hits = 0;
-    for (int p = p0; p < p1; ++p) hits += ids[p] == e;
+    for (int p = p0; p < p1; p += 4) {
+        int id[4];
+        four(p, id);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) hits += id[i] == e;
+    }
     int upto = hits;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1228,12 +1242,17 @@ moe_place_kernel(const int* __restrict__ ids, int n_pairs, int* counts_out, cons
     const int start = before[0], tile0 = before[1], mine = counts[e], from = padded ? tile0 * tm : start;
     int at = from + upto - hits;
     for (int w = 0; w < warp; ++w) at += wsum[w];
-    for (int p = p0; p < p1; ++p)
-        if (ids[p] == e) {
-            sorted[at] = p;
-            if (pos) pos[p] = at;
-            ++at;
-        }
+    for (int p = p0; p < p1; p += 4) {
+        int id[4];
+        four(p, id);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (id[i] == e) {
+                sorted[at] = p + i;
+                if (pos) pos[p + i] = at;
+                ++at;
+            }
+    }
     if (!given && threadIdx.x == 0) counts_out[e] = mine;
     if (padded)                                              // the holes behind its rows; the last expert's reach to the end
         for (int i = from + mine + (int)threadIdx.x; i < (e == E - 1 ? max_tiles : tile0 + (mine + tm - 1) / tm) * tm; i += blockDim.x) sorted[i] = -1;
