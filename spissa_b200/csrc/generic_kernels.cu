@@ -304,8 +304,8 @@ __device__ __forceinline__ float4 gs_load(const float* p, bool ok) {
 }
 // SPLIT: a cluster's CTAs share the columns, where there are too few rows of W to fill the chip (a product of 2,048 rows has
 // 256 CTAs, which keep half of the bytes in flight that the memory takes): the first adds the others' sums in their order.
-// 4 rows, 2,048 x 8,192: 18.5 us with one CTA for all of K, 16.5 with two. For 1 to 4 rows: beyond them
-// fewer CTAs fit an SM and the rows of a layer's products fill it.
+// 4 rows, 2,048 x 8,192: 20.3 us with one CTA for all of K, 15.2 with two. For 1 to 4 rows: beyond them
+// fewer CTAs fit an SM and the rows of a layer's products fill it. See gs_pieces for when.
 template <int MT, bool SPLIT>
 __global__ void __launch_bounds__(128, MT == 16 ? 5 : MT == 8 ? 3 : 4)
 gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
@@ -427,6 +427,20 @@ gemm_stream_f32_kernel(const float* A, const float* W, void* C, int c_dt,
         }
 }
 
+// CTAs that share the columns: a cluster's start and its barrier take 1 to 2.5 us, more with more rows of A, so only long sums pay
+// for them, and earlier where the rows of W come near to filling the chip. One CTA / this many, us: 512 rows of W (4 CTAs), K
+// 2,048: 1 row 2.6 / 2.8, 4 rows 3.5 / 4.9; 3,072: 5.0 / 3.5, 5.5 / 6.0; 4,096: 7.5 / 4.1, 7.9 / 6.4. 2,048 rows of W (2 CTAs), K
+// 1,536: 4.5 / 4.8, 5.6 / 6.8; 2,048: 5.8 / 5.2, 6.8 / 7.1; 3,072: 7.1 / 6.3, 8.7 / 8.4; 14,336: 28.2 / 20.5, 33.8 / 22.6. From these
+// lines on none of 32 to 2,048 rows of W is slower.
+static int gs_pieces(int M, int N, int K) {
+    const int blocks = (N + 4 * GS_ROWS - 1) / (4 * GS_ROWS), room = (sp_sm_count() > 0 ? sp_sm_count() : 148) * 4;
+    if (M > 4 || K < 1024 * (blocks >= 128 ? (M == 1 ? 2 : 3) : (M == 1 ? 3 : 4))) return 1;
+    int pieces = 1;
+    while (pieces < GS_PIECES && (long long)blocks * pieces * 2 <= room && K >= pieces * 2 * GS_KC) pieces *= 2;
+    return pieces;
+}
+SP_API int sp_gemm_f32_pieces(int M, int N, int K) { return gs_pieces(M, N, K); }
+
 SP_API int sp_gemm_generic(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt,
                            int M, int N, int K, int lda, int ldw, int ldc, int accumulate,
                            cudaStream_t stream) {
@@ -436,8 +450,7 @@ SP_API int sp_gemm_generic(const void* A, int a_dt, const void* W, int w_dt, voi
     if (M <= 16 && a_dt == SP_DT_F32 && w_dt == SP_DT_F32 && ((K | lda | ldw) & 3) == 0 &&
         ((((uintptr_t)A) | ((uintptr_t)W)) & 15) == 0) {
         const unsigned blocks = (unsigned)((N + 4 * GS_ROWS - 1) / (4 * GS_ROWS));
-        unsigned pieces = 1;
-        while (M <= 4 && pieces < GS_PIECES && blocks * pieces * 2 <= (unsigned)sp_sm_count() * 4 && (unsigned)K >= pieces * 2 * GS_KC) pieces *= 2;
+        const unsigned pieces = (unsigned)gs_pieces(M, N, K);
 #define GS_LAUNCH(MT, SPLIT) \
         SP_CHECK_CALL("gemm_stream_f32", sp_launch_cluster(gemm_stream_f32_kernel<MT, SPLIT>, dim3(blocks * pieces), dim3(128), 0, stream, -(int)pieces, \
                                                            (const float*)A, (const float*)W, C, c_dt, M, N, K, lda, ldw, ldc, accumulate, (int)pieces))

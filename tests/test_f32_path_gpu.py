@@ -92,7 +92,7 @@ def test_few_rows_slices_of_k(K, M, N, Kd):
 
 
 @pytest.mark.parametrize("M", [1, 4, 5, 16])
-@pytest.mark.parametrize("N,Kd", [(9, 1024), (24, 2048), (17, 2564), (3, 5000), (2048, 8192)])
+@pytest.mark.parametrize("N,Kd", [(9, 1024), (24, 2048), (17, 2564), (9, 3076), (24, 4096), (17, 4612), (3, 5000), (2048, 8192)])
 def test_few_rows_columns_shared_by_ctas(K, M, N, Kd):
     a, w = operands(M, N, Kd)
     c0 = torch.randn(M, N, device=DEV)
@@ -103,6 +103,15 @@ def test_few_rows_columns_shared_by_ctas(K, M, N, Kd):
     # a lane adds Kd / 32 terms or fewer in order, five rounds of sums, at most three sums of pieces
     assert bool(((out.double() - a.double() @ w.double().t()).abs() <= (Kd / 32 + 11) * 2.0 ** -24 * size).all())
     assert torch.equal(acc, out + c0)
+
+
+def test_short_sums_are_not_shared(K):
+    """Where a cluster costs more than it saves (the figures stand at the rule) one CTA takes all of K."""
+    pieces = K.load("generic").sp_gemm_f32_pieces
+    for N, one, more in ((32, 3072, 4096), (512, 3072, 4096), (1024, 2048, 3072), (2048, 2048, 3072)):
+        assert pieces(1, N, one - 1) == pieces(2, N, more - 1) == pieces(4, N, more - 1) == pieces(5, N, 14336) == 1
+        assert pieces(1, N, one) > 1 and pieces(2, N, more) > 1 and pieces(4, N, more) > 1
+    assert pieces(1, 100000, 8192) == 1
 
 
 @pytest.mark.parametrize("nh,nkv,hd,vd", [(4, 2, 64, 64), (3, 1, 32, 32), (2, 2, 20, 20), (8, 2, 128, 128), (8, 1, 96, 36), (10, 2, 4, 128)])
