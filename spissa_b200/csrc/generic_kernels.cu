@@ -1003,11 +1003,30 @@ attention_decode_f32_kernel(const float* q, const float* kpool, const float* vpo
     }
 }
 
+// Whether the clusters are the faster way for ``clusters`` (token, kv head) with at most ``keys`` keys each. About 70 of them are
+// on the chip at once; while they are, they win (us, the kernel above / clusters: 8 heads of 64, 64 keys 7.6 / 3.2, 2,048 keys
+// 79.6 / 8.4). More of them pay for their barriers in turn, which only longer sequences are worth: 32 heads of 64 on 8, 128
+// clusters: 16 keys 4.9 / 6.5, 128 13.1 / 10.5; 256: 64 keys 12.4 / 17.3, 256 31.5 / 20.6; 1,024: 128 keys 62.5 / 68.2, 512
+// 217 / 115; 8 heads of 32, 1,024: 512 keys 43.3 / 50.7. Longer rows are worth it sooner, groups of more than 4 heads, which
+// take longer to merge, later: 16 heads of 128 on 4, 256 clusters, 128 keys 28.3 / 20.9; 64 of 64 on 8, 32 clusters, 16 keys
+// 5.9 / 8.2, 128 10.0 / 8.2, 64 clusters 128 keys 11.0 / 12.0. (A decode step's ``keys`` are its bucket of lengths, of which the
+// smallest is 256: the lines for up to 256 keys are drawn at 128.)
+static bool ad_pays(long long clusters, int rep, int hd, int vd, int keys) {
+    const bool wide = hd > 64 || vd > 64, narrow = hd <= 32 && vd <= 32;
+    if (keys > 256) return !narrow || clusters <= 256 || keys > 512;
+    if (rep > 4) return clusters <= (keys <= 64 ? 16 : wide ? 64 : 32);
+    return clusters <= (keys <= 64 || (narrow && rep > 1) ? 64 : wide ? 256 : 128);
+}
+SP_API int sp_attention_decode_f32_pays(int T, int nh, int nkv, int hd, int vd, int keys) {
+    return nkv > 0 && nh % nkv == 0 && ad_pays((long long)T * nkv, nh / nkv, hd, vd, keys);
+}
+
+// ``longest``: how many keys the longest sequence may have (0: as many as the page table's rows); it only shapes the work.
 SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, const void* vpool, int cache_dt,
                                 void* out, const int* token_seq, const int* positions, const int* seq_slot,
                                 const int* page_table, int max_pages, int page_size, int T, int nh, int nkv,
                                 int hd, int vd, int window, float scale, const float* sink, const float* dist_bias,
-                                int dist_cap, cudaStream_t stream) {
+                                int dist_cap, int longest, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (dist_bias && dist_cap < 0) SP_FAIL("attention: a distance-bias table needs at least one entry per head");
     if (hd <= 0 || hd > AG_WIDE_HD) SP_FAIL("attention: head_dim %d is beyond this kernel's limit %d", hd, AG_WIDE_HD);
@@ -1019,7 +1038,8 @@ SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, cons
     // few (token, head) pairs (a decode step): a CTA per pair, its warps share the keys
     const bool split = warps <= 4096;
     const int rep = nh / nkv;
-    if (split && q_dt == SP_DT_F32 && cache_dt == SP_DT_F32 && rep <= 8 && hd <= 128 && vd <= 128 && ((hd | vd) & 3) == 0 &&
+    if (longest <= 0) longest = max_pages * page_size;
+    if (split && ad_pays((long long)T * nkv, rep, hd, vd, window > 0 && window < longest ? window : longest) && q_dt == SP_DT_F32 && cache_dt == SP_DT_F32 && rep <= 8 && hd <= 128 && vd <= 128 && ((hd | vd) & 3) == 0 &&
         (((uintptr_t)q | (uintptr_t)kpool | (uintptr_t)vpool | (uintptr_t)out) & 15) == 0) {
 #define AD_LAUNCH(LPR, REP)                                                                                            \
     SP_CHECK_CALL("attention_decode_f32", sp_launch_cluster(attention_decode_f32_kernel<LPR, REP>, dim3(AD_CLUSTER, nkv, T), dim3(128), 0, stream, \

@@ -223,11 +223,12 @@ def _dist_bias_args(dist_bias, nh):
     return c_void_p(_ptr(dist_bias)), int(dist_bias.shape[1]) - 1
 
 
-def attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, window, scale, vd=None, sink=None, dist_bias=None):
+def attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, window, scale, vd=None, sink=None, dist_bias=None, longest=0):
     """Causal attention of every token of the step over its sequence's cached keys; ``vd``: the size of a value row
     when it differs from a key row's (``out`` is then [T, nh·vd]). ``sink`` (float32 [nh]): per head a score that joins
     the softmax's denominator once and has no value. ``dist_bias`` (float32 [nh, entries]): a score added by the
-    distance between query and key, beyond the scale."""
+    distance between query and key, beyond the scale. ``longest``: the keys that the longest sequence may have (0: as many
+    as the page table's rows); it only shapes the work."""
     lib = load("generic")
     bias_ptr, bias_cap = _dist_bias_args(dist_bias, nh)
     if sink is not None and (sink.dtype != torch.float32 or sink.numel() != nh):
@@ -241,7 +242,7 @@ def attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, window, scale, 
         c_void_p(_ptr(out)), c_void_p(_ptr(meta.token_seq)), c_void_p(_ptr(meta.positions)),
         c_void_p(_ptr(meta.seq_slot)), c_void_p(_ptr(pt)), pt.shape[1], meta.page_size,
         T, nh, nkv, hd, int(vd or hd), int(window or 0), c_float(scale), c_void_p(_ptr(sink)), bias_ptr, bias_cap,
-        c_void_p(_stream())))
+        int(longest), c_void_p(_stream())))
 
 
 def attention_tile_f32_supported(q, k_pool, v_pool, n_seqs, nh, nkv, hd, vd) -> bool:

@@ -177,8 +177,10 @@ def attend_paged(q, step, cache, nh, nkv, hd, window, scale, sink=None, counters
                              scale, vd=vd, sink=sink, dist_bias=dist_bias)
         return ctx
     else:
+        # (a decode step by its length's bucket, as below: run directly and replayed from a graph it takes the same way)
+        longest = length_bucket(step.max_len, cache.page_size) if step.all_single else step.max_len
         K.attention_generic(q, cache.k_pool, cache.v_pool, ctx, cache, nh, nkv, hd, window, scale, vd=vd, sink=sink,
-                            dist_bias=dist_bias)
+                            dist_bias=dist_bias, longest=longest)
         return ctx
     if step.all_single:
         # the split is made for the length's bucket, not the length: a step run directly and the same step

@@ -151,6 +151,27 @@ def test_attention_of_a_decode_step(K, nh, nkv, hd, vd, window, extra):
     assert float((out.double().cpu() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
 
 
+def test_many_short_sequences_take_no_clusters(K):
+    """The lines of the rule (its figures stand there), and both ways' results on the same step."""
+    pays = K.load("generic").sp_attention_decode_f32_pays
+    for rep, hd, least, few in ((1, 64, 64, 128), (4, 64, 64, 128), (1, 32, 64, 128), (4, 32, 64, 64), (4, 128, 64, 256),
+                                (8, 64, 16, 32), (8, 128, 16, 64)):
+        for keys, most in ((1, least), (64, least), (65, few), (256, few)):
+            assert pays(most, rep, 1, hd, hd, keys) and not pays(most + 1, rep, 1, hd, hd, keys)
+        assert pays(256, rep, 1, hd, hd, 257) and bool(pays(257, rep, 1, hd, hd, 512)) == (hd > 32) and pays(9999, rep, 1, hd, hd, 513)
+    nh, nkv, hd, B = 4, 2, 64, 70
+    torch.manual_seed(3)
+    meta = KH.paged_meta([1] * B, [3 * i for i in range(B)], DEV, seed=3)
+    kv = [[torch.randn(t, nkv, hd) for t in meta.total_len] for _ in range(2)]
+    k_pool, v_pool = KH.fill_cache(meta, *kv, nkv, hd, torch.float32, DEV)
+    q = torch.randn(B, nh * hd, device=DEV)
+    outs = [torch.full((B, nh * hd), float("nan"), device=DEV) for _ in range(2)]
+    for out, longest in zip(outs, (210, 300)):
+        K.attention_generic(q, k_pool, v_pool, out, meta, nh, nkv, hd, None, 0.125, longest=longest)
+    # two orders of the same sums, each as near to them as the test above allows
+    assert float((outs[0] - outs[1]).abs().max()) <= 6e-6 * float(outs[1].abs().max())
+
+
 def test_a_value_that_is_not_finite_stays_with_its_group(K):
     """A decode step's NaN key and infinite value reach the heads and the sequence that see them, and no others."""
     nh, nkv, hd, before = 4, 2, 64, [600, 600]
