@@ -1450,6 +1450,10 @@ SP_API int sp_mingru_chunked(const float* proj, const void* zb, const void* xb, 
 
 // ============================================================== PolyNorm
 // out = a·z/rms(z) + b·z²/rms(z²) + c·z³/rms(z³) + e over each row of z (32-bit), rms with eps inside the root.
+// KEPT: the first 1,024·KEPT values of a row stay in registers, so that it is read once (2,000 rows of 8,192: 23 -> 18 us); as many
+// as the row needs, for the registers are those of other blocks (2,000 rows of 512 6.2 us, 10.4 with KEPT 8; of 2,048 8.6 and
+// 11.8). 0: rows that do not move in 16 bytes.
+template <int KEPT>
 __global__ void __launch_bounds__(256)
 polynorm_kernel(const float* __restrict__ z, const void* __restrict__ coef, int c_dt, void* __restrict__ out, int out_dt,
                 int T, int F, float eps) {
@@ -1458,9 +1462,8 @@ polynorm_kernel(const float* __restrict__ z, const void* __restrict__ coef, int 
     if (t >= T) return;
     const float* row = z + (size_t)t * F;
     float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
-    const bool vec = (F & 3) == 0 && (((uintptr_t)z) & 15) == 0;
-    // the first 8,192 values stay in registers: a row is read once (2,000 rows of 8,192: 23 -> 18 us)
-    float4 kept[8];
+    constexpr bool vec = KEPT > 0;
+    float4 kept[KEPT > 0 ? KEPT : 1];
     if (vec) {
         auto add = [&](const float4& q) {
             const float e[4] = {q.x, q.y, q.z, q.w};
@@ -1473,13 +1476,13 @@ polynorm_kernel(const float* __restrict__ z, const void* __restrict__ coef, int 
             }
         };
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < KEPT; ++u) {
             const int c = (threadIdx.x + 256 * u) * 4;
             kept[u] = c < F ? *(const float4*)(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) add(kept[u]);
-        for (int c = threadIdx.x * 4 + 8192; c < F; c += 1024) add(*(const float4*)(row + c));
+        for (int u = 0; u < KEPT; ++u) add(kept[u]);
+        for (int c = threadIdx.x * 4 + 1024 * KEPT; c < F; c += 1024) add(*(const float4*)(row + c));
     } else
     for (int c = threadIdx.x; c < F; c += blockDim.x) {
         const float v = row[c], v2 = v * v, v3 = v2 * v;
@@ -1503,10 +1506,13 @@ polynorm_kernel(const float* __restrict__ z, const void* __restrict__ coef, int 
             }
             sm_st4_dt(out, out_dt, (size_t)t * F + c, make_float4(o[0], o[1], o[2], o[3]));
         };
+        // (opaque here: else the squares and cubes are kept as well, 128 registers for KEPT 8)
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < KEPT; ++u) asm volatile("" : "+f"(kept[u].x), "+f"(kept[u].y), "+f"(kept[u].z), "+f"(kept[u].w));
+#pragma unroll
+        for (int u = 0; u < KEPT; ++u)
             if ((threadIdx.x + 256 * u) * 4 < F) put((threadIdx.x + 256 * u) * 4, kept[u]);
-        for (int c = threadIdx.x * 4 + 8192; c < F; c += 1024) put(c, *(const float4*)(row + c));
+        for (int c = threadIdx.x * 4 + 1024 * KEPT; c < F; c += 1024) put(c, *(const float4*)(row + c));
         return;
     }
     for (int c = threadIdx.x; c < F; c += blockDim.x) {
@@ -1518,7 +1524,9 @@ polynorm_kernel(const float* __restrict__ z, const void* __restrict__ coef, int 
 SP_API int sp_polynorm(const float* z, const void* coef, int c_dt, void* out, int out_dt, int T, int F, float eps,
                        cudaStream_t stream) {
     if (T <= 0) return 0;
-    polynorm_kernel<<<T, 256, 0, stream>>>(z, coef, c_dt, out, out_dt, T, F, eps);
+    const bool vec = (F & 3) == 0 && (((uintptr_t)z) & 15) == 0;
+    auto* kernel = !vec ? polynorm_kernel<0> : F <= 1024 ? polynorm_kernel<1> : F <= 2048 ? polynorm_kernel<2> : F <= 4096 ? polynorm_kernel<4> : polynorm_kernel<8>;
+    kernel<<<T, 256, 0, stream>>>(z, coef, c_dt, out, out_dt, T, F, eps);
     SP_CHECK_LAUNCH("polynorm");
     return 0;
 }

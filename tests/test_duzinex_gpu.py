@@ -150,7 +150,7 @@ def test_dynamic_tanh_and_polynorm_kernels(out_dtype):
     assert worst(rows32, x.double() + bias.double()) <= 1e-6
 
 
-@pytest.mark.parametrize("width", [4, 201, 1028, 8192, 8196])
+@pytest.mark.parametrize("width", [4, 201, 1024, 1028, 2048, 2052, 4096, 4100, 8192, 8196])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dynamic_tanh_and_polynorm_by_sixteen_bytes_and_by_elements(width, dtype):
     """Widths in fours and not, rows longer than what a block of PolyNorm holds."""
