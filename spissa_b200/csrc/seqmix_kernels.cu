@@ -891,19 +891,20 @@ SP_API int sp_retention(const float* proj, int ld, float* state, int n_slots, co
 template <typename Scale>
 __device__ __forceinline__ void rc_load(float* to, int st, int all_rows, int all_cols, const float* from, size_t ld, int rows, int cols,
                                         bool vec, Scale scale) {
+    const int bits = all_cols == 64 ? 6 : 7;                // columns: 64 or 128
     if (vec) {
-        const int per = all_cols / 4, n = all_rows * per;
+        const int n = all_rows << (bits - 2);
         for (int e0 = threadIdx.x; e0 < n; e0 += 8 * 256) {
             float4 v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int e = e0 + 256 * u, r = e / per, c = (e - r * per) * 4;
+                const int e = e0 + 256 * u, r = e >> (bits - 2), c = (e << 2) & (all_cols - 1);
                 v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (e < n && r < rows && c < cols) v[u] = *(const float4*)(from + (size_t)r * ld + c);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int e = e0 + 256 * u, r = e / per, c = (e - r * per) * 4;
+                const int e = e0 + 256 * u, r = e >> (bits - 2), c = (e << 2) & (all_cols - 1);
                 if (e >= n) break;
                 const float f = scale(r);
                 *(float4*)(to + r * st + c) = make_float4(v[u].x * f, v[u].y * f, v[u].z * f, v[u].w * f);
@@ -911,9 +912,19 @@ __device__ __forceinline__ void rc_load(float* to, int st, int all_rows, int all
         }
         return;
     }
-    for (int e = threadIdx.x; e < all_rows * all_cols; e += 256) {
-        const int r = e / all_cols, c = e - r * all_cols;
-        to[r * st + c] = r < rows && c < cols ? from[(size_t)r * ld + c] * scale(r) : 0.0f;
+    const int n = all_rows << bits;
+    for (int e0 = threadIdx.x; e0 < n; e0 += 8 * 256) {     // (whole rounds: all_rows is a multiple of 64)
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int e = e0 + 256 * u, r = e >> bits, c = e & (all_cols - 1);
+            v[u] = r < rows && c < cols ? from[(size_t)r * ld + c] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int e = e0 + 256 * u, r = e >> bits;
+            to[r * st + (e & (all_cols - 1))] = v[u] * scale(r);
+        }
     }
 }
 
@@ -1136,8 +1147,8 @@ __global__ void __launch_bounds__(256) retention_chunk_out_kernel(RcArgs a, int 
     }
     __syncwarp();                                           // a row of P is written and read by the same half warp
     float inter[4][4 * NB] = {}, intra[4][4 * NB] = {};
-    rc_rows_mm<NB>(Q, DS, S, NP, DP, inter, ty, tx);
-    rc_rows_mm<NB>(P, PS, vv, NP, RC_CHUNK, intra, ty, tx);
+    rc_rows_mm<NB>(Q, DS, S, NP, (d + 3) & ~3, inter, ty, tx);      // (behind d and n the arrays hold zeros)
+    rc_rows_mm<NB>(P, PS, vv, NP, (n + 3) & ~3, intra, ty, tx);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         const int i = ty + 16 * u;
@@ -1159,46 +1170,63 @@ __global__ void __launch_bounds__(256) retention_chunk_out_kernel(RcArgs a, int 
     }
 }
 
-// (D) unit rms over the head's values, the gate, the store: a warp per (token, head)
+// (D) unit rms over the head's values, the gate, the store: a warp per (token, head), grid (tokens / 8, H). A lane holds its first
+// HELD pieces of values and gates, of four (VEC) or one: as many as the rows have, for in a decode step fetching the
+// instructions is a good part of the kernel's time.
+template <bool VEC, int HELD>
 __global__ void __launch_bounds__(256) retention_finish_kernel(RcArgs a, int T) {
-    const int lane = threadIdx.x & 31;
-    const long long at = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (at >= (long long)T * a.H) return;
-    const int t = (int)(at / a.H), h = (int)(at % a.H);
+    const int lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5), h = blockIdx.y;
+    if (t >= T) return;
     const int vd = a.vd, Hv = a.H * vd;
     const float* o = a.o_raw + (size_t)t * Hv + h * vd;
     const float* g = a.proj + (size_t)t * a.ld + 2 * a.H * a.d + Hv + h * vd;
     const size_t to = (size_t)t * Hv + h * vd;
     float ss = 0.0f;
-    if (a.vec) {
-        float4 v[4], z[4];                                   // rows of up to 512 values are held, with their gates
+    if constexpr (VEC) {
+        float4 v[HELD], z[HELD];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < HELD; ++i) {
             const int c = 4 * lane + 128 * i;
             v[i] = z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (c < vd) { v[i] = *(const float4*)(o + c); z[i] = *(const float4*)(g + c); }
             ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
         }
-        for (int c = 4 * lane + 512; c < vd; c += 128) {
+        for (int c = 4 * lane + 128 * HELD; c < vd; c += 128) {
             const float4 w = *(const float4*)(o + c);
             ss = fmaf(w.x, w.x, fmaf(w.y, w.y, fmaf(w.z, w.z, fmaf(w.w, w.w, ss))));
         }
         const float inv = 1.0f / sqrtf(sp_warp_sum(ss) / (float)vd + a.eps);
         auto put = [&](int c, const float4& x, const float4& y) {
-            const float4 r = make_float4(x.x * inv * sm_silu(y.x), x.y * inv * sm_silu(y.y), x.z * inv * sm_silu(y.z), x.w * inv * sm_silu(y.w));
-            if (a.out_dt == SP_DT_F32) { *(float4*)((float*)a.out + to + c) = r; return; }
-            const __nv_bfloat162 p0 = __floats2bfloat162_rn(r.x, r.y), p1 = __floats2bfloat162_rn(r.z, r.w);
-            *(uint2*)((__nv_bfloat16*)a.out + to + c) = make_uint2(*(const uint32_t*)&p0, *(const uint32_t*)&p1);
+            sm_st4_dt(a.out, a.out_dt, to + c, make_float4(x.x * inv * sm_silu(y.x), x.y * inv * sm_silu(y.y), x.z * inv * sm_silu(y.z), x.w * inv * sm_silu(y.w)));
         };
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < HELD; ++i)
             if (4 * lane + 128 * i < vd) put(4 * lane + 128 * i, v[i], z[i]);
-        for (int c = 4 * lane + 512; c < vd; c += 128) put(c, *(const float4*)(o + c), *(const float4*)(g + c));
-        return;
+#pragma unroll 1
+        for (int c = 4 * lane + 128 * HELD; c < vd; c += 128) put(c, *(const float4*)(o + c), *(const float4*)(g + c));
+    } else {
+        float v[HELD], z[HELD];
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = lane + 32 * i;
+            v[i] = z[i] = 0.0f;
+            if (c < vd) { v[i] = o[c]; z[i] = g[c]; }
+        }
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) ss = fmaf(v[i], v[i], ss);
+        for (int c = lane + 32 * HELD; c < vd; c += 32) ss = fmaf(o[c], o[c], ss);
+        const float inv = 1.0f / sqrtf(sp_warp_sum(ss) / (float)vd + a.eps);
+#pragma unroll
+        for (int i = 0; i < HELD; ++i)
+            if (lane + 32 * i < vd) sp_st_dt(a.out, a.out_dt, to + lane + 32 * i, v[i] * inv * sm_silu(z[i]));
+#pragma unroll 1
+        for (int c = lane + 32 * HELD; c < vd; c += 32) sp_st_dt(a.out, a.out_dt, to + c, o[c] * inv * sm_silu(g[c]));
     }
-    for (int c = lane; c < vd; c += 32) ss = fmaf(o[c], o[c], ss);
-    const float inv = 1.0f / sqrtf(sp_warp_sum(ss) / (float)vd + a.eps);
-    for (int c = lane; c < vd; c += 32) sp_st_dt(a.out, a.out_dt, to + c, o[c] * inv * sm_silu(g[c]));
+}
+static void retention_finish(const RcArgs& a, int T, cudaStream_t stream) {
+    auto* kernel = !a.vec ? (a.vd <= 64 ? retention_finish_kernel<false, 2> : retention_finish_kernel<false, 8>)
+                   : a.vd <= 128 ? retention_finish_kernel<true, 1> : a.vd <= 256 ? retention_finish_kernel<true, 2> : retention_finish_kernel<true, 4>;
+    kernel<<<dim3((T + 7) / 8, a.H), 256, 0, stream>>>(a, T);
 }
 
 SP_API int sp_retention_chunked_supported(int d, int vd) { return d > 0 && d <= 128 && vd > 0; }
@@ -1245,7 +1273,7 @@ SP_API int sp_retention_chunked(const float* proj, int ld, float* state, int n_s
     if (NB == 1) retention_chunk_out_kernel<1><<<grid, 256, smem_c, stream>>>(a, DP);
     else retention_chunk_out_kernel<2><<<grid, 256, smem_c, stream>>>(a, DP);
     SP_CHECK_LAUNCH("retention_chunk_out");
-    retention_finish_kernel<<<(unsigned)(((long long)T * H + 7) / 8), 256, 0, stream>>>(a, T);
+    retention_finish(a, T, stream);
     SP_CHECK_LAUNCH("retention_finish");
     return 0;
 }
@@ -1310,7 +1338,7 @@ SP_API int sp_retention_step(const float* proj, int ld, float* state, int n_slot
     if (smem > 48 * 1024) SP_FAIL("retention (step): key size %d is beyond this kernel's range", d);
     retention_step_kernel<<<dim3(B, H, (vd + 31) / 32), 256, smem, stream>>>(a);
     SP_CHECK_LAUNCH("retention_step");
-    retention_finish_kernel<<<(unsigned)(((long long)B * H + 7) / 8), 256, 0, stream>>>(a, B);
+    retention_finish(a, B, stream);
     SP_CHECK_LAUNCH("retention_finish");
     return 0;
 }

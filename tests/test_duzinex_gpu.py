@@ -203,7 +203,7 @@ def test_token_shift_kernel_carries_the_last_row_in_the_state():
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(3, 8, 16), (1, 40, 24), (2, 16, 70), (2, 128, 130), (1, 72, 256), (1, 130, 8),
-                                             (2, 100, 40), (2, 32, 32), (1, 20, 644)])
+                                             (2, 100, 40), (2, 32, 32), (1, 20, 644), (2, 32, 33), (1, 30, 301)])
 def test_retention_kernel(heads, dim, vdim):
     """Sequences of 50 and 39 tokens run in chunks (where the key size allows), the single token and the portions
     below token by token; a chunk boundary lies inside nothing here, the next test crosses several."""
