@@ -50,3 +50,19 @@ def test_graph_table_evicts_the_graph_used_longest_ago():
     for i in range(1000):                                              # sightings of keys that never come back
         t.wants_capture(("once", i))
     assert len(t.seen) <= 8 * 3 + 1
+
+
+def test_the_choice_of_a_kernel_is_kept_for_each_device(monkeypatch):
+    from types import SimpleNamespace
+    import torch
+    from spissa_b200.csrc import lib
+    sms = {0: 148, 1: 74}
+    at = [0]
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: at[0])
+    monkeypatch.setattr(lib, "load", lambda name: SimpleNamespace(sp_tc_mid_or_pairs=lambda *a: sms[at[0]]))
+    for device in (0, 1, 0):
+        at[0] = device
+        assert lib.tc_mid_or_pairs(lib.TC_STORE, 1111, 2222, 3333) == sms[device]
+    for name in ("tc_mid_or_pairs", "_mid_or_pairs"):
+        getattr(getattr(lib, name, None), "cache_clear", lambda: None)()
