@@ -491,9 +491,9 @@ bool fill_plan(Plan& p, int parts, int M, int num_kb) {
     return p.stages >= 1 && p.tmem_cols <= 512;
 }
 
-// The division of a product (``estimate``: its time), by an estimate of its time in nanoseconds that was fitted to 1,276 measured divisions of the
-// products of the 1B and 8B layer sizes at 17 to 1,000 tokens (its choices are 1.5 % slower than the best of them on
-// average, 11 % at worst). A CTA takes in its blocks of K at about 115 bytes a nanosecond, two on one SM together at 136;
+// The division of a product, by an estimate of its time in nanoseconds (``estimate``) that was fitted to 1,276 measured
+// divisions of the products of the 1B and 8B layer sizes at 17 to 1,000 tokens (its choices are 1.5 % slower than the best of
+// them on average, 11 % at worst). A CTA takes in its blocks of K at about 115 bytes a nanosecond, two on one SM together at 136;
 // every wave adds the epilogue: 42 ns a token of the tile, 12 per token of the share, a microsecond for the exchange of
 // pieces and 170 ns per piece. Clusters of 4 and 8 do not find room on every SM: 136 and 128 CTAs at a time.
 Plan plan_of(int mode, int M, int N, int K, double* estimate = nullptr) {
@@ -541,27 +541,35 @@ SP_API int sp_tc_mid_plan(int mode, int M, int N, int K, int* out) {
 }
 
 // Which kernel takes a product of more than 128 tokens that both this one and the tiles by pairs of CTAs of tc_gemm.cu (256
-// rows, 74 pairs on 148 SMs) could: the width of those tiles, a multiple of ``multiple``, or 0 for this kernel. By the two
-// estimates of time: a round of pair tiles takes 0.36 us per 64 of K at 256 columns, 0.335 at 192 and 0.31 at 128, and the
-// launch with its last epilogue 10 us (measured at 128 to 6,000 tokens of the 1B and 8B layer sizes: within 15 %).
+// rows, 74 pairs on 148 SMs) could: the width of those tiles, a multiple of ``multiple``, or 0 for this kernel. By two estimates of
+// time, compared with 2,902 measured products (N 512 to 32,000, K 256 to 14,336): the choice is 0.3 % slower than the better
+// kernel on average for gated ones and 3.5 % for the others.
+//   Pairs: a round of tiles takes 0.36 us per 64 of K at 256 columns, 0.335 at 192 and 0.31 at 128, the launch with its last
+// epilogue 10 us, less where one round of narrow tiles does and K is short (512 x 512, 2,048 tokens 7.9 us, this kernel 10.8); gated
+// ones 0.323, 3.5 for a round's epilogue and 5 for the launch.
+//   This kernel: plan_of's, which was made to compare divisions and is 10 % short for gated products on average.
 // Gated products are worth pairs as soon as their rounds come out full, for they have the most rows of W (us, this kernel /
-// pairs: 1B 200 tokens 24.8 / 21.1, 301: 27.7 / 31.6, 512: 37.4 / 32.6, 1,023: 71.8 / 58.2; 8B 512: 122 / 103, 768: 206 / 138); the
-// others from 1,024 tokens on, this kernel still where their pair tiles fill few SMs (1B, 1,280 tokens: output 16.1 / 20.2,
-// down 40.5 / 51.7, 1,700 QKV 22.6 / 30.3; 8B 1,280 down 125 / 168).
+// pairs: 1B 200 tokens 24.1 / 20.5, 301: 27.0 / 31.1, 512: 36.5 / 31.8, 1,023: 71.3 / 56.6; 3B 256: 32.0 / 27.3, 800 88.9 / 79.5; 8B
+// 257: 89 / 107, 512: 123 / 109, 768: 201 / 139, 800: 209 / 206, 1,100: 257 / 222, 1,281: 318 / 289); the others from 1,024 tokens
+// on, this kernel still where their pair tiles fill few SMs (1B, 1,280 tokens: output 15.6 / 26.4, down 38 / 84, 1,700 QKV 21.5 /
+// 28.9; 8B 1,280 down 120 / 155).
 SP_API int sp_tc_mid_or_pairs(int mode, int M, int N, int K, int multiple) {
     const bool gated = mode == MODE_SILU_MUL;
     if (M <= 128 || (!gated && M < 1024)) return 0;
     const int walkers = (sp_sm_count() > 0 ? sp_sm_count() : 148) / 2, row_tiles = (M + 255) / 256, num_kb = (K + BK - 1) / BK;
+    auto rounds = [&](int bn) { return (row_tiles * ((N + bn - 1) / bn) + walkers - 1) / walkers; };
+    const double start = rounds(128) > 1 || num_kb > 18 ? 10000.0 : 5500.0 + 250.0 * num_kb;
     int best = 0;
     double best_t = 0;
     for (const int bn : {256, 192, 128}) {
         if ((gated && bn != 256) || (multiple > 1 && bn % multiple)) continue;
-        const int rounds = (row_tiles * ((N + bn - 1) / bn) + walkers - 1) / walkers;
-        const double t = 10000.0 + (double)rounds * num_kb * (bn == 256 ? 360.0 : bn == 192 ? 335.0 : 310.0);
+        const double t = gated ? 5000.0 + rounds(bn) * (3500.0 + num_kb * 323.0)
+                               : start + (double)rounds(bn) * num_kb * (bn == 256 ? 360.0 : bn == 192 ? 335.0 : 310.0);
         if (!best || t < best_t) { best = bn; best_t = t; }
     }
     double mine = 0;
-    return M <= 2048 && plan_of(mode, M, N, K, &mine).nt && mine < best_t ? 0 : best;
+    if (M > 2048 || !plan_of(mode, M, N, K, &mine).nt) return best;
+    return (gated ? 1.1 : 1.0) * mine < best_t ? 0 : best;
 }
 
 // Whether this kernel takes the product (0) or another has to (1, the reason as the last error).

@@ -324,8 +324,14 @@ def test_the_choice_between_the_two_kernels(K):
                 assert width in (0, 128, 256) and not (width and M <= 128) and (width or M <= 2048)
                 assert mode == K.TC_SILU_MUL or not width or M >= 1024
                 assert mode != K.TC_SILU_MUL or width in (0, 256)
+    if torch.cuda.get_device_properties(DEV).multi_processor_count != 148:
+        return                                                          # what follows was measured on 148
     assert K.tc_mid_or_pairs(K.TC_ACCUMULATE, 1280, 2048, 8192) == 0 and K.tc_mid_or_pairs(K.TC_ACCUMULATE, 2048, 2048, 8192) == 256
     assert K.tc_mid_or_pairs(K.TC_SILU_MUL, 301, 16384, 2048) == 0 and K.tc_mid_or_pairs(K.TC_SILU_MUL, 512, 16384, 2048) == 256
+    assert [K.tc_mid_or_pairs(K.TC_STORE, M, 512, 512) for M in (1024, 1280, 1700, 2048)] == [0, 0, 128, 128]
+    # gated rows of the 3B and 8B layers: the kernel that the figures beside the rule show as the faster one
+    assert [K.tc_mid_or_pairs(K.TC_SILU_MUL, M, 16384, 3072) for M in (200, 256, 257, 800)] == [256, 256, 0, 256]
+    assert [K.tc_mid_or_pairs(K.TC_SILU_MUL, M, 28672, 4096) for M in (200, 257, 512, 768, 880, 1100, 1281)] == [0, 0] + 5 * [256]
 
 
 @pytest.mark.parametrize("M", [1024, 1279, 1537, 2048])
