@@ -23,9 +23,9 @@
 //     launch arguments or, for a launch replayed from a CUDA graph, as two words on the device), two groups of
 //     four warps per CTA with cp.async double buffering, the keys as the M of mma.sync and the query heads of
 //     the kv head as its N (flash_common.cuh: decode_step_t), then one warp per (token, head) combines the chunks.
-//     Where the split is into 1, 2 or 4 chunks (about as many items as warp groups: eight sequences of eight kv
-//     heads, for instance) the CTAs are launched as pairs (a thread-block cluster of two) and all chunks of a
-//     (sequence, kv head) sit in one pair: the groups leave their partial results in shared memory, the pair's first
+//     For layers of head size 64 and up to eight query heads a kv head the CTAs are launched as pairs (a thread-block
+//     cluster of two), and where the split is into 1, 2 or 4 chunks (plan_split: short sequences, or about as many items
+//     as warp groups) all chunks of a (sequence, kv head) sit in one pair: the groups leave their partial results in shared memory, the pair's first
 //     CTA reads its partner's through distributed shared memory behind a cluster-scope mbarrier and writes the
 //     heads' outputs itself, so the combination costs neither a phase of its own nor its grid barrier;
 //   * phases that need every CTA's result are separated by a grid barrier (cooperative launch; an atomic
@@ -1178,29 +1178,37 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// The most chunks of a (sequence, kv head) that T sequences can have combined within a CTA or a CTA pair, or 0. Fewer than eight
-// (sequence, kv head) in all would leave nearly every SM without keys: these keep the finer split, whatever the length.
-int pair_chunks(int G, int T, int hd, int max_nkv) {
-    const int items = T * (max_nkv > 0 ? max_nkv : 1);
+// The most chunks of a (sequence, kv head) that T sequences can have combined within a CTA or a CTA pair, or 0. The pair-wise
+// form is built for up to eight query heads a kv head; where a layer has more, the others have it as far as it fills three
+// quarters of the warp groups (what layers of more heads lose by fewer chunks is then small). Fewer than eight (sequence, kv head)
+// in all keep the finer split, although the other is faster there too (8 layers with one kv head, a sequence of 100 keys 419
+// us a step / 388 by two chunks, of 600 424 / 413, of 2,000 430 either way): a gain left open.
+int pair_chunks(int G, int T, int hd, int max_nkv, int max_heads_per_kv) {
+    const int groups = G * 2, items = T * (max_nkv > 0 ? max_nkv : 1), want = groups / items;
     if (hd != 64 || (G % 2) != 0 || items < 8) return 0;
-    const int want = G * 2 / items;
-    return want >= 4 ? 4 : (want >= 2 ? 2 : (want >= 1 ? 1 : 0));
+    const int c = want >= 4 ? 4 : (want >= 2 ? 2 : (want >= 1 ? 1 : 0));
+    return max_heads_per_kv <= 8 || 4 * items * c >= 3 * groups ? c : 0;
 }
 
 // The split of the keys. Either about one (sequence, kv head, chunk) item per warp group of the grid, whose results a phase of its
-// own behind one more grid barrier combines; or 1, 2 or 4 chunks of longer, combined within a CTA (two) or a CTA pair (four). By
-// an estimate in microseconds: a page costs a group 0.6 (0.9 with two stages), the phase and its barrier 5.4, the exchange
-// between the CTAs of a pair 1.5. Measured with 8 layers of the 1B shape, us a step by the first / by the estimate: 1 sequence of
-// 100 keys SPLIT_A, 600 SPLIT_B, 2,048 SPLIT_C; 4 of 1,000 SPLIT_D; 10 of 500 SPLIT_E, of 2,048 SPLIT_F; 13 of 600 SPLIT_G.
-int plan_split(int G, int T, int hd, int len_pages, int max_nkv, int* chunk_pages, int* n_chunks) {
+// own behind one more grid barrier combines; or 1, 2 or 4 chunks of longer, combined within a CTA (two) or a CTA pair (four), even
+// where that leaves most groups without keys. By an estimate in microseconds a layer: a page costs a group 0.6 (0.9 with two
+// stages), the phase and its barrier 5.4, the exchange between the CTAs of a pair 1.5. (A split into one item per group that
+// ends in 1, 2 or 4 chunks is charged the phase too: the same number of chunks is then among the others.) 8 layers 1B with the
+// head, us a step with the pair-wise form only where it fills three quarters of the groups / by the estimate: 1 sequence of 100
+// keys 442 / 407, 300 439 / 411, 600 445 / 426, 1,000 447 / 436, 2,000 447 / 447; 4 of 100 455 / 421, 1,000 462 / 450, 2,000 475 /
+// 473; 8 of 100 452 / 442, 2,000 495 / 494; 10 of 300 496 / 470, 1,000 518 / 498, 2,000 546 / 551; 13 of 600 529 / 499, 4,000 672 /
+// 643; 2 of 100 on four kv heads 445 / 413. At worst 4 of 2,000 keys on six kv heads, 453 / 461.
+int plan_split(int G, int T, int hd, int len_pages, int max_nkv, int max_heads_per_kv, int* chunk_pages, int* n_chunks) {
     if (len_pages < 1) len_pages = 1;
     const int groups = G * (hd == 64 ? 2 : 1);
     int want = groups / (T * (max_nkv > 0 ? max_nkv : 1));
     if (want < 1) want = 1;
     const double page = attention_stages(hd, T) == 3 ? 0.6 : 0.9;
-    double best = 5.4 + page * ((len_pages + want - 1) / want);
+    const int most = pair_chunks(G, T, hd, max_nkv, max_heads_per_kv);
+    double best = max_heads_per_kv <= 8 ? 5.4 + page * ((len_pages + want - 1) / want) : 1e30;
     int pages = 0, chunks = 0;
-    for (int c = 1; c <= pair_chunks(G, T, hd, max_nkv); c *= 2) {
+    for (int c = max_heads_per_kv <= 8 ? 1 : most; c && c <= most; c *= 2) {
         const int per = (len_pages + c - 1) / c;
         const double t = page * per + (c == 4 ? 1.5 : c == 2 ? 0.3 : 0.0);
         if (per <= 64 && t < best) { best = t; pages = per; chunks = c; }
@@ -1252,12 +1260,13 @@ SP_API int sp_decode_layers_map_bytes() { return (int)sizeof(CUtensorMap); }
 
 // CTAs of the kernel = SMs of the device: the host sizes ``ssq`` ([2][CTAs][16] floats) with it.
 SP_API int sp_decode_layers_ctas() { return sm_count(); }
-// out[0] = pages per chunk, out[1] = chunks, for ``T`` sequences of at most ``len_pages`` pages
-SP_API int sp_decode_layers_plan(int T, int hd, int len_pages, int max_nkv, int* out) {
+// out[0] = pages per chunk, out[1] = chunks, for ``T`` sequences of at most ``len_pages`` pages and layers of at most ``max_nkv``
+// kv heads and ``max_heads_per_kv`` query heads to each
+SP_API int sp_decode_layers_plan(int T, int hd, int len_pages, int max_nkv, int max_heads_per_kv, int* out) {
     const int G = sm_count();
     if (G <= 0) SP_FAIL("decode_layers: cannot read the number of SMs");
     if (T < 1) T = 1;
-    return plan_split(G, T, hd, len_pages, max_nkv, out, out + 1);
+    return plan_split(G, T, hd, len_pages, max_nkv, max_heads_per_kv, out, out + 1);
 }
 SP_API int sp_decode_layers_max_chunks() { return MAX_CHUNKS; }
 SP_API int sp_decode_layers_max_pages() { return MAX_CHUNKS * MAX_CHUNK_PAGES; }
@@ -1345,7 +1354,7 @@ SP_API int sp_decode_layers(const void* layers, const void* maps, int n_layers, 
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.n_stages = stages;
     p.plan = plan;
-    p.pairs = pair_chunks(G, T, hd, max_nkv) > 0 ? 1 : 0;      // CTA pairs only where that split can occur with T sequences
+    p.pairs = pair_chunks(G, T, hd, max_nkv, max_heads_per_kv) > 0 ? 1 : 0;      // CTA pairs only where that split can occur with T sequences
     p.head_mode = next_head.mode;
     p.head_w = (const __nv_bfloat16*)next_head.w;
     p.final_norm = (const __nv_bfloat16*)next_head.norm;
@@ -1366,7 +1375,7 @@ SP_API int sp_decode_layers(const void* layers, const void* maps, int n_layers, 
     next_head.mode = 0;                                        // for this call only
     next_greedy = GreedyArgs{nullptr, nullptr, 0, nullptr, nullptr};
     p.rg = sp_range_host;
-    if (plan_split(G, T, hd, len_pages, max_nkv, &p.chunk_pages, &p.n_chunks)) return 1;
+    if (plan_split(G, T, hd, len_pages, max_nkv, max_heads_per_kv, &p.chunk_pages, &p.n_chunks)) return 1;
     const int smem = stages * STAGE_BYTES + 2 * red_floats(T) * 4 + uni;
 
     void* args[] = {(void*)&p};

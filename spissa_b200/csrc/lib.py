@@ -1009,11 +1009,12 @@ def argmax_candidates(cand, rows: int, n_cand: int, out, note=None) -> None:
         c_void_p(_ptr(note.seq_len) if note is not None else None), c_void_p(_stream())))
 
 
-def decode_layers_plan(T: int, hd: int, len_pages: int, max_nkv: int) -> tuple:
-    """(pages per chunk, chunks) of the keys for ``T`` sequences of at most ``len_pages`` pages."""
+def decode_layers_plan(T: int, hd: int, len_pages: int, max_nkv: int, max_heads_per_kv: int = 8) -> tuple:
+    """(pages per chunk, chunks) of the keys for ``T`` sequences of at most ``len_pages`` pages, in layers of at most
+    ``max_nkv`` kv heads with ``max_heads_per_kv`` query heads each."""
     lib = load("decode_layers")
     out = (ctypes.c_int * 2)()
-    _check("decode_layers", lib.sp_decode_layers_plan(int(T), int(hd), int(len_pages), int(max_nkv), out))
+    _check("decode_layers", lib.sp_decode_layers_plan(int(T), int(hd), int(len_pages), int(max_nkv), int(max_heads_per_kv), out))
     return int(out[0]), int(out[1])
 
 

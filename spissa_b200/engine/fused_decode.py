@@ -156,7 +156,7 @@ class FusedDecode:
         if got is None:
             if len(self._splits) > 4096:
                 self._splits.clear()
-            got = self._splits[key] = K.decode_layers_plan(n_seqs, self.hd, key[1], self.max_nkv)
+            got = self._splits[key] = K.decode_layers_plan(n_seqs, self.hd, key[1], self.max_nkv, self.max_group)
         return got
 
     def _bind_cache(self, cache) -> None:

@@ -259,3 +259,46 @@ def test_chunks_of_several_pages(tmp_path, n_seqs):
         ref = P.model_logits(pcfg, w, q, torch.float64)
         err = float((rows[:, b].double() - ref[n:n + steps]).abs().max()) / float(ref.abs().max())
         assert err <= TOL, f"{n_seqs} sequences, sequence {b}: {err:.3e}"
+
+
+def test_the_split_of_the_keys():
+    """The choices around the lines of the rule (its figures stand there), on the 148 SMs that they were measured on."""
+    from spissa_b200.csrc import lib as K
+    if K.decode_layers_ctas() != 148:
+        pytest.skip("measured on 148 SMs")
+    plan = K.decode_layers_plan
+    # few pages: one or two chunks, no phase to combine them; more: four in a pair of CTAs, until one item a group is worth it
+    assert [plan(1, 64, n, 8) for n in (1, 2, 5, 10, 16, 32)] == [(1, 1), (1, 2), (3, 2), (5, 2), (4, 4), (1, 32)]
+    assert [plan(10, 64, n, 8) for n in (1, 10, 32, 63)] == [(1, 1), (5, 2), (16, 2), (21, 3)]
+    assert plan(8, 64, 32, 8) == (8, 4) and plan(13, 64, 63, 8) == (32, 2) and plan(16, 64, 200, 8) == (100, 2)
+    # fewer than eight (sequence, kv head); layers of more than eight heads a kv head; the other head size
+    assert plan(7, 64, 10, 1) == plan(1, 64, 10, 7) == plan(1, 64, 10, 8, 9) == plan(1, 128, 10, 8) == (1, 10)
+    assert plan(8, 64, 32, 8, 16) == (8, 4)
+    for T in range(1, 17):
+        for pages in (1, 2, 3, 7, 31, 64, 65, 129, 300, 1000):
+            for nkv in (1, 2, 6, 8, 16):
+                for heads in (8, 16):
+                    per, n = plan(T, 64, pages, nkv, heads)
+                    assert 1 <= n <= K.decode_layers_max_chunks() and per * n >= pages and (n - 1) * per < max(pages, n)
+
+
+@pytest.mark.parametrize("n_seqs,kv_heads", [(1, 8), (4, 2), (8, 1), (3, 3), (12, 8)])
+def test_few_chunks_with_many_idle_groups(tmp_path, n_seqs, kv_heads):
+    """Splits of one, two and four chunks on a grid that they fill to a fraction, and the finer one, by length."""
+    from spissa_b200.csrc import lib as K
+    cfg = dict(tiny.TINY_E, num_attention_heads=2 * kv_heads, num_key_value_heads=kv_heads, num_hidden_layers=2, max_position_embeddings=4096)
+    folder = tiny.make_folder(cfg, tiny.TINY_E_INIT, tmp_path / "chunks")
+    pcfg, w = P.read_model_folder(folder)
+    steps = 3
+    engine = Engine.from_folder(str(folder), dtype="bfloat16", max_tokens=64 * 420, max_seqs=16, use_graphs=False)
+    forms = set()
+    for longest in (20, 100, 620, 1000, 2100):
+        lens = [max(1, longest - 37 * b) for b in range(n_seqs)]
+        seqs = [tiny.random_prompt(cfg["vocab_size"], n + steps, 3 * n + b) for b, n in enumerate(lens)]
+        rows = decode_rows(engine, seqs, lens, steps)
+        forms.add(min(5, K.decode_layers_plan(n_seqs, 64, (longest + steps + 63) // 64, kv_heads)[1]))
+        for b in {0, n_seqs - 1}:
+            ref = P.model_logits(pcfg, w, seqs[b], torch.float64)
+            err = float((rows[:, b].double() - ref[lens[b]:lens[b] + steps]).abs().max()) / float(ref.abs().max())
+            assert err <= TOL, f"{n_seqs} sequences on {kv_heads} kv heads, {longest} keys, sequence {b}: {err:.3e}"
+    assert engine.model._fused.runs == 5 * steps and len(forms) >= 3
