@@ -192,13 +192,15 @@ int linear(const void* x, const void* W, void* out, int out_dt, int M, int N, in
 int fused_product(const void* x, const void* W, void* out, int out_dt, int N, int K, int ldo, int mode, int pair, EpiArgs* ep,
                   const HostStep& st, cudaStream_t stream) {
     const HostKernels& k = kernels;
-    ep->w_settled = 1;                                   // a model's weights: complete before the step's first kernel
+    // a model's weights are complete before the step's first kernel, norm_prepare, which is launched in the ordinary way: it begins
+    // when all that was on the stream before has ended
+    ep->w_settled = 1;
     ++launches;
     if (st.mid) {
-        const int width = k.mid_or_pairs(mode, st.T, N, K, mode == MODE_STREAM_QKV_ROPE ? ep->hd : 1);
+        // (up to 1,023 tokens only gated products are worth tiles by pairs of CTAs)
+        const int width = mode == MODE_SILU_MUL ? k.mid_or_pairs(mode, st.T, N, K, 1) : 0;
         if (width) {
-            // (the rotating epilogue has another number in tc_gemm.cu)
-            if (k.tc_gemm_fused(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode == MODE_STREAM_QKV_ROPE ? 3 : mode, width, ep, st.status, stream))
+            if (k.tc_gemm_fused(x, W, out, out_dt, st.T, N, K, K, K, ldo, mode, width, ep, st.status, stream))
                 return fail_from(k.err_tc_gemm, "host step");
             return 0;
         }

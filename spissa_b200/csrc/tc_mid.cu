@@ -308,7 +308,9 @@ tc_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             };
             // The ring's first tiles of W are asked for while the predecessor's epilogue runs. That is for weights which were
             // complete before the predecessor began, as in a step's layers (a kernel without a signal of its own, torch's for
-            // instance, lets this one in when its CTAs have left, before their writes need be visible): the caller says so.
+            // instance, lets this one in when its CTAs have left, before their writes need be visible): the caller says so. (In a
+            // step norm_prepare stands in front of the first product, launched in the ordinary way: what the stream held before, a
+            // copy into a weight for instance, has ended when it begins, and no kernel of a step writes a weight.)
             // A step of 40 tokens of the 1B shape 1,184 -> 1,147 us, 64: 1,236 -> 1,174, 301: 1,600 -> 1,564; a decode step of
             // 64 sequences 960 -> 945. (With the signal at the kernels' start it was 1,255 -> 1,272 for 40 tokens.)
             const int ahead = GROUPED || !ep.w_settled ? 0 : min(a.stages, kb1 - kb0);

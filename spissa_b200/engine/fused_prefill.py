@@ -119,6 +119,8 @@ class FusedPrefill:
                 return K.tc_mid_or_pairs(mode, T, w.shape[0], w.shape[1], multiple)
             return bn
 
+        # ``w_settled``: nothing that writes a weight is under way when a product's kernel comes in ahead of its predecessor's end,
+        # for ``norm_prepare`` in front of the first of them is launched in the ordinary way (behind all that the stream held)
         def product(a, w, out, mode, bn, pair=0, **kw):
             if (mid or paired) and not bn:
                 K.tc_mid_fused(a, w, out, mode, pair, w_settled=True, **kw)
