@@ -149,3 +149,36 @@ def test_decode_batches_beyond_the_one_kernel_path_at_real_layer_sizes(n_seqs, b
     toks = engine2.step([(sl, [s[n]], [0]) for sl, s, n in zip(slots, seqs, lens)], greedy=True).tolist()
     for b, (r, n) in enumerate(zip(refs, lens)):
         assert float(r[n].max() - r[n][toks[b]]) <= tiny.TOL["bfloat16"] * scale
+
+
+@pytest.mark.parametrize("base,tokens", [("1b", 200), ("1b", 512), ("1b", 800), ("1b", 1023), ("1b", 1300), ("1b", 2100), ("3b", 256),
+                                         ("3b", 1100), ("8b", 600), ("8b", 1281)])
+def test_prompts_whose_products_go_to_both_kernels(base, tokens):
+    """Prompt steps of the real layer sizes where tc_mid.cu takes some products and the tiles by pairs of CTAs the others (from
+    1,024 tokens on any of them): two ragged prompts in one step against the plain run in 64 bits on the device; up to 1,023
+    tokens the C++ and the Python runner give the same bits."""
+    from spissa_b200.csrc import lib as K
+    cfg = {"1b": {**LLAMA_1B_2L, "vocab_size": 20000}, "8b": LLAMA_8B_1L, "3b": LLAMA_3B_1L}[base]
+    H, I = cfg["hidden_size"], cfg["intermediate_size"]
+    nqkv = (cfg["num_attention_heads"] + 2 * cfg["num_key_value_heads"]) * cfg["head_dim"]
+    widths = [K.tc_mid_or_pairs(mode, tokens, N, Kd) for mode, N, Kd in (
+        (K.TC_QKV_ROPE, nqkv, H), (K.TC_ACCUMULATE, H, cfg["num_attention_heads"] * cfg["head_dim"]), (K.TC_SILU_MUL, 2 * I, H), (K.TC_ACCUMULATE, H, I))]
+    assert widths[2] == 256 and (tokens > 2048 or tokens < 1100 or base == "1b" or 0 in widths)
+    engine, w = _engine_and_plain_weights(cfg, 6, "bfloat16", 64 * (tokens // 64 + 4), 4)
+    V = cfg["vocab_size"]
+    seqs = [tiny.random_prompt(V, n, n) for n in (tokens - 37, 37)]
+    want = [sorted({0, min(130, len(s) - 1), len(s) // 2, len(s) - 1}) for s in seqs]
+    rows = {}
+    for host in (True, False):
+        engine.model.host_steps = host
+        slots = [engine.acquire() for _ in seqs]
+        rows[host] = engine.step([(slot, s, places) for slot, s, places in zip(slots, seqs, want)])
+        for slot in slots:
+            engine.release(slot)
+    assert torch.equal(rows[True], rows[False])
+    del engine
+    w = {k: v.cuda() for k, v in w.items()}
+    with torch.device("cuda:0"):
+        ref = torch.cat([P.model_logits(cfg, w, s, torch.float64)[places] for s, places in zip(seqs, want)])
+    worst = float((rows[True].double() - ref).abs().max() / ref.abs().max())
+    assert worst <= tiny.TOL["bfloat16"], f"worst error {worst:.3e} of the largest logit"

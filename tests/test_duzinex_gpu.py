@@ -169,6 +169,30 @@ def test_dynamic_tanh_and_polynorm_by_sixteen_bytes_and_by_elements(width, dtype
     assert worst(act, ref) <= (5e-6 if dtype == torch.float32 else 5e-3)
 
 
+@pytest.mark.parametrize("width,off", [(4, 0), (200, 0), (2048, 0), (201, 0), (64, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_the_output_bias_that_the_differential_store_adds(width, off, dtype):
+    """The stream's rows in fours on 16-byte boundaries and others, beside the store itself, which must not depend on them."""
+    import kernel_harness as KH
+    from spissa_b200.csrc import lib as K
+    G, H, d, vd, lens = 2, 4, 16, 24, [5, 70]
+    meta = KH.paged_meta(lens, [0, 3], DEV, seed=1)
+    T = sum(lens)
+    g = torch.Generator().manual_seed(width)
+    qkv = torch.randn(T, 2 * H * d + G * (2 * d + vd), generator=g).to(DEV)
+    bias, freq = torch.randn(qkv.shape[1], generator=g).to(dtype).to(DEV), torch.rand(d // 2, generator=g).to(DEV)
+    stream = torch.randn(T * width + off, generator=g).to(DEV)[off:].view(T, width)
+    add = torch.randn(width + off, generator=g).to(dtype).to(DEV)[off:]
+    before, outs = stream.clone(), []
+    for with_stream in (False, True):
+        q = torch.zeros(T, 2 * H * d, device=DEV)
+        k, v = torch.zeros(meta.n_pages, G, 64, 2 * d, device=DEV), torch.zeros(meta.n_pages, G, 64, vd, device=DEV)
+        K.diff_qkv_store(qkv, bias, q, k, v, meta, freq, 2 * H, 2 * G, G, d, vd, d, *((stream, add) if with_stream else ()))
+        outs.append((q, k, v))
+    assert torch.equal(stream, before + add.float())
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and float(outs[0][2].abs().max()) > 0
+
+
 def test_token_shift_kernel_carries_the_last_row_in_the_state():
     from spissa_b200.csrc import lib as K
     g = torch.Generator().manual_seed(2)

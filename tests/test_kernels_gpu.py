@@ -209,6 +209,22 @@ def test_silu_mul(K, dtype):
     close(out, ref, 2e-6 if dtype == torch.float32 else 4e-3)
 
 
+@pytest.mark.parametrize("rows,width,off", [(1, 4, 0), (3, 1023, 0), (5, 1024, 0), (7, 1028, 0), (600, 8192, 0), (66000, 4, 0), (9, 30, 0),
+                                            (4, 64, 1), (70000, 2, 0)])
+@pytest.mark.parametrize("dtype,act,mult", [(torch.float32, "silu", 1.0), (torch.float32, "gelu", 0.5), (torch.bfloat16, "gelu", 1.0)])
+def test_gated_mul_by_sixteen_bytes_and_by_elements(K, rows, width, off, dtype, act, mult):
+    """Rows in fours on 16-byte boundaries and others, more rows than a launch has in one dimension, factor and unit."""
+    torch.manual_seed(width)
+    gu = (torch.randn(rows * 2 * width + off, device=DEV) * 3).to(dtype)[off:].view(rows, 2 * width)
+    out = torch.full((rows + 1, width), 7.0, dtype=dtype, device=DEV)
+    K.gated_mul(gu, out[:rows], K.ACT_SILU if act == "silu" else K.ACT_GELU, mult)
+    g, u = gu[:, :width].double(), gu[:, width:].double()
+    ref = (P.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u * mult
+    # an exponential, a quotient and two products in 32 bits, on arguments of up to 15; the storage's rounding
+    bound = (24 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)) * ref.abs() + 1e-6 * u.abs() * mult
+    assert bool(((out[:rows].double() - ref).abs() <= bound).all()) and bool((out[rows] == 7.0).all())
+
+
 def test_add_inplace(K):
     torch.manual_seed(5)
     a, b = torch.randn(1000), torch.randn(1000).bfloat16()

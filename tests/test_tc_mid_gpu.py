@@ -388,3 +388,78 @@ def test_clamped_units_whose_quotient_lies_near_the_middle_of_two_floats(K, kern
     want = gate / (1.0 + float(torch.exp(torch.tensor(-slope * gate, dtype=torch.float64))))
     # half a unit, and an expf that is two units of 2^-24 off below 1
     assert float((outs[0][::2].double() - want).abs().max()) <= 4 * 2.0 ** -24 * want
+
+
+@pytest.mark.parametrize("M", [129, 200, 256, 257, 449, 512, 800, 1023])
+def test_gated_products_by_pairs_with_row_statistics(K, M):
+    """What a prompt's step asks of the pairs' tiles: the normed residual's 1/rms folded into the epilogue."""
+    H, N = 264, 768
+    torch.manual_seed(M)
+    x, weight = torch.randn(M, H, device=DEV) * 2.0, (1.0 + 0.1 * torch.randn(H, device=DEV)).bfloat16()
+    x[M // 2] *= 1e-3                                                   # a small row: its 1/rms is large
+    w = (torch.randn(N, H, device=DEV) * 0.1).bfloat16()
+    xw, ssq = torch.empty(M, H, dtype=torch.bfloat16, device=DEV), torch.empty(M, 1, device=DEV)
+    K.norm_prepare(x, weight, xw, ssq)
+    out = torch.full((M + 2, N // 2), 9.0, device=DEV)
+    K.tc_gemm_fused(xw, w, out[:M], K.TC_SILU_MUL, 256, row_ssq=ssq, norm_width=H, eps=1e-5)
+    rstd = 1.0 / torch.sqrt((x.double() ** 2).sum(1, keepdim=True) / H + 1e-5)
+    y = (xw.double() @ w.double().t() * rstd).view(M, 3, 2, 128)
+    g, u = y[:, :, 0].reshape(M, 384), y[:, :, 1].reshape(M, 384)
+    size = (xw.double().abs() @ w.double().abs().t() * rstd).amax(1, keepdim=True)
+    # the sums' error (H terms of 2^-23 each) and 1/rms's (H / 32 + 8 roundings of 2^-24) through an activation of slope 1.1
+    bound = 1.2 * (H + 16) * 2.0 ** -23 * size * (1.0 + g.abs() + u.abs())
+    assert bool(((out[:M].double() - g * torch.sigmoid(g) * u).abs() <= bound).all())
+    assert bool((out[M:] == 9.0).all())
+
+
+@pytest.mark.parametrize("M", [17, 64, 200, 301])
+@pytest.mark.parametrize("Kd", [8, 64, 136, 512, 1096, 4096])
+def test_weights_asked_for_ahead(K, M, Kd):
+    """The ring's first tiles of W fetched before the predecessor has ended, for fewer, as many and more blocks of K than the ring
+    holds: the same bits, behind a kernel that writes the other operand."""
+    H = Kd
+    torch.manual_seed(Kd + M)
+    x, weight = torch.randn(M, H, device=DEV), (1.0 + 0.1 * torch.randn(H, device=DEV)).bfloat16()
+    w_store, w_gate = ((torch.randn(n, H, device=DEV) * 0.1).bfloat16() for n in (2056, 1024))
+    stages = {K.tc_mid_plan(mode, M, w.shape[0], Kd)[2:] for mode, w in ((K.TC_STORE, w_store), (K.TC_SILU_MUL, w_gate))}
+    assert all(pieces >= 1 and n >= 1 for pieces, n in stages)
+    got = {}
+    for settled in (False, True):
+        rows = []
+        for _ in range(4):
+            xw, ssq = torch.zeros(M, H, dtype=torch.bfloat16, device=DEV), torch.empty(M, 1, device=DEV)
+            store = torch.full((M, 2056), float("nan"), dtype=torch.bfloat16, device=DEV)
+            acc, act = torch.zeros(M, 2056, device=DEV), torch.full((M, 512), float("nan"), dtype=torch.bfloat16, device=DEV)
+            K.norm_prepare(x, weight, xw, ssq)
+            kw = dict(row_ssq=ssq, norm_width=H, eps=1e-5, w_settled=settled)
+            K.tc_mid_fused(xw, w_gate, act, K.TC_SILU_MUL, 128, **kw)
+            K.tc_mid_fused(xw, w_store, store, K.TC_STORE, **kw)
+            K.tc_mid_fused(xw, w_store, acc, K.TC_ACCUMULATE, w_settled=settled)
+            rows.append((act, store, acc))
+        got[settled] = rows
+    for again in got[False][1:] + got[True]:
+        assert all(torch.equal(a, b) for a, b in zip(got[False][0], again))
+    within(got[True][0][2], xw, w_store)
+
+
+@pytest.mark.parametrize("block", [64, 128])
+@pytest.mark.parametrize("poison", [float("nan"), 3e4])
+def test_experts_do_not_read_what_the_memory_held(K, block, poison):
+    """The rows of holes among the gathered ones are not written: whatever stands there, the tokens' results have the same bits."""
+    E, W, F, top, T = 8, 256, 384, 2, 700
+    torch.manual_seed(block)
+    x = torch.randn(T, W, device=DEV).bfloat16()
+    gate, up = ((torch.randn(E, F // block, block, W, device=DEV) * 0.1).bfloat16() for _ in range(2))
+    both = torch.stack([gate, up], dim=2).reshape(E, 2 * F, W).contiguous()
+    down = (torch.randn(E, W, F, device=DEV) * 0.1).bfloat16()
+    ids, weights = torch.randint(0, E, (T, top), dtype=torch.int32, device=DEV), torch.rand(T, top, device=DEV)
+    ys = []
+    for fill in (0.0, poison):
+        torch.cuda.empty_cache()
+        held = [torch.full((n, W), fill, dtype=dt, device=DEV) for n in (1500, 2500, 4000) for dt in (torch.bfloat16, torch.float32)]
+        torch.cuda.synchronize()
+        del held
+        y = torch.zeros(T, W, device=DEV)
+        K.moe_experts(x, ids, weights, both, down, y, top, 7.0, 1.702, block)
+        ys.append(y)
+    assert bool(ys[0].isfinite().all()) and torch.equal(*ys)
