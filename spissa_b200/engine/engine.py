@@ -65,6 +65,17 @@ def _require_gpu(device) -> torch.device:
     return torch.device(device)
 
 
+def _own_tokens(tokens):
+    """The step's own copy of a caller's tokens: a prompt as an array of 32-bit integers where it is a list of such (which is
+    all that packing it takes: 2,048 tokens 24 us, as a list and from there as a tensor 100), else a list."""
+    if type(tokens) is list and len(tokens) > 32:
+        try:
+            return array("i", tokens)
+        except (TypeError, OverflowError):
+            pass                                         # not all of them integers of 32 bits: refused or taken when checked
+    return list(tokens)
+
+
 class Engine:
     """``Engine.from_folder(dir, dtype=..., max_tokens=...)`` or ``Engine.from_config(cfg, seed=...)``."""
 
@@ -199,14 +210,11 @@ class Engine:
 
     def _prompt_tensor(self, slot: int, toks) -> torch.Tensor:
         """A prompt's tokens as an int32 tensor, which the packing takes as it is; refused where one is out of range."""
-        try:
-            # a quarter of what torch.tensor takes for a list (2,048 tokens: 24 us, 92 there)
-            as_tensor = torch.frombuffer(array("i", toks), dtype=torch.int32)
+        if isinstance(toks, array):                      # (the step's own, of 32 bits)
+            as_tensor = torch.frombuffer(toks, dtype=torch.int32)
             low, high = torch.aminmax(as_tensor)
             if int(low) >= 0 and int(high) < self.vocab_size:
                 return as_tensor
-        except (TypeError, OverflowError):
-            pass                                         # not all of them integers of 32 bits: below
         try:
             as_tensor = torch.tensor(toks, dtype=torch.int64)
         except (TypeError, ValueError, RuntimeError, OverflowError):
@@ -323,8 +331,8 @@ class Engine:
         step, by ``check()`` or ``settle()``, and until then ``length`` counts them.
         """
         # (copies: what has been checked is what runs, whatever the caller's other threads do with their lists meanwhile)
-        ents = [(e.slot, list(e.tokens), list(e.want)) if isinstance(e, StepEntry)
-                else (e[0], list(e[1]), list(e[2])) for e in entries]
+        ents = [(e.slot, _own_tokens(e.tokens), list(e.want)) if isinstance(e, StepEntry)
+                else (e[0], _own_tokens(e[1]), list(e[2])) for e in entries]
         lengths, packed = self._validate(ents)
         counts = [(slot, len(toks)) for slot, toks, _ in ents]
         with torch.cuda.device(self.device):

@@ -208,6 +208,26 @@ def test_step_refusals_leave_the_cache_alone(folders):
     assert out.shape == (1, 256) and engine.length(s) == 4
 
 
+def test_tokens_of_a_prompt_in_every_form_that_is_taken_and_refused(folders):
+    """33 tokens and more travel as an array: what is no list of 32-bit integers is still refused or taken as it was."""
+    import numpy as np
+    from spissa_b200 import StepError
+    folder, _, _ = folders["A"]
+    engine = Engine.from_folder(folder, dtype="float32", max_tokens=256, max_seqs=2)
+    good = [(5 * i + 1) % 256 for i in range(40)]
+    slot = engine.acquire()
+    for bad in (256, -1, 2 ** 31, -2 ** 31 - 1, 2 ** 70, "7", None):
+        with pytest.raises(StepError):
+            engine.step([(slot, good[:20] + [bad] + good[21:], [0])])
+    assert engine.length(slot) == 0
+    rows = []
+    for form in (good, tuple(good), np.array(good), [np.int64(t) for t in good], torch.tensor(good), [True] + good[1:]):
+        slot = engine.acquire()
+        rows.append(engine.step([(slot, form, [39])]))
+        engine.release(slot)
+    assert all(torch.equal(rows[0], r) for r in rows[1:])
+
+
 @pytest.mark.parametrize("n", [3, 40])
 def test_a_callers_lists_may_change_once_their_step_is_checked(folders, n):
     """What has been checked is what runs, whatever another thread does with the lists meanwhile."""
