@@ -1081,8 +1081,10 @@ SP_API int sp_attention_generic(const void* q, int q_dt, const void* kpool, cons
 // at a time through shared memory, each of 256 threads 4 x 4 scores and 4 x 4 (per 64 value columns) sums. The kernel
 // above reads every key once per query; here a key is read once per 64 queries, and the next tile's rows are copied into a
 // second buffer under this one's products (500 tokens, 32 heads of 64 on 8 kv heads: 423 us by the kernel above, 114 us with a
-// tile's rows fetched in front of its products one piece after another, 66 us here; the products' FFMAs alone are 17).
-// Sums, softmax and exponentials are float32 as there; only their order differs.
+// tile's rows fetched in front of its products one piece after another, 66 us here; the products' FFMAs alone are 17). The second
+// buffer leaves heads of 72 to 124 one CTA an SM where there was room for two, which costs them less than it gives: 24 heads on 8,
+// 500 tokens, heads of 80 167 -> 89 us, of 112 199 -> 101, 1,500 tokens 757 -> 565 and 907 -> 645, three prompts of 500 in all 65 ->
+// 59 and 77 -> 67. Sums, softmax and exponentials are float32 as there; only their order differs.
 #define AT_TILE 64
 #define AT_MAX_D 128
 template <int VC>
@@ -1093,7 +1095,7 @@ attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__
                           int n_seqs, int sms) {
     extern __shared__ __align__(16) float at_smem[];
     // The tiles with the most keys first, all heads of them side by side; every second round of CTAs over the SMs goes backwards,
-    // so that an SM's two CTAs are one of many keys and one of few (500 tokens: 8 tiles of keys on every SM; tile by tile of a
+    // so that an SM's two CTAs are one of many keys and one of few (heads of 64, 500 tokens: 8 tiles of keys on every SM; tile by tile of a
     // head it was 12 on some and 5 on others: 94 us, and 66 so).
     int at_cta = blockIdx.x;
     const int turn_of = at_cta / sms, turn_from = turn_of * sms, turn_to = min((int)gridDim.x, turn_from + sms);
