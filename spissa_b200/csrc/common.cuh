@@ -60,9 +60,8 @@ static inline bool sp_gate_built(const SpGate& g) { return g.kind == SP_ACT_SILU
 
 // The tanh form of gelu, ½ z (1 + tanh(a)) with a = √(2/π)(z + 0.044715 z³), written with the logistic function:
 // ½ (1 + tanh(a)) = 1 / (1 + e^{−2a}).
-__device__ __forceinline__ float sp_gelu_tanh(float z) {
-    return z / (1.0f + expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
-}
+__device__ __forceinline__ float sp_gelu_exponent(float z) { return -1.5957691216057308f * (z + 0.044715f * z * z * z); }
+__device__ __forceinline__ float sp_gelu_tanh(float z) { return z / (1.0f + expf(sp_gelu_exponent(z))); }
 __device__ __forceinline__ float sp_gated(float gate, float up, const SpGate& ga) {
     float slope = 1.0f;
     if (ga.kind == SP_ACT_CLAMPED) {

@@ -111,9 +111,9 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_bmn(int m, int n) {
 // x / d for 1 <= d <= 2^100 and finite x: the remainder of a quotient by an approximate reciprocal (two units at most off)
 // corrects it to within half a unit and 2^-20 of one, with a REFINED reciprocal (a step of Newton's) to within half a unit
 // (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). No branch, unlike
-// the general quotient. Compared with that one for x = g and d = 1 + expf(-slope·g), all g with |slope·g| <= 60 (2.2 · 10^9): the
-// same bits for a slope of 1 as it is, for 172 slopes from 0.013 to 200 when refined (without: up to 3 g a slope differ in the
-// last bit); where g is -0 the quotient is +0.
+// the general quotient. Compared with that one for every gate g that comes here: x = g and d = 1 + expf(-slope·g), |slope·g| <= 60,
+// the same bits for a slope of 1 as it is, for 172 slopes from 0.013 to 200 when refined (without: up to 3 g a slope differ in
+// the last bit); the tanh form of gelu, |g| <= 8.6, the same bits when refined; where g is -0 the quotient is +0.
 template <bool REFINED>
 __device__ __forceinline__ float tc_quotient(float x, float d) {
     float r;
@@ -127,7 +127,8 @@ __device__ __forceinline__ float tc_quotient(float x, float d) {
 // tc_mid.cu, 301 tokens x 16,384 x 2,048: 27.3 us, 32.0 with the general quotient, 40 with a branch on the activation around
 // each value. In tc_gemm.cu the general quotient's way for a numerator of zero, which the rows behind the last token all take,
 // held up the tiles behind them: 16,384 x 2,048 on weights from HBM, 1,408 tokens 130 us, 82 here (2,048 tokens, without
-// such rows, 123 and 102; of the 8B shape, 28,672 x 4,096, 6,000 tokens 1,180 and 1,098).
+// such rows, 123 and 102; of the 8B shape, 28,672 x 4,096, 6,000 tokens 1,180 and 1,098); gelu's, on the same way until it
+// had this form, 200 tokens 40.9 and 21.7, 1,024 columns of 400 tokens x 8,192 34.5 and 15.7.
 // Both ways give a value the same bits, so a token's result depends neither on its neighbours in the warp nor on rows that nobody
 // reads (holes among the routed experts' rows hold what the memory held). Deciding for each value by its own gate in the
 // second loop as well makes that loop twice as long: 2,048 tokens x 16,384 x 2,048 by pairs 100.5 -> 103 us.
@@ -135,6 +136,7 @@ template <int KIND, typename Scale>
 __device__ __forceinline__ void tc_activate(uint32_t (&rg)[32], uint32_t (&ru)[32], Scale scale, int n, SpGate ga) {
     ga.kind = KIND;
     const float slope = KIND == SP_ACT_CLAMPED ? ga.slope : 1.0f;
+    constexpr float edge = KIND == SP_ACT_GELU ? 8.6f : 60.0f;   // the exponent stays within 60
     float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};                     // (NaN is left out: the quotient is NaN either way)
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -144,13 +146,13 @@ __device__ __forceinline__ void tc_activate(uint32_t (&rg)[32], uint32_t (&ru)[3
         rg[j] = __float_as_uint(g);
         ru[j] = __float_as_uint(__uint_as_float(ru[j]) * scale(j));
     }
-    if (KIND != SP_ACT_GELU && __all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= 60.0f)) {
+    if (__all_sync(0xffffffffu, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) <= edge)) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
             const float g = __uint_as_float(rg[j]);
             float u = __uint_as_float(ru[j]);
             if (KIND == SP_ACT_CLAMPED) u = fminf(fmaxf(u, -ga.limit), ga.limit) + 1.0f;
-            rg[j] = __float_as_uint(tc_quotient<KIND == SP_ACT_CLAMPED>(g, 1.0f + expf(-slope * g)) * u * ga.mult);
+            rg[j] = __float_as_uint(tc_quotient<KIND != SP_ACT_SILU>(g, 1.0f + expf(KIND == SP_ACT_GELU ? sp_gelu_exponent(g) : -slope * g)) * u * ga.mult);
         }
         return;
     }

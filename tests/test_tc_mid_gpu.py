@@ -328,7 +328,7 @@ def test_the_choice_between_the_two_kernels(K):
         return                                                          # what follows was measured on 148
     assert K.tc_mid_or_pairs(K.TC_ACCUMULATE, 1280, 2048, 8192) == 0 and K.tc_mid_or_pairs(K.TC_ACCUMULATE, 2048, 2048, 8192) == 256
     assert K.tc_mid_or_pairs(K.TC_SILU_MUL, 301, 16384, 2048) == 0 and K.tc_mid_or_pairs(K.TC_SILU_MUL, 512, 16384, 2048) == 256
-    assert [K.tc_mid_or_pairs(K.TC_STORE, M, 512, 512) for M in (1024, 1280, 1700, 2048)] == [0, 0, 128, 128]
+    assert [K.tc_mid_or_pairs(K.TC_STORE, M, 512, 512) for M in (1024, 1280, 1800, 2048)] == [0, 0, 128, 128]
     # gated rows of the 3B and 8B layers: the kernel that the figures beside the rule show as the faster one
     assert [K.tc_mid_or_pairs(K.TC_SILU_MUL, M, 16384, 3072) for M in (200, 256, 257, 800)] == [256, 256, 0, 256]
     assert [K.tc_mid_or_pairs(K.TC_SILU_MUL, M, 28672, 4096) for M in (200, 257, 512, 768, 880, 1100, 1281)] == [0, 0] + 5 * [256]
@@ -345,7 +345,7 @@ def test_linear_of_more_tokens(K, M, N, Kd):
     within(acc, a, w, extra=c0)
 
 
-@pytest.mark.parametrize("act", ["ACT_SILU", "ACT_CLAMPED"])
+@pytest.mark.parametrize("act", ["ACT_SILU", "ACT_GELU", "ACT_CLAMPED"])
 @pytest.mark.parametrize("kernel,width", [("tc_mid", 128), ("tc_gemm", 256), ("tc_gemm", 128)])
 def test_a_tokens_gated_values_do_not_depend_on_its_neighbours(K, act, kernel, width):
     """Gates beyond the branch-free range in every sixteenth token leave the others' bits as they are."""
@@ -366,9 +366,10 @@ def test_a_tokens_gated_values_do_not_depend_on_its_neighbours(K, act, kernel, w
 @pytest.mark.parametrize("slope,gate", [(0.2526956572140501, 0.020345522090792656), (0.5680828327219911, 0.007325529120862484),
                                         (0.7441885108658084, 0.0013069163542240858), (0.7441885108658084, 0.10660775750875473),
                                         (0.974886949234209, 0.012287044897675514), (2.8710412953340563, 0.0016809902153909206),
-                                        (4.926993966922774, 0.005847701337188482)])
-def test_clamped_units_whose_quotient_lies_near_the_middle_of_two_floats(K, kernel, width, slope, gate):
-    """Gates whose quotient by an unrefined reciprocal is a last bit off: the same value alone and beside a large gate."""
+                                        (4.926993966922774, 0.005847701337188482), (None, 0.050509825348854065)])
+def test_units_whose_quotient_lies_near_the_middle_of_two_floats(K, kernel, width, slope, gate):
+    """Gates whose quotient by an unrefined reciprocal is a last bit off (a clamped unit's slope, or gelu): the same value alone and
+    beside a large gate."""
     parts, left = [], torch.tensor(gate)
     for _ in range(3):                                                  # the gate as an exact sum of three bfloat16 numbers
         parts.append(left.bfloat16())
@@ -376,16 +377,21 @@ def test_clamped_units_whose_quotient_lies_near_the_middle_of_two_floats(K, kern
     assert float(left) == 0.0
     half = width if kernel == "tc_mid" else width // 2
     w = torch.zeros(512, 64, dtype=torch.bfloat16, device=DEV)
-    w.view(-1, 2, half, 64)[:, 0, :, :3] = 1.0                          # gate rows; the up rows are zero, so up + 1 is 1
+    w.view(-1, 2, half, 64)[:, 0, :, :3] = 1.0                          # gate rows
+    if slope is None:
+        w.view(-1, 2, half, 64)[:, 1, :, 3] = 1.0                       # up is 1; the clamped unit adds one to zero
     a = torch.zeros(130, 64, dtype=torch.bfloat16, device=DEV)
     a[:, :3] = torch.stack(parts).to(DEV)
+    a[:, 3] = 1.0
     b = a.clone()
     b[1::2, 0] = 512.0
     outs = [torch.empty(130, 256, device=DEV) for _ in range(2)]
     for x, out in zip((a, b), outs):
-        getattr(K, kernel)(x, w, out, K.TC_SILU_MUL, width, act=K.ACT_CLAMPED, limit=1000.0, slope=slope)
+        kw = dict(act=K.ACT_GELU) if slope is None else dict(act=K.ACT_CLAMPED, limit=1000.0, slope=slope)
+        getattr(K, kernel)(x, w, out, K.TC_SILU_MUL, width, **kw)
     assert torch.equal(outs[0][::2], outs[1][::2])
-    want = gate / (1.0 + float(torch.exp(torch.tensor(-slope * gate, dtype=torch.float64))))
+    exponent = -slope * gate if slope is not None else -1.5957691216057308 * (gate + 0.044715 * gate ** 3)
+    want = gate / (1.0 + float(torch.exp(torch.tensor(exponent, dtype=torch.float64))))
     # half a unit, and an expf that is two units of 2^-24 off below 1
     assert float((outs[0][::2].double() - want).abs().max()) <= 4 * 2.0 ** -24 * want
 
