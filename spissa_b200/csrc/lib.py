@@ -1098,14 +1098,16 @@ def tc_mid_plan(mode, M: int, N: int, K: int) -> tuple:
 
 @functools.lru_cache(maxsize=4096)
 def _mid_or_pairs(device: int, mode: int, M: int, N: int, K: int, multiple: int) -> int:
-    return int(load("tc_mid").sp_tc_mid_or_pairs(mode, M, N, K, multiple))
+    return int(load("tc_mid").sp_tc_mid_or_pairs(int(mode), int(M), int(N), int(K), int(multiple)))
 
 
-def tc_mid_or_pairs(mode, M: int, N: int, K: int, multiple: int = 1) -> int:
-    """For a product that ``tc_mid`` and ``tc_gemm``'s tiles by pairs of CTAs could both take: the faster one by its sizes (and
-    the current device's number of SMs), as the width of those tiles (a multiple of ``multiple``) or 0 for ``tc_mid``."""
-    device = torch.cuda.current_device() if torch.cuda.is_initialized() else -1
-    return _mid_or_pairs(device, int(mode), int(M), int(N), int(K), int(multiple))
+def tc_mid_or_pairs(mode, M: int, N: int, K: int, multiple: int = 1, device: int | None = None) -> int:
+    """For a product that ``tc_mid`` and ``tc_gemm``'s tiles by pairs of CTAs could both take: the faster one by its sizes and
+    the number of SMs of ``device`` (the index of the current CUDA device, asked for where it is not given: a microsecond),
+    as the width of those tiles (a multiple of ``multiple``) or 0 for ``tc_mid``."""
+    if device is None:
+        device = torch.cuda.current_device() if torch.cuda.is_initialized() else -1
+    return _mid_or_pairs(device, mode, M, N, K, multiple)
 
 
 # ------------------------------------------------------------------ seqmix: other mixers, their norm and activation

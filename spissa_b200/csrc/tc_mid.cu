@@ -545,11 +545,11 @@ SP_API int sp_tc_mid_plan(int mode, int M, int N, int K, int* out) {
 // Which kernel takes a product of more than 128 tokens that both this one and the tiles by pairs of CTAs of tc_gemm.cu (256
 // rows, 74 pairs on 148 SMs) could: the width of those tiles, a multiple of ``multiple``, or 0 for this kernel. By two estimates of
 // time, compared with 2,902 measured products (N 512 to 32,000, K 256 to 14,336): the choice is 0.3 % slower than the better
-// kernel on average for gated ones and 3.5 % for the others.
+// kernel on average for gated ones and 2.8 % for the others.
 //   Pairs: a round of tiles takes 0.36 us per 64 of K at 256 columns, 0.335 at 192 and 0.31 at 128, the launch with its last
 // epilogue 10 us, less where one round of narrow tiles does and K is short (512 x 512, 2,048 tokens 7.9 us, this kernel 10.8); gated
-// ones 0.323, 3.5 for a round's epilogue and 5 for the launch.
-//   This kernel: plan_of's, which was made to compare divisions and is 10 % short for gated products on average.
+// ones 0.36 in the first round and 0.323 in the others, 3.5 for a round's epilogue and 5 for the launch.
+//   This kernel: plan_of's, which was made to compare divisions and is 12 % short for gated products on average.
 // Gated products are worth pairs as soon as their rounds come out full, for they have the most rows of W (us, this kernel /
 // pairs: 1B 200 tokens 24.1 / 20.5, 301: 27.0 / 31.1, 512: 36.5 / 31.8, 1,023: 71.3 / 56.6; 3B 256: 32.0 / 27.3, 800 88.9 / 79.5; 8B
 // 257: 89 / 107, 512: 123 / 109, 768: 201 / 139, 800: 209 / 206, 1,100: 257 / 222, 1,281: 318 / 289); the others from 1,024 tokens
@@ -560,18 +560,18 @@ SP_API int sp_tc_mid_or_pairs(int mode, int M, int N, int K, int multiple) {
     if (M <= 128 || (!gated && M < 1024)) return 0;
     const int walkers = (sp_sm_count() > 0 ? sp_sm_count() : 148) / 2, row_tiles = (M + 255) / 256, num_kb = (K + BK - 1) / BK;
     auto rounds = [&](int bn) { return (row_tiles * ((N + bn - 1) / bn) + walkers - 1) / walkers; };
-    const double start = rounds(128) > 1 || num_kb > 18 ? 10000.0 : 5500.0 + 250.0 * num_kb;
+    const double start = rounds(128) > 1 || num_kb > 16 ? 10000.0 : 6000.0 + 250.0 * num_kb;
     int best = 0;
     double best_t = 0;
     for (const int bn : {256, 192, 128}) {
         if ((gated && bn != 256) || (multiple > 1 && bn % multiple)) continue;
-        const double t = gated ? 5000.0 + rounds(bn) * (3500.0 + num_kb * 323.0)
+        const double t = gated ? 5000.0 + rounds(bn) * 3500.0 + num_kb * (360.0 + 323.0 * (rounds(bn) - 1))
                                : start + (double)rounds(bn) * num_kb * (bn == 256 ? 360.0 : bn == 192 ? 335.0 : 310.0);
         if (!best || t < best_t) { best = bn; best_t = t; }
     }
     double mine = 0;
     if (M > 2048 || !plan_of(mode, M, N, K, &mine).nt) return best;
-    return (gated ? 1.1 : 1.0) * mine < best_t ? 0 : best;
+    return (gated ? 1.12 : 1.0) * mine < best_t ? 0 : best;
 }
 
 // Whether this kernel takes the product (0) or another has to (1, the reason as the last error).

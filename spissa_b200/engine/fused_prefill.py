@@ -116,7 +116,7 @@ class FusedPrefill:
         def width_of(mode, w, bn, multiple=1):
             """The width of tc_gemm's tiles; 0 where tc_mid takes the product."""
             if mid or paired:
-                return K.tc_mid_or_pairs(mode, T, w.shape[0], w.shape[1], multiple)
+                return K.tc_mid_or_pairs(mode, T, w.shape[0], w.shape[1], multiple, dev.index)
             return bn
 
         # ``w_settled``: nothing that writes a weight is under way when a product's kernel comes in ahead of its predecessor's end,

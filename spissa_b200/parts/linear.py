@@ -42,7 +42,7 @@ MOST_MID_TOKENS = 2048    # the most that tc_mid.cu is built for
 
 def mid_takes(mode, x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether tc_mid.cu is the faster one for a product that tc_gemm.cu's tiles could take as well."""
-    return (x.shape[0] <= MID_TOKENS and mode != K.TC_SILU_MUL) or not K.tc_mid_or_pairs(mode, x.shape[0], w.shape[0], w.shape[1])
+    return (x.shape[0] <= MID_TOKENS and mode != K.TC_SILU_MUL) or not K.tc_mid_or_pairs(mode, x.shape[0], w.shape[0], w.shape[1], 1, x.device.index)
 
 
 def tile_width(M: int, N: int, sms: int | None = None) -> int:
@@ -89,7 +89,7 @@ class Linear:
         elif x.shape[0] <= STREAM_TOKENS and K.tc_stream_supported(x, self.weight, mode):
             K.tc_stream(x, self.weight, out, mode)
         elif K.tc_gemm_supported(x, self.weight):
-            width = x.shape[0] >= PAIR_TOKENS and K.tc_mid_or_pairs(mode, x.shape[0], self.out_features, self.in_features)
+            width = x.shape[0] >= PAIR_TOKENS and K.tc_mid_or_pairs(mode, x.shape[0], self.out_features, self.in_features, 1, x.device.index)
             K.tc_gemm(x, self.weight, out, mode, width or tile_width(x.shape[0], self.out_features, sm_count(x.device)))
         elif x.shape[0] > GEMV_TOKENS and x.shape[1] >= F32_PARTS_K and K.tc_f32_supported(x, self.weight, out):
             K.tc_f32(x, self.weight, out, accumulate=accumulate)
